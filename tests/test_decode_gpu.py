@@ -228,3 +228,34 @@ def test_rope_position_interpolation_and_paged_row_copies(torch_cuda, oracle):
     L.launch_paged_copy_row(tr.data_ptr(), pool.data_ptr(), 5, page, page, dm)  # offset outside the page
     assert L.df_attn_last_status() != 0
     p.sync_status()
+
+
+@pytest.mark.parametrize("H,D,T,bf16,page,scratch", [
+    (12, 64, 63, False, 0, False), (12, 64, 64, False, 0, False), (3, 64, 65, False, 16, False),  # edges of a stage (64 tokens)
+    (12, 64, 4096, False, 0, False), (12, 64, 4097, False, 0, False),  # the line between short and long caches
+    (2, 64, 9001, True, 16, True), (2, 128, 9001, True, 7, True), (1, 128, 16, True, 16, False),  # split form, odd page size
+    (20, 128, 5000, True, 16, False), (40, 128, 2500, False, 32, False), (300, 8, 4500, False, 0, False),  # many heads, small clusters
+    (5, 20, 5001, True, 16, False), (6, 100, 4999, True, 0, True), (6, 80, 4999, False, 0, True), (4, 10, 4200, True, 0, True)])  # granules of 8 bytes, two slots, scalar loads
+def test_decode_forms_and_edges(torch_cuda, oracle, H, D, T, bf16, page, scratch):
+    torch = torch_cuda
+    p = pkg()
+    rows = (T + page - 1) // page * page if page else T
+    q = oracle.fill_normal((H * D,), 9000 + T, 0)
+    k, v = (oracle.fill_normal((rows, H * D), 9000 + T, st) for st in (1, 2))
+    table = None
+    if page:
+        k, v, table = _paged(torch, k, v, page, T)
+    if bf16:
+        k, v = oracle.round_bf16(k)[0], oracle.round_bf16(v)[0]
+    scale = 1.0 / np.sqrt(D)
+    ref, _ = oracle.decode(q, k, v, H, T, scale, block_table=table, page_size=page) if page else oracle.decode(q, k, v, H, T, scale)
+    tq, tk, tv = to_dev(q, k, v)
+    if bf16:
+        tk, tv = tk.to(torch.bfloat16), tv.to(torch.bfloat16)
+    chunks = (T + 127) // 128
+    parts = tuple(torch.empty(H * chunks * n, device="cuda") for n in (1, 1, D)) if scratch else None
+    out = torch.full((H * D + 64,), 7.0, device="cuda")
+    p.decode(tq, tk, tv, H, T, scale, block_table=torch.from_numpy(table).cuda() if page else None, page_size=page, partials=parts,
+             max_chunks=chunks if scratch else 0, out=out[:H * D])
+    assert p.sync_status() == 0
+    assert np.abs(out[:H * D].cpu().numpy() - ref).max() <= TOL and float(out[H * D:].min()) == 7.0
