@@ -2,9 +2,10 @@
 
 The product is the C-ABI library ``lib/libdarkforest_kernels.so`` (declared in
 ``include/darkforest_kernels.h``). This Python module is only the thin loader that the tests
-and the benchmark use to reach that ABI: ctypes prototypes plus ``AttentionContext``, a mirror
-of the reference's ``darkforest_cuda::AttentionContext`` (darkforest-cuda/src/lib.rs:1949-2368)
-working on torch CUDA tensors. torch is used for device memory and streams, nothing else.
+and the benchmark use to reach that ABI: ctypes prototypes, functions on torch CUDA tensors whose
+checks and calls run in native code (``host/python_calls.cpp``), and ``AttentionContext``, a mirror
+of the reference's ``darkforest_cuda::AttentionContext`` (darkforest-cuda/src/lib.rs:1949-2368).
+torch is used for device memory and streams, nothing else.
 
 There is no CPU path: loading fails loudly when the CUDA library has not been built, and every
 call needs CUDA tensors.
@@ -20,6 +21,7 @@ import subprocess
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "lib", "libdarkforest_kernels.so")
+CALLS_PATH = os.path.join(_HERE, "lib", "df_python_calls.so")
 HEADER_PATH = os.path.join(_HERE, "..", "include", "darkforest_kernels.h")
 
 DF_OK = 0
@@ -138,6 +140,31 @@ class AttentionError(RuntimeError):
     pass
 
 
+def load_calls():
+    """The native host path (host/python_calls.cpp): loaded with the first call on tensors, bound to the library of lib()."""
+    global _calls
+    if isinstance(_calls, _CallsOnFirstUse):
+        import importlib.util
+        import torch  # noqa: F401  (the module is linked against torch's libraries)
+        L = lib()
+        if not os.path.exists(CALLS_PATH):
+            raise RuntimeError(f"{CALLS_PATH} is missing: build it with `make -C {_HERE}`")
+        spec = importlib.util.spec_from_file_location("df_python_calls", CALLS_PATH)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        mod.bind({name: ctypes.cast(getattr(L, name), ctypes.c_void_p).value for name in PROTOTYPES}, AttentionError)
+        _calls = mod
+    return _calls
+
+
+class _CallsOnFirstUse:
+    def __getattr__(self, name):
+        return getattr(load_calls(), name)
+
+
+_calls = _CallsOnFirstUse()
+
+
 def _check(status: int) -> None:
     if status != DF_OK:
         raise AttentionError(f"attention call failed: {lib().df_attn_status_string(status).decode()} ({status})")
@@ -188,17 +215,7 @@ def launch_count(reset: bool = False) -> int:
 # Batched, stream-aware calls on torch tensors: q,k,v,out [B,S,H*D] fp32, lse/delta [B,H,S] fp32
 # ------------------------------------------------------------------------------------------
 def forward(q, k, v, n_heads, scale, causal=True, out=None, lse=None, causal_shift=0, stream=None):
-    import torch
-    B, Sq, dm = q.shape
-    Sk = k.shape[1]
-    D = dm // n_heads
-    if out is None:
-        out = torch.empty_like(q)
-    if lse is None:
-        lse = torch.empty((B, n_heads, Sq), dtype=torch.float32, device=q.device)
-    _check(lib().df_attn_forward_block(_ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(lse), B, n_heads, Sq, Sk, D,
-                                       float(scale), int(bool(causal)), int(causal_shift), _stream_ptr(stream)))
-    return out, lse
+    return _calls.forward(q, k, v, n_heads, scale, causal, out, lse, causal_shift, stream)
 
 
 def decode(q, k, v, n_heads, cur_seq_len, scale, block_table=None, page_size=0, partials=None, max_chunks=0,
@@ -206,104 +223,39 @@ def decode(q, k, v, n_heads, cur_seq_len, scale, block_table=None, page_size=0, 
     """One-token decode: q [H*D] fp32, k/v a contiguous cache [T_max, H*D] or, with block_table (int32
     tensor), a pool of pages of page_size rows; bf16 caches are recognised by dtype. partials =
     (m, l, o) scratch tensors for max_chunks states per head selects the split form."""
-    import torch
-    D = q.numel() // n_heads
-    if out is None:
-        out = torch.empty_like(q)
-    pm, pl, po = partials if partials is not None else (None, None, None)
-    _check(lib().df_attn_decode(_ptr(q), _ptr(k), _ptr(v), _ptr(block_table) if block_table is not None else None,
-                                _ptr(out), _ptr(pm) if pm is not None else None, _ptr(pl) if pl is not None else None,
-                                _ptr(po) if po is not None else None, int(max_chunks), n_heads, int(cur_seq_len), D,
-                                float(scale), int(page_size), 1 if k.dtype == torch.bfloat16 else 0, _stream_ptr(stream)))
-    return out
+    return _calls.decode(q, k, v, n_heads, cur_seq_len, scale, block_table, page_size, partials, max_chunks, out, stream)
 
 
 def forward_bf16(q, k, v, n_heads, scale, causal=True, out=None, lse=None, causal_shift=0, out_fp32=False, stream=None):
     """bf16 variant: q, k, v are torch.bfloat16 [B,S,H*D] (D = 64 or 128); out is bf16, or fp32 with
     out_fp32=True (ring partial results); lse is fp32."""
-    import torch
-    if q.dtype != torch.bfloat16:
-        raise AttentionError("forward_bf16 needs bfloat16 tensors")
-    B, Sq, dm = q.shape
-    Sk = k.shape[1]
-    if out is None:
-        out = torch.empty(q.shape, dtype=torch.float32 if out_fp32 else torch.bfloat16, device=q.device)
-    if out.dtype != (torch.float32 if out_fp32 else torch.bfloat16):
-        raise AttentionError("forward_bf16: out dtype does not match out_fp32")
-    if lse is None:
-        lse = torch.empty((B, n_heads, Sq), dtype=torch.float32, device=q.device)
-    _check(lib().df_attn_forward_bf16(_ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(lse), B, n_heads, Sq, Sk,
-                                      dm // n_heads, float(scale), int(bool(causal)), int(causal_shift),
-                                      int(bool(out_fp32)), _stream_ptr(stream)))
-    return out, lse
+    return _calls.forward_bf16(q, k, v, n_heads, scale, causal, out, lse, causal_shift, out_fp32, stream)
 
 
 def delta_bf16(out, d_out, n_heads, delta_buf=None, stream=None):
-    import torch
-    B, S, dm = out.shape
-    if delta_buf is None:
-        delta_buf = torch.empty((B, n_heads, S), dtype=torch.float32, device=out.device)
-    _check(lib().df_attn_delta_bf16(_ptr(out), _ptr(d_out), _ptr(delta_buf), B, n_heads, S, dm // n_heads,
-                                    _stream_ptr(stream)))
-    return delta_buf
+    return _calls.delta_bf16(out, d_out, n_heads, delta_buf, stream)
 
 
 def backward_block_bf16(q, k, v, d_out, lse, delta_buf, n_heads, scale, causal=True, causal_shift=0, d_q=None, d_k=None,
                         d_v=None, out_fp32=False, stream=None):
     """Block form of the bf16 backward; gradients are bf16, or fp32 with out_fp32=True."""
-    import torch
-    B, Sq, dm = q.shape
-    Sk = k.shape[1]
-    gdt = torch.float32 if out_fp32 else torch.bfloat16
-    d_q = torch.empty(q.shape, dtype=gdt, device=q.device) if d_q is None else d_q
-    d_k = torch.empty(k.shape, dtype=gdt, device=q.device) if d_k is None else d_k
-    d_v = torch.empty(v.shape, dtype=gdt, device=q.device) if d_v is None else d_v
-    _check(lib().df_attn_backward_block_bf16(_ptr(q), _ptr(k), _ptr(v), _ptr(d_out), _ptr(lse), _ptr(delta_buf), _ptr(d_q),
-                                             _ptr(d_k), _ptr(d_v), B, n_heads, Sq, Sk, dm // n_heads, float(scale),
-                                             int(bool(causal)), int(causal_shift), int(bool(out_fp32)),
-                                             _stream_ptr(stream)))
-    return d_q, d_k, d_v
+    return _calls.backward_block_bf16(q, k, v, d_out, lse, delta_buf, n_heads, scale, causal, causal_shift, d_q, d_k, d_v, out_fp32,
+                                      stream)
 
 
 def backward_bf16(q, k, v, out, d_out, lse, n_heads, scale, causal=True, d_q=None, d_k=None, d_v=None, delta_buf=None,
                   stream=None):
     """bf16 variant of backward(): every [B,S,H*D] tensor is torch.bfloat16, lse and delta are fp32."""
-    import torch
-    B, S, dm = q.shape
-    d_q = torch.empty_like(q) if d_q is None else d_q
-    d_k = torch.empty_like(k) if d_k is None else d_k
-    d_v = torch.empty_like(v) if d_v is None else d_v
-    if delta_buf is None:
-        delta_buf = torch.empty((B, n_heads, S), dtype=torch.float32, device=q.device)
-    _check(lib().df_attn_backward_bf16(_ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(d_out), _ptr(lse), _ptr(d_q), _ptr(d_k),
-                                       _ptr(d_v), _ptr(delta_buf), B, n_heads, S, dm // n_heads, float(scale),
-                                       int(bool(causal)), _stream_ptr(stream)))
-    return d_q, d_k, d_v
+    return _calls.backward_bf16(q, k, v, out, d_out, lse, n_heads, scale, causal, d_q, d_k, d_v, delta_buf, stream)
 
 
 def delta(out, d_out, n_heads, delta_buf=None, stream=None):
-    import torch
-    B, S, dm = out.shape
-    if delta_buf is None:
-        delta_buf = torch.empty((B, n_heads, S), dtype=torch.float32, device=out.device)
-    _check(lib().df_attn_delta(_ptr(out), _ptr(d_out), _ptr(delta_buf), B, n_heads, S, dm // n_heads,
-                               _stream_ptr(stream)))
-    return delta_buf
+    return _calls.delta(out, d_out, n_heads, delta_buf, stream)
 
 
 def backward(q, k, v, out, d_out, lse, n_heads, scale, causal=True, d_q=None, d_k=None, d_v=None,
              delta_buf=None, stream=None):
-    import torch
-    B, S, dm = q.shape
-    d_q = torch.empty_like(q) if d_q is None else d_q
-    d_k = torch.empty_like(k) if d_k is None else d_k
-    d_v = torch.empty_like(v) if d_v is None else d_v
-    if delta_buf is None:
-        delta_buf = torch.empty((B, n_heads, S), dtype=torch.float32, device=q.device)
-    _check(lib().df_attn_backward(_ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(d_out), _ptr(lse), _ptr(d_q),
-                                  _ptr(d_k), _ptr(d_v), _ptr(delta_buf), B, n_heads, S, dm // n_heads,
-                                  float(scale), int(bool(causal)), _stream_ptr(stream)))
-    return d_q, d_k, d_v
+    return _calls.backward(q, k, v, out, d_out, lse, n_heads, scale, causal, d_q, d_k, d_v, delta_buf, stream)
 
 
 def backward_profile(q, k, v, out, d_out, lse, n_heads, scale, causal=True, d_q=None, d_k=None, d_v=None,
@@ -331,76 +283,33 @@ def backward_static_scratch(q, k, v, out, d_out, lse, n_heads, scale, causal=Tru
     """Backward through the entry point that takes no scratch argument and allocates nothing
     itself (the gradient tensors are allocated here, by the caller's side, only when not given).
     Raises AttentionError when batch*heads*seq_len exceeds STATIC_SCRATCH_MAX_ROWS."""
-    import torch
-    B, S, dm = q.shape
-    d_q = torch.empty_like(q) if d_q is None else d_q
-    d_k = torch.empty_like(k) if d_k is None else d_k
-    d_v = torch.empty_like(v) if d_v is None else d_v
-    _check(lib().df_attn_backward_static_scratch(_ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(d_out), _ptr(lse),
-                                                 _ptr(d_q), _ptr(d_k), _ptr(d_v), B, n_heads, S, dm // n_heads,
-                                                 float(scale), int(bool(causal)), _stream_ptr(stream)))
-    return d_q, d_k, d_v
+    return _calls.backward_static_scratch(q, k, v, out, d_out, lse, n_heads, scale, causal, d_q, d_k, d_v, stream)
 
 
 def backward_block(q, k, v, d_out, lse, delta_buf, n_heads, scale, causal=True, causal_shift=0, d_q=None,
                    d_k=None, d_v=None, stream=None):
-    import torch
-    B, Sq, dm = q.shape
-    Sk = k.shape[1]
-    d_q = torch.empty_like(q) if d_q is None else d_q
-    d_k = torch.empty_like(k) if d_k is None else d_k
-    d_v = torch.empty_like(v) if d_v is None else d_v
-    _check(lib().df_attn_backward_block(_ptr(q), _ptr(k), _ptr(v), _ptr(d_out), _ptr(lse), _ptr(delta_buf),
-                                        _ptr(d_q), _ptr(d_k), _ptr(d_v), B, n_heads, Sq, Sk, dm // n_heads,
-                                        float(scale), int(bool(causal)), int(causal_shift),
-                                        _stream_ptr(stream)))
-    return d_q, d_k, d_v
+    return _calls.backward_block(q, k, v, d_out, lse, delta_buf, n_heads, scale, causal, causal_shift, d_q, d_k, d_v, stream)
 
 
 def linear_qkv(x, wq, wk, wv, bq=None, bk=None, bv=None, q=None, k=None, v=None, stream=None):
     """q, k, v = x wq^T + bq, x wk^T + bk, x wv^T + bv in one launch. x [rows, in], w* [out, in], b* [out]."""
-    import torch
-    rows, fin = x.shape
-    fout = wq.shape[0]
-    q, k, v = (torch.empty((rows, fout), dtype=torch.float32, device=x.device) if t is None else t for t in (q, k, v))
-    _check(lib().df_linear_qkv_forward(_ptr(x), _ptr(wq), _ptr(wk), _ptr(wv), _ptr(bq), _ptr(bk), _ptr(bv), _ptr(q), _ptr(k),
-                                       _ptr(v), rows, fin, fout, _stream_ptr(stream)))
-    return q, k, v
+    return _calls.linear_qkv(x, wq, wk, wv, bq, bk, bv, q, k, v, stream)
 
 
 def linear(x, w, bias=None, residual=None, out=None, stream=None):
     """out = x w^T + bias + residual (bias, residual optional). x [rows, in], w [out, in]."""
-    import torch
-    rows, fin = x.shape
-    fout = w.shape[0]
-    if out is None:
-        out = torch.empty((rows, fout), dtype=torch.float32, device=x.device)
-    _check(lib().df_linear_forward(_ptr(x), _ptr(w), _ptr(bias), _ptr(residual), _ptr(out), rows, fin, fout,
-                                   _stream_ptr(stream)))
-    return out
+    return _calls.linear(x, w, bias, residual, out, stream)
 
 
 def linear_gelu(x, w, bias=None, pre_activation=None, out=None, keep_pre_activation=True, stream=None):
     """pre = x w^T + bias and out = gelu(pre) in one launch; returns (pre, out) (pre None with keep_pre_activation False)."""
-    import torch
-    rows, fin = x.shape
-    fout = w.shape[0]
-    if out is None:
-        out = torch.empty((rows, fout), dtype=torch.float32, device=x.device)
-    if pre_activation is None and keep_pre_activation:
-        pre_activation = torch.empty((rows, fout), dtype=torch.float32, device=x.device)
-    _check(lib().df_linear_gelu_forward(_ptr(x), _ptr(w), _ptr(bias), _ptr(pre_activation), _ptr(out), rows, fin, fout,
-                                        _stream_ptr(stream)))
-    return pre_activation, out
+    return _calls.linear_gelu(x, w, bias, pre_activation, out, keep_pre_activation, stream)
 
 
 def chunked_logit_ce(logits, targets, loss, total_rows, grad_logits=None, stream=None):
     """Softmax + cross-entropy over a chunk: logits [rows, cols] fp32 (overwritten with probabilities when
     grad_logits is given), targets [rows] int32/uint32 token ids, loss [1] fp32 accumulator. grad_logits None: eval form."""
-    rows, cols = logits.shape
-    _check(lib().df_chunked_logit_ce(_ptr(logits), _ptr(targets), _ptr(grad_logits), _ptr(loss), rows, cols, int(total_rows),
-                                     _stream_ptr(stream)))
-    return loss
+    return _calls.chunked_logit_ce(logits, targets, loss, total_rows, grad_logits, stream)
 
 
 # ------------------------------------------------------------------------------------------
@@ -410,49 +319,30 @@ def chunked_logit_ce(logits, targets, loss, total_rows, grad_logits=None, stream
 def layernorm(x, gamma=None, beta=None, out=None, means=None, rstds=None, stream=None):
     """LayerNorm over the last dimension of x [rows, cols] (fp32): returns (out, means, rstds), the statistics the
     backward needs (DeviceTensor::layernorm_into, lib.rs:1010-1040)."""
-    import torch
-    rows, cols = x.shape
-    out = torch.empty_like(x) if out is None else out
-    means = torch.empty(rows, dtype=torch.float32, device=x.device) if means is None else means
-    rstds = torch.empty(rows, dtype=torch.float32, device=x.device) if rstds is None else rstds
-    _check(lib().df_layernorm_forward(_ptr(x), _ptr(gamma), _ptr(beta), _ptr(out), _ptr(means), _ptr(rstds), rows, cols,
-                                      _stream_ptr(stream)))
-    return out, means, rstds
+    return _calls.layernorm(x, gamma, beta, out, means, rstds, stream)
 
 
 def layernorm_backward(grad_out, x, gamma, means, rstds, grad_x=None, grad_gamma=None, grad_beta=None, stream=None):
     """Backward of layernorm (DeviceTensor::layernorm_backward_into, lib.rs:1074-1100): returns grad_x; the column sums
     are ADDED to grad_gamma / grad_beta when given (the caller zeroes them)."""
-    import torch
-    rows, cols = x.shape
-    grad_x = torch.empty_like(x) if grad_x is None else grad_x
-    _check(lib().df_layernorm_backward(_ptr(grad_out), _ptr(x), _ptr(gamma), _ptr(means), _ptr(rstds), _ptr(grad_x),
-                                       _ptr(grad_gamma), _ptr(grad_beta), rows, cols, _stream_ptr(stream)))
-    return grad_x
+    return _calls.layernorm_backward(grad_out, x, gamma, means, rstds, grad_x, grad_gamma, grad_beta, stream)
 
 
 def gelu(x, out=None, stream=None):
     """tanh-form GELU (DeviceTensor::gelu_into, lib.rs:775-790)."""
-    import torch
-    out = torch.empty_like(x) if out is None else out
-    _check(lib().df_gelu_forward(_ptr(x), _ptr(out), x.numel(), _stream_ptr(stream)))
-    return out
+    return _calls.gelu(x, out, stream)
 
 
 def gelu_backward(grad_out, x, grad_x=None, stream=None):
     """grad_x = grad_out * gelu'(x) (DeviceTensor::gelu_backward_into, lib.rs:894-910)."""
-    import torch
-    grad_x = torch.empty_like(x) if grad_x is None else grad_x
-    _check(lib().df_gelu_backward(_ptr(grad_out), _ptr(x), _ptr(grad_x), x.numel(), _stream_ptr(stream)))
-    return grad_x
+    return _calls.gelu_backward(grad_out, x, grad_x, stream)
 
 
 def adamw_update(parameter, first_moment, second_moment, gradient, lr, beta1, beta2, eps, weight_decay, bias_correction1,
                  bias_correction2, stream=None):
     """One AdamW step on one tensor, in place (DeviceTensor::adamw_update, lib.rs:1755-1800)."""
-    _check(lib().df_adamw_update(_ptr(parameter), _ptr(first_moment), _ptr(second_moment), _ptr(gradient), parameter.numel(),
-                                 float(lr), float(beta1), float(beta2), float(eps), float(weight_decay), float(bias_correction1),
-                                 float(bias_correction2), _stream_ptr(stream)))
+    _calls.adamw_update(parameter, first_moment, second_moment, gradient, lr, beta1, beta2, eps, weight_decay, bias_correction1,
+                        bias_correction2, stream)
 
 
 class AdamwTensor(ctypes.Structure):
@@ -480,21 +370,16 @@ class AdamwPlan:
         self.table = host.to(self.tensors[0][0].device) if n else host
 
     def step(self, lr, beta1, beta2, eps, weight_decay, bias_correction1, bias_correction2, stream=None):
-        _check(lib().df_adamw_update_multi(_ptr(self.table), self.n_tensors, self.total_chunks, float(lr), float(beta1),
-                                           float(beta2), float(eps), float(weight_decay), float(bias_correction1),
-                                           float(bias_correction2), _stream_ptr(stream)))
+        _calls.adamw_step(self.table, self.n_tensors, self.total_chunks, lr, beta1, beta2, eps, weight_decay, bias_correction1,
+                          bias_correction2, stream)
 
 
 def merge_partials(o_a, lse_a, o_b, lse_b, n_heads, stream=None):
-    B, S, dm = o_a.shape
-    _check(lib().df_attn_merge_partials(_ptr(o_a), _ptr(lse_a), _ptr(o_b), _ptr(lse_b), B, n_heads, S,
-                                        dm // n_heads, _stream_ptr(stream)))
-    return o_a, lse_a
+    return _calls.merge_partials(o_a, lse_a, o_b, lse_b, n_heads, stream)
 
 
 def accumulate(dst, src, stream=None):
-    _check(lib().df_attn_accumulate(_ptr(dst), _ptr(src), dst.numel(), _stream_ptr(stream)))
-    return dst
+    return _calls.accumulate(dst, src, stream)
 
 
 # ------------------------------------------------------------------------------------------
@@ -523,22 +408,9 @@ class AttentionContext:
             holder[0] = torch.empty(max(n, 1), dtype=torch.float32, device=device)
         return holder[0]
 
-    def _check_shape(self, t, what):
-        if tuple(t.shape) != (self.seq_len, self.d_model):  # lib.rs:2051, 2252-2257
-            raise AttentionError(f"attention {what} shape mismatch")
-
     def forward_device_into(self, q, k, v, scale, causal, out):
-        self._check_shape(out, "output")
-        L = lib()
-        import torch
-        ptrs = [_ptr(t) for t in (q, k, v, out)]
-        torch.cuda.current_stream().synchronize()  # the legacy symbols run on the legacy default stream
-        if self.n_heads == 1:  # lib.rs:2055-2065
-            L.launch_fused_attention(*ptrs, self.seq_len, self.d_head, float(scale), int(bool(causal)))
-        else:
-            L.launch_fused_mha_forward(*ptrs, self.n_heads, self.seq_len, self.d_head, float(scale),
-                                       int(bool(causal)))
-        _check(L.df_attn_last_status())
+        # the legacy symbols run on the legacy default stream: a caller on another stream is waited for
+        _calls.context_forward(self.n_heads, self.seq_len, self.d_head, q, k, v, scale, causal, out)
 
     def forward_device(self, q, k, v, scale, causal):
         import torch
@@ -547,19 +419,8 @@ class AttentionContext:
         return out
 
     def backward_device_into(self, q, k, v, d_out, scale, causal, d_q, d_k, d_v):
-        for t, n in ((d_q, "d_q"), (d_k, "d_k"), (d_v, "d_v")):
-            self._check_shape(t, n)
-        L = lib()
-        import torch
-        ptrs = [_ptr(t) for t in (q, k, v, d_out, d_q, d_k, d_v)]
-        ptrs.append(_ptr(self._ensure_probabilities(q.device)))
-        torch.cuda.current_stream().synchronize()
-        if self.n_heads == 1:  # lib.rs:2260-2274
-            L.launch_attention_backward(*ptrs, self.seq_len, self.d_head, float(scale), int(bool(causal)))
-        else:
-            L.launch_fused_mha_backward(*ptrs, self.n_heads, self.seq_len, self.d_head, float(scale),
-                                        int(bool(causal)))
-        _check(L.df_attn_last_status())
+        _calls.context_backward(self.n_heads, self.seq_len, self.d_head, q, k, v, d_out, scale, causal, d_q, d_k, d_v,
+                                self._ensure_probabilities(q.device))
 
     def backward_device(self, q, k, v, d_out, scale, causal):
         import torch
