@@ -159,6 +159,11 @@ int tensor_linear(const float *x, const float *const *w, const float *const *bia
                   float *gelu_out,
                   int n_mats, uint32_t M, uint32_t K, uint32_t N, cudaStream_t s);
 
+// The same for at most kLinearRowsMax rows, one warp or a few per output feature (linear_rows.cu); tensor_linear calls it.
+constexpr uint32_t kLinearRowsMax = 8;
+int rows_linear(const float *x, const float *const *w, const float *const *bias, float *const *out, const float *residual, float *gelu_out,
+                int n_mats, uint32_t M, uint32_t K, uint32_t N, int n_sm, cudaStream_t s);
+
 // tanh-form GELU of the reference (kernels/elementwise.cu:180-215), shared by the elementwise kernels and the projection
 // kernel's epilogue so that the fused and the separate form give the same bits:
 // gelu(v) = 0.5 v (1 + tanh u), u = sqrt(2/pi) (v + 0.044715 v^3); with s = 1 / (1 + exp(-2u)): tanh u = 2s - 1,
