@@ -104,9 +104,7 @@ int backward_dispatch(const AttnParams &p, cudaStream_t s) {
   const bool tensor_ok = tensor_backward_supported(p);
   if (t_variant == DF_VARIANT_TENSOR && !tensor_ok) return DF_ERR_UNSUPPORTED;
   if (t_variant != DF_VARIANT_SIMT && tensor_ok) return tensor_backward(p, s);
-  int st = generic_backward_dkdv(p, s);
-  if (st != DF_OK) return st;
-  return generic_backward_dq(p, s);
+  return generic_backward(p, s);
 }
 
 int finish(int st) {

@@ -77,10 +77,9 @@ __device__ __forceinline__ size_t df_checked_index(size_t i, size_t n, unsigned 
 #define DF_IDX(i, n, status) (i)
 #endif
 
-// ---- SIMT kernels, any shape (attn_generic.cu) ----
+// ---- fp32 SIMT kernels, any shape (attn_simt.cu), and helper passes (attn_generic.cu) ----
 int generic_forward(const AttnParams &p, cudaStream_t s);            // out/lse and/or delta (stats mode)
-int generic_backward_dkdv(const AttnParams &p, cudaStream_t s);      // needs lse_in, delta_in
-int generic_backward_dq(const AttnParams &p, cudaStream_t s);
+int generic_backward(const AttnParams &p, cudaStream_t s);           // dQ, dK, dV; needs lse_in, delta_in
 int delta_prepass(const AttnParams &p, cudaStream_t s);              // delta = rowsum(dO * O)
 int merge_partials(float *o_a, float *lse_a, const float *o_b, const float *lse_b, uint32_t B,
                    uint32_t H, uint32_t S, uint32_t D, cudaStream_t s);

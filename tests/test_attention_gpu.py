@@ -119,6 +119,37 @@ def test_shape_sweep_simt(torch_cuda, oracle, causal):
             assert np.abs(g - r).max() <= 1e-4 * max(1.0, np.abs(r).max()), tag
 
 
+# heads enough for 64-row blocks; lengths around the 64-row tiles; every class of head size (32, 64, 96, 128 dims), 16- and 4-byte copies
+@pytest.mark.parametrize("Sq,Sk,shift", [(64, 64, 0), (65, 65, 0), (130, 130, 0), (193, 193, 0), (100, 164, 64), (164, 100, -64), (70, 200, 129)])
+@pytest.mark.parametrize("D", [20, 31, 48, 80, 97, 128])
+def test_simt_blocks_of_64_rows(torch_cuda, oracle, Sq, Sk, shift, D):
+    p = pkg()
+    B, H = 8, 20
+    q, k, v, go = _inputs(oracle, B, H, Sq, D, 7000 + Sq * 7 + Sk + D, Sk=Sk)
+    scale = hp.default_scale(D)
+    prev = p.set_variant(p.VARIANT_SIMT)
+    try:
+        tq, tk, tv, tg = to_dev(q, k, v, go)
+        out, lse = p.forward(tq, tk, tv, H, scale, True, causal_shift=shift)
+        delta = p.delta(out, tg, H)
+        dq, dk, dv = p.backward_block(tq, tk, tv, tg, lse, delta, H, scale, True, causal_shift=shift)
+        assert p.sync_status() == 0
+    finally:
+        p.set_variant(prev)
+    q4, k4, v4, g4 = (t.double().view(B, -1, H, D).transpose(1, 2) for t in (tq, tk, tv, tg))
+    s = q4 @ k4.transpose(2, 3) * scale
+    vis = torch_cuda.arange(Sk, device="cuda")[None, :] <= torch_cuda.arange(Sq, device="cuda")[:, None] + shift
+    pr = torch_cuda.where(vis, torch_cuda.exp(s - torch_cuda.where(vis, s, -torch_cuda.inf).amax(-1, keepdim=True).clamp_min(-1e30)), 0.0)
+    pr = pr / pr.sum(-1, keepdim=True).clamp_min(1e-300)
+    o = pr @ v4
+    dp = g4 @ v4.transpose(2, 3)
+    ds = pr * (dp - (g4 * o).sum(-1, keepdim=True))
+    want = (o, ds @ k4 * scale, ds.transpose(2, 3) @ q4 * scale, pr.transpose(2, 3) @ g4)
+    for got, ref, name in zip((out, dq, dk, dv), want, ("out", "dq", "dk", "dv")):
+        ref = ref.transpose(1, 2).reshape(got.shape)
+        assert float((got.double() - ref).abs().max()) <= 2e-5 * max(1.0, float(ref.abs().max())), name
+
+
 @pytest.mark.parametrize("persist", [0, 2])
 @pytest.mark.parametrize("causal", [True, False])
 def test_shape_sweep_tensor_forward(torch_cuda, oracle, causal, persist):
