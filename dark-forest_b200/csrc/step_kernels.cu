@@ -404,14 +404,40 @@ struct AdamHyper {
   float lr, beta1, beta2, eps, weight_decay, bias_correction1, bias_correction2;
 };
 
-// One element, in the reference's order of operations (matmul.cu:310-316).
+// One element, in the reference's order of operations (matmul.cu:310-316). The fused multiply-adds are written out, so that
+// every place this is inlined gives the same bits.
 __device__ __forceinline__ void adamw_one(float &p, float &m, float &v, float g, const AdamHyper &h) {
-  m = h.beta1 * m + (1.0f - h.beta1) * g;
-  v = h.beta2 * v + (1.0f - h.beta2) * (g * g);
+  m = fmaf(h.beta1, m, __fmul_rn(1.0f - h.beta1, g));
+  v = fmaf(h.beta2, v, __fmul_rn(1.0f - h.beta2, __fmul_rn(g, g)));
   const float m_hat = m / h.bias_correction1;
   const float v_hat = v / h.bias_correction2;
-  const float decay_factor = 1.0f - h.lr * h.weight_decay;
-  p = p * decay_factor - h.lr * m_hat / (sqrtf(v_hat) + h.eps);
+  const float decay_factor = fmaf(-h.lr, h.weight_decay, 1.0f);
+  p = fmaf(p, decay_factor, -(__fmul_rn(h.lr, m_hat) / __fadd_rn(sqrtf(v_hat), h.eps)));
+}
+
+// kAdamChunk elements, 16-byte aligned, by 256 threads: all eight loads of a thread are in flight before the first is used,
+// and nothing of it is wanted again (streaming accesses).
+constexpr int kAdamVec = kAdamChunk / (4 * 256);
+__device__ __forceinline__ void adamw_full_chunk(float *__restrict__ p, float *__restrict__ m, float *__restrict__ v,
+                                                 const float *__restrict__ g, uint32_t t, const AdamHyper &h) {
+  float4 pp[kAdamVec], mm[kAdamVec], vv[kAdamVec], gg[kAdamVec];
+#pragma unroll
+  for (int i = 0; i < kAdamVec; ++i) {
+    pp[i] = __ldcs(reinterpret_cast<const float4 *>(p) + i * 256 + t);
+    mm[i] = __ldcs(reinterpret_cast<const float4 *>(m) + i * 256 + t);
+    vv[i] = __ldcs(reinterpret_cast<const float4 *>(v) + i * 256 + t);
+    gg[i] = __ldcs(reinterpret_cast<const float4 *>(g) + i * 256 + t);
+  }
+#pragma unroll
+  for (int i = 0; i < kAdamVec; ++i) {
+    adamw_one(pp[i].x, mm[i].x, vv[i].x, gg[i].x, h);
+    adamw_one(pp[i].y, mm[i].y, vv[i].y, gg[i].y, h);
+    adamw_one(pp[i].z, mm[i].z, vv[i].z, gg[i].z, h);
+    adamw_one(pp[i].w, mm[i].w, vv[i].w, gg[i].w, h);
+    __stcs(reinterpret_cast<float4 *>(p) + i * 256 + t, pp[i]);
+    __stcs(reinterpret_cast<float4 *>(m) + i * 256 + t, mm[i]);
+    __stcs(reinterpret_cast<float4 *>(v) + i * 256 + t, vv[i]);
+  }
 }
 
 // `n` elements starting at the four pointers; the calling threads are `nthreads` wide with index `t`.
@@ -464,7 +490,12 @@ k_adamw_multi(const df_adamw_tensor_t *__restrict__ tensors, uint32_t n_tensors,
     const uint64_t off = (u - t.first_chunk) * kAdamChunk;
     if (off >= t.n) continue;  // a table whose first_chunk values leave gaps
     const uint64_t len = t.n - off < kAdamChunk ? t.n - off : kAdamChunk;
-    adamw_span(t.parameter + off, t.first_moment + off, t.second_moment + off, t.gradient + off, len, threadIdx.x, blockDim.x, h);
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(t.parameter) | reinterpret_cast<uintptr_t>(t.first_moment) |
+                           reinterpret_cast<uintptr_t>(t.second_moment) | reinterpret_cast<uintptr_t>(t.gradient);
+    if (len == kAdamChunk && (bits & 15u) == 0)
+      adamw_full_chunk(t.parameter + off, t.first_moment + off, t.second_moment + off, t.gradient + off, threadIdx.x, h);
+    else
+      adamw_span(t.parameter + off, t.first_moment + off, t.second_moment + off, t.gradient + off, len, threadIdx.x, blockDim.x, h);
   }
 }
 
@@ -637,7 +668,10 @@ int adamw_update_multi(const df_adamw_tensor_t *tensors_device, uint32_t n_tenso
   if (!tensors_device || bc1 == 0.0f || bc2 == 0.0f) return DF_ERR_INVALID_ARG;
   const int n_sm = sm_count();
   if (n_sm <= 0) return DF_ERR_CUDA;
-  const uint64_t cap = (uint64_t)n_sm * 16;
+  // State that goes through DRAM (more than about 96 MB of it) streams best with a block per chunk: blocks start as others end
+  // and loads and stores stay mixed (GPT-2 small, 124 M parameters: 520 us = 6.7 TB/s, 545 with a grid of 16 blocks per SM that
+  // walks the chunks, 612 before). What fits L2 is 5 % faster with the walking grid.
+  const uint64_t cap = total_chunks * kAdamChunk * 16 > (96ull << 20) ? 0x7fffffffull : (uint64_t)n_sm * 16;
   k_adamw_multi<<<(unsigned)(total_chunks < cap ? total_chunks : cap), 256, 0, s>>>(tensors_device, n_tensors, total_chunks,
                                                                                     hyper(lr, beta1, beta2, eps, weight_decay, bc1, bc2));
   note_launch();
