@@ -8,25 +8,26 @@
 //   launch_chunked_ce_eval         (softmax.cu:415-480)  loss += sum_rows (log(sum) - (z_target - max)) / total_rows
 // Same arithmetic (max-subtracted softmax in fp32 with __expf / __logf); what differs is the traffic. The
 // reference walks each row of [chunk_rows, vocab] three times through global memory (max; exp + write; normalise +
-// two writes: 3 reads, 3 writes of the 200 KB row). Here a CTA keeps the whole row in shared memory (a 50257-entry
-// row is 201 KB of the 227 KB an SM offers), so the training form reads the logits once and writes probabilities
-// and gradients once each (1 read + 2 writes, the algorithmic minimum), and the eval form reads once with an online
-// (max, sum) pair and writes nothing. The kernels are HBM-bound; grids are persistent (one CTA per SM, rows dealt
-// round robin). Rows of an odd-length vocabulary are not 16-byte aligned: every row is processed as a scalar head up
-// to the next 16-byte boundary, a float4 body and a scalar tail. Rows too long for shared memory take a two-pass
-// form from global memory (online max/sum, then the write pass).
+// two writes: 3 reads, 3 writes of the 200 KB row). Here a cluster of CTAs keeps the row in its shared memory, so
+// the training form reads the logits once and writes probabilities and gradients once each (1 read + 2 writes, the
+// algorithmic minimum); the eval form reads once with an online (max, sum) pair and writes nothing. Rows of an odd-length vocabulary are not
+// 16-byte aligned: every row is processed as a scalar head up to the next 16-byte boundary, a float4 body and a scalar
+// tail. Rows too long for a cluster's shared memory are walked in global memory.
+#include <cooperative_groups.h>
 #include <float.h>
 #include <math.h>
 
 #include <mutex>
 
 #include "df_common.cuh"
+#include "sm100_ptx.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace df {
 namespace {
 
 constexpr int kCeThreads = 1024;
-constexpr uint32_t kMaxSmemCols = 56 * 1024;  // 224 KB of floats: 57344 entries
 
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
@@ -65,85 +66,153 @@ __device__ __forceinline__ void split_row(const float *row, uint32_t cols, uint3
   *n4 = (cols - h) >> 2;
 }
 
-// Training form, row resident in shared memory.
-__global__ void __launch_bounds__(kCeThreads, 1)
-k_chunked_logit_ce_smem(float *__restrict__ logits, const uint32_t *__restrict__ targets, float *__restrict__ grad_logits,
-                        float *__restrict__ loss, uint32_t chunk_rows, uint32_t cols, float inv_total_rows) {
-  extern __shared__ __align__(16) float srow[];  // cols floats (+ up to 3 of padding in front), then 32 reduction slots
-  float *red = srow + ((cols + 3u + 3u) & ~3u);
-  float cta_loss = 0.0f;
-  for (uint32_t row = blockIdx.x; row < chunk_rows; row += gridDim.x) {
+// Training form, the row resident in the shared memory of a cluster of CTAs. What bounds it is HBM (1 read and 2 writes of
+// the row); a CTA that owns a whole SM and a whole row, as before, alternates between reading and writing and leaves the
+// last round of rows half empty (512 rows on 148 SMs). Here a row is cut into slices of at most 53 KB, one per CTA of
+// a cluster (short rows: several rows per cluster), and four CTAs share an SM, so that one row's loads run under another's
+// exponentials and stores. A thread copies its own 16-byte groups in with cp.async and reads back only those: no barrier until
+// the CTAs exchange one (max, sum) each. A running cluster takes over rows whose cluster has not started yet (claim_request): with
+// rows dealt out in advance the slowest SMs end 25 % after the others (2048 x 50257: 250 against 200 us), and with a cluster per
+// row the loss would be rounded once per row. Probabilities go in place, gradients out, with streaming stores; SAME_PHASE: the
+// gradient row lies at the same 16-byte phase as the logits row. Measured on B200 against the kernel before: 512 x 50257
+// 76.0 -> 56.2 us (5.5 TB/s), 2048 x 50257 268 -> 200 us (6.2 TB/s), 32 x 50257 15.3 -> 8.2 us, 512 x 5000 11.4 -> 10.0 us.
+constexpr int kSliceThreads = 256;
+constexpr int kMaxCeCluster = 8;
+constexpr uint32_t kSliceGroups = 13;     // groups of four floats per thread: 52 KB per CTA, four CTAs per SM
+constexpr uint32_t kMaxSliceGroups = 54;  // one CTA per SM
+
+template <bool SAME_PHASE>
+__global__ void __launch_bounds__(kSliceThreads, 4)
+k_logit_ce_cluster(float *__restrict__ logits, const uint32_t *__restrict__ targets, float *__restrict__ grad_logits,
+                   float *__restrict__ loss, uint32_t chunk_rows, uint32_t cols, uint32_t slices, uint32_t groups, uint32_t more,
+                   float inv_total_rows, unsigned int *status) {
+  extern __shared__ __align__(16) float4 slice[];  // [groups][kSliceThreads]
+  __shared__ float red[kSliceThreads / 32];
+  __shared__ float2 part[2][kMaxCeCluster];  // (max, sum) of every CTA of the cluster, for rows in turn
+  __shared__ uint32_t next_unit[2];
+  __shared__ __align__(16) uint4 claim;
+  __shared__ uint64_t claim_bar;
+  __shared__ uint32_t give_up;
+  __shared__ float cluster_loss;  // of the cluster's rows (in its first CTA)
+  cg::cluster_group cluster = cg::this_cluster();
+  const uint32_t n_cta = cluster.num_blocks(), rank = cluster.block_rank(), t = threadIdx.x;
+  const uint32_t slot = rank / slices, part_rank = rank - slot * slices, rows_per_cluster = n_cta / slices;
+  const uint32_t a_claim = ptx::smem_u32(&claim), a_bar = ptx::smem_u32(&claim_bar);
+  if (t == 0) {
+    ptx::mbar_init(a_bar, 1);
+    ptx::mbar_init_fence();
+    give_up = 0;
+    cluster_loss = 0.0f;
+  }
+  cluster.barrier_arrive();  // waited for before the first write to another CTA's shared memory
+  auto reduce = [&](float v, bool is_max) {
+    v = is_max ? warp_max(v) : warp_sum(v);
+    __syncthreads();  // the previous use of `red` is over
+    if ((t & 31) == 0) red[t >> 5] = v;
+    __syncthreads();
+    float r = red[0];
+#pragma unroll
+    for (int w = 1; w < kSliceThreads / 32; ++w) r = is_max ? fmaxf(r, red[w]) : r + red[w];
+    return r;
+  };
+  const bool one_row = rows_per_cluster == 1 && !more;
+  uint32_t turn = 0;
+  for (uint32_t unit = blockIdx.x / n_cta; unit != ~0u; unit = more ? next_unit[turn] : ~0u, turn ^= 1) {
+    if (more && rank == 0 && t == 0) {  // asked now, answered long before the exchange below
+      ptx::fence_proxy_async_smem();
+      ptx::mbar_arrive_expect_tx(a_bar, 16);
+      ptx::claim_request(a_claim, a_bar);
+    }
+    const bool has = unit * rows_per_cluster + slot < chunk_rows;  // else this CTA only keeps the cluster's barriers company
+    const uint32_t row = has ? unit * rows_per_cluster + slot : 0;
     float *grow = logits + (size_t)row * cols;
-    float *ggrad = grad_logits + (size_t)row * cols;
     const uint32_t target = __ldg(targets + row);
     uint32_t head, n4;
     split_row(grow, cols, &head, &n4);
-    // the shared copy is shifted so that the float4 body is 16-byte aligned on both sides
-    float *s = srow + ((4u - head) & 3u);
-    const uint32_t body_end = head + 4u * n4;
-    // ---- pass 1: global -> shared, running maximum
-    float tmax = -FLT_MAX;
-    if (threadIdx.x < head) {
-      const float x = grow[threadIdx.x];
-      s[threadIdx.x] = x;
-      tmax = x;
+    // this CTA: float4 groups [g0, g1) of the body; the first also has the row's scalar head, the last its scalar tail
+    const uint32_t per = groups * kSliceThreads, g0 = min(n4, part_rank * per), g1 = has ? min(n4, g0 + per) : g0;
+    const uint32_t body = head + 4u * n4;
+    uint32_t extra = cols;  // the scalar element of this thread, if any
+    if (has && part_rank == 0 && t < head) extra = t;
+    if (has && part_rank == slices - 1 && t >= 32 && t - 32 < cols - body) extra = body + (t - 32);
+    const float x_extra = extra < cols ? grow[extra] : 0.0f;
+    const float4 *src = reinterpret_cast<const float4 *>(grow + head);
+    const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(slice + t));
+    for (uint32_t i = 0; i < groups; ++i) {
+      const uint32_t g = g0 + i * kSliceThreads + t;
+      if (g < g1) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i * kSliceThreads * 16u), "l"(src + g) : "memory");
     }
-    {
-      const float4 *g4 = reinterpret_cast<const float4 *>(grow + head);
-      float4 *s4 = reinterpret_cast<float4 *>(s + head);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    const uint32_t mine = g1 > g0 + t ? (g1 - g0 - t + kSliceThreads - 1) / kSliceThreads : 0;  // groups of this thread
+    float top = extra < cols ? x_extra : -FLT_MAX;
 #pragma unroll 4
-      for (uint32_t i = threadIdx.x; i < n4; i += kCeThreads) {
-        const float4 x = __ldcs(g4 + i);  // read once: do not keep it in L2
-        s4[i] = x;
-        tmax = fmaxf(tmax, fmaxf(fmaxf(x.x, x.y), fmaxf(x.z, x.w)));
+    for (uint32_t i = 0; i < mine; ++i) {
+      const float4 x = slice[i * kSliceThreads + t];
+      top = fmaxf(top, fmaxf(fmaxf(x.x, x.y), fmaxf(x.z, x.w)));
+    }
+    const float cta_max = reduce(top, true);
+    float sum = extra < cols ? __expf(x_extra - cta_max) : 0.0f;
+#pragma unroll 4
+    for (uint32_t i = 0; i < mine; ++i) {
+      const float4 x = slice[i * kSliceThreads + t];
+      sum += (__expf(x.x - cta_max) + __expf(x.y - cta_max)) + (__expf(x.z - cta_max) + __expf(x.w - cta_max));
+    }
+    const float cta_sum = reduce(sum, false);
+    if (unit == blockIdx.x / n_cta) cluster.barrier_wait();
+    if (t < slices) cluster.map_shared_rank(&part[turn][0], slot * slices + t)[part_rank] = make_float2(cta_max, cta_sum);
+    if (more && rank == 0 && t == 0) {
+      const bool answered = ptx::mbar_wait(a_bar, turn, &give_up);
+      const uint32_t first = answered ? ptx::claim_result(a_claim) : ~0u;
+      if (!answered && status) atomicOr(status, DEV_STATUS_WAIT_EXPIRED);
+      for (uint32_t r = 0; r < n_cta; ++r) cluster.map_shared_rank(next_unit, r)[turn] = first == ~0u ? ~0u : first / n_cta;
+    }
+    cluster.sync();
+    float row_max = -FLT_MAX, row_sum = 0.0f;
+    for (uint32_t r = 0; r < slices; ++r) row_max = fmaxf(row_max, part[turn][r].x);
+    for (uint32_t r = 0; r < slices; ++r) row_sum += part[turn][r].y * __expf(part[turn][r].x - row_max);
+    const float inv_sum = 1.0f / row_sum, g_scale = inv_total_rows;
+    float *ggrad = grad_logits + (size_t)row * cols;
+    float p_target = -1.0f;
+    if (extra < cols) {
+      const float p = __expf(x_extra - row_max) * inv_sum;
+      grow[extra] = p;
+      ggrad[extra] = (p - (extra == target ? 1.0f : 0.0f)) * g_scale;
+      if (extra == target) p_target = p;
+    }
+    float4 *out = reinterpret_cast<float4 *>(grow + head);
+#pragma unroll 2
+    for (uint32_t i = 0; i < mine; ++i) {
+      const uint32_t g = g0 + i * kSliceThreads + t;
+      const float4 x = slice[i * kSliceThreads + t];
+      const float4 p = make_float4(__expf(x.x - row_max) * inv_sum, __expf(x.y - row_max) * inv_sum, __expf(x.z - row_max) * inv_sum,
+                                   __expf(x.w - row_max) * inv_sum);
+      __stcs(out + g, p);
+      // the target column (if it lies in this group of four) takes the scalar formula, (p - 1) * scale
+      const uint32_t k = target - (head + 4u * g);  // unsigned: 4 or more when the target is elsewhere
+      const float4 d = make_float4((p.x - (k == 0u ? 1.0f : 0.0f)) * g_scale, (p.y - (k == 1u ? 1.0f : 0.0f)) * g_scale,
+                                   (p.z - (k == 2u ? 1.0f : 0.0f)) * g_scale, (p.w - (k == 3u ? 1.0f : 0.0f)) * g_scale);
+      if (k < 4u) p_target = k == 0u ? p.x : (k == 1u ? p.y : (k == 2u ? p.z : p.w));
+      float *gd = ggrad + head + 4u * g;
+      if (SAME_PHASE) {
+        __stcs(reinterpret_cast<float4 *>(gd), d);
+      } else {
+        gd[0] = d.x; gd[1] = d.y; gd[2] = d.z; gd[3] = d.w;
       }
     }
-    if (body_end + threadIdx.x < cols) {
-      const float x = grow[body_end + threadIdx.x];
-      s[body_end + threadIdx.x] = x;
-      tmax = fmaxf(tmax, x);
-    }
-    const float row_max = block_max(tmax, red);
-    // ---- pass 2 (shared memory only): e = exp(x - max), sum
-    float tsum = 0.0f;
-    for (uint32_t i = threadIdx.x; i < cols; i += kCeThreads) {
-      const float e = __expf(s[i] - row_max);
-      s[i] = e;
-      tsum += e;
-    }
-    const float inv_sum = 1.0f / block_sum(tsum, red);
-    // ---- pass 3: probabilities and gradients out (streaming stores)
-    const float g_scale = inv_total_rows;
-    auto emit = [&](uint32_t i) {
-      const float p = s[i] * inv_sum;
-      grow[i] = p;
-      ggrad[i] = (p - (i == target ? 1.0f : 0.0f)) * g_scale;
-    };
-    if (threadIdx.x < head) emit(threadIdx.x);
-    {
-      float4 *g4 = reinterpret_cast<float4 *>(grow + head);
-      float4 *d4 = reinterpret_cast<float4 *>(ggrad + head);  // same 16-byte phase as the logits row (the launcher checks)
-      const float4 *s4 = reinterpret_cast<const float4 *>(s + head);
-#pragma unroll 4
-      for (uint32_t i = threadIdx.x; i < n4; i += kCeThreads) {
-        float4 p = s4[i];
-        p.x *= inv_sum; p.y *= inv_sum; p.z *= inv_sum; p.w *= inv_sum;
-        __stcs(g4 + i, p);
-        // the target column (if it lies in this group of four) takes the scalar formula, (p - 1) * scale
-        const uint32_t k = target - (head + 4u * i);  // unsigned: 4 or more when the target is elsewhere
-        const float4 g = make_float4((p.x - (k == 0u ? 1.0f : 0.0f)) * g_scale, (p.y - (k == 1u ? 1.0f : 0.0f)) * g_scale,
-                                     (p.z - (k == 2u ? 1.0f : 0.0f)) * g_scale, (p.w - (k == 3u ? 1.0f : 0.0f)) * g_scale);
-        __stcs(d4 + i, g);
-      }
-    }
-    if (body_end + threadIdx.x < cols) emit(body_end + threadIdx.x);
-    if (threadIdx.x == 0 && target < cols) cta_loss += -__logf(fmaxf(s[target] * inv_sum, 1e-12f)) * inv_total_rows;
-    __syncthreads();  // the row buffer is reused by the next row
+    if (p_target >= 0.0f)
+      atomicAdd(one_row ? loss : cluster.map_shared_rank(&cluster_loss, 0), -__logf(fmaxf(p_target, 1e-12f)) * inv_total_rows);
   }
-  if (threadIdx.x == 0 && cta_loss != 0.0f) atomicAdd(loss, cta_loss);
+  if (one_row) return;
+  // one addition per cluster: every further one would round the running loss once more
+  cluster.barrier_arrive();
+  if (rank == 0) {
+    cluster.barrier_wait();
+    if (t == 0 && cluster_loss != 0.0f) atomicAdd(loss, cluster_loss);
+  }
 }
 
-// Training form for rows that do not fit shared memory: online (max, sum) pass, then the write pass.
+// Training form for rows that do not fit a cluster's shared memory: max pass, sum pass and write pass from global memory.
 __global__ void __launch_bounds__(kCeThreads, 1)
 k_chunked_logit_ce_global(float *__restrict__ logits, const uint32_t *__restrict__ targets, float *__restrict__ grad_logits,
                           float *__restrict__ loss, uint32_t chunk_rows, uint32_t cols, float inv_total_rows) {
@@ -260,7 +329,7 @@ k_chunked_logit_ce_l2(float *__restrict__ logits, const uint32_t *__restrict__ t
 }
 
 // Eval form: one read of the row, online (max, sum) per thread, nothing written but the loss. One row per CTA, four
-// CTAs per SM.
+// CTAs per SM. (The cluster form above, with the row in shared memory, was slower: 26 against 18 us at 512 x 50257.)
 __global__ void __launch_bounds__(kCeL2Threads, 4)
 k_chunked_ce_eval(const float *__restrict__ logits, const uint32_t *__restrict__ targets, float *__restrict__ loss,
                   uint32_t chunk_rows, uint32_t cols, float inv_total_rows) {
@@ -321,7 +390,9 @@ int device_info(int *n_sm) {
   if (check_cuda(cudaGetDevice(&dev)) != DF_OK || dev < 0 || dev >= 64) return DF_ERR_CUDA;
   DeviceInfo &d = g_dev[dev];
   std::call_once(d.once, [&]() {
-    d.ok = cudaFuncSetAttribute(k_chunked_logit_ce_smem, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) == cudaSuccess &&
+    const int smem = (int)(kMaxSliceGroups * kSliceThreads * 16);
+    d.ok = cudaFuncSetAttribute(k_logit_ce_cluster<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+           cudaFuncSetAttribute(k_logit_ce_cluster<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
            cudaDeviceGetAttribute(&d.n_sm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && d.n_sm > 0;
   });
   if (!d.ok) {
@@ -340,32 +411,55 @@ int chunked_logit_ce(float *logits, const uint32_t *targets, float *grad_logits,
   if (!logits || !targets || !loss || total_rows == 0) return DF_ERR_INVALID_ARG;
   int n_sm = 0;
   if (device_info(&n_sm) != DF_OK) return DF_ERR_CUDA;
-  const unsigned grid = chunk_rows < (uint32_t)n_sm ? chunk_rows : (unsigned)n_sm;
   const float inv = 1.0f / (float)total_rows;
   if (!grad_logits) {
     k_chunked_ce_eval<<<chunk_rows, kCeL2Threads, 0, s>>>(logits, targets, loss, chunk_rows, cols, inv);
     note_launch();
     return check_cuda(cudaGetLastError());
   }
-  // the vector path of the resident-row kernel needs logits and grad_logits rows to be misaligned alike
-  const bool same_phase = ((reinterpret_cast<uintptr_t>(logits) ^ reinterpret_cast<uintptr_t>(grad_logits)) & 15u) == 0 &&
-                          (reinterpret_cast<uintptr_t>(logits) & 3u) == 0;
-  // DF_OPT_CE_VARIANT: 0 / 1 = resident row (default), 2 = two passes with the second out of L2
-  const int variant = option(DF_OPT_CE_VARIANT);
-  if (same_phase && variant == 2) {
+  // whether logits and grad_logits rows are misaligned alike (both stored with 16-byte accesses)
+  const bool same_phase = ((reinterpret_cast<uintptr_t>(logits) ^ reinterpret_cast<uintptr_t>(grad_logits)) & 15u) == 0;
+  // DF_OPT_CE_VARIANT: 0 / 1 = row resident in shared memory (default), 2 = two passes with the second out of L2
+  if (same_phase && option(DF_OPT_CE_VARIANT) == 2) {
     k_chunked_logit_ce_l2<<<chunk_rows, kCeL2Threads, 0, s>>>(logits, targets, grad_logits, loss, chunk_rows, cols, inv);
     note_launch();
     return check_cuda(cudaGetLastError());
   }
-  if (cols <= kMaxSmemCols && same_phase) {
-    const size_t smem = ((size_t)((cols + 6u) & ~3u) + 32) * sizeof(float);
-    k_chunked_logit_ce_smem<<<grid, kCeThreads, smem, s>>>(logits, targets, grad_logits, loss, chunk_rows, cols, inv);
+  // The smallest number of slices per row that leaves room for four CTAs per SM; more while the rows alone do not give every SM
+  // two CTAs; beyond eight slices' worth of columns (106000) the slices grow to a whole SM each. From 257 rows on, clusters of
+  // four CTAs take as many rows as they have slices for, which keeps the additions to the loss at 256 or fewer.
+  const uint32_t n4 = cols / 4 + 1;
+  uint32_t slices = 1;
+  auto groups_of = [&](uint32_t c) { return (n4 + c * kSliceThreads - 1) / (c * kSliceThreads); };
+  while (slices < (uint32_t)kMaxCeCluster && (groups_of(slices) > kSliceGroups ||
+                                              ((uint64_t)chunk_rows * slices < 2u * (uint64_t)n_sm && groups_of(slices) > 2)))
+    slices *= 2;
+  const uint32_t groups = groups_of(slices), cluster = slices < 4 && chunk_rows > 256 ? 4 : slices;
+  const uint32_t rows_per_cluster = cluster / slices, units = (chunk_rows + rows_per_cluster - 1) / rows_per_cluster;
+  if (groups > kMaxSliceGroups || (uint64_t)units * cluster > 0x7fffffffull) {
+    const unsigned grid = chunk_rows < (uint32_t)n_sm ? chunk_rows : (unsigned)n_sm;
+    k_chunked_logit_ce_global<<<grid, kCeThreads, 0, s>>>(logits, targets, grad_logits, loss, chunk_rows, cols, inv);
     note_launch();
     return check_cuda(cudaGetLastError());
   }
-  k_chunked_logit_ce_global<<<grid, kCeThreads, 0, s>>>(logits, targets, grad_logits, loss, chunk_rows, cols, inv);
+  // running clusters take over further rows only where there are more than two machines full of them: asking costs about 1.5 us
+  const uint32_t more = (uint64_t)units * cluster > 8u * (uint64_t)n_sm ? 1u : 0u;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(units * cluster);
+  cfg.blockDim = dim3(kSliceThreads);
+  cfg.dynamicSmemBytes = (size_t)groups * kSliceThreads * 16;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const int st = check_cuda(cudaLaunchKernelEx(&cfg, same_phase ? k_logit_ce_cluster<true> : k_logit_ce_cluster<false>, logits, targets,
+                                               grad_logits, loss, chunk_rows, cols, slices, groups, more, inv, device_status_ptr()));
   note_launch();
-  return check_cuda(cudaGetLastError());
+  return st;
 }
 
 }  // namespace df

@@ -167,6 +167,25 @@ __device__ __forceinline__ void tc_fence_after_sync() {
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Dynamic scheduling by the hardware's own block queue (cluster launch control): a running block takes over the index of a
+// block (cluster) that has not started yet. claim_request writes a 16-byte answer to shared memory and counts it on an mbarrier;
+// claim_result is the first block index of the cluster taken over, or ~0 when none was left (do not ask again then).
+__device__ __forceinline__ void claim_request(uint32_t answer, uint32_t bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(answer), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ uint32_t claim_result(uint32_t answer) {
+  uint32_t x;
+  asm volatile(
+      "{\n\t.reg .b128 h;\n\t.reg .pred p;\n\tld.shared.b128 h, [%1];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\tmov.u32 %0, 0xffffffff;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, h;\n\t}"
+      : "=r"(x)
+      : "r"(answer)
+      : "memory");
+  return x;
+}
+
 // ------------------------------------------------------------------ TMA (tiled, no multicast)
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap *m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");

@@ -104,3 +104,27 @@ def test_chunked_cross_entropy_matches_reference_cuda_kernels(oracle):
     probs_ref, grad_ref, loss_ref = oracle.chunked_ce(z, tg, total, train=True)   # and the oracle agrees with the reference
     assert _close(tz_b.cpu().numpy(), probs_ref) <= 1.0
     assert abs(float(lb) - loss_ref) <= 1e-5 * abs(loss_ref)
+
+
+@pytest.mark.parametrize("rows,cols,shift", [(3, 13311, 0), (3, 13313, 1), (600, 3000, 2), (5, 106493, 0), (2, 106501, 3), (1, 442400, 0)])
+def test_row_slices_over_clusters(rows, cols, shift):
+    """Rows at the edges of one to eight slices, of the largest slices and beyond them; gradient rows at another 16-byte phase."""
+    import torch
+    p = pkg()
+    g = torch.Generator(device="cuda")
+    g.manual_seed(rows + cols)
+    z = torch.randn((rows, cols), generator=g, device="cuda") * 3
+    tg = torch.randint(0, cols, (rows,), generator=g, device="cuda", dtype=torch.int32)
+    tg[0] = cols - 1
+    buf = torch.full((rows * cols + 8,), 7.0, device="cuda")
+    grad = buf[shift:shift + rows * cols].view(rows, cols)
+    want = torch.softmax(z.double(), 1)
+    loss = torch.zeros(1, device="cuda")
+    p.chunked_logit_ce(z, tg, loss, 2 * rows, grad_logits=grad)
+    assert p.sync_status() == 0
+    assert float((z.double() / want - 1).abs().max()) <= 2e-5
+    picked = want.gather(1, tg.long()[:, None])
+    assert abs(float(loss) + float(picked.log().sum()) / (2 * rows)) <= 1e-5 * max(1.0, float(loss))
+    want.scatter_add_(1, tg.long()[:, None], torch.full_like(picked, -1.0))
+    assert float((grad.double() * (2 * rows) - want).abs().max()) <= 2e-5
+    assert float(buf[:shift].sum()) == 7.0 * shift and float(buf[shift + rows * cols:].sum()) == 7.0 * (8 - shift)
