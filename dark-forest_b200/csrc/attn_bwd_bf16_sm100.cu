@@ -164,6 +164,7 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_holder;
+  pdl_wait();  // everything above touched only this CTA's shared and tensor memory
   const uint32_t tS = tmem, tDP = tmem + 128, tDV = tmem + 256, tDK = tmem + 256 + HD;
 
   if (warp == 8) {
@@ -428,6 +429,7 @@ k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_holder;
+  pdl_wait();  // everything above touched only this CTA's shared and tensor memory
   const uint32_t tS = tmem, tDP = tmem + 128, tDQ = tmem + 256;
 
   if (warp == 8) {
@@ -603,6 +605,7 @@ template <int LPS>  // lanes per (row, head) segment = D / 8
 __global__ void __launch_bounds__(256) k_delta_vec_bf16(const uint4 *__restrict__ o, const uint4 *__restrict__ g,
                                                         float *__restrict__ delta, uint32_t H, uint32_t S,
                                                         uint32_t tiles_per_batch) {
+  pdl_wait();
   extern __shared__ float s_sum[];  // [H][32]
   const uint32_t b = blockIdx.x / tiles_per_batch;
   const uint32_t i0 = (blockIdx.x % tiles_per_batch) * 32u;
@@ -669,11 +672,11 @@ int launch_backward(const AttnParams &p, cudaStream_t s) {
   bp.shift = p.shift;
   bp.status = device_status_ptr();
   const dim3 grid_kv(((p.Sk + BT - 1) / BT) * p.B * p.H);
-  k_attn_bwd_dkdv_bf16<C><<<grid_kv, kThreads, kv16::smem_total<C>(), s>>>(tmK, tmV, tmQ, tmG, bp);
+  launch_kernel(k_attn_bwd_dkdv_bf16<C>, grid_kv, dim3(kThreads), kv16::smem_total<C>(), s, tmK, tmV, tmQ, tmG, bp);
   note_launch();
   if (check_cuda(cudaGetLastError()) != DF_OK) return DF_ERR_CUDA;
   const dim3 grid_q(((p.Sq + BT - 1) / BT) * p.B * p.H);
-  k_attn_bwd_dq_bf16<C><<<grid_q, kThreads, dq16::smem_total<C>(), s>>>(tmQ, tmG, tmK, tmV, bp);
+  launch_kernel(k_attn_bwd_dq_bf16<C>, grid_q, dim3(kThreads), dq16::smem_total<C>(), s, tmQ, tmG, tmK, tmV, bp);
   note_launch();
   return check_cuda(cudaGetLastError());
 }
@@ -709,8 +712,8 @@ int delta_prepass_bf16(const AttnParams &p, cudaStream_t s) {
   const size_t smem = (size_t)p.H * 32 * sizeof(float);
   const uint4 *o4 = reinterpret_cast<const uint4 *>(p.o_in);
   const uint4 *g4 = reinterpret_cast<const uint4 *>(p.d_out);
-  if (p.D == 64) k_delta_vec_bf16<8><<<grid, 256, smem, s>>>(o4, g4, p.delta, p.H, p.Sq, tiles);
-  else k_delta_vec_bf16<16><<<grid, 256, smem, s>>>(o4, g4, p.delta, p.H, p.Sq, tiles);
+  if (p.D == 64) launch_kernel(k_delta_vec_bf16<8>, grid, dim3(256), smem, s, o4, g4, p.delta, p.H, p.Sq, tiles);
+  else launch_kernel(k_delta_vec_bf16<16>, grid, dim3(256), smem, s, o4, g4, p.delta, p.H, p.Sq, tiles);
   note_launch();
   return check_cuda(cudaGetLastError());
 }

@@ -261,7 +261,6 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
   // S^T / P^T is double-buffered (steps alternate between the two): S^T of step g+2 is issued as soon as dV of step g
   // has been, two steps ahead of the compute warps, so they never wait for it
   const uint32_t tS0 = tmem, tDP = tmem + 128, tDV = tmem + 256, tDK = tmem + 320, tS1 = tmem + 384;
-  pdl_trigger();
   pdl_wait();  // everything above touched only this CTA's shared and tensor memory
 
   // Counters every role keeps for itself: g = steps (query tiles) done over all items, n = items
@@ -746,7 +745,6 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 #endif
   int tr_n = 0;
 #endif
-  pdl_trigger();
   pdl_wait();  // everything above touched only this CTA's shared and tensor memory
 
   // g = steps (key tiles) done over all items, n = items done (see the dK/dV kernel)
@@ -1192,7 +1190,6 @@ int tensor_backward(const AttnParams &p, cudaStream_t s) {
   const dim3 grid_kv(items_kv < n_sm ? items_kv : n_sm);
   const dim3 grid_q(items_q < n_sm ? items_q : n_sm);
   cudaEvent_t *prof = t_profile_events;
-  const bool pdl = option(DF_OPT_PDL) != 0 && prof == nullptr;
   SideStreams::Side *sd = (!fuse && prof == nullptr && option(DF_OPT_BWD_OVERLAP) != 0) ? t_side.get() : nullptr;
   cudaStream_t s_dq = s;
   if (sd) {
@@ -1207,9 +1204,9 @@ int tensor_backward(const AttnParams &p, cudaStream_t s) {
   const int reps = prof ? kProfileReps : 1;
   for (int rep = 0; (fuse || prof) && rep < reps; ++rep) {
     // (a profiled call with ready-made row sums runs its dQ kernel here too, so that the events split the two kernels)
-    const cudaError_t e = fuse ? launch_kernel(k_attn_bwd_dq_tf32_d64<true>, grid_q, dim3(kBwdThreads), dq::kSmemTotal, s, pdl,
+    const cudaError_t e = fuse ? launch_kernel(k_attn_bwd_dq_tf32_d64<true>, grid_q, dim3(kBwdThreads), dq::kSmemTotal, s,
                                                tmQk, tmGk, tmKk, tmVk, tmKm, tmDQ, tmO, bp, items_q)
-                               : launch_kernel(k_attn_bwd_dq_tf32_d64<false>, grid_q, dim3(kBwdThreads), dq::kSmemTotal, s, pdl,
+                               : launch_kernel(k_attn_bwd_dq_tf32_d64<false>, grid_q, dim3(kBwdThreads), dq::kSmemTotal, s,
                                                tmQk, tmGk, tmKk, tmVk, tmKm, tmDQ, tmO, bp, items_q);
     note_launch();
 #if defined(DF_ATTN_TRACE) && defined(DF_ATTN_TRACE_DQ)
@@ -1227,7 +1224,7 @@ int tensor_backward(const AttnParams &p, cudaStream_t s) {
   }
   if (prof && check_cuda(cudaEventRecord(prof[1], s)) != DF_OK) return DF_ERR_CUDA;
   for (int rep = 0; rep < reps; ++rep) {
-    const cudaError_t e = launch_kernel(k_attn_bwd_dkdv_tf32_d64<DF_KV_NSUB>, grid_kv, dim3(kKvThreads), kv::kSmemTotal, s, pdl, tmKk, tmVk,
+    const cudaError_t e = launch_kernel(k_attn_bwd_dkdv_tf32_d64<DF_KV_NSUB>, grid_kv, dim3(kKvThreads), kv::kSmemTotal, s, tmKk, tmVk,
                                         tmQk, tmGk, tmQm, tmGm, tmDK, tmDV, bp, items_kv);
     note_launch();
 #if defined(DF_ATTN_TRACE) && !defined(DF_ATTN_TRACE_DQ)
@@ -1246,7 +1243,7 @@ int tensor_backward(const AttnParams &p, cudaStream_t s) {
   if (!fuse && !prof) {
     // with ready-made row sums the dQ kernel is independent of the dK/dV kernel
     const cudaError_t e = launch_kernel(k_attn_bwd_dq_tf32_d64<false>, grid_q, dim3(kBwdThreads), dq::kSmemTotal, s_dq,
-                                        pdl && !sd, tmQk, tmGk, tmKk, tmVk, tmKm, tmDQ, tmO, bp, items_q);
+                                        tmQk, tmGk, tmKk, tmVk, tmKm, tmDQ, tmO, bp, items_q);
     note_launch();
     if (check_cuda(e) != DF_OK) return DF_ERR_CUDA;
   }

@@ -28,6 +28,7 @@
 #include <mutex>
 
 #include "df_common.cuh"
+#include "sm100_ptx.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -147,6 +148,7 @@ __device__ __forceinline__ void read_granule(uint32_t addr, float2 (&f)[GB / (BF
 // 16: 386 -> 85 us (6.3 TB/s); 12 heads of 64 fp32 dims, 131072 contiguous tokens: 186 -> 115 us (7.0 TB/s).
 template <bool BF16, int GB, int LPT, int SLOTS, int kThreads, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 512 / kThreads) k_attn_decode_ring(const DecParams p) {
+  ptx::pdl_wait();
   constexpr int kWarps = kThreads / 32;
   constexpr int G = 32 / LPT, VE = GB / (BF16 ? 2 : 4), U = SLOTS == 1 ? 4 : 2, STAGES = 3;
   constexpr int kRound = kWarps * G;                  // tokens between a group's consecutive tokens
@@ -313,6 +315,7 @@ __device__ __forceinline__ float load1(const void *base, size_t e) {
 // Any d_head <= 128 and alignment: a half-warp per token, lane i owns dims i, i + 16, ..., two tokens a round.
 template <bool BF16, bool SPLIT>
 __global__ void __launch_bounds__(256) k_attn_decode_any(const DecParams p) {
+  ptx::pdl_wait();
   constexpr int kThreads = 256, kSlots = 8, TOK = 2, kHalfWarps = kThreads / 16;
   __shared__ MergeSmem sm;
   if (!SPLIT) cg::this_cluster().barrier_arrive();
@@ -394,8 +397,6 @@ __global__ void __launch_bounds__(256) k_attn_decode_any(const DecParams p) {
 // Merges the partial states of one head: grid = n_heads, 128 threads. The chunk maxima and sums
 // are staged in shared memory with coalesced loads, then thread d accumulates output dim d over the
 // chunks with independent, unrolled loads (a plain loop of dependent loads cost 11 us for 25 chunks).
-// Launched with programmatic stream serialization: its set-up overlaps the tail of the split kernel,
-// and griddepcontrol.wait orders it after that kernel's stores.
 constexpr int kMaxChunks = 1024;
 __global__ void __launch_bounds__(128) k_attn_decode_reduce(const float *__restrict__ pm, const float *__restrict__ pl,
                                                             const float *__restrict__ po, float *__restrict__ out,
@@ -403,7 +404,7 @@ __global__ void __launch_bounds__(128) k_attn_decode_reduce(const float *__restr
   __shared__ float s_w[kMaxChunks];
   __shared__ float s_red[4];
   const uint32_t h = blockIdx.x, d = threadIdx.x;
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  ptx::pdl_wait();
   float mx = -INFINITY;
   for (uint32_t c = d; c < n_chunks; c += 128) {
     const float mc = pm[(size_t)h * n_chunks + c];
@@ -436,17 +437,7 @@ __global__ void __launch_bounds__(128) k_attn_decode_reduce(const float *__restr
 }
 
 int launch_reduce(const DecParams &p, cudaStream_t s) {
-  cudaLaunchConfig_t rc = {};
-  rc.gridDim = dim3(p.H);
-  rc.blockDim = dim3(128);
-  rc.stream = s;
-  cudaLaunchAttribute ra[1];
-  ra[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  ra[0].val.programmaticStreamSerializationAllowed = 1;
-  rc.attrs = ra;
-  rc.numAttrs = 1;
-  const int st = check_cuda(cudaLaunchKernelEx(&rc, k_attn_decode_reduce, (const float *)p.pm, (const float *)p.pl,
-                                               (const float *)p.po, p.out, p.n_chunks, p.D));
+  const int st = check_cuda(launch_kernel(k_attn_decode_reduce, dim3(p.H), dim3(128), 0, s, p.pm, p.pl, p.po, p.out, p.n_chunks, p.D));
   note_launch();
   return st;
 }
@@ -469,21 +460,6 @@ struct DeviceInfo {
 
 using DecKernel = void (*)(const DecParams);
 
-cudaLaunchConfig_t cluster_config(cudaLaunchAttribute *attr, uint32_t cluster, uint32_t heads, int threads, size_t smem, cudaStream_t s) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(cluster, heads);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  attr->id = cudaLaunchAttributeClusterDimension;
-  attr->val.clusterDim.x = cluster;
-  attr->val.clusterDim.y = 1;
-  attr->val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cfg;
-}
-
 // One kernel in its two forms; `split` may be null when the caller never splits it.
 struct DecForm {
   DecKernel split, cluster;
@@ -502,8 +478,16 @@ const DeviceInfo *device_info(const DecForm &f) {
       ok = ok && (!k || cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem) == cudaSuccess);
     ok = ok && cudaFuncSetAttribute(f.cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
     for (int c = 1; ok && c <= kMaxCluster; ++c) {
+      cudaLaunchConfig_t cfg = {};
       cudaLaunchAttribute attr[1];
-      const cudaLaunchConfig_t cfg = cluster_config(attr, c, 64, f.threads, f.smem, nullptr);
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = c;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cfg.gridDim = dim3(c, 64);
+      cfg.blockDim = dim3(f.threads);
+      cfg.dynamicSmemBytes = f.smem;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
       ok = cudaOccupancyMaxActiveClusters(&di.resident[c], f.cluster, &cfg) == cudaSuccess;
     }
     di.ok = ok;
@@ -515,9 +499,7 @@ const DeviceInfo *device_info(const DecForm &f) {
 int launch_cluster(const DecForm &f, DecParams &p, uint32_t cluster, cudaStream_t s) {
   p.chunk = (p.T + cluster - 1) / cluster;
   p.n_chunks = cluster;
-  cudaLaunchAttribute attr[1];
-  const cudaLaunchConfig_t cfg = cluster_config(attr, cluster, p.H, f.threads, f.smem, s);
-  const int st = check_cuda(cudaLaunchKernelEx(&cfg, f.cluster, (const DecParams)p));
+  const int st = check_cuda(launch_clusters(f.cluster, cluster, dim3(cluster, p.H), dim3(f.threads), f.smem, s, p));
   note_launch();
   return st;
 }
@@ -558,7 +540,7 @@ int launch_form(const DecForm &narrow, const DecForm *wide, DecParams &p, uint32
     if (want > (uint32_t)kMaxChunks) want = kMaxChunks;
     p.chunk = (p.T + want - 1) / want;
     p.n_chunks = (p.T + p.chunk - 1) / p.chunk;
-    narrow.split<<<dim3(p.n_chunks, p.H), narrow.threads, narrow.smem, s>>>(p);
+    launch_kernel(narrow.split, dim3(p.n_chunks, p.H), dim3(narrow.threads), narrow.smem, s, p);
     note_launch();
     if (check_cuda(cudaGetLastError()) != DF_OK) return DF_ERR_CUDA;
     return launch_reduce(p, s);

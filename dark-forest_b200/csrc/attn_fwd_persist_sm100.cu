@@ -173,7 +173,6 @@ k_attn_fwd_persist_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __gri
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_holder;
-  pdl_trigger();
   pdl_wait();  // everything above touched only this CTA's shared and tensor memory
   DF_PTRACE(warp == kWarpMma ? 0 : (warp == 0 ? 1 : 2), 2);
 
@@ -639,9 +638,9 @@ int tensor_forward_persistent(const AttnParams &p, cudaStream_t s) {
   // measured on B200 (B*H = 96 / 12): S = 1024 0.0536 vs 0.0559 ms with the loop inline; S = 8192 0.2644 vs 0.2609, S = 16384
   // 1.001 vs 0.968 with one out-of-line copy
   const cudaError_t launch_err =
-      p.Sq <= 2048 ? launch_kernel(k_attn_fwd_persist_tf32_d64<true, DF_FWD_HALVES>, grid, dim3(kThreadsOf(DF_FWD_HALVES)), kSmemTotal, s, option(DF_OPT_PDL) != 0, tmQ,
+      p.Sq <= 2048 ? launch_kernel(k_attn_fwd_persist_tf32_d64<true, DF_FWD_HALVES>, grid, dim3(kThreadsOf(DF_FWD_HALVES)), kSmemTotal, s, tmQ,
                                    tmK, tmV, tmO, tab, fp)
-                   : launch_kernel(k_attn_fwd_persist_tf32_d64<false, DF_FWD_HALVES>, grid, dim3(kThreadsOf(DF_FWD_HALVES)), kSmemTotal, s, option(DF_OPT_PDL) != 0, tmQ,
+                   : launch_kernel(k_attn_fwd_persist_tf32_d64<false, DF_FWD_HALVES>, grid, dim3(kThreadsOf(DF_FWD_HALVES)), kSmemTotal, s, tmQ,
                                    tmK, tmV, tmO, tab, fp);
   note_launch();
 #ifdef DF_ATTN_TRACE

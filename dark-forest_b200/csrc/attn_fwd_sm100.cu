@@ -183,6 +183,7 @@ k_attn_fwd(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
   const int n_kv[2] = {visible_kv_tiles(p, q0), visible_kv_tiles(p, q0 + BM)};
   const int n_max = n_kv[0] > n_kv[1] ? n_kv[0] : n_kv[1];
 
+  pdl_wait();
   // Rows that exist but see no key at all: O = 0, lse = -inf (reference guard, attention_fused.cu:104).
   if (warp < 16) {
     const int t = warp >> 3;
@@ -689,7 +690,7 @@ int launch_forward(const AttnParams &p, cudaStream_t s) {
   fp.debug_mode = getenv("DF_ATTN_FWD_DEBUG") ? atoi(getenv("DF_ATTN_FWD_DEBUG")) : 0;
 #endif
   const dim3 grid(((p.Sq + 2 * BM - 1) / (2 * BM)) * p.B * p.H);
-  k_attn_fwd<C><<<grid, kFwdThreads, C::kSmemTotal, s>>>(tmQ, tmK, tmV, tmO, fp);
+  launch_kernel(k_attn_fwd<C>, grid, dim3(kFwdThreads), C::kSmemTotal, s, tmQ, tmK, tmV, tmO, fp);
   note_launch();
 #ifdef DF_ATTN_TRACE
   if (getenv("DF_ATTN_TRACE_DUMP")) {

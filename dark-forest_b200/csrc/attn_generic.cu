@@ -3,6 +3,7 @@
 #include <math.h>
 
 #include "df_common.cuh"
+#include "sm100_ptx.cuh"
 
 namespace df {
 
@@ -20,6 +21,7 @@ __global__ void __launch_bounds__(256) k_delta_vec(const float4 *__restrict__ o,
                                                    const float4 *__restrict__ g,
                                                    float *__restrict__ delta, uint32_t H,
                                                    uint32_t S, uint32_t tiles_per_batch, uint32_t R) {
+  ptx::pdl_wait();
   extern __shared__ float s_sum[];  // [H][R], R = rows per block (32, or 8 when the grid would be too small)
   const uint32_t b = blockIdx.x / tiles_per_batch;
   const uint32_t i0 = (blockIdx.x % tiles_per_batch) * R;
@@ -61,6 +63,7 @@ __global__ void __launch_bounds__(256) k_delta_vec(const float4 *__restrict__ o,
 template <bool VEC>
 __global__ void __launch_bounds__(256) k_delta_any(const float *__restrict__ o, const float *__restrict__ g, float *__restrict__ delta,
                                                    uint32_t B, uint32_t H, uint32_t S, uint32_t D) {
+  ptx::pdl_wait();
   const size_t n = (size_t)B * H * S;
   const uint32_t lane = threadIdx.x & 7u;
   for (size_t u0 = blockIdx.x * (size_t)32; u0 < n; u0 += (size_t)gridDim.x * 32) {
@@ -87,6 +90,7 @@ __global__ void __launch_bounds__(256) k_delta_any(const float *__restrict__ o, 
 __global__ void k_merge_partials(float *__restrict__ o_a, float *__restrict__ lse_a,
                                  const float *__restrict__ o_b, const float *__restrict__ lse_b,
                                  uint32_t B, uint32_t H, uint32_t S, uint32_t D) {
+  ptx::pdl_wait();
   const size_t n = (size_t)B * S * H * D;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n;
        e += (size_t)gridDim.x * blockDim.x) {
@@ -107,6 +111,7 @@ __global__ void k_merge_partials(float *__restrict__ o_a, float *__restrict__ ls
 // Second pass of the merge: the statistics themselves (kept separate so that every element
 // thread of the first pass reads the un-merged lse_a).
 __global__ void k_merge_lse(float *__restrict__ lse_a, const float *__restrict__ lse_b, size_t n) {
+  ptx::pdl_wait();
   for (size_t u = blockIdx.x * (size_t)blockDim.x + threadIdx.x; u < n;
        u += (size_t)gridDim.x * blockDim.x) {
     const float la = lse_a[u], lb = __ldg(lse_b + u);
@@ -116,6 +121,7 @@ __global__ void k_merge_lse(float *__restrict__ lse_a, const float *__restrict__
 }
 
 __global__ void k_accumulate(float *__restrict__ dst, const float *__restrict__ src, size_t n) {
+  ptx::pdl_wait();
   for (size_t u = blockIdx.x * (size_t)blockDim.x + threadIdx.x; u < n;
        u += (size_t)gridDim.x * blockDim.x)
     dst[u] += __ldg(src + u);
@@ -143,17 +149,17 @@ int delta_prepass(const AttnParams &p, cudaStream_t s) {
     const float4 *o4 = reinterpret_cast<const float4 *>(p.o_in);
     const float4 *g4 = reinterpret_cast<const float4 *>(p.d_out);
     switch (D / 4) {
-      case 1: k_delta_vec<1><<<grid, 256, smem, s>>>(o4, g4, p.delta, H, S, tiles, R); break;
-      case 2: k_delta_vec<2><<<grid, 256, smem, s>>>(o4, g4, p.delta, H, S, tiles, R); break;
-      case 4: k_delta_vec<4><<<grid, 256, smem, s>>>(o4, g4, p.delta, H, S, tiles, R); break;
-      case 8: k_delta_vec<8><<<grid, 256, smem, s>>>(o4, g4, p.delta, H, S, tiles, R); break;
-      case 16: k_delta_vec<16><<<grid, 256, smem, s>>>(o4, g4, p.delta, H, S, tiles, R); break;
-      default: k_delta_vec<32><<<grid, 256, smem, s>>>(o4, g4, p.delta, H, S, tiles, R); break;
+      case 1: launch_kernel(k_delta_vec<1>, grid, dim3(256), smem, s, o4, g4, p.delta, H, S, tiles, R); break;
+      case 2: launch_kernel(k_delta_vec<2>, grid, dim3(256), smem, s, o4, g4, p.delta, H, S, tiles, R); break;
+      case 4: launch_kernel(k_delta_vec<4>, grid, dim3(256), smem, s, o4, g4, p.delta, H, S, tiles, R); break;
+      case 8: launch_kernel(k_delta_vec<8>, grid, dim3(256), smem, s, o4, g4, p.delta, H, S, tiles, R); break;
+      case 16: launch_kernel(k_delta_vec<16>, grid, dim3(256), smem, s, o4, g4, p.delta, H, S, tiles, R); break;
+      default: launch_kernel(k_delta_vec<32>, grid, dim3(256), smem, s, o4, g4, p.delta, H, S, tiles, R); break;
     }
   } else {
     const size_t n = (size_t)p.B * H * S;
-    if (D % 4 == 0 && aligned) k_delta_any<true><<<grid_1d(n * 8, 256), 256, 0, s>>>(p.o_in, p.d_out, p.delta, p.B, H, S, D);
-    else k_delta_any<false><<<grid_1d(n * 8, 256), 256, 0, s>>>(p.o_in, p.d_out, p.delta, p.B, H, S, D);
+    if (D % 4 == 0 && aligned) launch_kernel(k_delta_any<true>, dim3(grid_1d(n * 8, 256)), dim3(256), 0, s, p.o_in, p.d_out, p.delta, p.B, H, S, D);
+    else launch_kernel(k_delta_any<false>, dim3(grid_1d(n * 8, 256)), dim3(256), 0, s, p.o_in, p.d_out, p.delta, p.B, H, S, D);
   }
   note_launch();
   return check_cuda(cudaGetLastError());
@@ -163,15 +169,15 @@ int merge_partials(float *o_a, float *lse_a, const float *o_b, const float *lse_
                    uint32_t H, uint32_t S, uint32_t D, cudaStream_t s) {
   const size_t n = (size_t)B * S * H * D;
   if (n == 0) return DF_OK;
-  k_merge_partials<<<grid_1d(n, 256), 256, 0, s>>>(o_a, lse_a, o_b, lse_b, B, H, S, D);
-  k_merge_lse<<<grid_1d((size_t)B * H * S, 256), 256, 0, s>>>(lse_a, lse_b, (size_t)B * H * S);
+  launch_kernel(k_merge_partials, dim3(grid_1d(n, 256)), dim3(256), 0, s, o_a, lse_a, o_b, lse_b, B, H, S, D);
+  launch_kernel(k_merge_lse, dim3(grid_1d((size_t)B * H * S, 256)), dim3(256), 0, s, lse_a, lse_b, (size_t)B * H * S);
   note_launch(2);
   return check_cuda(cudaGetLastError());
 }
 
 int accumulate(float *dst, const float *src, uint64_t n, cudaStream_t s) {
   if (n == 0) return DF_OK;
-  k_accumulate<<<grid_1d(n, 256), 256, 0, s>>>(dst, src, (size_t)n);
+  launch_kernel(k_accumulate, dim3(grid_1d(n, 256)), dim3(256), 0, s, dst, src, (size_t)n);
   note_launch();
   return check_cuda(cudaGetLastError());
 }

@@ -220,6 +220,7 @@ __device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %
 
 template <int R, int VW, int CG>
 __global__ void __launch_bounds__(256, 1) k_simt_fwd(const AttnParams p, const Order order, const int ld, const int vec) {
+  ptx::pdl_wait();
   constexpr int BM = TY * R, LDT = BM + 4;
   extern __shared__ __align__(16) float smem[];
   const int group = threadIdx.x / NT, tid = threadIdx.x % NT, tx = tid % TX, ty = tid / TX;
@@ -539,6 +540,7 @@ __device__ __forceinline__ void backward_block(const AttnParams &p, uint32_t til
 template <int R, int VW, int CG>
 __global__ void __launch_bounds__(256, 1) k_simt_bwd(const AttnParams p, const uint32_t key_tiles, const uint32_t query_tiles, const int ld,
                                                      const int vec) {
+  ptx::pdl_wait();
   extern __shared__ __align__(16) float smem[];
   const uint32_t heads = p.B * p.H, slot = blockIdx.x / heads, bh = blockIdx.x - slot * heads;
   const uint32_t both = 2 * min(key_tiles, query_tiles);
@@ -610,8 +612,7 @@ int forward_form(const AttnParams &p, cudaStream_t s) {
   order.heavy_last = p.causal != 0;
   const uint64_t blocks = (uint64_t)order.tiles * order.heads;
   if (blocks > 0x7fffffffull) return DF_ERR_UNSUPPORTED;
-  k_simt_fwd<R, VW, CG><<<(unsigned)blocks, 256, (q + kv + kt + second + kSlack) * sizeof(float), s>>>(
-      with_status(p), order, ld, aligned_rows(p.D, {p.q, p.k, p.v}));
+  launch_kernel(k_simt_fwd<R, VW, CG>, dim3((unsigned)blocks), dim3(256), (q + kv + kt + second + kSlack) * sizeof(float), s, with_status(p), order, ld, aligned_rows(p.D, {p.q, p.k, p.v}));
   note_launch();
   return check_cuda(cudaGetLastError());
 }
@@ -626,7 +627,7 @@ int backward_form(const AttnParams &p, cudaStream_t s) {
   const uint32_t key_tiles = (p.Sk + BM - 1) / BM, query_tiles = (p.Sq + BM - 1) / BM;
   const uint64_t blocks = ((uint64_t)key_tiles + query_tiles) * p.B * p.H;
   if (blocks > 0x7fffffffull) return DF_ERR_UNSUPPORTED;
-  k_simt_bwd<R, VW, CG><<<(unsigned)blocks, 256, floats * sizeof(float), s>>>(with_status(p), key_tiles, query_tiles, ld,
+  launch_kernel(k_simt_bwd<R, VW, CG>, dim3((unsigned)blocks), dim3(256), floats * sizeof(float), s, with_status(p), key_tiles, query_tiles, ld,
                                                                             aligned_rows(p.D, {p.q, p.k, p.v, p.d_out}));
   note_launch();
   return check_cuda(cudaGetLastError());

@@ -8,6 +8,7 @@
 // elements (eight 16-byte loads per lane in flight) and as short as it takes to have eight warps per SM, down to 256.
 // Measured on B200, 1 row: 768 -> 768 15.6 -> 2.6 us, 768 -> 3 x 768 15.9 -> 3.0, 768 -> 3072 16.1 -> 3.2, 3072 -> 768 40 -> 3.2.
 #include "df_common.cuh"
+#include "sm100_ptx.cuh"
 
 namespace df {
 namespace {
@@ -25,6 +26,7 @@ struct RowsParams {
 // MR: rows held per warp (M rounded up to a power of two); KS: warps per output feature.
 template <int MR, int KS>
 __global__ void __launch_bounds__(kThreads) k_linear_rows(const RowsParams p) {
+  ptx::pdl_wait();
   __shared__ float part[kWarps][MR];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t f = blockIdx.x * (kWarps / KS) + warp / KS;
@@ -87,10 +89,10 @@ template <int MR>
 void launch(const RowsParams &p, int ks, cudaStream_t s) {
   const unsigned grid = (p.features * (unsigned)ks + kWarps - 1) / kWarps;
   switch (ks) {
-    case 1: k_linear_rows<MR, 1><<<grid, kThreads, 0, s>>>(p); break;
-    case 2: k_linear_rows<MR, 2><<<grid, kThreads, 0, s>>>(p); break;
-    case 4: k_linear_rows<MR, 4><<<grid, kThreads, 0, s>>>(p); break;
-    default: k_linear_rows<MR, 8><<<grid, kThreads, 0, s>>>(p); break;
+    case 1: launch_kernel(k_linear_rows<MR, 1>, grid, dim3(kThreads), 0, s, p); break;
+    case 2: launch_kernel(k_linear_rows<MR, 2>, grid, dim3(kThreads), 0, s, p); break;
+    case 4: launch_kernel(k_linear_rows<MR, 4>, grid, dim3(kThreads), 0, s, p); break;
+    default: launch_kernel(k_linear_rows<MR, 8>, grid, dim3(kThreads), 0, s, p); break;
   }
 }
 

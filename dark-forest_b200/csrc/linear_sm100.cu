@@ -93,6 +93,7 @@ k_linear_tf32(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_holder;
+  pdl_wait();  // everything above touched only this CTA's shared and tensor memory
   const int n_kb = (int)((p.K + TK - 1) / TK);
 
   // tile number -> (row tile, matrix, feature tile); the feature tile runs fastest
@@ -320,7 +321,7 @@ int tensor_linear(const float *x, const float *const *w, const float *const *bia
   p.tiles = (long long)((M + TM - 1) / TM) * p.n_tiles_total;
   p.status = device_status_ptr();
   const dim3 grid((unsigned)(p.tiles < di.n_sm ? p.tiles : di.n_sm));
-  k_linear_tf32<<<grid, kLinThreads, kSmemTotal, s>>>(tmX, tmW[0], tmW[1], tmW[2], tmO[0], tmO[1], tmO[2], p);
+  launch_kernel(k_linear_tf32, grid, dim3(kLinThreads), kSmemTotal, s, tmX, tmW[0], tmW[1], tmW[2], tmO[0], tmO[1], tmO[2], p);
   note_launch();
   return check_cuda(cudaGetLastError());
 }

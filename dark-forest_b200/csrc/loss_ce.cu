@@ -86,6 +86,7 @@ __global__ void __launch_bounds__(kSliceThreads, 4)
 k_logit_ce_cluster(float *__restrict__ logits, const uint32_t *__restrict__ targets, float *__restrict__ grad_logits,
                    float *__restrict__ loss, uint32_t chunk_rows, uint32_t cols, uint32_t slices, uint32_t groups, uint32_t more,
                    float inv_total_rows, unsigned int *status) {
+  ptx::pdl_wait();
   extern __shared__ __align__(16) float4 slice[];  // [groups][kSliceThreads]
   __shared__ float red[kSliceThreads / 32];
   __shared__ float2 part[2][kMaxCeCluster];  // (max, sum) of every CTA of the cluster, for rows in turn
@@ -216,6 +217,7 @@ k_logit_ce_cluster(float *__restrict__ logits, const uint32_t *__restrict__ targ
 __global__ void __launch_bounds__(kCeThreads, 1)
 k_chunked_logit_ce_global(float *__restrict__ logits, const uint32_t *__restrict__ targets, float *__restrict__ grad_logits,
                           float *__restrict__ loss, uint32_t chunk_rows, uint32_t cols, float inv_total_rows) {
+  ptx::pdl_wait();
   __shared__ float red[32];
   float cta_loss = 0.0f;
   for (uint32_t row = blockIdx.x; row < chunk_rows; row += gridDim.x) {
@@ -251,6 +253,7 @@ constexpr int kCeL2Threads = 512;
 __global__ void __launch_bounds__(kCeL2Threads, 3)
 k_chunked_logit_ce_l2(float *__restrict__ logits, const uint32_t *__restrict__ targets, float *__restrict__ grad_logits,
                       float *__restrict__ loss, uint32_t chunk_rows, uint32_t cols, float inv_total_rows) {
+  ptx::pdl_wait();
   __shared__ float red[32];
   const uint32_t row = blockIdx.x;
   if (row >= chunk_rows) return;
@@ -333,6 +336,7 @@ k_chunked_logit_ce_l2(float *__restrict__ logits, const uint32_t *__restrict__ t
 __global__ void __launch_bounds__(kCeL2Threads, 4)
 k_chunked_ce_eval(const float *__restrict__ logits, const uint32_t *__restrict__ targets, float *__restrict__ loss,
                   uint32_t chunk_rows, uint32_t cols, float inv_total_rows) {
+  ptx::pdl_wait();
   __shared__ float red[32];
   const uint32_t row = blockIdx.x;
   if (row >= chunk_rows) return;
@@ -413,7 +417,7 @@ int chunked_logit_ce(float *logits, const uint32_t *targets, float *grad_logits,
   if (device_info(&n_sm) != DF_OK) return DF_ERR_CUDA;
   const float inv = 1.0f / (float)total_rows;
   if (!grad_logits) {
-    k_chunked_ce_eval<<<chunk_rows, kCeL2Threads, 0, s>>>(logits, targets, loss, chunk_rows, cols, inv);
+    launch_kernel(k_chunked_ce_eval, dim3(chunk_rows), dim3(kCeL2Threads), 0, s, logits, targets, loss, chunk_rows, cols, inv);
     note_launch();
     return check_cuda(cudaGetLastError());
   }
@@ -421,7 +425,7 @@ int chunked_logit_ce(float *logits, const uint32_t *targets, float *grad_logits,
   const bool same_phase = ((reinterpret_cast<uintptr_t>(logits) ^ reinterpret_cast<uintptr_t>(grad_logits)) & 15u) == 0;
   // DF_OPT_CE_VARIANT: 0 / 1 = row resident in shared memory (default), 2 = two passes with the second out of L2
   if (same_phase && option(DF_OPT_CE_VARIANT) == 2) {
-    k_chunked_logit_ce_l2<<<chunk_rows, kCeL2Threads, 0, s>>>(logits, targets, grad_logits, loss, chunk_rows, cols, inv);
+    launch_kernel(k_chunked_logit_ce_l2, dim3(chunk_rows), dim3(kCeL2Threads), 0, s, logits, targets, grad_logits, loss, chunk_rows, cols, inv);
     note_launch();
     return check_cuda(cudaGetLastError());
   }
@@ -438,26 +442,15 @@ int chunked_logit_ce(float *logits, const uint32_t *targets, float *grad_logits,
   const uint32_t rows_per_cluster = cluster / slices, units = (chunk_rows + rows_per_cluster - 1) / rows_per_cluster;
   if (groups > kMaxSliceGroups || (uint64_t)units * cluster > 0x7fffffffull) {
     const unsigned grid = chunk_rows < (uint32_t)n_sm ? chunk_rows : (unsigned)n_sm;
-    k_chunked_logit_ce_global<<<grid, kCeThreads, 0, s>>>(logits, targets, grad_logits, loss, chunk_rows, cols, inv);
+    launch_kernel(k_chunked_logit_ce_global, grid, dim3(kCeThreads), 0, s, logits, targets, grad_logits, loss, chunk_rows, cols, inv);
     note_launch();
     return check_cuda(cudaGetLastError());
   }
   // running clusters take over further rows only where there are more than two machines full of them: asking costs about 1.5 us
   const uint32_t more = (uint64_t)units * cluster > 8u * (uint64_t)n_sm ? 1u : 0u;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(units * cluster);
-  cfg.blockDim = dim3(kSliceThreads);
-  cfg.dynamicSmemBytes = (size_t)groups * kSliceThreads * 16;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = cluster;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  const int st = check_cuda(cudaLaunchKernelEx(&cfg, same_phase ? k_logit_ce_cluster<true> : k_logit_ce_cluster<false>, logits, targets,
-                                               grad_logits, loss, chunk_rows, cols, slices, groups, more, inv, device_status_ptr()));
+  const int st = check_cuda(launch_clusters(same_phase ? k_logit_ce_cluster<true> : k_logit_ce_cluster<false>, cluster, dim3(units * cluster),
+                                            dim3(kSliceThreads), (size_t)groups * kSliceThreads * 16, s, logits, targets, grad_logits, loss,
+                                            chunk_rows, cols, slices, groups, more, inv, device_status_ptr()));
   note_launch();
   return st;
 }

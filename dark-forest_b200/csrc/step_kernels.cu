@@ -48,6 +48,7 @@ template <int VPL>
 __global__ void __launch_bounds__(kRowThreads)
 k_layernorm_fwd(const float *__restrict__ x, const float *__restrict__ gamma, const float *__restrict__ beta,
                 float *__restrict__ out, float *__restrict__ means, float *__restrict__ rstds, uint32_t rows, uint32_t cols) {
+  pdl_wait();
   const uint32_t lane = threadIdx.x & 31u, nvec = cols >> 2;
   const uint32_t warps = gridDim.x * (kRowThreads / 32);
   const float inv_n = 1.0f / (float)cols;
@@ -108,6 +109,7 @@ __device__ __forceinline__ float block_sum(float v, float *red) {
 __global__ void __launch_bounds__(kRowThreads)
 k_layernorm_fwd_any(const float *__restrict__ x, const float *__restrict__ gamma, const float *__restrict__ beta,
                     float *__restrict__ out, float *__restrict__ means, float *__restrict__ rstds, uint32_t rows, uint32_t cols) {
+  pdl_wait();
   __shared__ float red[kRowThreads / 32];
   const float inv_n = 1.0f / (float)cols;
   for (uint32_t row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -142,6 +144,7 @@ __global__ void __launch_bounds__(kRowThreads, VPL <= 6 ? 2 : 1)
 k_layernorm_bwd(const float *__restrict__ grad_out, const float *__restrict__ x, const float *__restrict__ gamma,
                 const float *__restrict__ means, const float *__restrict__ rstds, float *__restrict__ grad_x,
                 float *__restrict__ grad_gamma, float *__restrict__ grad_beta, uint32_t rows, uint32_t cols) {
+  pdl_wait();
   extern __shared__ float col_sums[];  // [cols] grad_gamma partials, [cols] grad_beta partials
   const uint32_t lane = threadIdx.x & 31u, nvec = cols >> 2;
   const uint32_t warps = gridDim.x * (kRowThreads / 32);
@@ -214,6 +217,7 @@ k_layernorm_bwd_staged(const float *__restrict__ grad_out, const float *__restri
                        const float *__restrict__ means, const float *__restrict__ rstds, float *__restrict__ grad_x,
                        float *__restrict__ grad_gamma, float *__restrict__ grad_beta, uint32_t rows, uint32_t cols, uint32_t stages,
                        unsigned int *status) {
+  pdl_wait();
   extern __shared__ __align__(128) uint8_t staged_smem[];
   const uint32_t n_warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, nvec = cols >> 2;
   const uint32_t row_bytes = cols * 4u;
@@ -338,6 +342,7 @@ __global__ void __launch_bounds__(kRowThreads)
 k_layernorm_bwd_any(const float *__restrict__ grad_out, const float *__restrict__ x, const float *__restrict__ gamma,
                     const float *__restrict__ means, const float *__restrict__ rstds, float *__restrict__ grad_x,
                     float *__restrict__ grad_gamma, float *__restrict__ grad_beta, uint32_t rows, uint32_t cols) {
+  pdl_wait();
   __shared__ float red[kRowThreads / 32];
   const float n = (float)cols;
   for (uint32_t row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -369,6 +374,7 @@ __device__ __forceinline__ float gelu_grad_f(float v) { return gelu_slope(v); }
 
 template <bool VEC>
 __global__ void __launch_bounds__(256) k_gelu_fwd(const float *__restrict__ x, float *__restrict__ out, uint64_t n) {
+  pdl_wait();
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (VEC) {
     const uint64_t nv = n >> 2;
@@ -385,6 +391,7 @@ __global__ void __launch_bounds__(256) k_gelu_fwd(const float *__restrict__ x, f
 template <bool VEC>
 __global__ void __launch_bounds__(256)
 k_gelu_bwd(const float *__restrict__ grad_out, const float *__restrict__ x, float *__restrict__ grad_x, uint64_t n) {
+  pdl_wait();
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (VEC) {
     const uint64_t nv = n >> 2;
@@ -473,6 +480,7 @@ __device__ __forceinline__ void adamw_span(float *__restrict__ p, float *__restr
 
 __global__ void __launch_bounds__(256)
 k_adamw(float *__restrict__ p, float *__restrict__ m, float *__restrict__ v, const float *__restrict__ g, uint64_t n, AdamHyper h) {
+  pdl_wait();
   adamw_span(p, m, v, g, n, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, (uint64_t)gridDim.x * blockDim.x, h);
 }
 
@@ -480,6 +488,7 @@ k_adamw(float *__restrict__ p, float *__restrict__ m, float *__restrict__ v, con
 // first_chunk[t] <= u < first_chunk[t + 1] (found by bisection over the table, which sits in L1/L2 after the first units).
 __global__ void __launch_bounds__(256)
 k_adamw_multi(const df_adamw_tensor_t *__restrict__ tensors, uint32_t n_tensors, uint64_t total_chunks, AdamHyper h) {
+  pdl_wait();
   for (uint64_t u = blockIdx.x; u < total_chunks; u += gridDim.x) {
     uint32_t lo = 0, hi = n_tensors - 1;
     while (lo < hi) {
@@ -556,13 +565,13 @@ int layernorm_forward(const float *x, const float *gamma, const float *beta, flo
   // as they free up: with a grid sized to the machine and 3.5 rows per warp the last round ran a quarter full)
   const uint32_t cap = vec && cols <= 4096 ? row_blocks : (uint32_t)n_sm * 8u;
   if (vec && cols <= 768) {
-    k_layernorm_fwd<6><<<row_blocks < cap ? row_blocks : cap, kRowThreads, 0, s>>>(x, gamma, beta, out, means, rstds, rows, cols);
+    launch_kernel(k_layernorm_fwd<6>, dim3(row_blocks < cap ? row_blocks : cap), dim3(kRowThreads), 0, s, x, gamma, beta, out, means, rstds, rows, cols);
   } else if (vec && cols <= 1024) {
-    k_layernorm_fwd<8><<<row_blocks < cap ? row_blocks : cap, kRowThreads, 0, s>>>(x, gamma, beta, out, means, rstds, rows, cols);
+    launch_kernel(k_layernorm_fwd<8>, dim3(row_blocks < cap ? row_blocks : cap), dim3(kRowThreads), 0, s, x, gamma, beta, out, means, rstds, rows, cols);
   } else if (vec && cols <= 4096) {
-    k_layernorm_fwd<32><<<row_blocks < cap ? row_blocks : cap, kRowThreads, 0, s>>>(x, gamma, beta, out, means, rstds, rows, cols);
+    launch_kernel(k_layernorm_fwd<32>, dim3(row_blocks < cap ? row_blocks : cap), dim3(kRowThreads), 0, s, x, gamma, beta, out, means, rstds, rows, cols);
   } else {
-    k_layernorm_fwd_any<<<rows < cap ? rows : cap, kRowThreads, 0, s>>>(x, gamma, beta, out, means, rstds, rows, cols);
+    launch_kernel(k_layernorm_fwd_any, dim3(rows < cap ? rows : cap), dim3(kRowThreads), 0, s, x, gamma, beta, out, means, rstds, rows, cols);
   }
   note_launch();
   return check_cuda(cudaGetLastError());
@@ -589,26 +598,26 @@ int layernorm_backward(const float *grad_out, const float *x, const float *gamma
     if (option(DF_OPT_LN_STAGED) != 0 && stages >= 2u && rows >= (uint32_t)n_sm * warps && staged_ready()) {
       const size_t bytes = ((warps * stages * 8u + 16u + 127u) & ~127u) + (size_t)warps * stages * 2u * row_bytes;
       if (cols <= 768)
-        k_layernorm_bwd_staged<6><<<n_sm, warps * 32, bytes, s>>>(grad_out, x, gamma, means, rstds, grad_x, grad_gamma, grad_beta, rows,
+        launch_kernel(k_layernorm_bwd_staged<6>, dim3(n_sm), dim3(warps * 32), bytes, s, grad_out, x, gamma, means, rstds, grad_x, grad_gamma, grad_beta, rows,
                                                                   cols, stages, device_status_ptr());
       else
-        k_layernorm_bwd_staged<8><<<n_sm, warps * 32, bytes, s>>>(grad_out, x, gamma, means, rstds, grad_x, grad_gamma, grad_beta, rows,
+        launch_kernel(k_layernorm_bwd_staged<8>, dim3(n_sm), dim3(warps * 32), bytes, s, grad_out, x, gamma, means, rstds, grad_x, grad_gamma, grad_beta, rows,
                                                                   cols, stages, device_status_ptr());
       note_launch();
       return check_cuda(cudaGetLastError());
     }
     if (cols <= 768) {
       const uint32_t cap = (uint32_t)n_sm * resident_blocks(k_layernorm_bwd<6>, 0);
-      k_layernorm_bwd<6><<<row_blocks < cap ? row_blocks : cap, kRowThreads, smem, s>>>(grad_out, x, gamma, means, rstds, grad_x,
+      launch_kernel(k_layernorm_bwd<6>, dim3(row_blocks < cap ? row_blocks : cap), dim3(kRowThreads), smem, s, grad_out, x, gamma, means, rstds, grad_x,
                                                                                       grad_gamma, grad_beta, rows, cols);
     } else {
       const uint32_t cap = (uint32_t)n_sm * resident_blocks(k_layernorm_bwd<8>, 1);
-      k_layernorm_bwd<8><<<row_blocks < cap ? row_blocks : cap, kRowThreads, smem, s>>>(grad_out, x, gamma, means, rstds, grad_x,
+      launch_kernel(k_layernorm_bwd<8>, dim3(row_blocks < cap ? row_blocks : cap), dim3(kRowThreads), smem, s, grad_out, x, gamma, means, rstds, grad_x,
                                                                                       grad_gamma, grad_beta, rows, cols);
     }
   } else {
     const uint32_t cap = (uint32_t)n_sm * 8u;
-    k_layernorm_bwd_any<<<rows < cap ? rows : cap, kRowThreads, 0, s>>>(grad_out, x, gamma, means, rstds, grad_x, grad_gamma,
+    launch_kernel(k_layernorm_bwd_any, dim3(rows < cap ? rows : cap), dim3(kRowThreads), 0, s, grad_out, x, gamma, means, rstds, grad_x, grad_gamma,
                                                                         grad_beta, rows, cols);
   }
   note_launch();
@@ -622,8 +631,8 @@ int gelu_forward(const float *x, float *out, uint64_t n, cudaStream_t s) {
   if (n_sm <= 0) return DF_ERR_CUDA;
   const uint64_t want = (n / 4 + 255) / 256 + 1, cap = (uint64_t)n_sm * 16;
   const unsigned grid = (unsigned)(want < cap ? want : cap);
-  if (aligned16(x) && aligned16(out)) k_gelu_fwd<true><<<grid, 256, 0, s>>>(x, out, n);
-  else k_gelu_fwd<false><<<grid, 256, 0, s>>>(x, out, n);
+  if (aligned16(x) && aligned16(out)) launch_kernel(k_gelu_fwd<true>, grid, dim3(256), 0, s, x, out, n);
+  else launch_kernel(k_gelu_fwd<false>, grid, dim3(256), 0, s, x, out, n);
   note_launch();
   return check_cuda(cudaGetLastError());
 }
@@ -635,8 +644,8 @@ int gelu_backward(const float *grad_out, const float *x, float *grad_x, uint64_t
   if (n_sm <= 0) return DF_ERR_CUDA;
   const uint64_t want = (n / 4 + 255) / 256 + 1, cap = (uint64_t)n_sm * 16;
   const unsigned grid = (unsigned)(want < cap ? want : cap);
-  if (aligned16(x) && aligned16(grad_out) && aligned16(grad_x)) k_gelu_bwd<true><<<grid, 256, 0, s>>>(grad_out, x, grad_x, n);
-  else k_gelu_bwd<false><<<grid, 256, 0, s>>>(grad_out, x, grad_x, n);
+  if (aligned16(x) && aligned16(grad_out) && aligned16(grad_x)) launch_kernel(k_gelu_bwd<true>, grid, dim3(256), 0, s, grad_out, x, grad_x, n);
+  else launch_kernel(k_gelu_bwd<false>, grid, dim3(256), 0, s, grad_out, x, grad_x, n);
   note_launch();
   return check_cuda(cudaGetLastError());
 }
@@ -648,7 +657,7 @@ int adamw_update(float *p, float *m, float *v, const float *g, uint64_t n, float
   const int n_sm = sm_count();
   if (n_sm <= 0) return DF_ERR_CUDA;
   const uint64_t want = (n / 4 + 255) / 256 + 1, cap = (uint64_t)n_sm * 16;
-  k_adamw<<<(unsigned)(want < cap ? want : cap), 256, 0, s>>>(p, m, v, g, n, hyper(lr, beta1, beta2, eps, weight_decay, bc1, bc2));
+  launch_kernel(k_adamw, dim3((unsigned)(want < cap ? want : cap)), dim3(256), 0, s, p, m, v, g, n, hyper(lr, beta1, beta2, eps, weight_decay, bc1, bc2));
   note_launch();
   return check_cuda(cudaGetLastError());
 }
@@ -672,7 +681,7 @@ int adamw_update_multi(const df_adamw_tensor_t *tensors_device, uint32_t n_tenso
   // and loads and stores stay mixed (GPT-2 small, 124 M parameters: 520 us = 6.7 TB/s, 545 with a grid of 16 blocks per SM that
   // walks the chunks, 612 before). What fits L2 is 5 % faster with the walking grid.
   const uint64_t cap = total_chunks * kAdamChunk * 16 > (96ull << 20) ? 0x7fffffffull : (uint64_t)n_sm * 16;
-  k_adamw_multi<<<(unsigned)(total_chunks < cap ? total_chunks : cap), 256, 0, s>>>(tensors_device, n_tensors, total_chunks,
+  launch_kernel(k_adamw_multi, dim3((unsigned)(total_chunks < cap ? total_chunks : cap)), dim3(256), 0, s, tensors_device, n_tensors, total_chunks,
                                                                                     hyper(lr, beta1, beta2, eps, weight_decay, bc1, bc2));
   note_launch();
   return check_cuda(cudaGetLastError());
