@@ -150,3 +150,30 @@ def test_projection_with_gelu_epilogue(oracle, rows, fin, fout):
         with pytest.raises(p.AttentionError):   # in_features not a multiple of 4
             p.linear_gelu(tx[:, : fin - 1].contiguous(), tw[:, : fin - 1].contiguous(), tb)
         p.lib().df_attn_last_status()
+
+
+# CTA pairs at every tile width, contractions split over clusters, and the edges between the forms (8 / 9 rows: linear_rows)
+@pytest.mark.parametrize("rows,fin,fout", [(8, 260, 772), (9, 768, 768), (9, 3072, 100), (100, 768, 768), (129, 1028, 260), (257, 3072, 768),
+                                           (511, 256, 512), (1000, 3072, 768), (2049, 768, 2308), (4100, 516, 772), (9000, 260, 196), (3000, 1024, 1024)])
+def test_projection_forms(rows, fin, fout):
+    import torch
+    torch.cuda.set_device(0)
+    p = pkg()
+    g = torch.Generator(device="cuda")
+    g.manual_seed(rows + fin)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    x, w, b, r = rnd(rows, fin), [rnd(fout, fin) * 0.02 for _ in range(3)], [rnd(fout) for _ in range(3)], rnd(rows, fout)
+    buf = torch.full((rows * fout + 64,), 777.0, device="cuda")
+    out = buf[32:-32].view(rows, fout)
+    want = [x.double() @ wi.double().t() + bi.double() for wi, bi in zip(w, b)]
+    p.linear(x, w[0], b[0], residual=r, out=out)
+    assert p.sync_status() == 0
+    tol = 2e-3 * max(1.0, float(want[0].abs().max()))
+    assert float((out.double() - want[0] - r.double()).abs().max()) <= tol
+    assert bool((buf[:32] == 777.0).all()) and bool((buf[-32:] == 777.0).all())
+    assert torch.equal(out, p.linear(x, w[0], b[0], residual=r))
+    for got, ref in zip(p.linear_qkv(x, *w, *b), want):
+        assert float((got.double() - ref).abs().max()) <= tol
+    pre, act = p.linear_gelu(x, w[1], b[1])
+    assert p.sync_status() == 0
+    assert float((pre.double() - want[1]).abs().max()) <= tol and torch.equal(act, p.gelu(pre))
