@@ -642,12 +642,14 @@ int backward_form(const AttnParams &p, cudaStream_t s) {
 
 int generic_forward(const AttnParams &p, cudaStream_t s) {
   if (p.Sq == 0 || p.B == 0 || p.H == 0) return DF_OK;
+  if ((uint64_t)p.B * p.H > 65535u) return DF_ERR_UNSUPPORTED;  // refused before any CUDA call, as callers were told
   return wide_blocks(p.Sq, p) ? DF_BY_HEAD_DIM(forward_form, 8) : DF_BY_HEAD_DIM(forward_form, 4);
 }
 
 // dQ, dK and dV from lse_in and delta_in; with no keys (or no queries) the other side's gradients are zero.
 int generic_backward(const AttnParams &p, cudaStream_t s) {
   if ((p.Sq == 0 && p.Sk == 0) || p.B == 0 || p.H == 0) return DF_OK;
+  if ((uint64_t)p.B * p.H > 65535u) return DF_ERR_UNSUPPORTED;  // refused before any CUDA call, as callers were told
   return wide_blocks((uint64_t)p.Sq + p.Sk, p) ? DF_BY_HEAD_DIM(backward_form, 8) : DF_BY_HEAD_DIM(backward_form, 4);
 }
 
