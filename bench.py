@@ -483,7 +483,7 @@ def run_ours(args):
                 "peak_source": "cuBLAS TF32 8192^3 burst (best of 10) measured in this run; 4 s sustained figure and half of "
                                f"MEASURED_PEAKS.json's bf16 burst ({peaks.get('bf16_tflops')} TFLOP/s {peak_kind}) in `peaks`",
                 "ms_per_launch": ms_dkdv,
-                "other_kernels": {"k_attn_fwd_persist_tf32_d64": {"ms": ms_fwd, "tflops": fwd_tf, "frac": fwd_tf / tf32_peak,
+                "other_kernels": {"k_attn_fwd_tf32_d64": {"ms": ms_fwd, "tflops": fwd_tf, "frac": fwd_tf / tf32_peak,
                                                                  "fracs": fracs(fwd_tf), "traffic": TRAFFIC["fwd"]},
                                   "k_attn_bwd_dq_tf32_d64": {"ms": ms_dq, "tflops": dq_tf, "frac": dq_tf / tf32_peak,
                                                              "fracs": fracs(dq_tf), "traffic": TRAFFIC["dq"],

@@ -25,6 +25,18 @@ thread_local uint64_t t_launches = 0;
 __device__ unsigned int g_device_status_word = 0;
 }  // namespace
 
+int sm_count() {
+  static std::once_flag once[64];
+  static int count[64];
+  int dev = 0;
+  if (check_cuda(cudaGetDevice(&dev)) != DF_OK || dev < 0 || dev >= 64) return 0;
+  std::call_once(once[dev], [&]() {
+    int n = 0;
+    count[dev] = (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0) ? n : 0;
+  });
+  return count[dev];
+}
+
 void note_status(int status) {
   if (status != DF_OK && t_status == DF_OK) t_status = status;
 }

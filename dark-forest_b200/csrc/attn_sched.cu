@@ -1,7 +1,6 @@
-// attn_sched.cu — host side of the explicit work lists of the persistent kernels: a MULTIFIT
-// assignment of weighted items to CTAs, cached per shape. Nothing here touches the GPU.
+// attn_sched.cu — explicit work lists for kernels that deal their items out in advance: a MULTIFIT
+// assignment of weighted items to CTAs. Nothing here touches the GPU.
 #include <algorithm>
-#include <mutex>
 #include <numeric>
 #include <vector>
 
@@ -9,22 +8,6 @@
 
 namespace df {
 namespace {
-
-struct Entry {
-  SchedKey key;
-  int n_items;
-  SchedTable table;
-  bool valid = false;
-};
-constexpr int kEntries = 16;
-Entry g_cache[kEntries];
-int g_next = 0;
-std::mutex g_mutex;
-
-bool same(const SchedKey &a, const SchedKey &b) {
-  return a.kind == b.kind && a.bh == b.bh && a.sq == b.sq && a.sk == b.sk && a.causal == b.causal && a.shift == b.shift &&
-         a.grid == b.grid;
-}
 
 // First-fit decreasing under capacity `cap`: bin_of[i] for the items in `order`; false if one does not fit.
 bool first_fit(const std::vector<uint32_t> &w, const std::vector<int> &order, int grid, uint64_t cap, std::vector<int> *bin_of) {
@@ -77,33 +60,11 @@ void build(const std::vector<uint32_t> &w, int grid, SchedTable *out) {
 
 }  // namespace
 
-void schedule_for(const SchedKey &key, int n_items, uint32_t (*weight)(const void *ctx, int item), const void *ctx,
-                  SchedTable *out) {
-  out->used = 0;
-  if (n_items <= key.grid || n_items > kSchedMaxItems || key.grid > kSchedMaxCtas || !key.causal) return;
-  if (option(DF_OPT_SCHED_TABLE) == 0) return;
-  std::lock_guard<std::mutex> guard(g_mutex);
-  for (const Entry &e : g_cache)
-    if (e.valid && e.n_items == n_items && same(e.key, key)) {
-      *out = e.table;
-      return;
-    }
-  std::vector<uint32_t> w(n_items);
-  for (int i = 0; i < n_items; ++i) w[i] = weight(ctx, i);
-  Entry &e = g_cache[g_next];
-  g_next = (g_next + 1) % kEntries;
-  e.key = key;
-  e.n_items = n_items;
-  build(w, key.grid, &e.table);
-  e.valid = true;
-  *out = e.table;
-}
-
 }  // namespace df
 
-// Host-only probe of the builder (tests): the work lists for `n` items of the given weights on `grid`
-// CTAs. Returns 1 and fills off[grid + 1], items[n] when a table is produced, 0 when the launchers
-// would fall back to the snake order.
+// The builder: the work lists for `n` items of the given weights on `grid`
+// CTAs. Returns 1 and fills off[grid + 1], items[n] when a table is produced, 0 when the
+// snake order is as good.
 extern "C" int df_attn_schedule_build(const uint32_t *weights, int n, int grid, uint16_t *off, uint16_t *items) {
   if (!weights || !off || !items || n <= 0 || grid <= 0) return 0;
   static thread_local df::SchedTable t;

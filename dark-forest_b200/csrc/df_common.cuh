@@ -88,6 +88,7 @@ int accumulate(float *dst, const float *src, uint64_t n, cudaStream_t s);
 // ---- tcgen05 kernels (attn_fwd_sm100.cu / attn_bwd_sm100.cu) ----
 bool tensor_forward_supported(const AttnParams &p);
 int tensor_forward(const AttnParams &p, cudaStream_t s);
+int tensor_forward_row2(const AttnParams &p, cudaStream_t s);  // bf16, two threads per query row (attn_fwd_row2_sm100.cu)
 bool tensor_backward_supported(const AttnParams &p);
 int tensor_backward(const AttnParams &p, cudaStream_t s);
 // Creates, for the calling thread and the current device, what the block backward would otherwise
@@ -107,49 +108,22 @@ __host__ __device__ inline long long snake_item(int r, int grid, int cta, long l
   return idx < n_items ? idx : -1;
 }
 
-// Optional explicit work lists for the persistent kernels. The snake formula is as good as greedy
-// longest-first, but with few heavy items per CTA (one long sequence, a dozen heads) neither is
-// close to the average load: at S = 8192, B*H = 12 the heaviest CTA carries 96 steps against an
-// average of 85.6. For up to kSchedMaxItems items the forward launcher therefore computes a MULTIFIT
-// assignment on the host (first-fit decreasing under a binary-searched capacity, cached per shape)
-// and passes it to the kernel as a parameter: CTA c runs items[off[c] .. off[c+1]) in that order
-// (measured on B200, B=1, H=12: forward at S = 8192 351 -> 381 TFLOP/s, S = 16384 404 -> 410). The
-// backward kernels keep the snake order: the same tables made them slower (S = 4096: 0.34 -> 0.38-0.43
-// ms, S = 8192: 0.96 -> 1.03-1.05 ms, whatever weight the change of tile was given).
+// Explicit work lists: a MULTIFIT assignment of weighted items to CTAs (df_attn_schedule_build, attn_sched.cu): CTA c runs
+// items[off[c] .. off[c+1]) in that order.
 constexpr int kSchedMaxItems = 2048;
 constexpr int kSchedMaxCtas = 160;
 struct SchedTable {
-  uint32_t used;                       // 0: no table, the kernel uses snake_item
+  uint32_t used;                       // 0: no table
   uint16_t off[kSchedMaxCtas + 2];
   uint16_t items[kSchedMaxItems];
 };
-__host__ __device__ inline long long sched_item(const SchedTable &t, int r, int grid, int cta, long long n_items) {
-  if (t.used) {
-    const int i = (int)t.off[cta] + r;
-    return i < (int)t.off[cta + 1] ? (long long)t.items[i] : -1;
-  }
-  return snake_item(r, grid, cta, n_items);
-}
-// Fills `out` for `n_items` items of the given weights (any order) on `grid` CTAs; out->used = 0 when
-// the table does not apply (too many items, one round at most, or no better than the snake order).
-// `key` identifies the shape for the per-process cache (attn_sched.cu).
-struct SchedKey {
-  int kind;  // 0 forward pairs (the only user so far)
-  uint32_t bh, sq, sk;
-  int causal;
-  long long shift;
-  int grid;
-};
-void schedule_for(const SchedKey &key, int n_items, uint32_t (*weight)(const void *ctx, int item), const void *ctx,
-                  SchedTable *out);
+
+int sm_count();  // of the current device; 0 when it cannot be asked
 
 // one-token decode over a contiguous or paged KV cache (attn_decode.cu)
 int decode_dispatch(const float *q, const void *k, const void *v, const int32_t *block_table, float *out,
                     float *partial_m, float *partial_l, float *partial_o, uint32_t max_chunks, uint32_t H,
                     uint32_t T, uint32_t D, float scale, uint32_t page_size, bool kv_bf16, cudaStream_t s);
-// persistent TF32 forward for whole sequences with head dimension 64 (attn_fwd_persist_sm100.cu)
-bool tensor_forward_persistent_supported(const AttnParams &p);
-int tensor_forward_persistent(const AttnParams &p, cudaStream_t s);
 
 // ---- projections around the attention op (linear_sm100.cu): out_j = X W_j^T + b_j (+ residual), j < n_mats <= 3 ----
 bool tensor_linear_supported(const float *x, const float *const *w, const float *const *bias, float *const *out,

@@ -508,18 +508,6 @@ k_adamw_multi(const df_adamw_tensor_t *__restrict__ tensors, uint32_t n_tensors,
   }
 }
 
-std::once_flag g_sm_once[64];
-int g_sm_count[64];
-int sm_count() {
-  int dev = 0;
-  if (check_cuda(cudaGetDevice(&dev)) != DF_OK || dev < 0 || dev >= 64) return 0;
-  std::call_once(g_sm_once[dev], [&]() {
-    int n = 0;
-    g_sm_count[dev] = (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0) ? n : 0;
-  });
-  return g_sm_count[dev];
-}
-
 // Blocks of a backward LayerNorm kernel that fit on one SM (queried once per kernel; 8 KB of shared memory assumed).
 template <typename K>
 uint32_t resident_blocks(K kernel, int slot) {

@@ -142,7 +142,7 @@ DF_API void launch_paged_copy_row_f32_to_bf16(const float *src, void *pool, int3
 DF_API int df_attn_apply_rope_rows(float *qk, uint32_t first_pos, uint32_t rows, uint32_t n_heads, uint32_t d_head,
                             float base_freq, void *stream);
 
-/* Host-only probe of the explicit work lists that the persistent kernels receive when the round-robin
+/* Host-only: explicit work lists for a kernel whose items are dealt to `grid` CTAs in advance and whose round-robin
  * order would leave a heavy tail (up to 2048 items): first-fit decreasing under a binary-searched
  * capacity. Fills off[grid + 1] and items[n] (CTA c runs items[off[c] .. off[c+1]) in that order) and
  * returns 1, or returns 0 when no table is used (n <= grid, n > 2048, grid > 160, or nothing better than
@@ -397,10 +397,10 @@ DF_API int df_attn_set_variant(int variant);  /* per calling thread; returns the
  * environment variable named beside it, read ONCE when the library first looks an option up; after
  * that only df_attn_set_option changes it (returns the previous value, -1 for an unknown option).
  * None of them changes results beyond rounding order; no launcher reads the environment. */
-#define DF_OPT_FWD_PERSIST 0     /* DF_ATTN_FWD_PERSIST: persistent TF32 forward 0 never, 1 up to S = 2048 (default), 2 always */
+#define DF_OPT_FWD_PERSIST 0     /* DF_ATTN_FWD_PERSIST: forward items 0 pairs of query tiles, 1 by size (default), 2 split tiles  */
 #define DF_OPT_FUSE_DELTA 1      /* DF_ATTN_FUSE_DELTA: 1 (default) the dQ kernel forms delta itself, 0 separate pre-pass    */
 #define DF_OPT_BWD_OVERLAP 2     /* DF_ATTN_BWD_OVERLAP: 1 (default) block backward runs dQ on the thread's side stream      */
-#define DF_OPT_SCHED_TABLE 3     /* DF_ATTN_SCHED_TABLE: 1 (default) explicit work lists for the persistent forward          */
+#define DF_OPT_SCHED_TABLE 3     /* DF_ATTN_SCHED_TABLE: kept for callers; the forward no longer deals items out in advance   */
 #define DF_OPT_DISABLE_TENSOR 4  /* DF_ATTN_DISABLE_TENSOR: 1 = SIMT kernels only, 2 = SIMT backward only (default 0)        */
 #define DF_OPT_PDL 5             /* DF_ATTN_PDL: 1 (default) kernels are launched with programmatic stream serialization (each waits for
                                     its predecessor before its first access to global memory), 0 = ordinary launches           */

@@ -722,3 +722,37 @@ def test_ring_driver_bf16_backend_single_rank(torch_cuda, oracle):
     finally:
         if created:
             dist.destroy_process_group()
+
+
+# both kinds of forward items (0 pairs of query tiles, 2 split tiles): one item per SM and CTAs that take over items, odd and even
+# numbers of tiles, edges of tiles, rows without a key, every head dimension and element type
+@pytest.mark.parametrize("items", [0, 2])
+@pytest.mark.parametrize("dtype,D", [("fp32", 64), ("bf16", 64), ("bf16", 128)])
+@pytest.mark.parametrize("B,H,Sq,Sk,shift,causal", [
+    (1, 3, 1, 1, 0, True), (1, 2, 128, 128, 0, True), (2, 3, 129, 129, 0, True), (1, 5, 257, 257, 0, False), (1, 4, 640, 640, 0, True),
+    (9, 20, 300, 300, 0, True), (12, 30, 130, 130, 0, False), (3, 25, 700, 700, 0, True), (2, 40, 513, 257, -256, True),
+    (2, 30, 200, 900, 700, True), (1, 3, 384, 100, 0, False)])
+def test_forward_items(torch_cuda, items, dtype, D, B, H, Sq, Sk, shift, causal):
+    p = pkg()
+    gen = torch_cuda.Generator(device="cuda")
+    gen.manual_seed(Sq * 7 + Sk + D)
+    dt = torch_cuda.float32 if dtype == "fp32" else torch_cuda.bfloat16
+    q, k, v = (torch_cuda.randn(B, s, H * D, generator=gen, device="cuda").to(dt) for s in (Sq, Sk, Sk))
+    prev = p.set_option(p.OPT_FWD_PERSIST, items)
+    try:
+        out, lse = (p.forward if dtype == "fp32" else p.forward_bf16)(q, k, v, H, D ** -0.5, causal, causal_shift=shift)
+        assert p.sync_status() == 0
+    finally:
+        p.set_option(p.OPT_FWD_PERSIST, prev)
+    q4, k4, v4 = (t.double().view(B, -1, H, D).transpose(1, 2) for t in (q, k, v))
+    s = q4 @ k4.transpose(2, 3) * D ** -0.5
+    if causal:
+        s = s.masked_fill(torch_cuda.arange(Sk, device="cuda")[None, :] > torch_cuda.arange(Sq, device="cuda")[:, None] + shift, -math.inf)
+    want_lse = torch_cuda.logsumexp(s, -1)
+    seen = want_lse > -math.inf
+    pr = torch_cuda.where(seen[..., None], torch_cuda.exp(s - torch_cuda.where(seen, want_lse, 0.0)[..., None]), 0.0)
+    want = (pr @ v4).transpose(1, 2).reshape(out.shape)
+    tol = hp.TOL_O_TF32 if dtype == "fp32" else 2e-2
+    assert float((out.double() - want).abs().max()) <= tol * max(1.0, float(want.abs().max()))
+    assert bool((torch_cuda.isinf(lse) == ~seen).all())
+    assert float((lse.double() - want_lse)[seen].abs().max()) <= (hp.TOL_LSE_TF32 if dtype == "fp32" else 1e-3)
