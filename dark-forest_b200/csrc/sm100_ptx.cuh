@@ -168,6 +168,8 @@ __device__ __forceinline__ void tc_fence_after_sync() {
 // instead, its blocks sit on SMs that this kernel still wants (forward + backward of 12 heads, 1024 rows: 59 us this way, 65
 // with early triggers, 66 without programmatic launch).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the dependent grid start where SMs have room, once every CTA of this grid has said so or ended.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Dynamic scheduling by the hardware's own block queue (cluster launch control): a running block takes over the index of a
 // block (cluster) that has not started yet. claim_request writes a 16-byte answer to shared memory and counts it on an mbarrier;
