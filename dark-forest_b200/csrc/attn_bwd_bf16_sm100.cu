@@ -10,6 +10,10 @@
 //     columns, and each compute thread packs into the first half of the columns it has itself read
 //     (columns [0,32) and [64,96)), so nobody overwrites scores another thread still needs;
 //   * head dimension 64 or 128 (template parameter); gradients are written as bf16.
+// What bounds it: at head dimension 128 the compute warps' two phases per step (tensor pipe 51 % busy), at 64 the same and the
+// exponentials. The dQ kernel needs nothing of the dK/dV kernel and starts on SMs that it leaves. Backward on B200 with the delta
+// pass, causal, us: D = 64, H = 16, S = 8192 691 -> 580, 8 x 1024 (H = 12) 129 -> 115, S = 512 26.4 -> 15.8; D = 128 S = 8192 848 -> 836,
+// S = 2048 93 -> 78, S = 512 37 -> 24.
 // Every wait is bounded (mbar_wait); there is no TMA multicast.
 #include <math.h>
 
@@ -22,7 +26,6 @@ namespace {
 using namespace ptx;
 
 constexpr int BT = 128;
-constexpr int kThreads = 352;  // warps 0-7 compute, 8-9 TMA producers, 10 MMA issuer
 constexpr uint32_t kSlab = 128 * 128;
 constexpr uint32_t kTmemCols = 512;
 constexpr float kLog2e = 1.4426950408889634f;
@@ -35,6 +38,7 @@ struct Bwd16Params {
   float scale, scale_log2;
   int causal;
   long long shift;
+  int early;  // the dQ kernel begins where the dK/dV kernel leaves SMs and waits for it at its end
   unsigned int *status;
 };
 
@@ -46,6 +50,10 @@ struct Cfg16 {
   static constexpr uint32_t kSlabs = HD_ * 2 / 128;        // 1 (D=64) or 2 (D=128)
   static constexpr uint32_t kTile = kSlabs * kSlab;        // 128 rows x HD bf16
   static constexpr int kKSteps = HD_ / 16;                 // K-steps of an SS MMA over the head dimension
+  static constexpr int kRing = HD_ == 64 ? 4 : 2;          // stages of the per-step tiles
+  static constexpr int kSBufs = HD_ == 64 ? 2 : 1;         // dK/dV: S^T buffers in tensor memory
+  static constexpr int kIssuers = HD_ == 64 ? 2 : 1;       // warps that issue MMAs
+  static constexpr int kThreads = 32 * (10 + kIssuers);    // warps 0-7 compute, 8-9 TMA producers, then the issuers
 };
 
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
@@ -102,15 +110,16 @@ __device__ __forceinline__ void store_bf16x32(uint8_t *dst, const uint32_t (&r)[
 // dK / dV  (a CTA owns 128 keys; TMEM lanes = keys, columns = queries)
 // =========================================================================================
 namespace kv16 {
-enum Bar { KV_FULL = 0, Q_FULL = 1, Q_EMPTY = 3, G_FULL = 5, G_EMPTY = 7,   // + ring stage
-           S_FULL = 9, DP_FULL, P_FULL, DS_FULL, STAT_FULL, ACC_FULL, DRAIN, NUM };
-template <class C> __host__ __device__ constexpr uint32_t stats_off() { return 6 * C::kTile; }   // K, V, Q[2], dO[2]
-template <class C> __host__ __device__ constexpr uint32_t bars_off() { return stats_off<C>() + 4 * 128 * 4; }
+enum Bar { KV_FULL = 0, Q_FULL = 1, Q_EMPTY = 5, G_FULL = 9, G_EMPTY = 13,   // + ring stage
+           S_FULL = 17, P_FULL = 19,                                         // + S^T buffer
+           DP_FULL = 21, DS_FULL, STAT_FULL, ACC_FULL, DRAIN, NUM };
+template <class C> __host__ __device__ constexpr uint32_t stats_off() { return (2 + 2 * C::kRing) * C::kTile; }   // K, V, Q ring, dO ring
+template <class C> __host__ __device__ constexpr uint32_t bars_off() { return stats_off<C>() + 6 * 128 * 4; }
 template <class C> __host__ __device__ constexpr uint32_t smem_total() { return bars_off<C>() + 256 + 1024; }
 }  // namespace kv16
 
 template <class C>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(C::kThreads, 1)
 k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                      const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmG, const Bwd16Params p) {
   using namespace kv16;
@@ -118,12 +127,12 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
   constexpr uint32_t kTile = C::kTile;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const uint32_t aK = smem_u32(smem), aV = aK + kTile, aQ = aK + 2 * kTile, aG = aK + 4 * kTile;  // rings: + stage * kTile
+  const uint32_t aK = smem_u32(smem), aV = aK + kTile, aQ = aK + 2 * kTile, aG = aQ + C::kRing * kTile;  // rings: + stage * kTile
   float *sLse2 = reinterpret_cast<float *>(smem + stats_off<C>());
-  float *sDelta = sLse2 + 256;
+  float *sDelta = sLse2 + 384;   // both [3][128]
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + bars_off<C>());
-  volatile uint32_t *abort_flag = reinterpret_cast<volatile uint32_t *>(smem + bars_off<C>() + 160);
-  uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(smem + bars_off<C>() + 164);
+  volatile uint32_t *abort_flag = reinterpret_cast<volatile uint32_t *>(smem + bars_off<C>() + 224);
+  uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(smem + bars_off<C>() + 228);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t n_bh = p.B * p.H, bh = blockIdx.x % n_bh;
@@ -138,6 +147,7 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
   const int n_it = (int)(((long long)p.Sq + BT - 1) / BT - i_begin);
 
   if (n_it <= 0) {  // no query sees these keys: dK = dV = 0
+    pdl_wait();
     if (warp < 8) {
       const long long kj = k0 + (warp & 3) * 32 + lane;
       if (kj < (long long)p.Sk) {
@@ -152,7 +162,12 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
 
   auto bar = [&](int id) { return smem_u32(&bars[id]); };
   if (threadIdx.x == 0) {
-    for (int i = 0; i < NUM; ++i) mbar_init(bar(i), (i == P_FULL || i == DS_FULL || i == STAT_FULL) ? 256 : 1);
+    for (int i = 0; i < NUM; ++i) {
+      const bool compute = i == P_FULL || i == P_FULL + 1 || i == DS_FULL || i == STAT_FULL;
+      // a Q (dO) tile is read by a product of either issuer; both have to be done with it
+      const bool both = (i >= Q_EMPTY && i < Q_EMPTY + 4) || (i >= G_EMPTY && i < G_EMPTY + 4) || i == ACC_FULL || i == DRAIN;
+      mbar_init(bar(i), compute ? 256 : both ? C::kIssuers : 1);
+    }
     *abort_flag = 0;
     mbar_init_fence();
   }
@@ -165,7 +180,8 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_holder;
   pdl_wait();  // everything above touched only this CTA's shared and tensor memory
-  const uint32_t tS = tmem, tDP = tmem + 128, tDV = tmem + 256, tDK = tmem + 256 + HD;
+  if (p.early && threadIdx.x == 0) pdl_trigger();  // the dQ kernel needs nothing from this one: it may start where SMs are free
+  const uint32_t tS0 = tmem, tDP = tmem + 128, tDV = tmem + 256, tDK = tmem + 256 + HD, tS1 = C::kSBufs == 2 ? tmem + 384 : tmem;
 
   if (warp == 8) {
     // producer: K, V once, then the Q ring
@@ -176,7 +192,7 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
         tma_load_4d(aV + sl * kSlab, &tmV, bar(KV_FULL), (int)(sl * 64), (int)h, (int)k0, (int)b);
       }
       for (int it = 0; it < n_it; ++it) {
-        const int s = it & 1, use = it >> 1;
+        const int s = it % C::kRing, use = it / C::kRing;
         if (use > 0 && !mbar_wait(bar(Q_EMPTY + s), (use - 1) & 1, abort_flag)) break;
         load_tile<C>(aQ + s * kTile, &tmQ, bar(Q_FULL + s), (int)h, (int)((i_begin + it) * BT), (int)b);
       }
@@ -185,61 +201,64 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
     // producer: the dO ring
     if (lane == 0) {
       for (int it = 0; it < n_it; ++it) {
-        const int s = it & 1, use = it >> 1;
+        const int s = it % C::kRing, use = it / C::kRing;
         if (use > 0 && !mbar_wait(bar(G_EMPTY + s), (use - 1) & 1, abort_flag)) break;
         load_tile<C>(aG + s * kTile, &tmG, bar(G_FULL + s), (int)h, (int)((i_begin + it) * BT), (int)b);
       }
     }
-  } else if (warp == 10) {
-    // The whole warp runs this role, warp-uniformly; one elected lane issues the MMA and commit instructions and
-    // every wait returns the same answer in all lanes (see elect_one).
-    {
-      const uint32_t idesc_ss = make_idesc(kFmtBF16, BT, BT, 0, 0);
-      const uint32_t idesc_ts = make_idesc(kFmtBF16, BT, HD, 0, 1);
-      const uint64_t dK = make_smem_desc(aK, 16, 1024, kSwz128), dV = make_smem_desc(aV, 16, 1024, kSwz128);
-      // the same Q / dO tile serves as K-major B (S^T, dP^T) and as MN-major B (dK, dV)
-      const uint64_t dQk[2] = {make_smem_desc(aQ, 16, 1024, kSwz128), make_smem_desc(aQ + kTile, 16, 1024, kSwz128)};
-      const uint64_t dGk[2] = {make_smem_desc(aG, 16, 1024, kSwz128), make_smem_desc(aG + kTile, 16, 1024, kSwz128)};
-      const uint64_t dQm[2] = {make_smem_desc(aQ, kSlab, 1024, kSwz128), make_smem_desc(aQ + kTile, kSlab, 1024, kSwz128)};
-      const uint64_t dGm[2] = {make_smem_desc(aG, kSlab, 1024, kSwz128), make_smem_desc(aG + kTile, kSlab, 1024, kSwz128)};
-      bool ok = mbar_wait_warp(bar(KV_FULL), 0, abort_flag) && mbar_wait_warp(bar(Q_FULL), 0, abort_flag);
-      if (ok) {
-        tc_fence_after_sync();
-        issue_ss<C>(tS, dK, dQk[0], idesc_ss);  // S^T_0 = K Q^T
-        commit_elected(bar(S_FULL));
-        ok = mbar_wait_warp(bar(G_FULL), 0, abort_flag);
-      }
-      if (ok) {
-        tc_fence_after_sync();
-        issue_ss<C>(tDP, dV, dGk[0], idesc_ss);  // dP^T_0 = V dO^T
-        commit_elected(bar(DP_FULL));
-      }
+  } else if (warp >= 10) {
+    // Two chains of products that share no tensor memory (an issuer runs its role warp-uniformly; one elected lane issues the MMA and
+    // commit instructions):
+    //   S / dV: .., dV_i (needs P_i), S_{i+1} (overwrites P^T_i after dV_i has read it; two steps ahead where S^T has two buffers), ..
+    //   dP / dK: .., dK_i (needs dS_i), dP_{i+1} (overwrites dS^T_i after dK_i has read it), ..
+    // Head dimension 64: a warp each (with S^T ahead and the statistics staged ahead 691 -> 591 us at S = 8192, H = 16). Head
+    // dimension 128: one warp, in the order dV S dK dP: each product then has the tensor pipe to itself when the compute warps wait
+    // for it (a warp each: 834 -> 892 us).
+    const uint32_t idesc_ss = make_idesc(kFmtBF16, BT, BT, 0, 0), idesc_ts = make_idesc(kFmtBF16, BT, HD, 0, 1);
+    // the same Q / dO tile serves as K-major B (S^T, dP^T) and as MN-major B (dK, dV)
+    const uint64_t dK = make_smem_desc(aK, 16, 1024, kSwz128), dV = make_smem_desc(aV, 16, 1024, kSwz128);
+    const uint64_t dQk = make_smem_desc(aQ, 16, 1024, kSwz128), dGk = make_smem_desc(aG, 16, 1024, kSwz128);
+    const uint64_t dQm = make_smem_desc(aQ, kSlab, 1024, kSwz128), dGm = make_smem_desc(aG, kSlab, 1024, kSwz128);
+    auto scores = [&](bool chain_s, int it) -> bool {
+      const int st = it % C::kRing;
+      const uint64_t off = (uint64_t)(st * (kTile >> 4));
+      if (!mbar_wait_warp(bar((chain_s ? Q_FULL : G_FULL) + st), (it / C::kRing) & 1, abort_flag)) return false;
+      tc_fence_after_sync();
+      const bool second = C::kSBufs == 2 && (it & 1);
+      issue_ss<C>(chain_s ? (second ? tS1 : tS0) : tDP, chain_s ? dK : dV, (chain_s ? dQk : dGk) + off, idesc_ss);
+      commit_elected(bar(chain_s ? S_FULL + (second ? 1 : 0) : DP_FULL));
+      if (C::kIssuers == 2) commit_elected(bar((chain_s ? Q_EMPTY : G_EMPTY) + st));
+      return true;
+    };
+    auto gradient = [&](bool chain_s, int it) -> bool {
+      const int st = it % C::kRing;
+      const bool second = C::kSBufs == 2 && (it & 1);
+      if (C::kIssuers == 2 && !mbar_wait_warp(bar((chain_s ? G_FULL : Q_FULL) + st), (it / C::kRing) & 1, abort_flag)) return false;
+      if (!(chain_s ? mbar_wait_warp(bar(P_FULL + (second ? 1 : 0)), (it / C::kSBufs) & 1, abort_flag)
+                    : mbar_wait_warp(bar(DS_FULL), it & 1, abort_flag)))
+        return false;
+      tc_fence_after_sync();
+      issue_ts<C>(chain_s ? tDV : tDK, chain_s ? (second ? tS1 : tS0) : tDP, (chain_s ? dGm : dQm) + (uint64_t)(st * (kTile >> 4)), idesc_ts, it > 0);
+      commit_elected(bar((chain_s ? G_EMPTY : Q_EMPTY) + st));  // one issuer: the score product of this tile came before
+      return true;
+    };
+    bool ok = mbar_wait_warp(bar(KV_FULL), 0, abort_flag);
+    if (C::kIssuers == 2) {
+      const bool chain_s = warp == 10;
+      const int ahead = chain_s ? C::kSBufs : 1;
+      for (int it = 0; ok && it < ahead && it < n_it; ++it) ok = scores(chain_s, it);
       for (int it = 0; ok && it < n_it; ++it) {
-        const int s = it & 1, ns = (it + 1) & 1;
-        const uint32_t ph = it & 1, nring = ((it + 1) >> 1) & 1;
-        if (!mbar_wait_warp(bar(P_FULL), ph, abort_flag)) break;
-        tc_fence_after_sync();
-        issue_ts<C>(tDV, tS, dGm[s], idesc_ts, it > 0);  // dV += P^T dO
-        commit_elected(bar(G_EMPTY + s));
-        if (it + 1 < n_it) {
-          if (!mbar_wait_warp(bar(Q_FULL + ns), nring, abort_flag)) break;
-          tc_fence_after_sync();
-          issue_ss<C>(tS, dK, dQk[ns], idesc_ss);  // S^T_{i+1} (after dV_i has read P^T_i)
-          commit_elected(bar(S_FULL));
-        }
-        if (!mbar_wait_warp(bar(DS_FULL), ph, abort_flag)) break;
-        tc_fence_after_sync();
-        issue_ts<C>(tDK, tDP, dQm[s], idesc_ts, it > 0);  // dK += dS^T Q
-        commit_elected(bar(Q_EMPTY + s));
-        if (it + 1 < n_it) {
-          if (!mbar_wait_warp(bar(G_FULL + ns), nring, abort_flag)) break;
-          tc_fence_after_sync();
-          issue_ss<C>(tDP, dV, dGk[ns], idesc_ss);  // dP^T_{i+1}
-          commit_elected(bar(DP_FULL));
-        }
+        ok = gradient(chain_s, it);
+        if (ok && it + ahead < n_it) ok = scores(chain_s, it + ahead);
       }
-      commit_elected(bar(ACC_FULL));
+    } else {
+      ok = ok && scores(true, 0) && scores(false, 0);
+      for (int it = 0; ok && it < n_it; ++it) {
+        const bool more = it + 1 < n_it;
+        ok = gradient(true, it) && (!more || scores(true, it + 1)) && gradient(false, it) && (!more || scores(false, it + 1));
+      }
     }
+    commit_elected(bar(ACC_FULL));
   } else {
     // compute warps: lanes = keys; warps 0-3 own query columns 0-63, warps 4-7 columns 64-127
     const int quarter = warp & 3, half = warp >> 2;
@@ -258,20 +277,29 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
       }
       return __ldg(p.delta + s_base + q);
     };
-    float stat_next = fetch_stat(0);
+    // Row statistics are staged one step ahead in one of three buffers and published by a split barrier: every thread arrives in
+    // the middle of step i-1 and waits at the start of step i. A thread past that wait knows the others are at least in step i-1,
+    // whose readers use buffers (i-1) % 3 and i % 3, so writing (i+1) % 3 in step i is safe.
+    auto stage_stat = [&](int buf, float v) {
+      if (tid < 128) sLse2[buf * 128 + tid] = v; else sDelta[buf * 128 + tid - 128] = v;
+      mbar_arrive(bar(STAT_FULL));
+    };
+    stage_stat(0, fetch_stat(0));
     bool ok = true;
+    int sb = 0;
     for (int it = 0; it < n_it; ++it) {
       const uint32_t ph = it & 1;
       const long long q0 = (i_begin + it) * BT;
-      float *lse2 = sLse2 + ph * 128, *dlt = sDelta + ph * 128;
-      if (tid < 128) lse2[tid] = stat_next; else dlt[tid - 128] = stat_next;
-      mbar_arrive(bar(STAT_FULL));
+      const float *lse2 = sLse2 + sb * 128, *dlt = sDelta + sb * 128;
+      sb = sb == 2 ? 0 : sb + 1;
+      const float stat_next = fetch_stat(it + 1);
       if (!mbar_wait(bar(STAT_FULL), ph, abort_flag)) { ok = false; break; }
-      stat_next = fetch_stat(it + 1);
       const bool need_mask = p.causal && (q0 + p.shift < k0 + (BT - 1));
       const long long cmin_ll = kj - p.shift - q0;  // visible iff column >= cmin
       const int cmin = !need_mask ? 0 : (cmin_ll > BT ? BT : (cmin_ll < 0 ? 0 : (int)cmin_ll));
-      if (!mbar_wait(bar(S_FULL), ph, abort_flag)) { ok = false; break; }
+      const bool second = C::kSBufs == 2 && ph;
+      const uint32_t tS = second ? tS1 : tS0;
+      if (!mbar_wait(bar(S_FULL + (second ? 1 : 0)), (it / C::kSBufs) & 1, abort_flag)) { ok = false; break; }
       tc_fence_after_sync();
       float pr[64];
       uint32_t packed[32];
@@ -302,7 +330,8 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
       tmem_st32(tS + lane_base + col0, packed);  // packed P^T over the first half of this thread's own columns
       tmem_wait_st();
       tc_fence_before_sync();
-      mbar_arrive(bar(P_FULL));
+      mbar_arrive(bar(P_FULL + (second ? 1 : 0)));
+      if (it + 1 < n_it) stage_stat(sb, stat_next);
       if (!mbar_wait(bar(DP_FULL), ph, abort_flag)) { ok = false; break; }
       tc_fence_after_sync();
 #pragma unroll
@@ -347,7 +376,7 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
   tc_fence_before_sync();
   __syncthreads();
   if (*abort_flag != 0u) {
-    if (warp == 10) {
+    if (warp >= 10) {
       commit_elected(bar(DRAIN));  // by the lane that issued the MMAs: the election is deterministic
       for (int n = 0; n < (1 << 16) && !mbar_try_wait(bar(DRAIN), 0); ++n) {
       }
@@ -370,14 +399,15 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
 // dQ  (a CTA owns 128 queries; TMEM lanes = queries, columns = keys)
 // =========================================================================================
 namespace dq16 {
-enum Bar { QG_FULL = 0, K_FULL = 1, K_EMPTY = 3, V_FULL = 5, V_EMPTY = 7,   // + ring stage
-           S_FULL = 9, S_FREE, DP_FULL, DS_FULL, ACC_FULL, DRAIN, NUM };
-template <class C> __host__ __device__ constexpr uint32_t bars_off() { return 6 * C::kTile; }     // Q, dO, K[2], V[2]
+enum Bar { QG_FULL = 0, K_FULL = 1, K_EMPTY = 5, V_FULL = 9, V_EMPTY = 13,   // + ring stage
+           DP_FULL = 17,                                                     // + dP buffer
+           S_FULL = 19, S_FREE, DS_FULL, ACC_FULL, DRAIN, NUM };
+template <class C> __host__ __device__ constexpr uint32_t bars_off() { return (2 + 2 * C::kRing) * C::kTile; }     // Q, dO, K ring, V ring
 template <class C> __host__ __device__ constexpr uint32_t smem_total() { return bars_off<C>() + 256 + 1024; }
 }  // namespace dq16
 
 template <class C>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(C::kThreads, 1)
 k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmG,
                    const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const Bwd16Params p) {
   using namespace dq16;
@@ -385,10 +415,10 @@ k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   constexpr uint32_t kTile = C::kTile;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const uint32_t aQ = smem_u32(smem), aG = aQ + kTile, aK = aQ + 2 * kTile, aV = aQ + 4 * kTile;  // rings: + stage * kTile
+  const uint32_t aQ = smem_u32(smem), aG = aQ + kTile, aK = aQ + 2 * kTile, aV = aK + C::kRing * kTile;  // rings: + stage * kTile
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + bars_off<C>());
-  volatile uint32_t *abort_flag = reinterpret_cast<volatile uint32_t *>(smem + bars_off<C>() + 160);
-  uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(smem + bars_off<C>() + 164);
+  volatile uint32_t *abort_flag = reinterpret_cast<volatile uint32_t *>(smem + bars_off<C>() + 224);
+  uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(smem + bars_off<C>() + 228);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t n_bh = p.B * p.H, bh = blockIdx.x % n_bh;
@@ -403,6 +433,7 @@ k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const int n_kv = (int)((kv_end + BT - 1) / BT);
 
   if (n_kv == 0) {
+    pdl_wait();
     if (warp < 8) {
       const long long i = q0 + (warp & 3) * 32 + lane;
       if (i < (long long)p.Sq) {
@@ -417,7 +448,7 @@ k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
   auto bar = [&](int id) { return smem_u32(&bars[id]); };
   if (threadIdx.x == 0) {
-    for (int i = 0; i < NUM; ++i) mbar_init(bar(i), (i == S_FREE || i == DS_FULL) ? 256 : 1);
+    for (int i = 0; i < NUM; ++i) mbar_init(bar(i), (i == S_FREE || i == DS_FULL) ? 256 : i == DRAIN ? C::kIssuers : 1);
     *abort_flag = 0;
     mbar_init_fence();
   }
@@ -429,8 +460,9 @@ k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_holder;
-  pdl_wait();  // everything above touched only this CTA's shared and tensor memory
-  const uint32_t tS = tmem, tDP = tmem + 128, tDQ = tmem + 256;
+  if (!p.early) pdl_wait();  // everything above touched only this CTA's shared and tensor memory
+  // head dimension 64: dP / dS has two buffers, steps alternate
+  const uint32_t tS = tmem, tDP0 = tmem + 128, tDQ = tmem + 256, tDP1 = C::kIssuers == 2 ? tmem + 384 : tmem + 128;
 
   if (warp == 8) {
     if (lane == 0) {
@@ -440,7 +472,7 @@ k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tma_load_4d(aG + sl * kSlab, &tmG, bar(QG_FULL), (int)(sl * 64), (int)h, (int)q0, (int)b);
       }
       for (int j = 0; j < n_kv; ++j) {
-        const int s = j & 1, use = j >> 1;
+        const int s = j % C::kRing, use = j / C::kRing;
         if (use > 0 && !mbar_wait(bar(K_EMPTY + s), (use - 1) & 1, abort_flag)) break;
         load_tile<C>(aK + s * kTile, &tmK, bar(K_FULL + s), (int)h, j * BT, (int)b);
       }
@@ -448,31 +480,34 @@ k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   } else if (warp == 9) {
     if (lane == 0) {
       for (int j = 0; j < n_kv; ++j) {
-        const int s = j & 1, use = j >> 1;
+        const int s = j % C::kRing, use = j / C::kRing;
         if (use > 0 && !mbar_wait(bar(V_EMPTY + s), (use - 1) & 1, abort_flag)) break;
         load_tile<C>(aV + s * kTile, &tmV, bar(V_FULL + s), (int)h, j * BT, (int)b);
       }
     }
-  } else if (warp == 10) {
-    // The whole warp runs this role, warp-uniformly; one elected lane issues the MMA and commit instructions and
-    // every wait returns the same answer in all lanes (see elect_one).
-    {
-      const uint32_t idesc_ss = make_idesc(kFmtBF16, BT, BT, 0, 0);
-      const uint32_t idesc_ts = make_idesc(kFmtBF16, BT, HD, 0, 1);
-      const uint64_t dQ = make_smem_desc(aQ, 16, 1024, kSwz128), dG = make_smem_desc(aG, 16, 1024, kSwz128);
+  } else if (warp >= 10) {
+    // S_{j+1} = Q K^T as soon as the scores before are in registers; dQ += dS_j K; dP_{j+1} = dO V^T. (Issuers run warp-uniformly;
+    // one elected lane issues the MMA and commit instructions.) Head dimension 64: S by a warp of its own, dP into the buffer that
+    // dQ_{j-1} has read, ahead of dQ_j. Head dimension 128: one warp, one dP buffer, S dQ dP: a product then runs while the compute
+    // warps are in their exponentials and not while they move dP and dS through tensor memory (dP ahead: 357 -> 420 us at
+    // S = 8192, H = 16).
+    const uint32_t idesc_ss = make_idesc(kFmtBF16, BT, BT, 0, 0), idesc_ts = make_idesc(kFmtBF16, BT, HD, 0, 1);
+    const uint64_t dQ = make_smem_desc(aQ, 16, 1024, kSwz128), dG = make_smem_desc(aG, 16, 1024, kSwz128);
+    bool ok = mbar_wait_warp(bar(QG_FULL), 0, abort_flag);
+    if constexpr (C::kIssuers == 1) {
       const uint64_t dKk[2] = {make_smem_desc(aK, 16, 1024, kSwz128), make_smem_desc(aK + kTile, 16, 1024, kSwz128)};
       const uint64_t dKm[2] = {make_smem_desc(aK, kSlab, 1024, kSwz128), make_smem_desc(aK + kTile, kSlab, 1024, kSwz128)};
       const uint64_t dVk[2] = {make_smem_desc(aV, 16, 1024, kSwz128), make_smem_desc(aV + kTile, 16, 1024, kSwz128)};
-      bool ok = mbar_wait_warp(bar(QG_FULL), 0, abort_flag) && mbar_wait_warp(bar(K_FULL), 0, abort_flag);
+      ok = ok && mbar_wait_warp(bar(K_FULL), 0, abort_flag);
       if (ok) {
         tc_fence_after_sync();
-        issue_ss<C>(tS, dQ, dKk[0], idesc_ss);  // S_0 = Q K^T
+        issue_ss<C>(tS, dQ, dKk[0], idesc_ss);
         commit_elected(bar(S_FULL));
         ok = mbar_wait_warp(bar(V_FULL), 0, abort_flag);
       }
       if (ok) {
         tc_fence_after_sync();
-        issue_ss<C>(tDP, dG, dVk[0], idesc_ss);  // dP_0 = dO V^T
+        issue_ss<C>(tDP0, dG, dVk[0], idesc_ss);
         commit_elected(bar(DP_FULL));
         commit_elected(bar(V_EMPTY));
       }
@@ -482,20 +517,52 @@ k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (j + 1 < n_kv) {
           if (!mbar_wait_warp(bar(S_FREE), ph, abort_flag) || !mbar_wait_warp(bar(K_FULL + ns), nring, abort_flag)) break;
           tc_fence_after_sync();
-          issue_ss<C>(tS, dQ, dKk[ns], idesc_ss);  // S_{j+1}: P_j already lives in registers
+          issue_ss<C>(tS, dQ, dKk[ns], idesc_ss);
           commit_elected(bar(S_FULL));
         }
         if (!mbar_wait_warp(bar(DS_FULL), ph, abort_flag)) break;
         tc_fence_after_sync();
-        issue_ts<C>(tDQ, tDP, dKm[s], idesc_ts, j > 0);  // dQ += dS K
+        issue_ts<C>(tDQ, tDP0, dKm[s], idesc_ts, j > 0);
         commit_elected(bar(K_EMPTY + s));
         if (j + 1 < n_kv) {
           if (!mbar_wait_warp(bar(V_FULL + ns), nring, abort_flag)) break;
           tc_fence_after_sync();
-          issue_ss<C>(tDP, dG, dVk[ns], idesc_ss);  // dP_{j+1} (after dQ_j has read dS_j)
+          issue_ss<C>(tDP0, dG, dVk[ns], idesc_ss);
           commit_elected(bar(DP_FULL));
           commit_elected(bar(V_EMPTY + ns));
         }
+      }
+      commit_elected(bar(ACC_FULL));
+    } else if (warp == 10) {
+      const uint64_t dKk = make_smem_desc(aK, 16, 1024, kSwz128);
+      for (int j = 0; ok && j < n_kv; ++j) {
+        const int st = j % C::kRing;
+        if (!mbar_wait_warp(bar(K_FULL + st), (j / C::kRing) & 1, abort_flag)) break;
+        if (j > 0 && !mbar_wait_warp(bar(S_FREE), (j - 1) & 1, abort_flag)) break;
+        tc_fence_after_sync();
+        issue_ss<C>(tS, dQ, dKk + (uint64_t)(st * (kTile >> 4)), idesc_ss);
+        commit_elected(bar(S_FULL));
+      }
+    } else {
+      const uint64_t dVk = make_smem_desc(aV, 16, 1024, kSwz128), dKm = make_smem_desc(aK, kSlab, 1024, kSwz128);
+      auto issue_dp = [&](int j) -> bool {
+        const int st = j % C::kRing;
+        if (!mbar_wait_warp(bar(V_FULL + st), (j / C::kRing) & 1, abort_flag)) return false;
+        tc_fence_after_sync();
+        issue_ss<C>((j & 1) ? tDP1 : tDP0, dG, dVk + (uint64_t)(st * (kTile >> 4)), idesc_ss);
+        commit_elected(bar(DP_FULL + (j & 1)));
+        commit_elected(bar(V_EMPTY + st));
+        return true;
+      };
+      ok = ok && issue_dp(0);
+      for (int j = 0; ok && j < n_kv; ++j) {
+        const int st = j % C::kRing;
+        if (j + 1 < n_kv && !issue_dp(j + 1)) break;
+        // S_j has read this K tile before its scores became dS_j
+        if (!mbar_wait_warp(bar(K_FULL + st), (j / C::kRing) & 1, abort_flag) || !mbar_wait_warp(bar(DS_FULL), j & 1, abort_flag)) break;
+        tc_fence_after_sync();
+        issue_ts<C>(tDQ, (j & 1) ? tDP1 : tDP0, dKm + (uint64_t)(st * (kTile >> 4)), idesc_ts, j > 0);
+        commit_elected(bar(K_EMPTY + st));
       }
       commit_elected(bar(ACC_FULL));
     }
@@ -542,7 +609,8 @@ k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       }
       tc_fence_before_sync();
       mbar_arrive(bar(S_FREE));
-      if (!mbar_wait(bar(DP_FULL), ph, abort_flag)) { ok = false; break; }
+      const uint32_t tDP = ph ? tDP1 : tDP0, dp_buf = C::kIssuers == 2 ? ph : 0;
+      if (!mbar_wait(bar(DP_FULL + dp_buf), (j / C::kIssuers) & 1, abort_flag)) { ok = false; break; }
       tc_fence_after_sync();
       uint32_t packed[32];
 #pragma unroll
@@ -577,10 +645,11 @@ k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     }
   }
 
+  if (p.early) pdl_wait();  // whoever waits for this kernel waits for the dK/dV kernel too
   tc_fence_before_sync();
   __syncthreads();
   if (*abort_flag != 0u) {
-    if (warp == 10) {
+    if (warp >= 10) {
       commit_elected(bar(DRAIN));  // by the lane that issued the MMAs: the election is deterministic
       for (int n = 0; n < (1 << 16) && !mbar_try_wait(bar(DRAIN), 0); ++n) {
       }
@@ -599,42 +668,54 @@ k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   }
 }
 
-// delta[b][h][i] = sum_d dO * O for bf16 tensors: same streaming pattern as the fp32 pre-pass
-// (32 rows x all heads per block, 16-byte loads = 8 bf16, transposed through shared memory).
+// delta[b][h][i] = sum_d dO * O for bf16 tensors: a block has 8 rows x all heads, a group of LPS lanes a (row, head) segment of 16-byte
+// loads, four segments in flight per thread. Bound by HBM; what counts is loads in flight: with 32 rows per block (1.7 blocks per
+// SM at S = 8192) and a segment at a time S = 8192, H = 16, D = 128 took 29.4 us (2.3 TB/s) and S = 1024, H = 12 11.1 us. The
+// sums pass through shared memory so that the [B][H][S] output is written in whole 32-byte sectors.
+constexpr uint32_t kDeltaRows = 8;
 template <int LPS>  // lanes per (row, head) segment = D / 8
 __global__ void __launch_bounds__(256) k_delta_vec_bf16(const uint4 *__restrict__ o, const uint4 *__restrict__ g,
                                                         float *__restrict__ delta, uint32_t H, uint32_t S,
                                                         uint32_t tiles_per_batch) {
   pdl_wait();
-  extern __shared__ float s_sum[];  // [H][32]
+  extern __shared__ float s_sum[];  // [kDeltaRows][H]
   const uint32_t b = blockIdx.x / tiles_per_batch;
-  const uint32_t i0 = (blockIdx.x % tiles_per_batch) * 32u;
-  const uint32_t rows = (S - i0) < 32u ? (S - i0) : 32u;
+  const uint32_t i0 = (blockIdx.x % tiles_per_batch) * kDeltaRows;
+  const uint32_t rows = (S - i0) < kDeltaRows ? (S - i0) : kDeltaRows;
   const uint32_t nseg = rows * H;
   const size_t chunk = ((size_t)b * S + i0) * H * LPS;
   const uint32_t grp = threadIdx.x / LPS, lane = threadIdx.x % LPS;
-  constexpr uint32_t kGroups = 256 / LPS;
-  for (uint32_t sg0 = 0; sg0 < nseg; sg0 += kGroups) {
-    const uint32_t sg = sg0 + grp;
-    float acc = 0.0f;
-    if (sg < nseg) {
-      const uint4 a = __ldg(o + chunk + (size_t)sg * LPS + lane);
-      const uint4 c = __ldg(g + chunk + (size_t)sg * LPS + lane);
-      const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, cw[4] = {c.x, c.y, c.z, c.w};
+  constexpr uint32_t kGroups = 256 / LPS, U = 4;
+  for (uint32_t sg0 = 0; sg0 < nseg; sg0 += kGroups * U) {
+    uint4 a[U], c[U];
+#pragma unroll
+    for (uint32_t u = 0; u < U; ++u) {
+      const uint32_t sg = sg0 + u * kGroups + grp;
+      a[u] = c[u] = make_uint4(0u, 0u, 0u, 0u);
+      if (sg < nseg) {
+        a[u] = __ldg(o + chunk + (size_t)sg * LPS + lane);
+        c[u] = __ldg(g + chunk + (size_t)sg * LPS + lane);
+      }
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < U; ++u) {
+      float acc = 0.0f;
+      const uint32_t aw[4] = {a[u].x, a[u].y, a[u].z, a[u].w}, cw[4] = {c[u].x, c[u].y, c[u].z, c[u].w};
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
         acc = fmaf(__uint_as_float(aw[w] << 16), __uint_as_float(cw[w] << 16), acc);
         acc = fmaf(__uint_as_float(aw[w] & 0xffff0000u), __uint_as_float(cw[w] & 0xffff0000u), acc);
       }
-    }
 #pragma unroll
-    for (int off = LPS / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-    if (lane == 0 && sg < nseg) s_sum[(sg % H) * 32u + sg / H] = acc;
+      for (int off = LPS / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+      const uint32_t sg = sg0 + u * kGroups + grp;
+      if (lane == 0 && sg < nseg) s_sum[sg] = acc;
+    }
   }
   __syncthreads();
-  for (uint32_t idx = threadIdx.x; idx < 32u * H; idx += 256u) {
-    const uint32_t h = idx >> 5, ii = idx & 31u;
-    if (ii < rows) delta[((size_t)b * H + h) * S + i0 + ii] = s_sum[idx];
+  for (uint32_t idx = threadIdx.x; idx < kDeltaRows * H; idx += 256u) {
+    const uint32_t h = idx / kDeltaRows, ii = idx % kDeltaRows;
+    if (ii < rows) delta[((size_t)b * H + h) * S + i0 + ii] = s_sum[ii * H + h];
   }
 }
 
@@ -671,12 +752,19 @@ int launch_backward(const AttnParams &p, cudaStream_t s) {
   bp.causal = p.causal;
   bp.shift = p.shift;
   bp.status = device_status_ptr();
+  // unless dQ overwrites what the dK/dV kernel reads
+  const uint64_t q_bytes = (uint64_t)p.B * p.Sq * p.H * C::HD, k_bytes = (uint64_t)p.B * p.Sk * p.H * C::HD;
+  auto overlaps_dq = [&](const void *in, uint64_t elements) {
+    const uintptr_t x = (uintptr_t)p.d_q, y = (uintptr_t)in;
+    return x < y + elements * 2 && y < x + q_bytes * C::kOutElt;
+  };
+  bp.early = option(DF_OPT_PDL) != 0 && !overlaps_dq(p.q, q_bytes) && !overlaps_dq(p.d_out, q_bytes) && !overlaps_dq(p.k, k_bytes) && !overlaps_dq(p.v, k_bytes);
   const dim3 grid_kv(((p.Sk + BT - 1) / BT) * p.B * p.H);
-  launch_kernel(k_attn_bwd_dkdv_bf16<C>, grid_kv, dim3(kThreads), kv16::smem_total<C>(), s, tmK, tmV, tmQ, tmG, bp);
+  launch_kernel(k_attn_bwd_dkdv_bf16<C>, grid_kv, dim3(C::kThreads), kv16::smem_total<C>(), s, tmK, tmV, tmQ, tmG, bp);
   note_launch();
   if (check_cuda(cudaGetLastError()) != DF_OK) return DF_ERR_CUDA;
   const dim3 grid_q(((p.Sq + BT - 1) / BT) * p.B * p.H);
-  launch_kernel(k_attn_bwd_dq_bf16<C>, grid_q, dim3(kThreads), dq16::smem_total<C>(), s, tmQ, tmG, tmK, tmV, bp);
+  launch_kernel(k_attn_bwd_dq_bf16<C>, grid_q, dim3(C::kThreads), dq16::smem_total<C>(), s, tmQ, tmG, tmK, tmV, bp);
   note_launch();
   return check_cuda(cudaGetLastError());
 }
@@ -707,9 +795,9 @@ int delta_prepass_bf16(const AttnParams &p, cudaStream_t s) {
   if (p.Sq == 0 || p.B == 0 || p.H == 0) return DF_OK;
   if ((p.D != 64 && p.D != 128) || p.H > 256) return DF_ERR_UNSUPPORTED;
   if ((reinterpret_cast<uintptr_t>(p.o_in) | reinterpret_cast<uintptr_t>(p.d_out)) & 15u) return DF_ERR_UNSUPPORTED;
-  const uint32_t tiles = (p.Sq + 31) / 32;
+  const uint32_t tiles = (p.Sq + kDeltaRows - 1) / kDeltaRows;
   const dim3 grid(p.B * tiles);
-  const size_t smem = (size_t)p.H * 32 * sizeof(float);
+  const size_t smem = (size_t)p.H * kDeltaRows * sizeof(float);
   const uint4 *o4 = reinterpret_cast<const uint4 *>(p.o_in);
   const uint4 *g4 = reinterpret_cast<const uint4 *>(p.d_out);
   if (p.D == 64) launch_kernel(k_delta_vec_bf16<8>, grid, dim3(256), smem, s, o4, g4, p.delta, p.H, p.Sq, tiles);

@@ -756,3 +756,33 @@ def test_forward_items(torch_cuda, items, dtype, D, B, H, Sq, Sk, shift, causal)
     assert float((out.double() - want).abs().max()) <= tol * max(1.0, float(want.abs().max()))
     assert bool((torch_cuda.isinf(lse) == ~seen).all())
     assert float((lse.double() - want_lse)[seen].abs().max()) <= (hp.TOL_LSE_TF32 if dtype == "fp32" else 1e-3)
+
+
+# backward items: more of them than SMs (taken over at run time), keys that no query sees (some, none), few tiles (the two kernels overlap)
+@pytest.mark.parametrize("dtype,D", [("fp32", 64), ("bf16", 64), ("bf16", 128)])
+@pytest.mark.parametrize("B,H,Sq,Sk,shift", [(1, 2, 65, 65, 0), (9, 20, 300, 300, 0), (2, 3, 700, 700, 0), (30, 8, 129, 640, 0),
+                                             (2, 3, 300, 1000, -100), (1, 2, 64, 512, -200), (1, 3, 400, 130, 270)])
+def test_backward_items(torch_cuda, dtype, D, B, H, Sq, Sk, shift):
+    p = pkg()
+    gen = torch_cuda.Generator(device="cuda")
+    gen.manual_seed(Sq * 5 + Sk + D)
+    dt = torch_cuda.float32 if dtype == "fp32" else torch_cuda.bfloat16
+    q, k, v, go = (torch_cuda.randn(B, s, H * D, generator=gen, device="cuda").to(dt) for s in (Sq, Sk, Sk, Sq))
+    scale, suffix = D ** -0.5, "" if dtype == "fp32" else "_bf16"
+    out, lse = getattr(p, "forward" + suffix)(q, k, v, H, scale, True, causal_shift=shift)
+    if Sq == Sk and shift == 0:
+        got = getattr(p, "backward" + suffix)(q, k, v, out, go, lse, H, scale, True)
+    else:
+        delta = getattr(p, "delta" + suffix)(out, go, H)
+        got = getattr(p, "backward_block" + suffix)(q, k, v, go, lse, delta, H, scale, True, causal_shift=shift)
+    assert p.sync_status() == 0
+    q4, k4, v4, g4 = (t.double().view(B, -1, H, D).transpose(1, 2) for t in (q, k, v, go))
+    vis = torch_cuda.arange(Sk, device="cuda")[None, :] <= torch_cuda.arange(Sq, device="cuda")[:, None] + shift
+    s = (q4 @ k4.transpose(2, 3) * scale).masked_fill(~vis, -math.inf)
+    top = torch_cuda.logsumexp(s, -1, keepdim=True)
+    pr = torch_cuda.where(vis, torch_cuda.exp(s - torch_cuda.where(top > -math.inf, top, 0.0)), 0.0)
+    ds = pr * (g4 @ v4.transpose(2, 3) - (g4 * (pr @ v4)).sum(-1, keepdim=True))
+    want = (ds @ k4 * scale, ds.transpose(2, 3) @ q4 * scale, pr.transpose(2, 3) @ g4)
+    for g, w, name in zip(got, want, ("dq", "dk", "dv")):
+        w = w.transpose(1, 2).reshape(g.shape)
+        assert float((g.double() - w).norm()) <= (2e-3 if dtype == "fp32" else 1e-2) * float(w.norm()) + 1e-6, name
