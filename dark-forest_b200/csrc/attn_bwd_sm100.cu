@@ -154,6 +154,44 @@ __device__ __forceinline__ void load_tile(uint32_t dst, const CUtensorMap *m, ui
   tma_load_4d(dst + kSlab, m, bar, 32, h, row0, b);
 }
 
+__device__ __forceinline__ void store_cluster(uint32_t addr, float4 v) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+// SPLIT kernels: one thread's N accumulator columns (one row) into the other CTA's staging tile of 128 rows of N floats, and
+// back as the sum with this CTA's own columns. 16-byte chunk c of row r sits at c ^ (r % 8).
+template <int N>
+__device__ __forceinline__ void send_row(uint32_t peer_tile, int row, uint32_t taddr) {
+#pragma unroll 1
+  for (int c = 0; c < N; c += 32) {
+    uint32_t rr[32];
+    tmem_ld32(taddr + c, rr);
+    tmem_wait_ld();
+#pragma unroll
+    for (int x = 0; x < 8; ++x)
+      store_cluster(peer_tile + row * (N * 4) + (uint32_t)((c / 4 + x) ^ (row & 7)) * 16,
+                    make_float4(__uint_as_float(rr[4 * x]), __uint_as_float(rr[4 * x + 1]), __uint_as_float(rr[4 * x + 2]), __uint_as_float(rr[4 * x + 3])));
+  }
+}
+template <int N>
+__device__ __forceinline__ void finish_row(const uint8_t *tile, int row, uint32_t taddr, bool own, bool other, float mul, float *dst, bool store) {
+#pragma unroll 1
+  for (int c = 0; c < N; c += 32) {
+    uint32_t rr[32];
+    tmem_ld32(taddr + c, rr);
+    tmem_wait_ld();
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+      float4 a = make_float4(__uint_as_float(rr[4 * x]), __uint_as_float(rr[4 * x + 1]), __uint_as_float(rr[4 * x + 2]), __uint_as_float(rr[4 * x + 3]));
+      if (!own) a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (other) {
+        const float4 b = *reinterpret_cast<const float4 *>(tile + row * (N * 4) + ((c / 4 + x) ^ (row & 7)) * 16);
+        a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+      }
+      if (store) *reinterpret_cast<float4 *>(dst + c + 4 * x) = make_float4(a.x * mul, a.y * mul, a.z * mul, a.w * mul);
+    }
+  }
+}
+
 // =========================================================================================
 // Work distribution shared by both kernels
 // =========================================================================================
@@ -207,7 +245,10 @@ __device__ __forceinline__ Item decode(const BwdParams &p, int idx) {
 // NSUB = column groups of the compute warps: 4 * NSUB compute warps (warp w: TMEM lanes 32 * (w % 4).., query
 // columns (w / 4) * 128 / NSUB ..), then two producer warps and two MMA warps. (Which warp number issues the MMAs
 // makes no difference: with the MMA role on warp 0 instead of the last warp the kernel took the same time.)
-template <int NSUB>
+// SPLIT: a cluster of two CTAs shares an item. Each takes every other query tile; at the end rank 0 finishes dV and rank 1 dK, each
+// from its own accumulator and the other's, which comes through distributed shared memory. For problems whose items leave SMs
+// without work or are long against an SM's share (split_backward).
+template <int NSUB, bool SPLIT>
 __global__ void __launch_bounds__((4 * NSUB + 4) * 32, 1)
 k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                          const __grid_constant__ CUtensorMap tmQk, const __grid_constant__ CUtensorMap tmGk,
@@ -232,6 +273,8 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
   constexpr int NCH = CPT / 32;        // 32-column chunks per compute thread
   constexpr int kWarpLoadK = kCW, kWarpLoadM = kCW + 1, kWarpMma = kCW + 2, kWarpMma2 = kCW + 3, kWarpCompute0 = 0;
   const size_t dm = (size_t)p.H * HD;
+  constexpr int ST = SPLIT ? 2 : 1;  // query tiles from one step to the next
+  const uint32_t rank = SPLIT ? cluster_rank() : 0u;
 #ifdef DF_ATTN_TRACE
 #ifdef DF_ATTN_TRACE_DQ
   const bool trace_on = false;
@@ -243,11 +286,36 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
   DF_BTRACE(warp == kWarpMma ? 0 : 1, 1);
 
   auto bar = [&](int id) { return smem_u32(&bars[id]); };
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < NUM; ++i)
+  // Items: blockIdx.x first, then those of CTAs that have not started (claimed by the first producer). take(k) is item k of this
+  // CTA; false when there is none (or a wait gave up).
+  auto take = [&](uint32_t k, Item *out) -> bool {
+    uint32_t idx = blockIdx.x / ST;
+    if (SPLIT && k > 0) return false;
+    if (!SPLIT && k > 0) {
+      const int c = (int)((k - 1) % kClaims);
+      if (!mbar_wait(bar(CLAIM + c), ((k - 1) / kClaims) & 1, abort_flag)) return false;
+      idx = claim_result(smem_u32(smem) + kAnswers + 16 * c);
+      if (idx == ~0u) return false;
+    }
+    *out = decode(p, (int)idx);
+    if (SPLIT) {
+      out->i_begin += rank;
+      out->n_it = (out->n_it + 1 - (int)rank) / 2;
+    }
+    return !SPLIT || out->n_it > 0;
+  };
+  if (warp == kWarpLoadK) {
+    for (int i = lane; i < NUM; i += 32)
       mbar_init(bar(i), (i == P_FULL0 || i == P_FULL1 || i == DS_FULL || i == STAT_FULL || i == EPI_FULL) ? kArrivals : ((i == ACC_FULL || i == DRAIN) ? 2 : 1));
-    *abort_flag = 0;
+    if (lane == 0) *abort_flag = 0;
     mbar_init_fence();
+    __syncwarp();
+    Item first;
+    if (lane == 0 && take(0, &first)) {  // the first tiles are under way while the others set up
+      if (!p.early) pdl_wait();
+      load_tile(aK, &tmK, bar(K_FULL), (int)first.h, (int)first.k0, (int)first.b);
+      load_tile(aQk, &tmQk, bar(QK_FULL), (int)first.h, (int)(first.i_begin * BT), (int)first.b);
+    }
   }
   if (warp == kWarpMma) {
     tmem_alloc(smem_u32(tmem_holder), kTmemCols);
@@ -262,19 +330,6 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
   const uint32_t tS0 = tmem, tDP = tmem + 128, tDV = tmem + 256, tDK = tmem + 320, tS1 = tmem + 384;
   if (!p.early) pdl_wait();  // everything above touched only this CTA's shared and tensor memory
 
-  // Items: blockIdx.x first, then those of CTAs that have not started (claimed by the first producer). take(k) is item k of this
-  // CTA; false when there is none (or a wait gave up).
-  auto take = [&](uint32_t k, Item *out) -> bool {
-    uint32_t idx = blockIdx.x;
-    if (k > 0) {
-      const int c = (int)((k - 1) % kClaims);
-      if (!mbar_wait(bar(CLAIM + c), ((k - 1) / kClaims) & 1, abort_flag)) return false;
-      idx = claim_result(smem_u32(smem) + kAnswers + 16 * c);
-      if (idx == ~0u) return false;
-    }
-    *out = decode(p, (int)idx);
-    return true;
-  };
   auto take_warp = [&](uint32_t k, Item *out) -> bool { return __all_sync(0xffffffffu, take(k, out)) != 0; };
 
   // Counters every role keeps for itself: g = steps (query tiles) done over all items, n = items
@@ -290,12 +345,10 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
         // K and V land on barriers of their own: the next item's first S^T needs only K, and V can be replaced only
         // after the item's last dP^T, a step later. On one barrier the S^T / dV warp stood waiting for V at the end of
         // every item, with the item's last dV (whose P^T was ready) queued behind that wait: 2 K cycles per item.
-        mbar_arrive_expect_tx(bar(K_FULL), kTile);
-        tma_load_4d(aK, &tmK, bar(K_FULL), 0, (int)cur.h, (int)cur.k0, (int)cur.b);
-        tma_load_4d(aK + kSlab, &tmK, bar(K_FULL), 32, (int)cur.h, (int)cur.k0, (int)cur.b);
+        if (n > 0) load_tile(aK, &tmK, bar(K_FULL), (int)cur.h, (int)cur.k0, (int)cur.b);  // the first: during set-up
         for (int it = 0; it < cur.n_it; ++it, ++g) {
-          const int q0 = (int)((cur.i_begin + it) * BT);
-          if (it == (cur.n_it > 1 ? cur.n_it - 2 : 0)) {  // ask for the next item: S^T of its first step is due two steps before the end
+          const int q0 = (int)((cur.i_begin + it * ST) * BT);
+          if (!SPLIT && it == (cur.n_it > 1 ? cur.n_it - 2 : 0)) {  // ask for the next item: S^T of its first step is due two steps before the end
             const int c = (int)(n % kClaims);
             fence_proxy_async_smem();
             mbar_arrive_expect_tx(bar(CLAIM + c), 16);
@@ -304,7 +357,7 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
           // the K-major Q (dO) buffer is free once the S^T (dP^T) product that read it has completed: the
           // barrier that hands that product to the compute warps tells this thread too
           if (g > 0 && !mbar_wait(bar(S_FULL0 + ((g - 1) & 1)), ((g - 1) >> 1) & 1, abort_flag)) { ok = false; break; }
-          load_tile(aQk, &tmQk, bar(QK_FULL), (int)cur.h, q0, (int)cur.b);
+          if (g > 0) load_tile(aQk, &tmQk, bar(QK_FULL), (int)cur.h, q0, (int)cur.b);
           if (it == 0) {  // V follows the item's first Q tile: that one, like K, does not have to wait for V's buffer
             if (n > 0 && !mbar_wait(bar(V_EMPTY), (n - 1) & 1, abort_flag)) { ok = false; break; }
             mbar_arrive_expect_tx(bar(V_FULL), kTile);
@@ -325,7 +378,7 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
       for (; take(n, &cur); ++n) {
         bool ok = true;
         for (int it = 0; it < cur.n_it; ++it, ++g) {
-          const int q0 = (int)((cur.i_begin + it) * BT);
+          const int q0 = (int)((cur.i_begin + it * ST) * BT);
           // the MN-major dO (Q) buffer is released by a commit of its own right after dV (dK) of the step before:
           // waiting for the next S^T (dP^T) product instead delayed these loads and measured 1-3 % slower
           if (g > 0 && !mbar_wait(bar(GM_EMPTY), (g - 1) & 1, abort_flag)) { ok = false; break; }
@@ -333,6 +386,7 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
           if (g > 0 && !mbar_wait(bar(QM_EMPTY), (g - 1) & 1, abort_flag)) { ok = false; break; }
           load_tile(aQm, &tmQm, bar(QM_FULL), (int)cur.h, q0, (int)cur.b);
         }
+        if (SPLIT) break;
         // The compute warps stage the item's dV and dK tiles in these two buffers; this thread
         // hands them to the copy engine (key rows beyond Sk are dropped) and may refill the
         // buffers for the next item once the store has read them.
@@ -504,7 +558,7 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
     // The value comes back RAW: nothing is computed from it here, so the thread does not stall on the load; it is
     // turned into what the phases use (`staged`) only when it is written to shared memory, a P phase later.
     auto fetch_stat = [&](const Item &im, int it) -> float {
-      const long long q = (im.i_begin + it) * BT + (tid & 127);
+      const long long q = (im.i_begin + it * ST) * BT + (tid & 127);
       if (q >= (long long)p.Sq || tid >= 256) return (tid < 128) ? -INFINITY : 0.0f;
       const size_t s_base = ((size_t)im.b * p.H + im.h) * p.Sq;
       return __ldcg((tid < 128 ? p.lse : p.delta) + s_base + q);  // delta may still be being written when this kernel starts: not cached
@@ -559,7 +613,7 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
       if (p.zero_tiles > 0) zero_unseen(cur);
       for (int it = 0; it < cur.n_it; ++it, ++g) {
         const uint32_t ph = g & 1;
-        const long long q0 = (cur.i_begin + it) * BT;
+        const long long q0 = (cur.i_begin + it * ST) * BT;
         const long long kj = cur.k0 + row;
         const float *lse2 = sLse2 + gb * 128, *dlt = sDelta + gb * 128;
         const uint32_t gb_next = gb == 2 ? 0 : gb + 1;
@@ -643,10 +697,34 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
         mbar_arrive(bar(DS_FULL));
         DF_BTRACE(1, 54);
       }
+      if (SPLIT) {
+        if (ok) ok = mbar_wait(bar(ACC_FULL), n & 1, abort_flag);
+        break;
+      }
       if (!ok || !hand_over(n)) { ok = false; break; }
       cur = nxt;
       ++n;
     }
+  }
+  if constexpr (SPLIT) {
+    __syncwarp();
+    tc_fence_before_sync();
+    cluster_sync();  // both CTAs' products are done and their operand buffers free
+    tc_fence_after_sync();
+    const Item it = decode(p, (int)(blockIdx.x / 2));
+    const bool own = it.n_it + 1 - (int)rank >= 2, other = it.n_it + (int)rank >= 2;
+    const int row = (warp & 3) * 32 + lane, sub = warp >> 2;  // sub 0 holds the thread's row of dV, sub 1 of dK
+    const uint32_t taddr = (sub ? tDK : tDV) + ((uint32_t)((warp & 3) * 32) << 16);
+    if (warp < kCW && sub != (int)rank && own) send_row<HD>(map_to_rank(aGm, rank ^ 1), row, taddr);
+    __syncwarp();
+    cluster_sync();
+    if (warp < kCW && sub == (int)rank) {
+      const long long kj = it.k0 + row;
+      const bool in = kj < (long long)p.Sk;
+      finish_row<HD>(smem + 5 * kTile, row, taddr, own, other, sub ? p.scale : 1.0f,
+                     (sub ? p.dk : p.dv) + ((size_t)it.b * p.Sk + (size_t)(in ? kj : 0)) * dm + it.h * HD, in);
+    }
+    tc_fence_before_sync();
   }
   if (p.early) pdl_wait();  // whoever waits for this kernel waits for the dQ kernel too
 
@@ -714,7 +792,8 @@ __device__ __forceinline__ int next_round(const BwdParams &p, int r, int n_items
 // FUSE_DELTA: the kernel also fetches the O tile of its queries, computes delta = rowsum(dO o O)
 // itself (dO as rounded to TF32 by its tensor map, the same values the dP product sees) and
 // writes it to p.delta_out for the dK/dV kernel, which then has to run after this one.
-template <bool FUSE_DELTA>
+// SPLIT (with FUSE_DELTA): as in the dK/dV kernel, two CTAs take every other key tile of an item; rank r finishes dims 32 r...
+template <bool FUSE_DELTA, bool SPLIT>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmG,
                        const __grid_constant__ CUtensorMap tmKk, const __grid_constant__ CUtensorMap tmVk,
@@ -732,13 +811,31 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t dm = (size_t)p.H * HD;
+  constexpr int ST = SPLIT ? 2 : 1;  // key tiles from one step to the next
+  const int rank = SPLIT ? (int)cluster_rank() : 0;
   const int n_qt = (int)(((long long)p.Sq + BT - 1) / BT);
 
   auto bar = [&](int id) { return smem_u32(&bars[id]); };
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < NUM; ++i) mbar_init(bar(i), (i == S_FREE || i == DS_FULL || i == EPI_FULL || i == O_FREE || i == DX_FULL || i == DELTA_DONE) ? 256 : 1);
-    *abort_flag = 0;
+  // item of the first round >= r that has work for this CTA
+  auto pick = [&](int r, Item *out) -> int {
+    if (!SPLIT) return next_round(p, r, n_items, n_qt, out);
+    if (r > 0) return -1;
+    *out = decode(p, (int)(blockIdx.x / 2), n_qt);
+    out->n_kv = (out->n_kv + 1 - rank) / 2;
+    return out->n_kv > 0 ? 0 : -1;
+  };
+  if (warp == 8) {
+    if (lane < NUM) mbar_init(bar(lane), (lane == S_FREE || lane == DS_FULL || lane == EPI_FULL || lane == O_FREE || lane == DX_FULL || lane == DELTA_DONE) ? 256 : 1);
+    static_assert(NUM <= 32, "a lane per barrier");
+    if (lane == 0) *abort_flag = 0;
     mbar_init_fence();
+    __syncwarp();
+    Item first;
+    if (lane == 0 && pick(0, &first) >= 0) {  // the first tiles are under way while the others set up
+      pdl_wait();
+      load_tile(aQ, &tmQ, bar(Q_FULL), (int)first.h, (int)first.q0, (int)first.b);
+      load_tile(aKk, &tmKk, bar(KK_FULL), (int)first.h, rank * BT, (int)first.b);
+    }
   }
   if (warp == 10) {
     tmem_alloc(smem_u32(tmem_holder), kTmemCols);
@@ -768,19 +865,17 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     if (lane == 0) {
       Item cur;
       uint32_t g = 0, n = 0;
-      for (int r = next_round(p, 0, n_items, n_qt, &cur); r >= 0; r = next_round(p, r + 1, n_items, n_qt, &cur), ++n) {
+      for (int r = pick(0, &cur); r >= 0; r = pick(r + 1, &cur), ++n) {
         bool ok = true;
         if (n > 0 && !mbar_wait(bar(Q_EMPTY), (n - 1) & 1, abort_flag)) break;
         // Q lands on a barrier of its own, dO (and O) on another: the next item's first S needs only Q, whose buffer
         // is free a step before dO's. On one barrier the MMA warp stood waiting for all three tiles at the end of every
         // item with the item's last dQ queued behind that wait, and the compute warps behind it.
-        mbar_arrive_expect_tx(bar(Q_FULL), kTile);
-        tma_load_4d(aQ, &tmQ, bar(Q_FULL), 0, (int)cur.h, (int)cur.q0, (int)cur.b);
-        tma_load_4d(aQ + kSlab, &tmQ, bar(Q_FULL), 32, (int)cur.h, (int)cur.q0, (int)cur.b);
+        if (n > 0) load_tile(aQ, &tmQ, bar(Q_FULL), (int)cur.h, (int)cur.q0, (int)cur.b);  // the first: during set-up
         for (int j = 0; j < cur.n_kv; ++j, ++g) {
           // a K-major K (V) buffer is free once the S (dP) product that read it has completed
           if (g > 0 && !mbar_wait(bar(S_FULL), (g - 1) & 1, abort_flag)) { ok = false; break; }
-          load_tile(aKk, &tmKk, bar(KK_FULL), (int)cur.h, j * BT, (int)cur.b);
+          if (g > 0) load_tile(aKk, &tmKk, bar(KK_FULL), (int)cur.h, (j * ST + rank) * BT, (int)cur.b);
           if (j == 0) {  // dO (and O) follow the item's first K tile, which does not have to wait for their buffers
             if (n > 0 && !mbar_wait(bar(G_EMPTY), (n - 1) & 1, abort_flag)) { ok = false; break; }
             // with fused row sums the compute warps read the dO and O tiles too: both are replaced
@@ -795,7 +890,7 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             }
           }
           if (g > 0 && !mbar_wait(bar(DP_FULL0 + ((g - 1) & 1)), ((g - 1) >> 1) & 1, abort_flag)) { ok = false; break; }
-          load_tile(aVk, &tmVk, bar(VK_FULL), (int)cur.h, j * BT, (int)cur.b);
+          load_tile(aVk, &tmVk, bar(VK_FULL), (int)cur.h, (j * ST + rank) * BT, (int)cur.b);
         }
         if (!ok) break;
       }
@@ -805,13 +900,14 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     if (lane == 0) {
       Item cur;
       uint32_t g = 0, n = 0;
-      for (int r = next_round(p, 0, n_items, n_qt, &cur); r >= 0; r = next_round(p, r + 1, n_items, n_qt, &cur), ++n) {
+      for (int r = pick(0, &cur); r >= 0; r = pick(r + 1, &cur), ++n) {
         bool ok = true;
         for (int j = 0; j < cur.n_kv; ++j, ++g) {
           // the buffer is released by a commit of its own right after dQ of the step before
           if (g > 0 && !mbar_wait(bar(KM_EMPTY), (g - 1) & 1, abort_flag)) { ok = false; break; }
-          load_tile(aKm, &tmKm, bar(KM_FULL), (int)cur.h, j * BT, (int)cur.b);
+          load_tile(aKm, &tmKm, bar(KM_FULL), (int)cur.h, (j * ST + rank) * BT, (int)cur.b);
         }
+        if (SPLIT) break;
         // the compute warps stage the item's dQ tile in this buffer; hand it to the copy engine
         // (rows beyond Sq are dropped) and refill the buffer once the store has read it
         if (!ok || !mbar_wait(bar(EPI_FULL), n & 1, abort_flag)) break;
@@ -831,7 +927,7 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       const uint64_t dQ_ = kmajor_desc(aQ), dG_ = kmajor_desc(aG), dKk = kmajor_desc(aKk), dVk = kmajor_desc(aVk), dKm = mnmajor_desc(aKm);
       Item cur, nxt;
       uint32_t g = 0, n = 0;
-      int r = next_round(p, 0, n_items, n_qt, &cur);
+      int r = pick(0, &cur);
       bool ok = r >= 0;
       // `last` = last step of its item: Q (for S) or dO (for dP) may then be replaced
       // `landed`: the caller has already seen the operand tile's barrier complete
@@ -858,7 +954,7 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       if (ok) ok = mbar_wait_warp(bar(GO_FULL), 0, abort_flag);
       if (ok) ok = issue_dp(0, cur.n_kv == 1);
       while (ok) {
-        const int rn = next_round(p, r + 1, n_items, n_qt, &nxt);
+        const int rn = pick(r + 1, &nxt);
         for (int j = 0; ok && j < cur.n_kv; ++j, ++g) {
           const bool last = j + 1 == cur.n_kv;
           const bool has_next = !last || rn >= 0;
@@ -910,7 +1006,7 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     const int col0 = half * 64;
     // query rows that see no key: dQ = 0
-    for (int r0 = 0;; ++r0) {
+    for (int r0 = 0; !SPLIT; ++r0) {
       const int idx = item_of_round(r0, n_items);
       if (idx < 0) break;
       const Item z = decode(p, idx, n_qt);
@@ -959,18 +1055,19 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       if (!mbar_wait(bar(DX_FULL), nn & 1, abort_flag)) return false;
       *out = xs[row] + xs[128 + row];
       const long long i = im.q0 + row;
-      if (half == 0 && i < (long long)p.Sq) p.delta_out[((size_t)im.b * p.H + im.h) * p.Sq + (size_t)i] = *out;
+      if (half == 0 && rank == 0 && i < (long long)p.Sq) p.delta_out[((size_t)im.b * p.H + im.h) * p.Sq + (size_t)i] = *out;
       return true;
     };
     Item cur, nxt;
     uint32_t g = 0, n = 0;
-    int r = next_round(p, 0, n_items, n_qt, &cur);
+    int r = pick(0, &cur);
     bool ok = true;
+    if (SPLIT && r < 0 && p.early && threadIdx.x == 0) pdl_trigger();  // no step for this CTA
     float lse_raw = -INFINITY, dlt = 0.0f, lse_raw_next = -INFINITY, dlt_next = 0.0f;
     if (r >= 0) fetch_stats(cur, &lse_raw, &dlt);
     if (FUSE_DELTA && r >= 0) ok = fused_delta(cur, 0, &dlt);
     while (r >= 0 && ok) {
-      const int rn = next_round(p, r + 1, n_items, n_qt, &nxt);
+      const int rn = pick(r + 1, &nxt);
       if (FUSE_DELTA && p.early && rn < 0) {
         // All row sums of this CTA are written: the dK/dV kernel may start on SMs that have run out of items.
         __threadfence();
@@ -986,7 +1083,7 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       const int kmax = (int)kmax_ll;
       for (int j = 0; j < cur.n_kv; ++j, ++g) {
         const uint32_t ph = g & 1;
-        const int key0 = j * BT;
+        const int key0 = (j * ST + rank) * BT;
         const bool need_mask = key0 + BT > kmax;
         DF_BTRACE(1, 50);
         if (!mbar_wait(bar(S_FULL), ph, abort_flag)) { ok = false; break; }
@@ -1037,6 +1134,7 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       if (!ok || !mbar_wait(bar(ACC_FULL), n & 1, abort_flag)) { ok = false; break; }
       DF_BTRACE(1, 60);
       tc_fence_after_sync();
+      if (SPLIT) break;
       {
         uint32_t rr[32];
         tmem_ld32(tDQ + lane_base + half * 32, rr);  // each half handles 32 of the 64 dims = one 128-byte slab
@@ -1062,6 +1160,25 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     }
   }
 
+  if constexpr (SPLIT) {
+    __syncwarp();
+    tc_fence_before_sync();
+    cluster_sync();  // both CTAs' products are done and their operand buffers free
+    tc_fence_after_sync();
+    const Item it = decode(p, (int)(blockIdx.x / 2), n_qt);
+    const bool own = it.n_kv + 1 - rank >= 2, other = it.n_kv + rank >= 2;
+    const int row = (warp & 3) * 32 + lane, half = warp >> 2;
+    const uint32_t taddr = tDQ + half * 32 + ((uint32_t)((warp & 3) * 32) << 16);
+    if (warp < 8 && half != rank && own) send_row<32>(map_to_rank(aKm, (uint32_t)(rank ^ 1)), row, taddr);
+    __syncwarp();
+    cluster_sync();
+    if (warp < 8 && half == rank) {
+      const long long i = it.q0 + row;
+      const bool in = i < (long long)p.Sq;
+      finish_row<32>(smem + 4 * kTile, row, taddr, own, other, p.scale,
+                     p.dq + ((size_t)it.b * p.Sq + (size_t)(in ? i : 0)) * dm + it.h * HD + half * 32, in);
+    }
+  }
   tc_fence_before_sync();
   __syncthreads();
   if (*abort_flag != 0u) {
@@ -1115,9 +1232,11 @@ int device_info(int *n_sm) {
   if (check_cuda(cudaGetDevice(&dev)) != DF_OK || dev < 0 || dev >= 64) return DF_ERR_CUDA;
   DeviceInfo &d = g_dev[dev];
   std::call_once(d.once, [&]() {
-    d.ok = cudaFuncSetAttribute(k_attn_bwd_dkdv_tf32_d64<DF_KV_NSUB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kv::kSmemTotal) == cudaSuccess &&
-           cudaFuncSetAttribute(k_attn_bwd_dq_tf32_d64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dq::kSmemTotal) == cudaSuccess &&
-           cudaFuncSetAttribute(k_attn_bwd_dq_tf32_d64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dq::kSmemTotal) == cudaSuccess &&
+    d.ok = cudaFuncSetAttribute(k_attn_bwd_dkdv_tf32_d64<DF_KV_NSUB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kv::kSmemTotal) == cudaSuccess &&
+           cudaFuncSetAttribute(k_attn_bwd_dkdv_tf32_d64<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kv::kSmemTotal) == cudaSuccess &&
+           cudaFuncSetAttribute(k_attn_bwd_dq_tf32_d64<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dq::kSmemTotal) == cudaSuccess &&
+           cudaFuncSetAttribute(k_attn_bwd_dq_tf32_d64<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dq::kSmemTotal) == cudaSuccess &&
+           cudaFuncSetAttribute(k_attn_bwd_dq_tf32_d64<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dq::kSmemTotal) == cudaSuccess &&
            cudaDeviceGetAttribute(&d.n_sm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && d.n_sm > 0;
   });
   if (!d.ok) {
@@ -1159,6 +1278,14 @@ struct SideStreams {
   }
 };
 thread_local SideStreams t_side;
+
+// Whether an item of the whole-sequence backward goes to a cluster of two CTAs: only where all halves run at once. A CTA costs
+// about 5 us beside its steps of 1.8 us, so with a second wave the halves lose (B200, H = 12, causal, both kernels, us, whole /
+// halves: S = 256 16.0 / 14.7, 512 22.3 / 18.7, 1024 34.8 / 37.7, 2048 60.8 / 80.3).
+bool split_backward(const AttnParams &p, int n_sm) {
+  if (p.Sq != p.Sk || p.shift != 0 || p.Sq <= BT) return false;
+  return 2ull * ((p.Sq + BT - 1) / BT) * p.B * p.H <= (uint64_t)n_sm;
+}
 
 // Events that df_attn_backward_profile asks the launcher to record around the two kernels.
 thread_local cudaEvent_t *t_profile_events = nullptr;
@@ -1218,6 +1345,7 @@ int tensor_backward(const AttnParams &p, cudaStream_t s) {
   const int items_q = (int)(((p.Sq + BT - 1) / BT) * p.B * p.H);
   const dim3 grid_q(items_q < n_sm ? items_q : n_sm);
   cudaEvent_t *prof = t_profile_events;
+  const bool split = fuse && split_backward(p, n_sm);
   SideStreams::Side *sd = (!fuse && prof == nullptr && option(DF_OPT_BWD_OVERLAP) != 0) ? t_side.get() : nullptr;
   cudaStream_t s_dq = s;
   if (sd) {
@@ -1244,9 +1372,11 @@ int tensor_backward(const AttnParams &p, cudaStream_t s) {
   const int reps = prof ? kProfileReps : 1;
   for (int rep = 0; (fuse || prof) && rep < reps; ++rep) {
     // (a profiled call with ready-made row sums runs its dQ kernel here too, so that the events split the two kernels)
-    const cudaError_t e = fuse ? launch_kernel(k_attn_bwd_dq_tf32_d64<true>, grid_q, dim3(kBwdThreads), dq::kSmemTotal, s,
+    const cudaError_t e = split ? launch_clusters(k_attn_bwd_dq_tf32_d64<true, true>, 2, dim3(2 * items_q), dim3(kBwdThreads), dq::kSmemTotal, s,
+                                                  tmQk, tmGk, tmKk, tmVk, tmKm, tmDQ, tmO, bp, items_q)
+                          : fuse ? launch_kernel(k_attn_bwd_dq_tf32_d64<true, false>, grid_q, dim3(kBwdThreads), dq::kSmemTotal, s,
                                                tmQk, tmGk, tmKk, tmVk, tmKm, tmDQ, tmO, bp, items_q)
-                               : launch_kernel(k_attn_bwd_dq_tf32_d64<false>, grid_q, dim3(kBwdThreads), dq::kSmemTotal, s,
+                               : launch_kernel(k_attn_bwd_dq_tf32_d64<false, false>, grid_q, dim3(kBwdThreads), dq::kSmemTotal, s,
                                                tmQk, tmGk, tmKk, tmVk, tmKm, tmDQ, tmO, bp, items_q);
     note_launch();
 #if defined(DF_ATTN_TRACE) && defined(DF_ATTN_TRACE_DQ)
@@ -1268,7 +1398,9 @@ int tensor_backward(const AttnParams &p, cudaStream_t s) {
       if (check_cuda(cudaMemsetAsync(p.d_k, 0, k_bytes, s)) != DF_OK || check_cuda(cudaMemsetAsync(p.d_v, 0, k_bytes, s)) != DF_OK) return DF_ERR_CUDA;
       continue;
     }
-    const cudaError_t e = launch_kernel(k_attn_bwd_dkdv_tf32_d64<DF_KV_NSUB>, dim3(items_kv), dim3(kKvThreads), kv::kSmemTotal, s, tmKk, tmVk,
+    const cudaError_t e = split ? launch_clusters(k_attn_bwd_dkdv_tf32_d64<2, true>, 2, dim3(2 * items_kv), dim3(12 * 32), kv::kSmemTotal, s, tmKk,
+                                                  tmVk, tmQk, tmGk, tmQm, tmGm, tmDK, tmDV, bp)
+                          : launch_kernel(k_attn_bwd_dkdv_tf32_d64<DF_KV_NSUB, false>, dim3(items_kv), dim3(kKvThreads), kv::kSmemTotal, s, tmKk, tmVk,
                                         tmQk, tmGk, tmQm, tmGm, tmDK, tmDV, bp);
     note_launch();
 #if defined(DF_ATTN_TRACE) && !defined(DF_ATTN_TRACE_DQ)
@@ -1286,7 +1418,7 @@ int tensor_backward(const AttnParams &p, cudaStream_t s) {
   }
   if (!fuse && !prof) {
     // with ready-made row sums the dQ kernel is independent of the dK/dV kernel
-    const cudaError_t e = launch_kernel(k_attn_bwd_dq_tf32_d64<false>, grid_q, dim3(kBwdThreads), dq::kSmemTotal, s_dq,
+    const cudaError_t e = launch_kernel(k_attn_bwd_dq_tf32_d64<false, false>, grid_q, dim3(kBwdThreads), dq::kSmemTotal, s_dq,
                                         tmQk, tmGk, tmKk, tmVk, tmKm, tmDQ, tmO, bp, items_q);
     note_launch();
     if (check_cuda(e) != DF_OK) return DF_ERR_CUDA;
