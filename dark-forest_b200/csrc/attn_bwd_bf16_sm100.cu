@@ -161,15 +161,25 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
   }
 
   auto bar = [&](int id) { return smem_u32(&bars[id]); };
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < NUM; ++i) {
-      const bool compute = i == P_FULL || i == P_FULL + 1 || i == DS_FULL || i == STAT_FULL;
+  if (warp == 8) {
+    static_assert(NUM <= 32, "a lane per barrier");
+    if (lane < NUM) {
+      const bool compute = lane == P_FULL || lane == P_FULL + 1 || lane == DS_FULL || lane == STAT_FULL;
       // a Q (dO) tile is read by a product of either issuer; both have to be done with it
-      const bool both = (i >= Q_EMPTY && i < Q_EMPTY + 4) || (i >= G_EMPTY && i < G_EMPTY + 4) || i == ACC_FULL || i == DRAIN;
-      mbar_init(bar(i), compute ? 256 : both ? C::kIssuers : 1);
+      const bool both = (lane >= Q_EMPTY && lane < Q_EMPTY + 4) || (lane >= G_EMPTY && lane < G_EMPTY + 4) || lane == ACC_FULL || lane == DRAIN;
+      mbar_init(bar(lane), compute ? 256 : both ? C::kIssuers : 1);
     }
-    *abort_flag = 0;
+    if (lane == 0) *abort_flag = 0;
     mbar_init_fence();
+    __syncwarp();
+    if (lane == 0) {  // the first tiles are under way while the others set up
+      pdl_wait();
+      mbar_arrive_expect_tx(bar(KV_FULL), 2 * kTile);
+      for (uint32_t sl = 0; sl < C::kSlabs; ++sl) tma_load_4d(aK + sl * kSlab, &tmK, bar(KV_FULL), (int)(sl * 64), (int)h, (int)k0, (int)b);
+      load_tile<C>(aQ, &tmQ, bar(Q_FULL), (int)h, (int)(i_begin * BT), (int)b);
+      for (uint32_t sl = 0; sl < C::kSlabs; ++sl) tma_load_4d(aV + sl * kSlab, &tmV, bar(KV_FULL), (int)(sl * 64), (int)h, (int)k0, (int)b);
+      load_tile<C>(aG, &tmG, bar(G_FULL), (int)h, (int)(i_begin * BT), (int)b);
+    }
   }
   if (warp == 10) {
     tmem_alloc(smem_u32(tmem_holder), kTmemCols);
@@ -184,14 +194,9 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
   const uint32_t tS0 = tmem, tDP = tmem + 128, tDV = tmem + 256, tDK = tmem + 256 + HD, tS1 = C::kSBufs == 2 ? tmem + 384 : tmem;
 
   if (warp == 8) {
-    // producer: K, V once, then the Q ring
+    // producer: the Q ring (K, V and the first Q and dO tiles were requested during set-up)
     if (lane == 0) {
-      mbar_arrive_expect_tx(bar(KV_FULL), 2 * kTile);
-      for (uint32_t sl = 0; sl < C::kSlabs; ++sl) {
-        tma_load_4d(aK + sl * kSlab, &tmK, bar(KV_FULL), (int)(sl * 64), (int)h, (int)k0, (int)b);
-        tma_load_4d(aV + sl * kSlab, &tmV, bar(KV_FULL), (int)(sl * 64), (int)h, (int)k0, (int)b);
-      }
-      for (int it = 0; it < n_it; ++it) {
+      for (int it = 1; it < n_it; ++it) {
         const int s = it % C::kRing, use = it / C::kRing;
         if (use > 0 && !mbar_wait(bar(Q_EMPTY + s), (use - 1) & 1, abort_flag)) break;
         load_tile<C>(aQ + s * kTile, &tmQ, bar(Q_FULL + s), (int)h, (int)((i_begin + it) * BT), (int)b);
@@ -200,7 +205,7 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
   } else if (warp == 9) {
     // producer: the dO ring
     if (lane == 0) {
-      for (int it = 0; it < n_it; ++it) {
+      for (int it = 1; it < n_it; ++it) {
         const int s = it % C::kRing, use = it / C::kRing;
         if (use > 0 && !mbar_wait(bar(G_EMPTY + s), (use - 1) & 1, abort_flag)) break;
         load_tile<C>(aG + s * kTile, &tmG, bar(G_FULL + s), (int)h, (int)((i_begin + it) * BT), (int)b);
@@ -447,10 +452,20 @@ k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   }
 
   auto bar = [&](int id) { return smem_u32(&bars[id]); };
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < NUM; ++i) mbar_init(bar(i), (i == S_FREE || i == DS_FULL) ? 256 : i == DRAIN ? C::kIssuers : 1);
-    *abort_flag = 0;
+  if (warp == 8) {
+    static_assert(NUM <= 32, "a lane per barrier");
+    if (lane < NUM) mbar_init(bar(lane), (lane == S_FREE || lane == DS_FULL) ? 256 : lane == DRAIN ? C::kIssuers : 1);
+    if (lane == 0) *abort_flag = 0;
     mbar_init_fence();
+    __syncwarp();
+    if (lane == 0) {  // the first tiles are under way while the others set up
+      if (!p.early) pdl_wait();
+      mbar_arrive_expect_tx(bar(QG_FULL), 2 * kTile);
+      for (uint32_t sl = 0; sl < C::kSlabs; ++sl) tma_load_4d(aQ + sl * kSlab, &tmQ, bar(QG_FULL), (int)(sl * 64), (int)h, (int)q0, (int)b);
+      load_tile<C>(aK, &tmK, bar(K_FULL), (int)h, 0, (int)b);
+      for (uint32_t sl = 0; sl < C::kSlabs; ++sl) tma_load_4d(aG + sl * kSlab, &tmG, bar(QG_FULL), (int)(sl * 64), (int)h, (int)q0, (int)b);
+      load_tile<C>(aV, &tmV, bar(V_FULL), (int)h, 0, (int)b);
+    }
   }
   if (warp == 10) {
     tmem_alloc(smem_u32(tmem_holder), kTmemCols);
@@ -466,12 +481,7 @@ k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
   if (warp == 8) {
     if (lane == 0) {
-      mbar_arrive_expect_tx(bar(QG_FULL), 2 * kTile);
-      for (uint32_t sl = 0; sl < C::kSlabs; ++sl) {
-        tma_load_4d(aQ + sl * kSlab, &tmQ, bar(QG_FULL), (int)(sl * 64), (int)h, (int)q0, (int)b);
-        tma_load_4d(aG + sl * kSlab, &tmG, bar(QG_FULL), (int)(sl * 64), (int)h, (int)q0, (int)b);
-      }
-      for (int j = 0; j < n_kv; ++j) {
+      for (int j = 1; j < n_kv; ++j) {
         const int s = j % C::kRing, use = j / C::kRing;
         if (use > 0 && !mbar_wait(bar(K_EMPTY + s), (use - 1) & 1, abort_flag)) break;
         load_tile<C>(aK + s * kTile, &tmK, bar(K_FULL + s), (int)h, j * BT, (int)b);
@@ -479,7 +489,7 @@ k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     }
   } else if (warp == 9) {
     if (lane == 0) {
-      for (int j = 0; j < n_kv; ++j) {
+      for (int j = 1; j < n_kv; ++j) {
         const int s = j % C::kRing, use = j / C::kRing;
         if (use > 0 && !mbar_wait(bar(V_EMPTY + s), (use - 1) & 1, abort_flag)) break;
         load_tile<C>(aV + s * kTile, &tmV, bar(V_FULL + s), (int)h, j * BT, (int)b);
