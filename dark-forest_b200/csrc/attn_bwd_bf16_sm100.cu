@@ -190,7 +190,7 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_holder;
   pdl_wait();  // everything above touched only this CTA's shared and tensor memory
-  if (p.early && threadIdx.x == 0) pdl_trigger();  // the dQ kernel needs nothing from this one: it may start where SMs are free
+  if (p.early && warp == 0) pdl_trigger();  // the dQ kernel needs nothing from this one: it may start where SMs are free
   const uint32_t tS0 = tmem, tDP = tmem + 128, tDV = tmem + 256, tDK = tmem + 256 + HD, tS1 = C::kSBufs == 2 ? tmem + 384 : tmem;
 
   if (warp == 8) {

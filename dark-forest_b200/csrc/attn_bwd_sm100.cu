@@ -1062,7 +1062,7 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     uint32_t g = 0, n = 0;
     int r = pick(0, &cur);
     bool ok = true;
-    if (SPLIT && r < 0 && p.early && threadIdx.x == 0) pdl_trigger();  // no step for this CTA
+    if (SPLIT && r < 0 && p.early && warp == 0) pdl_trigger();  // no step for this CTA
     float lse_raw = -INFINITY, dlt = 0.0f, lse_raw_next = -INFINITY, dlt_next = 0.0f;
     if (r >= 0) fetch_stats(cur, &lse_raw, &dlt);
     if (FUSE_DELTA && r >= 0) ok = fused_delta(cur, 0, &dlt);
@@ -1070,9 +1070,11 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       const int rn = pick(r + 1, &nxt);
       if (FUSE_DELTA && p.early && rn < 0) {
         // All row sums of this CTA are written: the dK/dV kernel may start on SMs that have run out of items.
+        // (Decided by a whole warp: the tensor-memory instructions that follow need their warps converged.)
         __threadfence();
         mbar_arrive(bar(DELTA_DONE));
-        if (threadIdx.x == 0 && mbar_wait(bar(DELTA_DONE), 0, abort_flag)) pdl_trigger();
+        if (warp == 0 && mbar_wait_warp(bar(DELTA_DONE), 0, abort_flag)) pdl_trigger();
+        __syncwarp();
       }
       if (rn >= 0) fetch_stats(nxt, &lse_raw_next, &dlt_next);  // in flight while this item computes
       const float lse2 = lse2_of(lse_raw);
