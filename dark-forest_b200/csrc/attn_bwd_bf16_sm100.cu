@@ -298,13 +298,13 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
       const float *lse2 = sLse2 + sb * 128, *dlt = sDelta + sb * 128;
       sb = sb == 2 ? 0 : sb + 1;
       const float stat_next = fetch_stat(it + 1);
-      if (!mbar_wait(bar(STAT_FULL), ph, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(bar(STAT_FULL), ph, abort_flag)) { ok = false; break; }
       const bool need_mask = p.causal && (q0 + p.shift < k0 + (BT - 1));
       const long long cmin_ll = kj - p.shift - q0;  // visible iff column >= cmin
       const int cmin = !need_mask ? 0 : (cmin_ll > BT ? BT : (cmin_ll < 0 ? 0 : (int)cmin_ll));
       const bool second = C::kSBufs == 2 && ph;
       const uint32_t tS = second ? tS1 : tS0;
-      if (!mbar_wait(bar(S_FULL + (second ? 1 : 0)), (it / C::kSBufs) & 1, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(bar(S_FULL + (second ? 1 : 0)), (it / C::kSBufs) & 1, abort_flag)) { ok = false; break; }
       tc_fence_after_sync();
       float pr[64];
       uint32_t packed[32];
@@ -337,7 +337,7 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
       tc_fence_before_sync();
       mbar_arrive(bar(P_FULL + (second ? 1 : 0)));
       if (it + 1 < n_it) stage_stat(sb, stat_next);
-      if (!mbar_wait(bar(DP_FULL), ph, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(bar(DP_FULL), ph, abort_flag)) { ok = false; break; }
       tc_fence_after_sync();
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
@@ -358,7 +358,7 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
       tc_fence_before_sync();
       mbar_arrive(bar(DS_FULL));
     }
-    if (ok && mbar_wait(bar(ACC_FULL), 0, abort_flag)) {
+    if (ok && mbar_wait_warp(bar(ACC_FULL), 0, abort_flag)) {
       tc_fence_after_sync();
       // warps 0-3 store dV, warps 4-7 store scale * dK
       const bool row_ok = kj < (long long)p.Sk;
@@ -599,7 +599,7 @@ k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       const uint32_t ph = j & 1;
       const int key0 = j * BT;
       const bool need_mask = key0 + BT > kmax;
-      if (!mbar_wait(bar(S_FULL), ph, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(bar(S_FULL), ph, abort_flag)) { ok = false; break; }
       tc_fence_after_sync();
       float pr[64];
 #pragma unroll
@@ -620,7 +620,7 @@ k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       tc_fence_before_sync();
       mbar_arrive(bar(S_FREE));
       const uint32_t tDP = ph ? tDP1 : tDP0, dp_buf = C::kIssuers == 2 ? ph : 0;
-      if (!mbar_wait(bar(DP_FULL + dp_buf), (j / C::kIssuers) & 1, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(bar(DP_FULL + dp_buf), (j / C::kIssuers) & 1, abort_flag)) { ok = false; break; }
       tc_fence_after_sync();
       uint32_t packed[32];
 #pragma unroll
@@ -638,7 +638,7 @@ k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       tc_fence_before_sync();
       mbar_arrive(bar(DS_FULL));
     }
-    if (ok && mbar_wait(bar(ACC_FULL), 0, abort_flag)) {
+    if (ok && mbar_wait_warp(bar(ACC_FULL), 0, abort_flag)) {
       tc_fence_after_sync();
       uint8_t *dst = reinterpret_cast<uint8_t *>(p.dq) +
                      (((size_t)b * p.Sq + (size_t)(row_ok ? i : 0)) * dm + h * HD + half * (HD / 2)) * C::kOutElt;

@@ -573,7 +573,7 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
     // the MN-major dO buffer stages dV and the MN-major Q buffer dK, in the 128-byte-swizzled
     // slab layout of the store's tensor map (16-byte chunk c of row r at c ^ (r % 8)).
     auto hand_over = [&](uint32_t nd) -> bool {
-      if (!mbar_wait(bar(ACC_FULL), nd & 1, abort_flag)) return false;
+      if (!mbar_wait_warp(bar(ACC_FULL), nd & 1, abort_flag)) return false;
       DF_BTRACE(1, 60);
       tc_fence_after_sync();
       const float mul = is_dk ? p.scale : 1.0f;
@@ -623,14 +623,14 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
         const bool has_next_step = !last || more;
         float stat_next = 0.0f;
         if (has_next_step) stat_next = last ? fetch_stat(nxt, 0) : fetch_stat(cur, it + 1);
-        if (!mbar_wait(bar(STAT_FULL), ph, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(bar(STAT_FULL), ph, abort_flag)) { ok = false; break; }
         // visible iff key <= query + shift  <=>  column >= kj - shift - q0
         const bool need_mask = p.causal && (q0 + p.shift < cur.k0 + (BT - 1));
         long long cmin_ll = kj - p.shift - q0;
         const int cmin = !need_mask ? 0 : (cmin_ll > BT ? BT : (cmin_ll < 0 ? 0 : (int)cmin_ll));
         DF_BTRACE(1, 50);
         const uint32_t tS = ph ? tS1 : tS0;
-        if (!mbar_wait(bar(S_FULL0 + ph), (g >> 1) & 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(bar(S_FULL0 + ph), (g >> 1) & 1, abort_flag)) { ok = false; break; }
         DF_BTRACE(1, 51);
         tc_fence_after_sync();
         float pr[CPT];
@@ -672,7 +672,7 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
         }
         gb = gb_next;
         DF_BTRACE(1, 52);
-        if (!mbar_wait(bar(DP_FULL), ph, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(bar(DP_FULL), ph, abort_flag)) { ok = false; break; }
         DF_BTRACE(1, 53);
         tc_fence_after_sync();
 #pragma unroll
@@ -1036,7 +1036,7 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     // dO and O tiles in shared memory. Each of the row's two threads sums its 32 dims (one
     // 128-byte slab row, 16-byte chunk c at c ^ (row % 8)); the halves meet in shared memory.
     auto fused_delta = [&](const Item &im, uint32_t nn, float *out) -> bool {
-      if (!mbar_wait(bar(GO_FULL), nn & 1, abort_flag)) return false;
+      if (!mbar_wait_warp(bar(GO_FULL), nn & 1, abort_flag)) return false;
       const uint8_t *g_row = smem + kTile + half * kSlab + row * 128;
       const uint8_t *o_row = smem + 5 * kTile + half * kSlab + row * 128;
       float acc0 = 0.0f, acc1 = 0.0f;
@@ -1052,7 +1052,7 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       xs[half * 128 + row] = acc0 + acc1;
       mbar_arrive(bar(O_FREE));
       mbar_arrive(bar(DX_FULL));
-      if (!mbar_wait(bar(DX_FULL), nn & 1, abort_flag)) return false;
+      if (!mbar_wait_warp(bar(DX_FULL), nn & 1, abort_flag)) return false;
       *out = xs[row] + xs[128 + row];
       const long long i = im.q0 + row;
       if (half == 0 && rank == 0 && i < (long long)p.Sq) p.delta_out[((size_t)im.b * p.H + im.h) * p.Sq + (size_t)i] = *out;
@@ -1088,7 +1088,7 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         const int key0 = (j * ST + rank) * BT;
         const bool need_mask = key0 + BT > kmax;
         DF_BTRACE(1, 50);
-        if (!mbar_wait(bar(S_FULL), ph, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(bar(S_FULL), ph, abort_flag)) { ok = false; break; }
         DF_BTRACE(1, 51);
         tc_fence_after_sync();
         float pr[64];
@@ -1110,7 +1110,7 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         tc_fence_before_sync();
         mbar_arrive(bar(S_FREE));
         DF_BTRACE(1, 52);
-        if (!mbar_wait(bar(DP_FULL0 + ph), (g >> 1) & 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(bar(DP_FULL0 + ph), (g >> 1) & 1, abort_flag)) { ok = false; break; }
         DF_BTRACE(1, 53);
         tc_fence_after_sync();
         const uint32_t tDP = ph ? tDP1 : tDP0;
@@ -1133,7 +1133,7 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       // and the row sums after it, measured the same)
       if (FUSE_DELTA && ok && rn >= 0) ok = fused_delta(nxt, n + 1, &dlt_next);
       DF_BTRACE(1, 59);
-      if (!ok || !mbar_wait(bar(ACC_FULL), n & 1, abort_flag)) { ok = false; break; }
+      if (!ok || !mbar_wait_warp(bar(ACC_FULL), n & 1, abort_flag)) { ok = false; break; }
       DF_BTRACE(1, 60);
       tc_fence_after_sync();
       if (SPLIT) break;
