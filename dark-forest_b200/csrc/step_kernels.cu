@@ -232,7 +232,13 @@ k_layernorm_bwd_staged(const float *__restrict__ grad_out, const float *__restri
   mbar_init_fence();
   fence_proxy_async_smem();
   __syncthreads();
-  const uint32_t total_warps = gridDim.x * n_warps, w0 = blockIdx.x * n_warps + warp;
+  // Sixteen warps and below eight rounds: rows go to the same warp of all blocks before the next warp, so that a last round that is not full is
+  // spread over the SMs (8192 rows: 55 or 56 per SM; dealt block by block 64 on 68 SMs and 48 on the others). With more rounds
+  // the remainder weighs less than neighbouring rows in one block do, and with eight warps (wide rows) it made no clear difference. B200, us, with the column sums below: 2400 x 768 9.6 -> 8.6,
+  // 4000 x 768 12.0 -> 11.6, 8192 x 768 20.0 -> 19.8, 12288 x 512 20.1 -> 19.4, 5000 x 1024 21.6 -> 20.6; 32768 x 768 57.4 block by block
+  // against 60.
+  const uint32_t total_warps = gridDim.x * n_warps;
+  const uint32_t w0 = n_warps == 16u && rows < 8u * total_warps ? warp * gridDim.x + blockIdx.x : blockIdx.x * n_warps + warp;
   const float n = (float)cols;
   // the copies of this warp's k-th row (row w0 + k * total_warps) into slot `st`
   // Lane `st` also fetches the row's mean and rstd now and hands them to the warp when the slot is consumed: loaded
@@ -309,7 +315,8 @@ k_layernorm_bwd_staged(const float *__restrict__ grad_out, const float *__restri
     }
   }
   // Column sums over the block: every warp parks its partial sums in its own ring (empty by now: every copy it issued
-  // has been consumed), then each thread adds up a few columns over the warps and sends one atomic per column.
+  // has been consumed), then each thread adds up four columns over the warps and sends them in one vector reduction (a scalar
+  // atomic per column where the gradients are not on 16-byte boundaries).
   // (Floating-point atomics on shared memory from sixteen warps at once cost a quarter of the kernel's time.)
   const bool want_cols = grad_gamma != nullptr || grad_beta != nullptr;
   float4 *park = reinterpret_cast<float4 *>(my_ring);  // [2][nvec]
@@ -327,11 +334,26 @@ k_layernorm_bwd_staged(const float *__restrict__ grad_out, const float *__restri
   if (want_cols) {
     const size_t warp_stride = (size_t)stages * 2u * row_bytes / sizeof(float);
     const float *base = reinterpret_cast<const float *>(ring);
-    for (uint32_t i = threadIdx.x; i < 2 * cols; i += blockDim.x) {
-      float t = 0.0f;
-      for (uint32_t w = 0; w < n_warps; ++w) t += base[w * warp_stride + i];
-      float *dst = i < cols ? grad_gamma : grad_beta;
-      if (dst) atomicAdd(dst + (i < cols ? i : i - cols), t);
+    // the blocks end together: each starts at a column of its own, so that they do not all add to the same line at once
+    const uint32_t first = (uint32_t)((uint64_t)blockIdx.x * 2u * nvec / gridDim.x);
+    for (uint32_t k = threadIdx.x; k < 2 * nvec; k += blockDim.x) {
+      const uint32_t i = k + first < 2 * nvec ? k + first : k + first - 2 * nvec;
+      float *dst = i < nvec ? grad_gamma : grad_beta;
+      if (!dst) continue;
+      dst += 4u * (i < nvec ? i : i - nvec);
+      float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (uint32_t w = 0; w < n_warps; ++w) {
+        const float4 v = *reinterpret_cast<const float4 *>(base + w * warp_stride + 4u * i);
+        t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w;
+      }
+      if ((reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
+        asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(t.x), "f"(t.y), "f"(t.z), "f"(t.w) : "memory");
+      } else {
+        atomicAdd(dst, t.x);
+        atomicAdd(dst + 1, t.y);
+        atomicAdd(dst + 2, t.z);
+        atomicAdd(dst + 3, t.w);
+      }
     }
   }
 }
