@@ -13,8 +13,8 @@
 //   warps 0-7   softmax of tile A, warps 8-15 of tile B: two threads per query row (64 keys each) read S from tensor memory, mask
 //               the diagonal tile, combine their maxima through shared memory, keep a lazily updated running maximum, write P as
 //               packed bf16 over S, and finally normalise O and store O and lse.
-// Every mbarrier wait is bounded; if one gives up, the CTA raises its abort flag, all roles fall through to the common teardown
-// and bit 0 of the device status word is set.
+// Every mbarrier wait is bounded and, in roles of whole warps, decided by the warp together; if one gives up, the CTA raises its abort
+// flag, all roles fall through to the common teardown and bit 0 of the device status word is set.
 #include <math.h>
 
 #include "df_common.cuh"
@@ -267,7 +267,7 @@ k_attn_fwd(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     float l0 = 0.0f, l1 = 0.0f, l2 = 0.0f, l3 = 0.0f;
     bool ok = nkv > 0;
     for (int j = 0; j < nkv; ++j) {
-      if (!mbar_wait(bar(S_FULL + t), j & 1, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(bar(S_FULL + t), j & 1, abort_flag)) { ok = false; break; }
       tc_fence_after_sync();
       const int key0 = j * BN + col0;
       const bool need_mask = key0 + 64 > kmax;
@@ -299,7 +299,7 @@ k_attn_fwd(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
       float *xmax = xch + (j & 1) * 256;
       xmax[half * 128 + row] = mx_half;
       mbar_arrive(bar(X_FULL + t));
-      if (!mbar_wait(bar(X_FULL + t), j & 1, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(bar(X_FULL + t), j & 1, abort_flag)) { ok = false; break; }
       const float mx = fmaxf(mx_half, xmax[(half ^ 1) * 128 + row]);
       m_run = fmaxf(m_run, mx * p.scale_log2);
       // lazy rescale, decided per warp so that the TMEM accesses stay warp-uniform; the partner
@@ -310,7 +310,7 @@ k_attn_fwd(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         l0 *= alpha; l1 *= alpha; l2 *= alpha; l3 *= alpha;
         m_used = m_run;
         if (j > 0) {
-          if (!mbar_wait(bar(O_FULL + t), (j - 1) & 1, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(bar(O_FULL + t), (j - 1) & 1, abort_flag)) { ok = false; break; }
           tc_fence_after_sync();
           // each half rescales HD/2 of the O columns, 16 at a time to stay within the register budget
 #pragma unroll 1
@@ -369,10 +369,10 @@ k_attn_fwd(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
       float *xl = xch + 512;
       xl[half * 128 + row] = l;
       mbar_arrive(bar(L_FULL + t));
-      if (!mbar_wait(bar(L_FULL + t), 0, abort_flag)) ok = false;
+      if (!mbar_wait_warp(bar(L_FULL + t), 0, abort_flag)) ok = false;
       else l += xl[(half ^ 1) * 128 + row];
     }
-    if (ok && mbar_wait(bar(O_FULL + t), (nkv - 1) & 1, abort_flag)) {
+    if (ok && mbar_wait_warp(bar(O_FULL + t), (nkv - 1) & 1, abort_flag)) {
       tc_fence_after_sync();
       const float inv = l > 0.0f ? 1.0f / l : 0.0f;
       const bool row_ok = i < (long long)p.Sq;

@@ -132,9 +132,12 @@ __device__ __forceinline__ bool elect_one() {
 
 // Bounded wait and barrier poll for a role that all 32 lanes of a warp run together: every lane gets the same answer,
 // so the lanes leave their loops together (a lane that gave up alone would leave the others waiting for it at the
-// next elect.sync).
+// next elect.sync, vote or tensor-memory instruction). The first poll is voted on by itself, so that the usual case has no
+// branch that lanes could take apart: with one vote around mbar_wait the bf16 forward at head dimension 128 took 1.5 to 5 % more
+// than with waits lane by lane, this way 1 % less (B200, 16 heads, S = 8192, causal: 275 us lane by lane, 280, 270).
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t *abort_flag) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)) != 0;
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return __all_sync(0xffffffffu, mbar_wait_slow(bar, parity, abort_flag, kWaitBudgetNs)) != 0;
 }
 __device__ __forceinline__ uint32_t mbar_test3_warp(uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1, uint32_t b2, uint32_t p2) {
   return __reduce_and_sync(0xffffffffu, mbar_test3(b0, p0, b1, p1, b2, p2));
