@@ -266,7 +266,9 @@ k_layernorm_bwd_staged(const float *__restrict__ grad_out, const float *__restri
   bool ok = true;
   uint32_t st = 0, phase = 0;
   for (uint32_t row = w0; row < rows; row += total_warps) {
-    if (!mbar_wait_warp(smem_u32(my_bars + st), phase, abort_flag)) { ok = false; break; }
+    // one vote around the whole wait: with mbar_wait_warp, whose first poll has a vote of its own, rows that mostly are not there
+    // yet cost 1 to 3 % more (12000 x 768: 20.4 against 21.0 us)
+    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(my_bars + st), phase, abort_flag))) { ok = false; break; }
     const float4 *sx = reinterpret_cast<const float4 *>(my_ring + (size_t)st * 2u * row_bytes), *sd = sx + nvec;
     const float mean = __shfl_sync(0xffffffffu, slot_mean, (int)st), rstd = __shfl_sync(0xffffffffu, slot_rstd, (int)st);
     float s1 = 0.0f, s2 = 0.0f;
