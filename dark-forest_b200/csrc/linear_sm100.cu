@@ -234,7 +234,7 @@ k_linear_tf32(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
         }
       };
       fetch(0);
-      if (!mbar_wait(bar(C::ACC_FULL + acc), (j >> 1) & 1, abort_flag)) break;
+      if (!mbar_wait_warp(bar(C::ACC_FULL + acc), (j >> 1) & 1, abort_flag)) break;
       tc_fence_after_sync();
 #pragma unroll 1
       for (int cg = 0; cg < kGroups; ++cg) {
@@ -287,7 +287,7 @@ k_linear_tf32(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
     constexpr int OW = C::kOwned, LD = C::kPartLd;
     bool ok = true;
     if (warp >= 2) {
-      ok = mbar_wait(bar(C::ACC_FULL), 0, abort_flag);
+      ok = mbar_wait_warp(bar(C::ACC_FULL), 0, abort_flag);
       tc_fence_after_sync();
     }
     __syncthreads();
