@@ -756,7 +756,7 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
 // =========================================================================================
 namespace dq {
 enum Bar { Q_FULL = 0, GO_FULL, Q_EMPTY, G_EMPTY, KK_FULL, VK_FULL, KM_FULL, KM_EMPTY, S_FULL, S_FREE, DP_FULL0, DP_FULL1,
-           DS_FULL, ACC_FULL, EPI_FULL, O_FREE, DX_FULL, DELTA_DONE, DRAIN, NUM };
+           DS_FULL0, DS_FULL1, ACC_FULL, EPI_FULL, O_FREE, DX_FULL, DELTA_DONE, DRAIN, NUM };
 constexpr uint32_t kBars = 6 * kTile;              // Q, dO, K (K-major), V, K (MN-major), O (only with fused row sums)
 constexpr uint32_t kXch = kBars + 256;             // partial row sums [2][128]
 constexpr uint32_t kSmemTotal = kXch + 1024 + 1024;
@@ -825,7 +825,7 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     return out->n_kv > 0 ? 0 : -1;
   };
   if (warp == 8) {
-    if (lane < NUM) mbar_init(bar(lane), (lane == S_FREE || lane == DS_FULL || lane == EPI_FULL || lane == O_FREE || lane == DX_FULL || lane == DELTA_DONE) ? 256 : 1);
+    if (lane < NUM) mbar_init(bar(lane), (lane == S_FREE || lane == DS_FULL0 || lane == DS_FULL1 || lane == EPI_FULL || lane == O_FREE || lane == DX_FULL || lane == DELTA_DONE) ? 256 : 1);
     static_assert(NUM <= 32, "a lane per barrier");
     if (lane == 0) *abort_flag = 0;
     mbar_init_fence();
@@ -974,8 +974,11 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             // dP_{g+1} of the same item goes out now, into the buffer dQ_{g-1} (issued a step ago by this thread) read
             if (!last && !issue_dp(g + 1, next_last)) { ok = false; break; }
           }
-          const uint32_t m = mbar_test3_warp(bar(DS_FULL), ph, bar(KM_FULL), ph, bar(KM_FULL), ph);
-          if ((!(m & 1u) && !mbar_wait_warp(bar(DS_FULL), ph, abort_flag)) || (!(m & 2u) && !mbar_wait_warp(bar(KM_FULL), ph, abort_flag))) {
+          // dS has a barrier per dP buffer: dP_{g+1} is out already, so dS_{g+1} may be complete before this warp has looked for
+          // dS_g, and on one barrier it would then wait for a phase that has come round again
+          const uint32_t ph2 = (g >> 1) & 1;
+          const uint32_t m = mbar_test3_warp(bar(DS_FULL0 + ph), ph2, bar(KM_FULL), ph, bar(KM_FULL), ph);
+          if ((!(m & 1u) && !mbar_wait_warp(bar(DS_FULL0 + ph), ph2, abort_flag)) || (!(m & 2u) && !mbar_wait_warp(bar(KM_FULL), ph, abort_flag))) {
             ok = false;
             break;
           }
@@ -1125,7 +1128,7 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         }
         tmem_wait_st();
         tc_fence_before_sync();
-        mbar_arrive(bar(DS_FULL));
+        mbar_arrive(bar(DS_FULL0 + ph));
         DF_BTRACE(1, 54);
       }
       // the next item's dO and O tiles are on their way or already here: its row sums are
