@@ -405,8 +405,8 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
 // =========================================================================================
 namespace dq16 {
 enum Bar { QG_FULL = 0, K_FULL = 1, K_EMPTY = 5, V_FULL = 9, V_EMPTY = 13,   // + ring stage
-           DP_FULL = 17,                                                     // + dP buffer
-           S_FULL = 19, S_FREE, DS_FULL, ACC_FULL, DRAIN, NUM };
+           DP_FULL = 17, DS_FULL = 19,                                       // + dP buffer
+           S_FULL = 21, S_FREE, ACC_FULL, DRAIN, NUM };
 template <class C> __host__ __device__ constexpr uint32_t bars_off() { return (2 + 2 * C::kRing) * C::kTile; }     // Q, dO, K ring, V ring
 template <class C> __host__ __device__ constexpr uint32_t smem_total() { return bars_off<C>() + 256 + 1024; }
 }  // namespace dq16
@@ -454,7 +454,7 @@ k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   auto bar = [&](int id) { return smem_u32(&bars[id]); };
   if (warp == 8) {
     static_assert(NUM <= 32, "a lane per barrier");
-    if (lane < NUM) mbar_init(bar(lane), (lane == S_FREE || lane == DS_FULL) ? 256 : lane == DRAIN ? C::kIssuers : 1);
+    if (lane < NUM) mbar_init(bar(lane), (lane == S_FREE || lane == DS_FULL || lane == DS_FULL + 1) ? 256 : lane == DRAIN ? C::kIssuers : 1);
     if (lane == 0) *abort_flag = 0;
     mbar_init_fence();
     __syncwarp();
@@ -568,8 +568,9 @@ k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       for (int j = 0; ok && j < n_kv; ++j) {
         const int st = j % C::kRing;
         if (j + 1 < n_kv && !issue_dp(j + 1)) break;
-        // S_j has read this K tile before its scores became dS_j
-        if (!mbar_wait_warp(bar(K_FULL + st), (j / C::kRing) & 1, abort_flag) || !mbar_wait_warp(bar(DS_FULL), j & 1, abort_flag)) break;
+        // S_j has read this K tile before its scores became dS_j. dS has a barrier per dP buffer: dP_{j+1} is out already, so dS_{j+1}
+        // may be complete before this warp has looked for dS_j, and on one barrier that phase would have come round again.
+        if (!mbar_wait_warp(bar(K_FULL + st), (j / C::kRing) & 1, abort_flag) || !mbar_wait_warp(bar(DS_FULL + (j & 1)), (j >> 1) & 1, abort_flag)) break;
         tc_fence_after_sync();
         issue_ts<C>(tDQ, (j & 1) ? tDP1 : tDP0, dKm + (uint64_t)(st * (kTile >> 4)), idesc_ts, j > 0);
         commit_elected(bar(K_EMPTY + st));
@@ -636,7 +637,7 @@ k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       tmem_st32(tDP + lane_base + col0, packed);
       tmem_wait_st();
       tc_fence_before_sync();
-      mbar_arrive(bar(DS_FULL));
+      mbar_arrive(bar(DS_FULL + dp_buf));
     }
     if (ok && mbar_wait_warp(bar(ACC_FULL), 0, abort_flag)) {
       tc_fence_after_sync();

@@ -102,6 +102,40 @@ def dq_tf32(items, ds_bars):
     return {"load_k": load_k, "load_m": load_m, "mma": mma, "compute 0": compute, "compute 1": compute}
 
 
+def dq_bf16(n_kv, ds_bars, ring=4):
+    """k_attn_bwd_dq_bf16 with two issuing warps (head dimension 64)."""
+    load_k, load_v, scores, dp_dq, compute = Role(), Role(), Role(), Role(), Role()
+    for j in range(n_kv):
+        for role, tile in ((load_k, "K"), (load_v, "V")):
+            if j >= ring:
+                role.wait("%s_EMPTY%d" % (tile, j % ring), j // ring - 1)
+            role.arrive("%s_FULL%d" % (tile, j % ring))
+        scores.wait("K_FULL%d" % (j % ring), j // ring)
+        if j > 0:
+            scores.wait("S_FREE", j - 1)
+        scores.arrive("S_FULL")
+
+    def dp(j):
+        dp_dq.wait("V_FULL%d" % (j % ring), j // ring)
+        dp_dq.arrive("DP_FULL%d" % (j % 2))
+        dp_dq.arrive("V_EMPTY%d" % (j % ring))
+
+    dp(0)
+    for j in range(n_kv):
+        if j + 1 < n_kv:
+            dp(j + 1)
+        dp_dq.wait("K_FULL%d" % (j % ring), j // ring)
+        dp_dq.wait("DS_FULL%d" % (j % ds_bars), j // ds_bars)
+        dp_dq.arrive("K_EMPTY%d" % (j % ring))
+        compute.wait("S_FULL", j)
+        compute.arrive("S_FREE")
+        compute.wait("DP_FULL%d" % (j % 2), j // 2)
+        compute.arrive("DS_FULL%d" % (j % ds_bars))
+    dp_dq.arrive("ACC_FULL")
+    compute.wait("ACC_FULL", 0)
+    return {"load_k": load_k, "load_v": load_v, "scores": scores, "dp_dq": dp_dq, "compute 0": compute, "compute 1": compute}
+
+
 def phases_missed(roles):
     """(role, barrier, phase) of every wait that can find its barrier two phases on; fails when a role does not reach its end."""
     counts = {}
@@ -137,7 +171,8 @@ def phases_missed(roles):
 
 
 def test_one_barrier_for_two_buffers_is_missed():
-    assert {m[:2] for m in phases_missed(dq_tf32([4], 1))} == {("mma", "DS_FULL0")}
+    assert ("mma", "DS_FULL0") in {m[:2] for m in phases_missed(dq_tf32([4], 1))}
+    assert ("dp_dq", "DS_FULL0") in {m[:2] for m in phases_missed(dq_bf16(4, 1))}
 
 
 @pytest.mark.parametrize("items", [[1], [2], [1, 1, 1], [5, 2, 1, 3], [7, 6]])
@@ -146,3 +181,16 @@ def test_tf32_dq_waits_see_every_phase(items):
         enum = re.search(r"namespace dq \{\s*enum Bar \{(.*?)\}", f.read(), re.S).group(1)
     ds_bars = len(re.findall(r"\bDS_FULL\d?\b", enum))
     assert phases_missed(dq_tf32(items, ds_bars)) == []
+
+
+@pytest.mark.parametrize("n_kv", [1, 2, 3, 9])
+def test_bf16_dq_waits_see_every_phase(n_kv):
+    with open(os.path.join(CSRC, "attn_bwd_bf16_sm100.cu")) as f:
+        enum = re.search(r"namespace dq16 \{\s*enum Bar \{(.*?)\}", f.read(), re.S).group(1)
+    enum = re.sub(r"//[^\n]*", "", enum)
+    at, value = {}, -1
+    for name, explicit in re.findall(r"(\w+)(?:\s*=\s*(\d+))?\s*(?:,|$)", enum):
+        value = int(explicit) if explicit else value + 1
+        at[name] = value
+    ds_bars = min(v for v in at.values() if v > at["DS_FULL"]) - at["DS_FULL"]
+    assert phases_missed(dq_bf16(n_kv, ds_bars)) == []
