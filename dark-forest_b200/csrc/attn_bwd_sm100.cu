@@ -698,7 +698,7 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
         DF_BTRACE(1, 54);
       }
       if (SPLIT) {
-        if (ok) ok = mbar_wait(bar(ACC_FULL), n & 1, abort_flag);
+        if (ok) ok = mbar_wait_warp(bar(ACC_FULL), n & 1, abort_flag);
         break;
       }
       if (!ok || !hand_over(n)) { ok = false; break; }

@@ -84,7 +84,7 @@ def test_the_rule_sees_what_it_is_about():
     assert lone_waits(kernel("if (take(1)) tmem_ld32(a, r);")) == [1]
 
 
-@pytest.mark.parametrize("name", ["attn_fwd_sm100.cu", "attn_fwd_row2_sm100.cu", "attn_bwd_bf16_sm100.cu", "linear_sm100.cu"])
+@pytest.mark.parametrize("name", ["attn_fwd_sm100.cu", "attn_fwd_row2_sm100.cu", "attn_bwd_sm100.cu", "attn_bwd_bf16_sm100.cu", "linear_sm100.cu"])
 def test_whole_warps_wait_as_warps(name):
     with open(os.path.join(CSRC, name)) as f:
         src = f.read()
