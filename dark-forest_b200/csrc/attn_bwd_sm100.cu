@@ -707,7 +707,6 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
     }
   }
   if constexpr (SPLIT) {
-    __syncwarp();
     tc_fence_before_sync();
     cluster_sync();  // both CTAs' products are done and their operand buffers free
     tc_fence_after_sync();
@@ -716,7 +715,6 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
     const int row = (warp & 3) * 32 + lane, sub = warp >> 2;  // sub 0 holds the thread's row of dV, sub 1 of dK
     const uint32_t taddr = (sub ? tDK : tDV) + ((uint32_t)((warp & 3) * 32) << 16);
     if (warp < kCW && sub != (int)rank && own) send_row<HD>(map_to_rank(aGm, rank ^ 1), row, taddr);
-    __syncwarp();
     cluster_sync();
     if (warp < kCW && sub == (int)rank) {
       const long long kj = it.k0 + row;
@@ -1166,7 +1164,6 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   }
 
   if constexpr (SPLIT) {
-    __syncwarp();
     tc_fence_before_sync();
     cluster_sync();  // both CTAs' products are done and their operand buffers free
     tc_fence_after_sync();
@@ -1175,7 +1172,6 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     const int row = (warp & 3) * 32 + lane, half = warp >> 2;
     const uint32_t taddr = tDQ + half * 32 + ((uint32_t)((warp & 3) * 32) << 16);
     if (warp < 8 && half != rank && own) send_row<32>(map_to_rank(aKm, (uint32_t)(rank ^ 1)), row, taddr);
-    __syncwarp();
     cluster_sync();
     if (warp < 8 && half == rank) {
       const long long i = it.q0 + row;

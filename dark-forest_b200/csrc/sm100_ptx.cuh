@@ -386,7 +386,9 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
   return a;
 }
+// Every thread of the cluster. The barrier is warp-aligned, and callers come from regions that single lanes run: the warp meets first.
 __device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // Arrives on a barrier of any CTA of the cluster (address from map_to_rank).

@@ -90,3 +90,10 @@ def test_whole_warps_wait_as_warps(name):
         src = f.read()
     assert "mbar_wait" in src and "tmem_ld32" in src
     assert lone_waits(src) == []
+
+
+def test_the_cluster_barrier_brings_its_warps_together():
+    """Its instructions are warp-aligned, and kernels come to it out of one-lane regions (set-up, producers)."""
+    with open(os.path.join(CSRC, "sm100_ptx.cuh")) as f:
+        body = re.search(r"void cluster_sync\(\) \{(.*?)\n\}", f.read(), re.S).group(1)
+    assert body.index("__syncwarp();") < body.index("barrier.cluster.arrive.release.aligned")
