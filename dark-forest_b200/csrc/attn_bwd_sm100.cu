@@ -756,8 +756,9 @@ namespace dq {
 enum Bar { Q_FULL = 0, GO_FULL, Q_EMPTY, G_EMPTY, KK_FULL, VK_FULL, KM_FULL, KM_EMPTY, S_FULL, S_FREE, DP_FULL0, DP_FULL1,
            DS_FULL0, DS_FULL1, ACC_FULL, EPI_FULL, O_FREE, DX_FULL, DELTA_DONE, DRAIN, NUM };
 constexpr uint32_t kBars = 6 * kTile;              // Q, dO, K (K-major), V, K (MN-major), O (only with fused row sums)
-constexpr uint32_t kXch = kBars + 256;             // partial row sums [2][128]
-constexpr uint32_t kSmemTotal = kXch + 1024 + 1024;
+constexpr uint32_t kXch = kBars + 256;             // partial row sums of two items in turn, [2][2][128]
+constexpr uint32_t kXchItem = 2 * 128 * 4;
+constexpr uint32_t kSmemTotal = kXch + 2 * kXchItem + 1024;  // 1024: the tiles begin on the next 1024-byte boundary
 
 // One work item: 128 queries of one head and the key tiles they can see.
 struct Item {
@@ -1049,7 +1050,7 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         acc0 = fmaf(gv.x, ov.x, acc0); acc1 = fmaf(gv.y, ov.y, acc1);
         acc0 = fmaf(gv.z, ov.z, acc0); acc1 = fmaf(gv.w, ov.w, acc1);
       }
-      float *xs = sXch + (nn & 1) * 256;
+      float *xs = sXch + (nn & 1) * (kXchItem / 4);
       xs[half * 128 + row] = acc0 + acc1;
       mbar_arrive(bar(O_FREE));
       mbar_arrive(bar(DX_FULL));
