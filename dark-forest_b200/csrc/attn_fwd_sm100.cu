@@ -705,6 +705,10 @@ int launch_items(const AttnParams &p, bool split, cudaStream_t s) {
   return split ? launch_forward<FwdCfg<HD, BF16, OUT_F32, true>>(p, s) : launch_forward<FwdCfg<HD, BF16, OUT_F32, false>>(p, s);
 }
 
+// tensor_forward_supported sees to it that a CTA per pair of query tiles is a valid grid; a CTA per tile can be one too many.
+constexpr bool split_grid_fits(uint64_t tiles, uint64_t n_bh) { return tiles * n_bh <= 0x7fffffffull; }
+static_assert(split_grid_fits(2, 0x3fffffff) && !split_grid_fits(2, 0x40000000) && split_grid_fits(1, 0x7fffffff), "");
+
 // Pairs of query tiles or split items? Split items are half as long and twice as many: they win where pairs leave SMs without
 // work, or a pair of tiles is longer than an SM's share; pairs read K and V half as often. Both times are estimated from
 // what an item costs in thousands of cycles (measured slopes over S = 1000..2000 on B200): pairs 8.5 + 1.72 per step,
@@ -713,8 +717,9 @@ int launch_items(const AttnParams &p, bool split, cudaStream_t s) {
 // 1 x 6000 96.8 / 102.6, 8 x 1000 37.4 / 45.9.
 bool split_items(const AttnParams &p, int n_sm) {
   const int mode = option(DF_OPT_FWD_PERSIST);
-  if (mode != 1) return mode == 2;
   const uint64_t tiles = (p.Sq + BM - 1) / BM, n_bh = (uint64_t)p.B * p.H;
+  if (!split_grid_fits(tiles, n_bh)) return false;
+  if (mode != 1) return mode == 2;
   if (tiles < 2) return false;
   FwdParams fp;
   fp.Sq = p.Sq; fp.Sk = p.Sk; fp.causal = p.causal; fp.shift = p.shift;
