@@ -232,13 +232,13 @@ k_layernorm_bwd_staged(const float *__restrict__ grad_out, const float *__restri
   mbar_init_fence();
   fence_proxy_async_smem();
   __syncthreads();
-  // Sixteen warps and below eight rounds: rows go to the same warp of all blocks before the next warp, so that a last round that is not full is
-  // spread over the SMs (8192 rows: 55 or 56 per SM; dealt block by block 64 on 68 SMs and 48 on the others). With more rounds
-  // the remainder weighs less than neighbouring rows in one block do, and with eight warps (wide rows) it made no clear difference. B200, us, with the column sums below: 2400 x 768 9.6 -> 8.6,
-  // 4000 x 768 12.0 -> 11.6, 8192 x 768 20.0 -> 19.8, 12288 x 512 20.1 -> 19.4, 5000 x 1024 21.6 -> 20.6; 32768 x 768 57.4 block by block
-  // against 60.
+  // Sixteen warps and below two and a half rounds: rows go to the same warp of all blocks before the next warp, so that a last round that
+  // is not full is spread over the SMs. With more rounds the remainder weighs less than neighbouring rows in one block do; with eight warps
+  // (wide rows) it made no difference. B200, the dealing alone, us, block by block / spread: 3000 x 768 (1.3 rounds) 9.0 / 8.0, 5000 x 768 (2.1)
+  // 11.8 / 11.4, 6000 x 768 (2.5) 12.3 / 12.2, 7000 x 768 (3.0) 12.5 / 13.1, 8192 x 768 14.6 / 15.4, 12000 x 768 (5.1) 19.2 / 20.8; 3000 x 512
+  // 6.7 / 6.0, 5000 x 512 8.9 / 8.2, 12288 x 512 15.1 / 15.7.
   const uint32_t total_warps = gridDim.x * n_warps;
-  const uint32_t w0 = n_warps == 16u && rows < 8u * total_warps ? warp * gridDim.x + blockIdx.x : blockIdx.x * n_warps + warp;
+  const uint32_t w0 = n_warps == 16u && 2u * (uint64_t)rows < 5u * (uint64_t)total_warps ? warp * gridDim.x + blockIdx.x : blockIdx.x * n_warps + warp;
   const float n = (float)cols;
   // the copies of this warp's k-th row (row w0 + k * total_warps) into slot `st`
   // Lane `st` also fetches the row's mean and rstd now and hands them to the warp when the slot is consumed: loaded
