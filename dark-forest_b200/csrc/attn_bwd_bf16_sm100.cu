@@ -28,7 +28,6 @@ using namespace ptx;
 constexpr int BT = 128;
 constexpr uint32_t kSlab = 128 * 128;
 constexpr uint32_t kTmemCols = 512;
-constexpr float kLog2e = 1.4426950408889634f;
 
 struct Bwd16Params {
   const float *lse;

@@ -59,7 +59,6 @@ constexpr int kKvThreads = (4 * DF_KV_NSUB + 4) * 32;
 constexpr uint32_t kSlab = 128 * 128;
 constexpr uint32_t kTile = 2 * kSlab;
 constexpr uint32_t kTmemCols = 512;
-constexpr float kLog2e = 1.4426950408889634f;
 
 // Optional phase trace (build with -DDF_ATTN_TRACE): (event id, SM clock) pairs recorded by the
 // MMA thread (slot 0) and lane 0 of compute warp 0 (slot 1) of CTA 0 of the dK/dV kernel; the

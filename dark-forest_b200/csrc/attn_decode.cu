@@ -35,9 +35,11 @@ namespace cg = cooperative_groups;
 namespace df {
 namespace {
 
+using ptx::ex2_approx;
+using ptx::fma2;
+
 constexpr int kMaxWarps = 16;
 constexpr int kMaxCluster = 16;     // CTAs per head in the scratch-free form (above 8: non-portable, asked of the device once)
-constexpr float kLog2e = 1.4426950408889634f;
 
 struct DecParams {
   const float *q;
@@ -50,12 +52,6 @@ struct DecParams {
   uint32_t n_chunks;
   float scale_log2;
 };
-
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 
 // What a CTA's warps leave behind, and (in the first CTA of a cluster) what the cluster's CTAs send.
 struct MergeSmem {
@@ -79,7 +75,7 @@ __device__ __forceinline__ void merge_and_write(const DecParams &p, MergeSmem *s
     for (int w = 0; w < kWarps; ++w) M = fmaxf(M, sm->m[w]);
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) {
-      const float wgt = ex2(sm->m[w] - M);
+      const float wgt = ex2_approx(sm->m[w] - M);
       L = fmaf(sm->l[w], wgt, L);
       O = fmaf(sm->o[w][d], wgt, O);
     }
@@ -101,7 +97,7 @@ __device__ __forceinline__ void merge_and_write(const DecParams &p, MergeSmem *s
     float Mg = -FLT_MAX, Lg = 0.0f, Og = 0.0f;
     for (unsigned r = 0; r < n; ++r) Mg = fmaxf(Mg, sm->cm[r]);
     for (unsigned r = 0; r < n; ++r) {
-      const float wgt = ex2(sm->cm[r] - Mg);
+      const float wgt = ex2_approx(sm->cm[r] - Mg);
       Lg = fmaf(sm->cl[r], wgt, Lg);
       Og = fmaf(sm->co[r][d], wgt, Og);
     }
@@ -115,15 +111,6 @@ __device__ __forceinline__ void cp_async(uint32_t dst, const void *src, bool val
   const int n = valid ? GB : 0;
   if (GB == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
   else asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
-}
-
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
-      "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-      : "=f"(d.x), "=f"(d.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-  return d;
 }
 
 // One granule (GB bytes) of a thread's ring slot as pairs of floats.
@@ -254,7 +241,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads) k_attn_decode_ring(c
 #pragma unroll
     for (int o = LPT / 2; o >= (LPT >> kSplit); o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
     if (__any_sync(0xffffffffu, top > m)) {
-      const float m_new = fmaxf(m, top), alpha = ex2(m - m_new);
+      const float m_new = fmaxf(m, top), alpha = ex2_approx(m - m_new);
       m = m_new;
       l *= alpha;
 #pragma unroll
@@ -262,7 +249,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads) k_attn_decode_ring(c
 #pragma unroll
         for (int x = 0; x < VE / 2; ++x) acc[s][x] = make_float2(acc[s][x].x * alpha, acc[s][x].y * alpha);
     }
-    const float my_p = ex2(sc[0] - m);
+    const float my_p = ex2_approx(sc[0] - m);
     l += my_p;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -282,7 +269,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads) k_attn_decode_ring(c
 #pragma unroll
   for (int o = LPT; o < 32; o <<= 1) {
     const float mo = __shfl_xor_sync(0xffffffffu, m, o), lo = __shfl_xor_sync(0xffffffffu, l, o);
-    const float mn = fmaxf(m, mo), wa = ex2(m - mn), wb = ex2(mo - mn);
+    const float mn = fmaxf(m, mo), wa = ex2_approx(m - mn), wb = ex2_approx(mo - mn);
     l = l * wa + lo * wb;
 #pragma unroll
     for (int s = 0; s < SLOTS; ++s)
@@ -369,8 +356,8 @@ __global__ void __launch_bounds__(256) k_attn_decode_any(const DecParams p) {
       for (int o = 8; o >= 1; o >>= 1) dot += __shfl_xor_sync(hmask, dot, o);
       const float s2 = dot * p.scale_log2;
       const float m_new = fmaxf(m, s2);
-      const float alpha = ex2(m - m_new);  // m = -FLT_MAX on the first token: 0
-      const float pe = ex2(s2 - m_new);
+      const float alpha = ex2_approx(m - m_new);  // m = -FLT_MAX on the first token: 0
+      const float pe = ex2_approx(s2 - m_new);
       l = fmaf(l, alpha, pe);
 #pragma unroll
       for (int i = 0; i < kSlots; ++i) acc[i] = fmaf(pe, vv[u][i], acc[i] * alpha);
@@ -380,7 +367,7 @@ __global__ void __launch_bounds__(256) k_attn_decode_any(const DecParams p) {
   __syncwarp();
   {  // the two half-warps of a warp
     const float mo = __shfl_xor_sync(0xffffffffu, m, 16), lo = __shfl_xor_sync(0xffffffffu, l, 16);
-    const float mn = fmaxf(m, mo), wa = ex2(m - mn), wb = ex2(mo - mn);
+    const float mn = fmaxf(m, mo), wa = ex2_approx(m - mn), wb = ex2_approx(mo - mn);
     l = l * wa + lo * wb;
 #pragma unroll
     for (int i = 0; i < kSlots; ++i) acc[i] = acc[i] * wa + __shfl_xor_sync(0xffffffffu, acc[i], 16) * wb;
@@ -419,7 +406,7 @@ __global__ void __launch_bounds__(128) k_attn_decode_reduce(const float *__restr
   __syncthreads();
   float lsum = 0.0f;
   for (uint32_t c = d; c < n_chunks; c += 128) {
-    const float w = M > -INFINITY ? ex2(s_w[c] - M) : 0.0f;
+    const float w = M > -INFINITY ? ex2_approx(s_w[c] - M) : 0.0f;
     s_w[c] = w;
     lsum = fmaf(pl[(size_t)h * n_chunks + c], w, lsum);
   }

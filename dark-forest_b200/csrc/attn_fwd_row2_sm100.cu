@@ -425,7 +425,7 @@ k_attn_fwd(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
       if (row_ok) {
         if (half == 0 && p.lse)
           p.lse[((size_t)b * p.H + h) * p.Sq + (size_t)i] =
-              l > 0.0f ? (m_used + lg2_approx(l)) * 0.6931471805599453f : -INFINITY;
+              l > 0.0f ? (m_used + lg2_approx(l)) * kLn2 : -INFINITY;
       }
       if (C::kStoreViaSmem) {
         // all 256 threads of the tile have staged their rows (second phase of the tile's
@@ -496,7 +496,7 @@ int launch_forward(const AttnParams &p, cudaStream_t s) {
   fp.out = p.out;
   fp.lse = p.lse;
   fp.B = p.B; fp.H = p.H; fp.Sq = p.Sq; fp.Sk = p.Sk;
-  fp.scale_log2 = p.scale * 1.4426950408889634f;
+  fp.scale_log2 = p.scale * kLog2e;
   fp.causal = p.causal;
   fp.shift = p.shift;
   fp.status = device_status_ptr();

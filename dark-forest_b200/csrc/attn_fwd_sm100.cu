@@ -598,7 +598,7 @@ k_attn_fwd(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(X_EMPTY));
-        if (row_ok && t == 0 && lse) *lse = l > 0.0f ? (m + lg2_approx(l)) * 0.6931471805599453f : -INFINITY;
+        if (row_ok && t == 0 && lse) *lse = l > 0.0f ? (m + lg2_approx(l)) * kLn2 : -INFINITY;
       } else {
         const float inv = l > 0.0f ? 1.0f / l : 0.0f;
 #pragma unroll 1
@@ -612,7 +612,7 @@ k_attn_fwd(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
           for (int x = 0; x < 32; ++x) v[x] = l > 0.0f ? __uint_as_float(ro[x]) * inv : 0.0f;
           if (row_ok) store_cols(c * 32, v);
         }
-        if (row_ok && lse) *lse = l > 0.0f ? (m_used + lg2_approx(l)) * 0.6931471805599453f : -INFINITY;
+        if (row_ok && lse) *lse = l > 0.0f ? (m_used + lg2_approx(l)) * kLn2 : -INFINITY;
       }
       tc_fence_before_sync();
       buf0 = (buf0 + it.n0 + it.n1) % NB;
@@ -684,7 +684,7 @@ int launch_forward(const AttnParams &p, cudaStream_t s) {
   fp.out = p.out;
   fp.lse = p.lse;
   fp.B = p.B; fp.H = p.H; fp.Sq = p.Sq; fp.Sk = p.Sk;
-  fp.scale_log2 = p.scale * 1.4426950408889634f;
+  fp.scale_log2 = p.scale * kLog2e;
   fp.causal = p.causal;
   fp.shift = p.shift;
   fp.wide = ((uintptr_t)p.out & 31u) == 0;

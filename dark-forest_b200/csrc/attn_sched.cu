@@ -9,6 +9,15 @@
 namespace df {
 namespace {
 
+constexpr int kSchedMaxItems = 2048;
+constexpr int kSchedMaxCtas = 160;
+// CTA c runs items[off[c] .. off[c+1]) in that order.
+struct SchedTable {
+  uint32_t used;  // 0: no table
+  uint16_t off[kSchedMaxCtas + 2];
+  uint16_t items[kSchedMaxItems];
+};
+
 // First-fit decreasing under capacity `cap`: bin_of[i] for the items in `order`; false if one does not fit.
 bool first_fit(const std::vector<uint32_t> &w, const std::vector<int> &order, int grid, uint64_t cap, std::vector<int> *bin_of) {
   std::vector<uint64_t> load(grid, 0);

@@ -30,26 +30,15 @@
 namespace df {
 namespace {
 
+using ptx::ex2_approx;
+using ptx::fma2;
+
 constexpr int kCols = 64;      // loop-side rows (keys, or queries in the dK/dV part) per step
 constexpr int NT = 128;        // threads of a group; a block is two groups
 constexpr int TX = 16, TY = 8; // a group's threads along the loop-side rows (and the head dimension), and along the resident rows
 constexpr int C = kCols / TX;
 
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
-      "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-      : "=f"(d.x), "=f"(d.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-  return d;
-}
 // Exponentials are taken as 2^x of scores scaled by scale * log2 e; maxima are in the same unit.
-constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 __device__ __forceinline__ int clamp_int(long long x) { return x > 1000 ? 1000 : (x < -1000 ? -1000 : (int)x); }
 __device__ __forceinline__ void cp16(uint32_t dst, const float *src, bool valid) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
@@ -281,7 +270,7 @@ __global__ void __launch_bounds__(256, 1) k_simt_fwd(const AttnParams p, const O
 #pragma unroll
       for (int o = TX / 2; o >= 1; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
       if (__any_sync(0xffffffffu, top > m[i])) {
-        const float mn = fmaxf(m[i], top), alpha = mn == -INFINITY ? 1.0f : ex2(m[i] - mn);  // m = -inf before the first visible key: 0
+        const float mn = fmaxf(m[i], top), alpha = mn == -INFINITY ? 1.0f : ex2_approx(m[i] - mn);  // m = -inf before the first visible key: 0
         m[i] = mn;
         l[i] *= alpha;
 #pragma unroll
@@ -290,7 +279,7 @@ __global__ void __launch_bounds__(256, 1) k_simt_fwd(const AttnParams p, const O
       const float ms = m[i] == -INFINITY ? 0.0f : m[i];
 #pragma unroll
       for (int j = 0; j < C; ++j) {
-        s2[i][j].x = ex2(s2[i][j].x - ms);
+        s2[i][j].x = ex2_approx(s2[i][j].x - ms);
         l[i] += s2[i][j].x;
       }
     }
@@ -335,7 +324,7 @@ __global__ void __launch_bounds__(256, 1) k_simt_fwd(const AttnParams p, const O
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     const float mo = sM[(2 * i) * NT + tid], lo = sM[(2 * i + 1) * NT + tid];
-    const float mn = fmaxf(m[i], mo), ms = mn == -INFINITY ? 0.0f : mn, wa = ex2(m[i] - ms), wb = ex2(mo - ms);
+    const float mn = fmaxf(m[i], mo), ms = mn == -INFINITY ? 0.0f : mn, wa = ex2_approx(m[i] - ms), wb = ex2_approx(mo - ms);
     m[i] = mn;
     l[i] = l[i] * wa + lo * wb;
 #pragma unroll
@@ -453,7 +442,7 @@ __device__ __forceinline__ void backward_block(const AttnParams &p, uint32_t til
           const int row = ty + TY * i;
           const bool vis = full || (DKDV ? (col >= row + off && row < keys_left) : (col <= row + off && col < keys_left));
           const float x = (s2[i][j].x + s2[i][j].y) * scale2 - stats[DKDV ? col : row];
-          pr[i] = vis ? ex2(x) : 0.0f;
+          pr[i] = vis ? ex2_approx(x) : 0.0f;
         }
         store_column<R>(sT1, LDT, col, ty, pr);
       }
@@ -553,15 +542,6 @@ __global__ void __launch_bounds__(256, 1) k_simt_bwd(const AttnParams p, const u
 // ---------------------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------------------
-int sm_count() {
-  static std::once_flag once[64];
-  static int n[64];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  std::call_once(once[dev], [&]() { cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev); });
-  return n[dev];
-}
-
 // Every kernel may use the whole shared memory of an SM (asked once per device and kernel).
 template <auto K>
 bool allow_smem() {

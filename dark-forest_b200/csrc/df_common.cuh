@@ -25,6 +25,8 @@ struct NvtxRange {
 
 namespace df {
 
+constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
+
 // One attention problem (or one block of a ring-partitioned problem).
 // Layout: q-side tensors [B][Sq][H*D], k-side tensors [B][Sk][H*D], row statistics [B][H][Sq].
 struct AttnParams {
@@ -107,16 +109,6 @@ __host__ __device__ inline long long snake_item(int r, int grid, int cta, long l
   const long long idx = (long long)r * grid + ((r & 1) ? (grid - 1 - cta) : cta);
   return idx < n_items ? idx : -1;
 }
-
-// Explicit work lists: a MULTIFIT assignment of weighted items to CTAs (df_attn_schedule_build, attn_sched.cu): CTA c runs
-// items[off[c] .. off[c+1]) in that order.
-constexpr int kSchedMaxItems = 2048;
-constexpr int kSchedMaxCtas = 160;
-struct SchedTable {
-  uint32_t used;                       // 0: no table
-  uint16_t off[kSchedMaxCtas + 2];
-  uint16_t items[kSchedMaxItems];
-};
 
 int sm_count();  // of the current device; 0 when it cannot be asked
 

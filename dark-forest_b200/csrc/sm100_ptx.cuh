@@ -90,29 +90,9 @@ static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity
   *abort_flag = 1u;
   return false;
 }
-// INLINE = true keeps the loop at the wait site: the persistent forward runs short sequences 4 % faster that way
-// (the out-of-line call makes it spill), and everything else 2-6 % slower.
-template <bool INLINE>
-__device__ __forceinline__ bool mbar_wait_sel(uint32_t bar, uint32_t parity, volatile uint32_t *abort_flag, uint64_t budget_ns) {
-  if (mbar_try_wait(bar, parity)) return true;
-  if constexpr (INLINE) {
-    const uint64_t t0 = global_timer_ns();
-    for (uint32_t polls = 1; polls < kWaitMaxPolls; ++polls) {
-      if (mbar_try_wait(bar, parity)) return true;
-      if ((polls & 255u) == 0u) {
-        if (*abort_flag != 0u) return false;
-        if (global_timer_ns() - t0 > budget_ns) break;
-      }
-    }
-    *abort_flag = 1u;
-    return false;
-  } else {
-    return mbar_wait_slow(bar, parity, abort_flag, budget_ns);
-  }
-}
 __device__ __forceinline__ bool mbar_wait_budget(uint32_t bar, uint32_t parity, volatile uint32_t *abort_flag,
                                                  uint64_t budget_ns) {
-  return mbar_wait_sel<false>(bar, parity, abort_flag, budget_ns);
+  return mbar_try_wait(bar, parity) || mbar_wait_slow(bar, parity, abort_flag, budget_ns);
 }
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t *abort_flag) {
   return mbar_wait_budget(bar, parity, abort_flag, kWaitBudgetNs);
@@ -482,6 +462,15 @@ __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+// two fp32 fused multiply-adds in one instruction: the pipe's rate is the same, the issue slots are half
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
+      "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
 }
 __device__ __forceinline__ float lg2_approx(float x) {
   float y;
