@@ -402,10 +402,10 @@ DF_API int df_attn_set_variant(int variant);  /* per calling thread; returns the
 #define DF_OPT_BWD_OVERLAP 2     /* DF_ATTN_BWD_OVERLAP: 1 (default) block backward runs dQ on the thread's side stream      */
 #define DF_OPT_SCHED_TABLE 3     /* DF_ATTN_SCHED_TABLE: kept for callers; the forward no longer deals items out in advance   */
 #define DF_OPT_DISABLE_TENSOR 4  /* DF_ATTN_DISABLE_TENSOR: 1 = SIMT kernels only, 2 = SIMT backward only (default 0)        */
-#define DF_OPT_PDL 5             /* DF_ATTN_PDL: 1 (default) kernels are launched with programmatic stream serialization (each waits for
-                                    its predecessor before its first access to global memory), 0 = ordinary launches           */
-#define DF_OPT_CE_VARIANT 6      /* DF_CE_VARIANT: loss-head training kernel 0 = automatic, 1 = row resident in shared memory,
-                                    2 = two passes, the second out of L2 */
+#define DF_OPT_PDL 5             /* DF_ATTN_PDL: 1 (default) kernels are launched with programmatic stream serialization: each waits for its
+                                    predecessor before its first access to global memory, but for the second kernel of a backward,
+                                    which starts on SMs that the first has left and waits at its end. 0 = ordinary launches     */
+#define DF_OPT_CE_VARIANT 6      /* DF_CE_VARIANT: kept for callers; the loss head has one training kernel for rows that fit       */
 #define DF_OPT_LN_STAGED 7       /* DF_LN_STAGED: 1 (default) the LayerNorm backward stages its rows in shared memory with bulk
                                     copies when there are enough rows to fill the machine, 0 = rows in registers only          */
 #define DF_OPT_COUNT 8

@@ -31,7 +31,7 @@ def test_chunked_cross_entropy_matches_oracle(oracle, rows, cols, variant):
     import torch
     torch.cuda.set_device(0)
     p = pkg()
-    prev_variant = p.set_option(p.OPT_CE_VARIANT, variant)  # 1: row resident in shared memory, 2: second pass out of L2
+    prev_variant = p.set_option(p.OPT_CE_VARIANT, variant)  # values that callers may still set: the kernel is the same
     z, tg = _case(oracle, rows, cols, 600 + rows + cols)
     total = max(rows, 512)
     tz, tt = to_dev(z, tg)
