@@ -30,7 +30,7 @@
 namespace df {
 namespace {
 
-using ptx::ex2_approx;
+using ptx::ex2_approx;  // exponentials are taken as 2^x of scores scaled by scale * log2 e; maxima are in the same unit
 using ptx::fma2;
 
 constexpr int kCols = 64;      // loop-side rows (keys, or queries in the dK/dV part) per step
@@ -38,7 +38,6 @@ constexpr int NT = 128;        // threads of a group; a block is two groups
 constexpr int TX = 16, TY = 8; // a group's threads along the loop-side rows (and the head dimension), and along the resident rows
 constexpr int C = kCols / TX;
 
-// Exponentials are taken as 2^x of scores scaled by scale * log2 e; maxima are in the same unit.
 __device__ __forceinline__ int clamp_int(long long x) { return x > 1000 ? 1000 : (x < -1000 ? -1000 : (int)x); }
 __device__ __forceinline__ void cp16(uint32_t dst, const float *src, bool valid) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");

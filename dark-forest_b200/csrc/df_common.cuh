@@ -101,7 +101,7 @@ int tensor_backward_init();
 // caller's stream (and run them strictly one after the other).
 void tensor_backward_set_profile_events(cudaEvent_t *three_events);
 constexpr int kProfileReps = 4;  // launches of each kernel between the events of a profiled backward
-// Static schedule of the persistent kernels: work items are numbered heaviest first and dealt to the
+// Static schedule of the TF32 dQ kernel: work items are numbered heaviest first and dealt to the
 // `grid` CTAs in rounds, odd rounds in reverse CTA order ("snake"), which on the causal triangle
 // balances as well as a greedy longest-first assignment and needs no counter that concurrent
 // launches could share. Returns the item of CTA `cta` in round `r`, or -1 when its list is exhausted.

@@ -73,6 +73,8 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
 // flag is raised by another thread, after kWaitBudgetNs of wall time, or after a hard number of
 // polls, whichever comes first. On giving up it raises the abort flag so that every other role
 // of the CTA leaves its loops too, and the caller unwinds to the common teardown.
+// A wait names its phase by a parity, so it can only be made where the barrier cannot complete the phase after the one
+// waited for before the waiter has looked: that phase would look as if it had not come, and never come again.
 constexpr uint64_t kWaitBudgetNs = 2000000000ull;  // 2 s: far above any legitimate wait
 constexpr uint32_t kWaitMaxPolls = 1u << 28;
 
@@ -145,11 +147,13 @@ __device__ __forceinline__ void tc_fence_after_sync() {
 
 // ------------------------------------------------------------------ programmatic dependent launch
 // pdl_wait: blocks until every kernel this one depends on has completed and its writes are visible; a no-op in a kernel
-// that was launched the ordinary way. Every kernel that launch_kernel starts executes it in all threads before its first
-// access to global memory. No kernel triggers its dependents early (griddepcontrol.launch_dependents): the next kernel then
-// starts as this one's last blocks leave, which saves the 2 us between two kernels of a stream; triggered at the start
-// instead, its blocks sit on SMs that this kernel still wants (forward + backward of 12 heads, 1024 rows: 59 us this way, 65
-// with early triggers, 66 without programmatic launch).
+// that was launched the ordinary way. A kernel that launch_kernel starts executes it in all threads before its first access to global
+// memory. It starts as the last blocks of the kernel before it leave, which saves the 2 us between two kernels of a stream.
+// One kind of kernel is started earlier, by its predecessor's pdl_trigger, and does not wait first: the second kernel of a backward (`early`:
+// dK/dV behind the TF32 dQ kernel, dQ behind the bf16 dK/dV kernel). What it reads was written before the trigger, its launcher keeps it
+// from starting early where it would write what the first kernel still reads, and it waits at its end, so that whoever waits
+// for it waits for both. Triggers elsewhere cost time: blocks of the next kernel then sit on SMs that this one still wants (forward +
+// backward of 12 heads, 1024 rows: 59 us without, 65 with early triggers everywhere, 66 without programmatic launch).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Lets the dependent grid start where SMs have room, once every CTA of this grid has said so or ended.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -161,7 +161,7 @@ DF_API int df_attn_schedule_build(const uint32_t *weights, int n, int grid, uint
 DF_API uint64_t df_attn_workspace_bytes(int kind, uint32_t batch, uint32_t n_heads, uint32_t seq_len, uint32_t d_head,
                                  uint32_t chunk_size);
 
-/* Host-side view of the static work distribution of the persistent kernels (no GPU involved; no
+/* Host-side view of the static work distribution of the fp32 dQ kernel (no GPU involved; no
  * counterpart in the reference): the index of the work item that CTA `cta` of `grid` processes in
  * round `round` when `n_items` items are numbered heaviest first, or -1 past the end of its list. */
 DF_API long long df_attn_schedule_item(int round, int grid, int cta, long long n_items);

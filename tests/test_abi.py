@@ -77,7 +77,7 @@ def test_attention_context_mirrors_reference_checks():
 
 
 def test_persistent_schedule_covers_every_item_once_and_balances_the_causal_triangle():
-    """df_attn_schedule_item is the function the persistent kernels use to pick their work: every item must be
+    """df_attn_schedule_item is the function the fp32 dQ kernel uses to pick its work: every item must be
     taken exactly once, each CTA's list must be contiguous in rounds, and on causal workloads (items numbered
     heaviest first) the heaviest CTA must stay close to the average load."""
     import heapq
@@ -109,7 +109,7 @@ def test_persistent_schedule_covers_every_item_once_and_balances_the_causal_tria
             heapq.heappush(h, heapq.heappop(h) + w)
         return max(h)
 
-    # forward: pairs of query tiles of B*H heads, weight = key tiles of the later tile; backward: key tiles
+    # "fwd": pairs of query tiles of B*H heads, weight = key tiles of the later tile; "bwd": one tile per item
     cases = {"fwd S=1024 B*H=96": [2 * (4 - p) for p in range(4) for _ in range(96)],
              "fwd S=32768 B*H=12": [2 * (128 - p) for p in range(128) for _ in range(12)],
              "bwd S=1024 B*H=96": [8 - k for k in range(8) for _ in range(96)],
@@ -134,9 +134,8 @@ def test_workspace_sizes():
 
 
 def test_explicit_work_lists_cover_every_item_and_beat_the_round_robin_order():
-    """df_attn_schedule_build (the MULTIFIT assignment the persistent kernels receive for mid-sized causal
-    problems): every item exactly once, the heaviest CTA within 2 % of the average load where the round-robin
-    order is 12 % off, and no table where it would not help."""
+    """df_attn_schedule_build (a MULTIFIT assignment of weighted items to CTAs): every item exactly once, the heaviest
+    CTA within 2 % of the average load where the round-robin order is 12 % off, and no table where it would not help."""
     import ctypes
     L = pkg().lib()
 
@@ -148,7 +147,7 @@ def test_explicit_work_lists_cover_every_item_and_beat_the_round_robin_order():
                                         ctypes.cast(items, ctypes.c_void_p))
         return used, list(off), list(items)
 
-    # forward at S = 8192, B*H = 12: 32 pairs per head, weight 4 * key tiles + 3
+    # pairs of query tiles at S = 8192, B*H = 12: 32 pairs per head, weight 4 * key tiles + 3
     w = [4 * (2 * (31 - p) + 2) + 3 for p in range(32) for _ in range(12)]
     used, off, items = build(w, 148)
     assert used == 1 and off[0] == 0 and off[148] == len(w)

@@ -153,8 +153,8 @@ def test_simt_blocks_of_64_rows(torch_cuda, oracle, Sq, Sk, shift, D):
 @pytest.mark.parametrize("persist", [0, 2])
 @pytest.mark.parametrize("causal", [True, False])
 def test_shape_sweep_tensor_forward(torch_cuda, oracle, causal, persist):
-    """tcgen05 forward at D=64 over ragged and tile-aligned S, several batch/head counts, through both
-    whole-sequence kernels: one CTA per pair of query tiles (0) and the persistent one (2)."""
+    """tcgen05 forward at D=64 over ragged and tile-aligned S, several batch/head counts, with both kinds of
+    items: pairs of query tiles (0) and query tiles whose key tiles are split over the two slots (2)."""
     p = pkg()
     prev_opt = p.set_option(p.OPT_FWD_PERSIST, persist)
     prev = p.set_variant(p.VARIANT_TENSOR)
@@ -382,9 +382,8 @@ def test_unaligned_slices_fall_back_to_the_generic_kernels(torch_cuda, oracle):
 
 # ------------------------------------------------------------------ benchmark-size properties
 def test_long_sequence_forward_row_sample(torch_cuda, oracle):
-    """S = 8192, H = 12, D = 64 (the sweep's first point): sampled rows against float64, through the kernel the
-    launcher picks at this length (one CTA per pair of query tiles) and through the persistent kernel with its
-    host-computed work lists (option value 2)."""
+    """S = 8192, H = 12, D = 64 (the sweep's first point): sampled rows against float64, with the items the
+    launcher picks at this length (pairs of query tiles) and with split query tiles (option value 2)."""
     p = pkg()
     B, H, S, D = 1, 12, 8192, 64
     q, k, v, _ = _inputs(oracle, B, H, S, D, 0xDF03)
@@ -433,9 +432,8 @@ def test_benchmark_configuration_full_parity(torch_cuda, oracle):
 
 @pytest.mark.parametrize("S", [16384, 32768])
 def test_long_sequence_forward_backward_row_samples(torch_cuda, oracle, S):
-    """The kernels that only long sequences reach, against float64 on sampled rows: S = 16384 takes the
-    persistent forward with explicit work lists, S = 32768 the one-CTA-per-pair forward; both take the
-    persistent backward kernels over 128 / 256 tiles per head. Forward rows, dQ rows and dK/dV rows are
+    """Long sequences against float64 on sampled rows: forward items of up to 256 and 512 steps, of which every CTA takes
+    over several at run time, and the backward kernels over 128 / 256 tiles per head. Forward rows, dQ rows and dK/dV rows are
     sampled at both ends of the sequence (the heaviest and the lightest tiles) and at random in between."""
     p = pkg()
     B, H, D = 1, 12, 64
@@ -507,8 +505,7 @@ def test_block_backward_from_two_host_threads(torch_cuda, oracle):
 # ------------------------------------------------------------------ ring driver on the CUDA backend
 @pytest.mark.parametrize("B,S", [(8, 1024), (1, 32768)])
 def test_full_size_gradient_identities(torch_cuda, B, S):
-    """Benchmark-size checks that need no oracle (H = 12, D = 64; the step shape and a long sequence that
-    takes the non-persistent forward): O is linear in V, so sum(dV o V) = sum(dO o O) = sum(delta); the
+    """Benchmark-size checks that need no oracle (H = 12, D = 64; the step shape and a long sequence): O is linear in V, so sum(dV o V) = sum(dO o O) = sum(delta); the
     scores depend on Q and K only through their products, so sum(dQ o Q) = sum(dK o K); and lse, delta
     come back finite. Sums are taken in float64; the bound is three times the TF32 gradient tolerance times the
     scale of a sum of independent per-term errors, which a gradient that is off by a few per cent exceeds."""
