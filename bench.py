@@ -31,8 +31,8 @@ sys.path.insert(0, ROOT)
 CFG = dict(B=8, H=12, S=1024, D=64)
 # DRAM bytes (read + write) of one launch of each kernel of the step at exactly the benchmark size, from one ncu
 # capture; TRAFFIC_CAPTURE names the build the capture was taken from
-TRAFFIC = {"fwd": 91.9e6, "dq": 148.3e6, "dkdv": 125.7e6}
-TRAFFIC_CAPTURE = "ncu --set full of bench.py --kernel-case fwd / bwd --batch 8 --seq 1024, backward kernels as of commit 875fe8b, forward as of 4239d77 (unchanged since)"
+TRAFFIC = {"fwd": 81.2e6, "dq": 148.9e6, "dkdv": 126.2e6}
+TRAFFIC_CAPTURE = "ncu, dram__bytes_read.sum + dram__bytes_write.sum of bench.py --kernel-case fwd / bwd --batch 8 --seq 1024 --iters 3, kernels as of commit 6cf3b5b"
 METRIC = "causal_attention_fwd_bwd_tflops"
 UNIT = "TFLOP/s"
 
@@ -483,7 +483,7 @@ def run_ours(args):
                 "peak_source": "cuBLAS TF32 8192^3 burst (best of 10) measured in this run; 4 s sustained figure and half of "
                                f"MEASURED_PEAKS.json's bf16 burst ({peaks.get('bf16_tflops')} TFLOP/s {peak_kind}) in `peaks`",
                 "ms_per_launch": ms_dkdv,
-                "other_kernels": {"k_attn_fwd_tf32_d64": {"ms": ms_fwd, "tflops": fwd_tf, "frac": fwd_tf / tf32_peak,
+                "other_kernels": {"k_attn_fwd": {"ms": ms_fwd, "tflops": fwd_tf, "frac": fwd_tf / tf32_peak,
                                                                  "fracs": fracs(fwd_tf), "traffic": TRAFFIC["fwd"]},
                                   "k_attn_bwd_dq_tf32_d64": {"ms": ms_dq, "tflops": dq_tf, "frac": dq_tf / tf32_peak,
                                                              "fracs": fracs(dq_tf), "traffic": TRAFFIC["dq"],
@@ -1001,14 +1001,19 @@ def run_kernel_case(args):
         print(json.dumps(step_kernels_case(pkg, torch, dev, B * S, H * D, args.iters)))
         return
     q, k, v, go = (torch.randn((B, S, H * D), device=dev, generator=gen) for _ in range(4))
-    if args.kernel_case == "fwd_bf16":
-        qb, kb, vb = (x.to(torch.bfloat16) for x in (q, k, v))
+    if args.kernel_case in ("fwd_bf16", "bwd_bf16"):
+        qb, kb, vb, gb = (x.to(torch.bfloat16) for x in (q, k, v, go))
         ob, lb = pkg.forward_bf16(qb, kb, vb, H, scale, True)
+        delta = torch.empty((B, H, S), device=dev)
+        grads = [torch.empty_like(qb) for _ in range(3)]
         torch.cuda.synchronize()
         a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         a.record()
         for _ in range(args.iters):
-            pkg.forward_bf16(qb, kb, vb, H, scale, True, out=ob, lse=lb)
+            if args.kernel_case == "fwd_bf16":
+                pkg.forward_bf16(qb, kb, vb, H, scale, True, out=ob, lse=lb)
+            else:
+                pkg.backward_bf16(qb, kb, vb, ob, gb, lb, H, scale, True, d_q=grads[0], d_k=grads[1], d_v=grads[2], delta_buf=delta)
         b.record()
         torch.cuda.synchronize()
         assert pkg.sync_status() == 0
@@ -1460,7 +1465,7 @@ def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--workload", default="attention", choices=["attention", "gpt2_step", "ring", "long_forward"],
                     help="gpt2_step: the full-training-step configuration (attention time share); not the headline metric")
-    ap.add_argument("--kernel-case", default=None, choices=["fwd", "bwd", "delta", "fwd_bf16", "decode", "linear_qkv", "loss_ce", "step_kernels"],
+    ap.add_argument("--kernel-case", default=None, choices=["fwd", "bwd", "delta", "fwd_bf16", "bwd_bf16", "decode", "linear_qkv", "loss_ce", "step_kernels"],
                     help="run one kernel of the path a few times on a small case (for ncu) and exit")
     ap.add_argument("--seq", type=int, default=16384)
     ap.add_argument("--batch", type=int, default=1)

@@ -690,8 +690,9 @@ int adamw_update_multi(const df_adamw_tensor_t *tensors_device, uint32_t n_tenso
   const int n_sm = sm_count();
   if (n_sm <= 0) return DF_ERR_CUDA;
   // State that goes through DRAM (more than about 96 MB of it) streams best with a block per chunk: blocks start as others end
-  // and loads and stores stay mixed (GPT-2 small, 124 M parameters, the whole call: 540 to 564 us from box to box = 6.2 to 6.45 TB/s; 5 % more
-  // with a grid of 16 blocks per SM that walks the chunks, 615 to 631 before). What fits L2 is 5 % faster with the walking grid.
+  // and loads and stores stay mixed (GPT-2 small, 124 M parameters: 519 us = 6.7 TB/s for one call after another, 540 to 564 us where each
+  // call meets buffers that the one before did not touch; 5 % more with a grid of 16 blocks per SM that walks the chunks, 615 to 631 before).
+  // What fits L2 is 5 % faster with the walking grid.
   const uint64_t cap = total_chunks * kAdamChunk * 16 > (96ull << 20) ? 0x7fffffffull : (uint64_t)n_sm * 16;
   launch_kernel(k_adamw_multi, dim3((unsigned)(total_chunks < cap ? total_chunks : cap)), dim3(256), 0, s, tensors_device, n_tensors, total_chunks,
                                                                                     hyper(lr, beta1, beta2, eps, weight_decay, bc1, bc2));
