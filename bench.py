@@ -947,7 +947,7 @@ def linear_case(pkg, torch, dev, rows, d_model, iters):
 
 def decode_case(pkg, torch, dev, H, T, D, iters):
     """One-token decode over a contiguous fp32 KV cache of T tokens (HBM-bound: K and V are read once): the
-    scratch-free form (clusters of 8 CTAs per head) and the split form with caller scratch for chunk_size 256.
+    scratch-free form (clusters of CTAs per head) and the split form with caller scratch for chunk_size 256.
     Eight caches are rotated so that every launch reads from DRAM (8 x 2 x T x H x D x 4 bytes > L2 for T >= 4096)."""
     gen = torch.Generator(device=dev)
     gen.manual_seed(2)

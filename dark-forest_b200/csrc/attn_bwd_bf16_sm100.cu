@@ -10,11 +10,11 @@
 //     columns, and each compute thread packs into the first half of the columns it has itself read
 //     (columns [0,32) and [64,96)), so nobody overwrites scores another thread still needs;
 //   * head dimension 64 or 128 (template parameter); gradients are written as bf16.
-// What bounds it: at head dimension 128 the compute warps' two phases per step (tensor pipe 51 % busy), at 64 the same and the
+// What bounds it: at head dimension 128 the compute warps' two phases per step (tensor pipe 57 to 59 % of active cycles, S = 8192), at 64 the same and the
 // exponentials. The dQ kernel needs nothing of the dK/dV kernel and starts on SMs that it leaves. Backward on B200 with the delta
 // pass, causal, us: D = 64, H = 16, S = 8192 691 -> 580, 8 x 1024 (H = 12) 129 -> 115, S = 512 26.4 -> 15.8; D = 128 S = 8192 848 -> 836,
 // S = 2048 93 -> 78, S = 512 37 -> 24.
-// Every wait is bounded (mbar_wait); there is no TMA multicast.
+// Every wait is bounded (mbar_wait) and, in roles of whole warps, decided by the warp together; there is no TMA multicast.
 #include <math.h>
 
 #include "df_common.cuh"

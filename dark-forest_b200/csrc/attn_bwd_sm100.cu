@@ -31,7 +31,8 @@
 // a tile of the next item that it does not need.
 //
 // Inputs are rounded to TF32 by the TFLOAT32 tensor maps (nearest even); P and dS are rounded
-// with cvt.rna before they are written back to TMEM. Every wait is bounded (see mbar_wait).
+// with cvt.rna before they are written back to TMEM. Every wait is bounded (see mbar_wait) and,
+// in roles of whole warps, decided by the warp together.
 #include <math.h>
 #include <stdio.h>
 #include <stdlib.h>

@@ -5,7 +5,7 @@
 // scores wait for its last PV product and the softmax of a step lies on the critical path; so it does where a sequence is one
 // tile. Two threads per query row (sixteen softmax warps) halve that path. One thread per row measured 8-10 % slower at head
 // dimension 128 (B200, S = 8192, H = 12: causal 216 against 206 us, all keys 436 against 391 us) and 6.9 against 5.4 us at head
-// dimension 64 and S = 96. One CTA per pair of query tiles, heaviest first; that chain bounds it (tensor pipe 48 % busy).
+// dimension 64 and S = 96. One CTA per pair of query tiles, heaviest first; that chain bounds it (tensor pipe 57 % of active cycles, S = 16384).
 //   warp 16     TMA producer: Q_A, Q_B once, then K_j / V_j tiles (128 keys, 128-byte swizzled slabs) through two-stage rings
 //               released by MMA commits
 //   warp 17     MMA issuer, order PV_A(j) QK_A(j+1) PV_B(j) QK_B(j+1) ... One election per MMA: batches of nothing but MMAs, which

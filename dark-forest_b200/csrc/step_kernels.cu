@@ -14,7 +14,7 @@
 //    normalise) forward and twice backward, with two float atomics per ELEMENT for grad_gamma / grad_beta. Here a warp
 //    owns a row and keeps it in registers (a 768-wide row is six float4 per lane): one read and one write of the
 //    activations forward, two reads and one write backward; grad_gamma / grad_beta are summed in registers over all rows
-//    a warp sees, then in shared memory over the block, and reach global memory as one atomic per column and BLOCK.
+//    a warp sees, then in shared memory over the block, and reach global memory as one vector reduction per four columns and BLOCK.
 //  * GELU: 16-byte accesses; tanh through one exponential, 0.5 * (1 + tanh(u)) = 1 / (1 + exp(-2u)).
 //  * AdamW: the reference launches once per parameter tensor (196 launches for a 12-layer GPT-2 small, most of them over a few
 //    thousand elements). df_adamw_update_multi walks a caller-built table of tensors in ONE launch, in chunks of 2048
