@@ -1,5 +1,5 @@
-// attn_simt.cu - fp32 attention kernels for every shape the tcgen05 path does not take (any S, 1 <= D <= 128, any
-// alignment): odd head sizes, unaligned slices, tiny problems such as the S=5,D=4 and S=4,D=3 cases that the
+// attn_simt.cu - fp32 attention kernels for every shape the tensor-core kernels do not take (any S, 1 <= D <= 128, any
+// alignment): short sequences with head sizes other than 64 (longer ones: attn_split_sm100.cu), unaligned slices, tiny problems such as the S=5,D=4 and S=4,D=3 cases that the
 // reference's own unit tests use (darkforest-cuda/src/lib.rs:2606-2628, 2753-2769).
 //
 // Arithmetic follows the reference definition (attention_fused.cu:41-159 forward, :390-516 backward) in full fp32, not

@@ -87,6 +87,12 @@ int merge_partials(float *o_a, float *lse_a, const float *o_b, const float *lse_
                    uint32_t H, uint32_t S, uint32_t D, cudaStream_t s);
 int accumulate(float *dst, const float *src, uint64_t n, cudaStream_t s);
 
+// ---- fp32 in full precision on the tensor cores (attn_split_sm100.cu): head sizes without a TF32 kernel, from 193 keys on ----
+bool split_forward_wanted(const AttnParams &p);   // out, and lse if asked for; no row sums
+bool split_backward_wanted(const AttnParams &p);
+int split_forward(const AttnParams &p, cudaStream_t s);
+int split_backward(const AttnParams &p, cudaStream_t s);  // needs lse_in, delta_in
+
 // ---- tcgen05 kernels (attn_fwd_sm100.cu / attn_bwd_sm100.cu) ----
 bool tensor_forward_supported(const AttnParams &p);
 int tensor_forward(const AttnParams &p, cudaStream_t s);

@@ -388,7 +388,7 @@ DF_API int df_chunked_logit_ce(float *logits, const uint32_t *targets, float *gr
                         uint32_t cols, uint32_t total_rows, void *stream);
 
 /* ---- variant selection and status ---- */
-#define DF_VARIANT_AUTO 0     /* tensor-core kernel where the shape allows, SIMT otherwise */
+#define DF_VARIANT_AUTO 0     /* tensor-core kernel where the shape allows (TF32 at d_head 64, full fp32 by bf16 parts at others), SIMT otherwise */
 #define DF_VARIANT_SIMT 1     /* force the shape-generic SIMT kernels                      */
 #define DF_VARIANT_TENSOR 2   /* force the tcgen05 kernels; unsupported shapes return DF_ERR_UNSUPPORTED */
 DF_API int df_attn_set_variant(int variant);  /* per calling thread; returns the previous value */
@@ -401,7 +401,7 @@ DF_API int df_attn_set_variant(int variant);  /* per calling thread; returns the
 #define DF_OPT_FUSE_DELTA 1      /* DF_ATTN_FUSE_DELTA: 1 (default) the dQ kernel forms delta itself, 0 separate pre-pass    */
 #define DF_OPT_BWD_OVERLAP 2     /* DF_ATTN_BWD_OVERLAP: 1 (default) block backward runs dQ on the thread's side stream      */
 #define DF_OPT_SCHED_TABLE 3     /* DF_ATTN_SCHED_TABLE: kept for callers; the forward no longer deals items out in advance   */
-#define DF_OPT_DISABLE_TENSOR 4  /* DF_ATTN_DISABLE_TENSOR: 1 = SIMT kernels only, 2 = SIMT backward only (default 0)        */
+#define DF_OPT_DISABLE_TENSOR 4  /* DF_ATTN_DISABLE_TENSOR: 1 = fp32 SIMT kernels only, 2 = SIMT backward only (default 0)        */
 #define DF_OPT_PDL 5             /* DF_ATTN_PDL: 1 (default) kernels are launched with programmatic stream serialization: each waits for its
                                     predecessor before its first access to global memory, but for the second kernel of a backward,
                                     which starts on SMs that the first has left and waits at its end. 0 = ordinary launches     */

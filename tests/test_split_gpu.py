@@ -1,0 +1,61 @@
+"""fp32 attention on the tensor cores with operands cut into three bf16 parts (head sizes other than 64, four steps of 64 keys or more): the forms
+that its rules choose between, at the edges of its tiles, against float64. The bar is that of the other fp32 kernels, 2e-5 of the result's scale."""
+import pytest
+
+import helpers as hp
+from helpers import pkg, to_dev
+
+pytestmark = pytest.mark.gpu
+
+
+def _reference(torch, q, k, v, go, H, scale, causal, shift):
+    q4, k4, v4, g4 = (t.double().view(t.shape[0], t.shape[1], H, -1).transpose(1, 2) for t in (q, k, v, go))
+    s = q4 @ k4.transpose(2, 3) * scale
+    if causal:
+        hidden = torch.arange(k.shape[1], device="cuda")[None, :] > torch.arange(q.shape[1], device="cuda")[:, None] + shift
+        s = s.masked_fill(hidden, -torch.inf)
+    lse = torch.logsumexp(s, -1)
+    pr = torch.exp(s - torch.where(torch.isinf(lse), 0.0, lse)[..., None])
+    o = pr @ v4
+    ds = pr * (g4 @ v4.transpose(2, 3) - (g4 * o).sum(-1, keepdim=True))
+    back = lambda t: t.transpose(1, 2).reshape(t.shape[0], t.shape[2], -1)
+    return back(o), lse, back(ds @ k4 * scale), back(ds.transpose(2, 3) @ q4 * scale), back(pr.transpose(2, 3) @ g4)
+
+
+# B x H: one CTA a block, two (few blocks), four (very few, and eight steps). Sequences: just over four steps, whole tiles, a row more, keys ahead of
+# the queries, queries that see no key, all keys visible.
+@pytest.mark.parametrize("B,H,Sq,Sk,causal,shift", [
+    (8, 20, 193, 193, True, 0), (8, 20, 257, 257, True, 0), (4, 20, 130, 320, False, 0),
+    (2, 3, 193, 193, True, 0), (2, 3, 256, 256, True, 0), (2, 3, 100, 321, True, 221), (2, 3, 300, 420, True, -100), (2, 3, 321, 100, True, -150),
+    (1, 1, 449, 449, True, 0), (1, 2, 640, 640, False, 0)])
+@pytest.mark.parametrize("D", [4, 32, 36, 80, 96, 100, 128])
+def test_split_against_float64(B, H, Sq, Sk, causal, shift, D):
+    import torch
+    p = pkg()
+    from oracle.attn_oracle import Oracle
+    orc = Oracle()
+    q, go = (orc.fill_normal((B, Sq, H * D), 900 + Sq + D, i) for i in (0, 3))
+    k, v = (orc.fill_normal((B, Sk, H * D), 900 + Sq + D, i) for i in (1, 2))
+    q, k, v, go = to_dev(q, k, v, go)
+    scale = hp.default_scale(D)
+
+    def run():
+        out, lse = p.forward(q, k, v, H, scale, causal, causal_shift=shift)
+        delta = p.delta(out, go, H)
+        got = (out, lse) + tuple(p.backward_block(q, k, v, go, lse, delta, H, scale, causal, causal_shift=shift))
+        assert p.sync_status() == 0
+        return got
+
+    got, again = run(), run()
+    for got_t, again_t, ref, name in zip(got, again, _reference(torch, q, k, v, go, H, scale, causal, shift), ("out", "lse", "dq", "dk", "dv")):
+        assert torch.equal(got_t, again_t), name  # no atomics: the same bits every time
+        seen = torch.isfinite(ref)
+        assert torch.equal(torch.isfinite(got_t), seen), name
+        ref = torch.where(seen, ref, 0.0)
+        assert float((torch.where(seen, got_t, 0.0).double() - ref).abs().max()) <= 2e-5 * max(1.0, float(ref.abs().max())), name
+    prev = p.set_variant(p.VARIANT_SIMT)
+    try:
+        other = run()
+    finally:
+        p.set_variant(prev)
+    assert not torch.equal(got[4], other[4])  # dV: the rule did choose another kernel
