@@ -7,20 +7,21 @@
 // with no S x S scratch, no atomics (bit-reproducible) and no memsets: two kernels (a whole-sequence call runs
 // dQ first, which also forms delta, then dK/dV), each recomputing P tile by tile on the tensor cores.
 //
-// dK/dV kernel: a CTA owns 128 keys (TMEM lanes = keys) and walks the 128-query tiles that can see
-//   them.  S^T = K Q^T and dP^T = V dO^T are SS MMAs (both operands K-major in shared memory);
-//   eight compute warps (two per lane quarter, splitting the 128 query columns) turn S^T into P^T
-//   and dP^T into dS^T in place in TMEM; dV += P^T dO and dK += dS^T Q are TS MMAs whose B operand
-//   (dO, Q as [query, d]) is MN-major.  A 32-bit MN-major operand needs a different shared-memory
-//   swizzle (32-byte atoms) than a K-major one, so Q and dO tiles are fetched twice by TMA, once
-//   per layout, through four independently recycled buffers.
+// dK/dV kernel: a CTA owns 128 keys (TMEM lanes = keys) and walks the 128-query tiles that can see them.  K and V lie in tensor memory from an item's
+//   second step on: S^T = K Q^T and dP^T = V dO^T are TS MMAs over K-major tiles of Q and dO in rings of two (SS in the first step, so that nothing waits
+//   for the move); dV += P^T dO and dK += dS^T Q are TS MMAs whose B operand (dO, Q as [query, d]) is MN-major.  A 32-bit MN-major operand needs a
+//   different shared-memory swizzle (32-byte atoms) than a K-major one, so Q and dO tiles are fetched twice by TMA, once per layout.  The queries'
+//   statistics come in as one more K-step of the first two products: S^T - lse / scale, dP^T - delta.  A step's queries are two halves with barriers of
+//   their own: warps 0-3 turn one half's S^T into P^T and dP^T into dS^T in place in TMEM, warps 4-7 the other's, and neither group waits for the other.
+//   What bounds it: the compute warps, two of which share a scheduler. Of a step's 3.4 K cycles 3.1 K were theirs when they read the statistics from
+//   shared memory (a quarter of their time) and went in step; now it takes 2.7 K, of which the tensor pipe needs 2.2 K.
+//   Backward on B200, us, before / now: 8 x 12 x 1024 causal 115 / 109, 1 x 12 x 8192 669 / 577, 2 x 16 x 2000 all keys 228 / 203, 1 x 12 x 512 18.0 / 17.4.
 // dQ kernel: a CTA owns 128 queries (lanes = queries) and walks the key tiles they can see:
 //   S = Q K^T, dP = dO V^T (SS), dS in TMEM, dQ += dS K (TS, K tile MN-major: K is fetched twice).
 // MMA issue: tcgen05 MMAs of one thread execute in issue order, which is what lets single shared-memory stages
 // suffice. The dQ kernel has one MMA warp that interleaves the phases of consecutive tiles (.., S_{j+1}, dP_{j+1},
 // dQ_j, ..: dP has two buffers in tensor memory and runs a step ahead of dQ); the dK/dV kernel has one MMA warp per
-// product chain (dV_i, S_{i+2} and dK_i, dP_{i+1}: they share
-// nothing) and a second S^T buffer in tensor memory, so the tensor pipe has work while the compute warps are busy.
+// product chain (dV_i, S_{i+1} and dK_i, dP_{i+1}, each half by half: they share nothing).
 // An MMA role is run by all 32 lanes of its warp, warp-uniformly, with elect.sync around the tensor instructions.
 // Both kernels run a CTA's tiles as one uninterrupted pipeline, heaviest tiles first, and hand finished tiles to the copy engine
 // through shared memory. The dQ kernel deals its tiles out in advance; dK/dV CTAs take over tiles whose CTA has not started, and in a
@@ -50,13 +51,9 @@ using namespace ptx;
 constexpr int BT = 128;  // tile edge: keys per CTA / queries per step (and vice versa)
 constexpr int HD = 64;
 constexpr int kBwdThreads = 352;  // dQ kernel: warps 0-7 compute, 8-9 TMA producers, 10 MMA issuer
-// column groups of the dK/dV kernel's compute warps (2: 8 compute warps, 4: 16). Measured on the B200 with the same
-// inputs and bit-identical results: 16 warps (96 registers each, the MMA warp sharing its scheduler with four of
-// them) are 13 % slower than 8 (S = 16384: 1.59 ms against 1.40 ms).
-#ifndef DF_KV_NSUB
-#define DF_KV_NSUB 2
-#endif
-constexpr int kKvThreads = (4 * DF_KV_NSUB + 4) * 32;
+// dK/dV kernel: warps 0-7 compute (two groups of four, each with half of a step's queries), 8-9 TMA producers, 10-11 MMA issuers. With sixteen compute
+// warps (96 registers each, some spilled) it took 362 us where eight take 348 (1 x 12 x 8192, causal).
+constexpr int kKvThreads = 384;
 constexpr uint32_t kSlab = 128 * 128;
 constexpr uint32_t kTile = 2 * kSlab;
 constexpr uint32_t kTmemCols = 512;
@@ -84,7 +81,7 @@ struct BwdParams {
   float *delta_out;  // dQ kernel with fused row sums: delta = rowsum(dO o O) is computed there and written here
   float *dq, *dk, *dv;
   uint32_t B, H, Sq, Sk;
-  float scale, scale_log2;
+  float scale, scale_log2, inv_scale;
   int causal;
   long long shift;
   uint32_t zero_tiles;  // dK/dV: key tiles (times heads) beyond the items, which no query sees
@@ -119,16 +116,29 @@ __device__ __forceinline__ TileMN tile_mn(uint32_t tile_smem) {
   return t;
 }
 // To be called by the elected lane only.
-// 8 K-steps of a 128x128x64 SS MMA, both operands K-major tiles.
-__device__ __forceinline__ void batch_ss_128x128(uint32_t d_tmem, const TileK &a, const TileK &b, uint32_t idesc) {
-#pragma unroll
-  for (int kk = 0; kk < HD / 8; ++kk) mma_tf32_ss_lohi(d_tmem, a.lo[kk], a.hi, b.lo[kk], b.hi, idesc, kk > 0 ? 1u : 0u);
+// 32 lanes x 16 columns of tensor memory from 16 registers per thread
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+               "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
+               "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+               : "memory");
 }
-// 16 K-steps of a 128x64x128 TS MMA: A = 128 TMEM columns, B = MN-major tile.
-__device__ __forceinline__ void batch_ts_128x64(uint32_t d_tmem, uint32_t a_tmem, const TileMN &b, uint32_t idesc, bool accumulate) {
-  mma_tf32_ts_lohi(d_tmem, a_tmem, b.lo[0], b.hi, idesc, accumulate ? 1u : 0u);
+// 8 K-steps added to a 128x64x64 TS MMA: A = 64 TMEM columns, B = 64 rows of a K-major tile of a ring (off: their descriptor offset).
+__device__ __forceinline__ void batch_ts_scores(uint32_t d_tmem, uint32_t a_tmem, const TileK &b, uint32_t off, uint32_t idesc) {
 #pragma unroll
-  for (int kk = 1; kk < BT / 8; ++kk) mma_tf32_ts_lohi_acc(d_tmem, a_tmem + kk * 8, b.lo[kk], b.hi, idesc);
+  for (int kk = 0; kk < HD / 8; ++kk) mma_tf32_ts_lohi_acc(d_tmem, a_tmem + kk * 8, b.lo[kk] + off, b.hi, idesc);
+}
+// The same with A, a whole tile, in shared memory too: what an item's first step takes, before its K (V) is in tensor memory.
+__device__ __forceinline__ void batch_ss_scores(uint32_t d_tmem, const TileK &t, uint32_t a_off, uint32_t b_off, uint32_t idesc) {
+#pragma unroll
+  for (int kk = 0; kk < HD / 8; ++kk) mma_tf32_ss_lohi(d_tmem, t.lo[kk] + a_off, t.hi, t.lo[kk] + b_off, t.hi, idesc, 1u);
+}
+// 8 K-steps from FROM on (half) of a 128x64x128 TS MMA: A = 128 TMEM columns, B = MN-major tile.
+template <int FROM>
+__device__ __forceinline__ void batch_ts_128x64(uint32_t d_tmem, uint32_t a_tmem, const TileMN &b, uint32_t idesc, bool accumulate) {
+  mma_tf32_ts_lohi(d_tmem, a_tmem + FROM * 8, b.lo[FROM], b.hi, idesc, accumulate ? 1u : 0u);
+#pragma unroll
+  for (int kk = FROM + 1; kk < FROM + BT / 16; ++kk) mma_tf32_ts_lohi_acc(d_tmem, a_tmem + kk * 8, b.lo[kk], b.hi, idesc);
 }
 // The dQ kernel keeps the other form - all lanes call these, one lane is elected per MMA, the descriptor is base +
 // constant: with pure-MMA batches it measured 1.5 % faster at S = 1024 but 4 % slower at S = 16384 (the dK/dV kernel
@@ -157,38 +167,38 @@ __device__ __forceinline__ void load_tile(uint32_t dst, const CUtensorMap *m, ui
 __device__ __forceinline__ void store_cluster(uint32_t addr, float4 v) {
   asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
-// SPLIT kernels: one thread's N accumulator columns (one row) into the other CTA's staging tile of 128 rows of N floats, and
-// back as the sum with this CTA's own columns. 16-byte chunk c of row r sits at c ^ (r % 8).
-template <int N>
-__device__ __forceinline__ void send_row(uint32_t peer_tile, int row, uint32_t taddr) {
-#pragma unroll 1
-  for (int c = 0; c < N; c += 32) {
-    uint32_t rr[32];
-    tmem_ld32(taddr + c, rr);
-    tmem_wait_ld();
-#pragma unroll
-    for (int x = 0; x < 8; ++x)
-      store_cluster(peer_tile + row * (N * 4) + (uint32_t)((c / 4 + x) ^ (row & 7)) * 16,
-                    make_float4(__uint_as_float(rr[4 * x]), __uint_as_float(rr[4 * x + 1]), __uint_as_float(rr[4 * x + 2]), __uint_as_float(rr[4 * x + 3])));
-  }
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+                 "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+               : "r"(taddr)
+               : "memory");
 }
-template <int N>
-__device__ __forceinline__ void finish_row(const uint8_t *tile, int row, uint32_t taddr, bool own, bool other, float mul, float *dst, bool store) {
-#pragma unroll 1
-  for (int c = 0; c < N; c += 32) {
-    uint32_t rr[32];
-    tmem_ld32(taddr + c, rr);
-    tmem_wait_ld();
+// SPLIT kernels: 16 accumulator columns of a thread's row (dims d0 .. d0 + 15) into the other CTA's staging tile, which has the layout of the store's
+// tensor map (slabs of 32 dims, 16-byte chunk c of row r at c ^ (r % 8)), and there, in place, the sum with the finishing CTA's own columns.
+__device__ __forceinline__ void send_cols(uint32_t peer_tile, int row, int d0, uint32_t taddr) {
+  uint32_t rr[16];
+  tmem_ld16(taddr + d0, rr);
+  tmem_wait_ld();
 #pragma unroll
-    for (int x = 0; x < 8; ++x) {
-      float4 a = make_float4(__uint_as_float(rr[4 * x]), __uint_as_float(rr[4 * x + 1]), __uint_as_float(rr[4 * x + 2]), __uint_as_float(rr[4 * x + 3]));
-      if (!own) a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      if (other) {
-        const float4 b = *reinterpret_cast<const float4 *>(tile + row * (N * 4) + ((c / 4 + x) ^ (row & 7)) * 16);
-        a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
-      }
-      if (store) *reinterpret_cast<float4 *>(dst + c + 4 * x) = make_float4(a.x * mul, a.y * mul, a.z * mul, a.w * mul);
+  for (int x = 0; x < 4; ++x)
+    store_cluster(peer_tile + (uint32_t)(d0 >> 5) * kSlab + row * 128 + (uint32_t)((((d0 & 31) >> 2) + x) ^ (row & 7)) * 16,
+                  make_float4(__uint_as_float(rr[4 * x]), __uint_as_float(rr[4 * x + 1]), __uint_as_float(rr[4 * x + 2]), __uint_as_float(rr[4 * x + 3])));
+}
+__device__ __forceinline__ void finish_cols(uint8_t *tile, int row, int d0, uint32_t taddr, bool own, bool other, float mul) {
+  uint32_t rr[16];
+  tmem_ld16(taddr + d0, rr);
+  tmem_wait_ld();
+#pragma unroll
+  for (int x = 0; x < 4; ++x) {
+    float4 *at = reinterpret_cast<float4 *>(tile + (d0 >> 5) * kSlab + row * 128 + ((((d0 & 31) >> 2) + x) ^ (row & 7)) * 16);
+    float4 a = make_float4(__uint_as_float(rr[4 * x]), __uint_as_float(rr[4 * x + 1]), __uint_as_float(rr[4 * x + 2]), __uint_as_float(rr[4 * x + 3]));
+    if (!own) a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (other) {
+      const float4 b = *at;
+      a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
     }
+    *at = make_float4(a.x * mul, a.y * mul, a.z * mul, a.w * mul);
   }
 }
 
@@ -211,13 +221,17 @@ __device__ __forceinline__ int item_of_round(int r, int n_items) {
 constexpr int kClaims = 8;  // answers to item claims kept in shared memory (the roles are at most three items apart)
 
 namespace kv {
-enum Bar { K_FULL = 0, V_FULL, K_EMPTY, V_EMPTY, QK_FULL, GK_FULL, QM_FULL, GM_FULL, QM_EMPTY, GM_EMPTY,
-           S_FULL0, S_FULL1, DP_FULL, P_FULL0, P_FULL1, DS_FULL, STAT_FULL, ACC_FULL, EPI_FULL, DRAIN,
+// *_FULL / *_EMPTY of the Q and dO rings: + slot; of the MN-major tiles: + half of the rows; S_FULL .. DS_FULL: + half of the step's queries
+enum Bar { QK_FULL = 0, QK_EMPTY = 2, GK_FULL = 4, GK_EMPTY = 6, QM_FULL = 8, QM_EMPTY = 10, GM_FULL = 12, GM_EMPTY = 14,
+           S_FULL = 16, P_FULL = 18, DP_FULL = 20, DS_FULL = 22, K_READY = 24, V_READY, K_FREE, V_FREE, FIRST, ACC_FULL, EPI_FULL, DRAIN,
            CLAIM, NUM = CLAIM + kClaims };  // CLAIM + answer
-constexpr uint32_t kStats = 6 * kTile;             // lse2[3][128], delta[3][128]
-constexpr uint32_t kAnswers = kStats + 6 * 128 * 4;
+constexpr uint32_t kOnes = 6 * kTile;              // A of the statistics' K-step: 128 rows of (1, 1, 1, 0, 0, 0, 0, 0)
+constexpr uint32_t kStats = kOnes + BT * 32;       // B: [lse, delta][half of the queries][64 rows of 8]
+constexpr uint32_t kStatTile = BT / 2 * 32;
+constexpr uint32_t kAnswers = kStats + 4 * kStatTile;
 constexpr uint32_t kBars = kAnswers + kClaims * 16;
-constexpr uint32_t kSmemTotal = kBars + 320 + 1024;
+constexpr uint32_t kSmemTotal = kBars + 336 + 1024;
+static_assert(NUM * 8 <= 320, "barriers");
 
 // One work item: 128 keys of one head and the query tiles that can see them.
 struct Item {
@@ -242,14 +256,11 @@ __device__ __forceinline__ Item decode(const BwdParams &p, int idx) {
 }
 }  // namespace kv
 
-// NSUB = column groups of the compute warps: 4 * NSUB compute warps (warp w: TMEM lanes 32 * (w % 4).., query
-// columns (w / 4) * 128 / NSUB ..), then two producer warps and two MMA warps. (Which warp number issues the MMAs
-// makes no difference: with the MMA role on warp 0 instead of the last warp the kernel took the same time.)
 // SPLIT: a cluster of two CTAs shares an item. Each takes every other query tile; at the end rank 0 finishes dV and rank 1 dK, each
 // from its own accumulator and the other's, which comes through distributed shared memory. For problems whose items leave SMs
 // without work or are long against an SM's share (split_backward).
-template <int NSUB, bool SPLIT>
-__global__ void __launch_bounds__((4 * NSUB + 4) * 32, 1)
+template <bool SPLIT>
+__global__ void __launch_bounds__(kKvThreads, 1)
 k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                          const __grid_constant__ CUtensorMap tmQk, const __grid_constant__ CUtensorMap tmGk,
                          const __grid_constant__ CUtensorMap tmQm, const __grid_constant__ CUtensorMap tmGm,
@@ -258,18 +269,15 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
   using namespace kv;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const uint32_t aK = smem_u32(smem), aV = aK + kTile, aQk = aK + 2 * kTile, aGk = aK + 3 * kTile,
-                 aQm = aK + 4 * kTile, aGm = aK + 5 * kTile;
-  float *sLse2 = reinterpret_cast<float *>(smem + kStats);   // [3][128]
-  float *sDelta = sLse2 + 384;                               // [3][128]
+  const uint32_t aQk = smem_u32(smem), aGk = aQk + 2 * kTile, aQm = aQk + 4 * kTile, aGm = aQk + 5 * kTile;  // rings of two; MN-major tiles
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kBars);
-  volatile uint32_t *abort_flag = reinterpret_cast<volatile uint32_t *>(smem + kBars + 304);
-  uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(smem + kBars + 308);
+  volatile uint32_t *abort_flag = reinterpret_cast<volatile uint32_t *>(smem + kBars + 320);
+  uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(smem + kBars + 324);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr int kCW = 4 * NSUB;        // compute warps
+  constexpr int kCW = 8;               // compute warps
   constexpr int kArrivals = kCW * 32;  // every compute thread arrives (one arrival per warp measured the same)
-  constexpr int CPT = BT / NSUB;       // query columns per compute thread
+  constexpr int CPT = BT / 2;          // query columns per compute thread
   constexpr int NCH = CPT / 32;        // 32-column chunks per compute thread
   constexpr int kWarpLoadK = kCW, kWarpLoadM = kCW + 1, kWarpMma = kCW + 2, kWarpMma2 = kCW + 3, kWarpCompute0 = 0;
   const size_t dm = (size_t)p.H * HD;
@@ -306,28 +314,34 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
   };
   if (warp == kWarpLoadK) {
     for (int i = lane; i < NUM; i += 32)
-      mbar_init(bar(i), (i == P_FULL0 || i == P_FULL1 || i == DS_FULL || i == STAT_FULL || i == EPI_FULL) ? kArrivals : ((i == ACC_FULL || i == DRAIN) ? 2 : 1));
+      mbar_init(bar(i), (i == K_READY || i == V_READY || i == FIRST || i == EPI_FULL) ? kArrivals : (i == P_FULL || i == P_FULL + 1 || i == DS_FULL || i == DS_FULL + 1) ? kArrivals / 2 : ((i == ACC_FULL || i == DRAIN) ? 2 : 1));
     if (lane == 0) *abort_flag = 0;
     mbar_init_fence();
     __syncwarp();
     Item first;
     if (lane == 0 && take(0, &first)) {  // the first tiles are under way while the others set up
       if (!p.early) pdl_wait();
-      load_tile(aK, &tmK, bar(K_FULL), (int)first.h, (int)first.k0, (int)first.b);
-      load_tile(aQk, &tmQk, bar(QK_FULL), (int)first.h, (int)(first.i_begin * BT), (int)first.b);
+      load_tile(aQk, &tmK, bar(QK_FULL), (int)first.h, (int)first.k0, (int)first.b);
+      load_tile(aQk + kTile, &tmQk, bar(QK_FULL + 1), (int)first.h, (int)(first.i_begin * BT), (int)first.b);
+      load_tile(aGk, &tmV, bar(GK_FULL), (int)first.h, (int)first.k0, (int)first.b);
+      load_tile(aGk + kTile, &tmGk, bar(GK_FULL + 1), (int)first.h, (int)(first.i_begin * BT), (int)first.b);
     }
   }
   if (warp == kWarpMma) {
     tmem_alloc(smem_u32(tmem_holder), kTmemCols);
     tmem_relinquish();
   }
+  // 16-byte units of the statistics' operands, unswizzled: chunk c (of two) of row r at (r / 8) * 256 + c * 128 + (r % 8) * 16
+  if (warp < kCW) {
+    for (uint32_t u = threadIdx.x; u < (BT * 32 + 4 * kStatTile) / 16; u += kCW * 32)
+      *reinterpret_cast<float4 *>(smem + kOnes + u * 16) = u < BT * 2 && !(u & 8) ? make_float4(1.0f, 1.0f, 1.0f, 0.0f) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    fence_proxy_async_smem();
+  }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_holder;
-  // S^T / P^T is double-buffered (steps alternate between the two): S^T of step g+2 is issued as soon as dV of step g
-  // has been, two steps ahead of the compute warps, so they never wait for it
-  const uint32_t tS0 = tmem, tDP = tmem + 128, tDV = tmem + 256, tDK = tmem + 320, tS1 = tmem + 384;
+  const uint32_t tK = tmem, tV = tmem + 64, tS = tmem + 128, tDP = tmem + 256, tDV = tmem + 384, tDK = tmem + 448;
   if (!p.early) pdl_wait();  // everything above touched only this CTA's shared and tensor memory
 
   auto take_warp = [&](uint32_t k, Item *out) -> bool { return __all_sync(0xffffffffu, take(k, out)) != 0; };
@@ -335,56 +349,52 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
   // Counters every role keeps for itself: g = steps (query tiles) done over all items, n = items
   // done. A barrier used once per step is in phase g & 1, one used once per item in phase n & 1.
   if (warp == kWarpLoadK) {
-    // ---------------------------------------------- producer: K, V per item; K-major Q and dO tiles per step
+    // ---------------------------------------------- producer: rings of K-major tiles: an item's K (V), then Q (dO) of every step
     if (lane == 0) {
       Item cur;
-      uint32_t g = 0, n = 0;
-      for (; take(n, &cur); ++n) {
-        bool ok = true;
-        if (n > 0 && !mbar_wait(bar(K_EMPTY), (n - 1) & 1, abort_flag)) break;
-        // K and V land on barriers of their own: the next item's first S^T needs only K, and V can be replaced only
-        // after the item's last dP^T, a step later. On one barrier the S^T / dV warp stood waiting for V at the end of
-        // every item, with the item's last dV (whose P^T was ready) queued behind that wait: 2 K cycles per item.
-        if (n > 0) load_tile(aK, &tmK, bar(K_FULL), (int)cur.h, (int)cur.k0, (int)cur.b);  // the first: during set-up
-        for (int it = 0; it < cur.n_it; ++it, ++g) {
-          const int q0 = (int)((cur.i_begin + it * ST) * BT);
-          if (!SPLIT && it == (cur.n_it > 1 ? cur.n_it - 2 : 0)) {  // ask for the next item: S^T of its first step is due two steps before the end
+      uint32_t n = 0, r = 0;  // r: tiles of either ring so far
+      bool ok = true;
+      auto ring = [&](const CUtensorMap *mq, const CUtensorMap *mg, int row) {  // the next tile of both
+        const uint32_t slot = r & 1;
+        if (r > 1 && !mbar_wait(bar(QK_EMPTY + slot), ((r >> 1) - 1) & 1, abort_flag)) return false;
+        if (r > 1) load_tile(aQk + slot * kTile, mq, bar(QK_FULL + slot), (int)cur.h, row, (int)cur.b);  // the first two: during set-up
+        if (r > 1 && !mbar_wait(bar(GK_EMPTY + slot), ((r >> 1) - 1) & 1, abort_flag)) return false;
+        if (r > 1) load_tile(aGk + slot * kTile, mg, bar(GK_FULL + slot), (int)cur.h, row, (int)cur.b);
+        ++r;
+        return true;
+      };
+      for (; ok && take(n, &cur); ++n) {
+        ok = ring(&tmK, &tmV, (int)cur.k0);
+        for (int it = 0; ok && it < cur.n_it; ++it) {
+          if (!SPLIT && it == (cur.n_it > 1 ? cur.n_it - 2 : 0)) {  // ask for the next item: its K and V follow this item's last tiles
             const int c = (int)(n % kClaims);
             fence_proxy_async_smem();
             mbar_arrive_expect_tx(bar(CLAIM + c), 16);
             claim_request(smem_u32(smem) + kAnswers + 16 * c, bar(CLAIM + c));
           }
-          // the K-major Q (dO) buffer is free once the S^T (dP^T) product that read it has completed: the
-          // barrier that hands that product to the compute warps tells this thread too
-          if (g > 0 && !mbar_wait(bar(S_FULL0 + ((g - 1) & 1)), ((g - 1) >> 1) & 1, abort_flag)) { ok = false; break; }
-          if (g > 0) load_tile(aQk, &tmQk, bar(QK_FULL), (int)cur.h, q0, (int)cur.b);
-          if (it == 0) {  // V follows the item's first Q tile: that one, like K, does not have to wait for V's buffer
-            if (n > 0 && !mbar_wait(bar(V_EMPTY), (n - 1) & 1, abort_flag)) { ok = false; break; }
-            mbar_arrive_expect_tx(bar(V_FULL), kTile);
-            tma_load_4d(aV, &tmV, bar(V_FULL), 0, (int)cur.h, (int)cur.k0, (int)cur.b);
-            tma_load_4d(aV + kSlab, &tmV, bar(V_FULL), 32, (int)cur.h, (int)cur.k0, (int)cur.b);
-          }
-          if (g > 0 && !mbar_wait(bar(DP_FULL), (g - 1) & 1, abort_flag)) { ok = false; break; }
-          load_tile(aGk, &tmGk, bar(GK_FULL), (int)cur.h, q0, (int)cur.b);
+          ok = ring(&tmQk, &tmGk, (int)((cur.i_begin + it * ST) * BT));
         }
-        if (!ok) break;
       }
     }
   } else if (warp == kWarpLoadM) {
-    // ---------------------------------------------- producer: MN-major dO and Q tiles per step, result stores per item
+    // ---------------------------------------------- producer: MN-major dO and Q tiles per step in halves, result stores per item
     if (lane == 0) {
       Item cur;
       uint32_t g = 0, n = 0;
       for (; take(n, &cur); ++n) {
         bool ok = true;
-        for (int it = 0; it < cur.n_it; ++it, ++g) {
+        for (int it = 0; ok && it < cur.n_it; ++it, ++g) {
           const int q0 = (int)((cur.i_begin + it * ST) * BT);
-          // the MN-major dO (Q) buffer is released by a commit of its own right after dV (dK) of the step before:
-          // waiting for the next S^T (dP^T) product instead delayed these loads and measured 1-3 % slower
-          if (g > 0 && !mbar_wait(bar(GM_EMPTY), (g - 1) & 1, abort_flag)) { ok = false; break; }
-          load_tile(aGm, &tmGm, bar(GM_FULL), (int)cur.h, q0, (int)cur.b);
-          if (g > 0 && !mbar_wait(bar(QM_EMPTY), (g - 1) & 1, abort_flag)) { ok = false; break; }
-          load_tile(aQm, &tmQm, bar(QM_FULL), (int)cur.h, q0, (int)cur.b);
+          // A tile has one buffer. Its halves are released by commits of their own in the middle and at the end of the product that reads them, so
+          // the next step's first half is on its way while this step's second one is still read.
+          auto half = [&](int full, int empty, uint32_t dst, const CUtensorMap *m, int x) {
+            if (g > 0 && !mbar_wait(bar(empty + x), (g - 1) & 1, abort_flag)) return false;
+            mbar_arrive_expect_tx(bar(full + x), kTile / 2);
+            for (int sl = 0; sl < 2; ++sl) tma_load_4d(dst + sl * kSlab + x * (kSlab / 2), m, bar(full + x), 32 * sl, (int)cur.h, q0 + x * (BT / 2), (int)cur.b);
+            return true;
+          };
+          ok = half(GM_FULL, GM_EMPTY, aGm, &tmGm, 0) && half(GM_FULL, GM_EMPTY, aGm, &tmGm, 1) && half(QM_FULL, QM_EMPTY, aQm, &tmQm, 0) &&
+               half(QM_FULL, QM_EMPTY, aQm, &tmQm, 1);
         }
         if (SPLIT) break;
         // The compute warps stage the item's dV and dK tiles in these two buffers; this thread
@@ -402,144 +412,92 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
   } else if (warp == kWarpMma || warp == kWarpMma2) {
     // ---------------------------------------------- MMA issuers
     // The step's four products form two chains that share neither tensor memory nor operand buffers nor barriers:
-    //   warp kWarpMma :  .., dV_g (needs P_g), S_{g+2} (overwrites P^T_g after dV_g has read it), ..
+    //   warp kWarpMma :  .., dV_g (needs P_g), S_{g+1} (overwrites P^T_g after dV_g has read it), ..
     //   warp kWarpMma2:  .., dK_g (needs dS_g), dP_{g+1} (overwrites dS^T_g after dK_g has read it), ..
-    // Each chain has its own warp: MMAs of one thread execute in issue order, which is all a chain needs, and while
-    // one warp sits between two batches (poll, fence, the first MMA's start-up) the other's MMAs keep the tensor
-    // pipe busy. Step g+1 may belong to the next item (new K and V), so the pipe never drains between items.
+    // Each chain has its own warp: MMAs of one thread execute in issue order, which is all a chain needs, and while one warp sits between two batches
+    // (poll, fence, the first MMA's start-up) the other's MMAs keep the tensor pipe busy.
     // The whole warp runs its role; only the MMA and commit instructions are issued by one elected lane.
-    const uint32_t idesc_ss = make_idesc(kFmtTF32, BT, BT, 0, 0);
-    const uint32_t idesc_ts = make_idesc(kFmtTF32, BT, HD, 0, 1);
-    if (warp == kWarpMma) {
-      // ---- chain S / dV. S^T runs two steps ahead of dV: a cursor of its own walks the flat sequence of steps.
-      const TileK dA = tile_k(aK), dB = tile_k(aQk);
-      const TileMN dM = tile_mn(aGm);
-      Item s_item;
-      int s_it = 0;
-      uint32_t gs = 0, ns = 0;  // flat index and item ordinal of the next S^T to issue
-      bool s_more = take_warp(0, &s_item);
-      // S^T of the cursor's step, if there is one, into buffer gs & 1; false when a wait gave up
-      auto issue_next_s = [&]() -> bool {
-        if (s_more && s_it == s_item.n_it) {
-          s_more = take_warp(++ns, &s_item);
-          s_it = 0;
-        }
-        if (!s_more) return *abort_flag == 0u;
-        DF_BTRACE(0, 10);
-        if (s_it == 0) {  // first step of an item: its K tile must have landed
-          if (!mbar_wait_warp(bar(K_FULL), ns & 1, abort_flag)) return false;
-        }
-        if (!mbar_wait_warp(bar(QK_FULL), gs & 1, abort_flag)) return false;
+    const bool s_chain = warp == kWarpMma;
+    const uint32_t idesc_st = make_idesc(kFmtTF32, BT, BT / 2, 0, 0), idesc_ts = make_idesc(kFmtTF32, BT, HD, 0, 1);
+    const uint32_t tA = s_chain ? tK : tV, tX = s_chain ? tS : tDP, tR = s_chain ? tDV : tDK;
+    const int full = s_chain ? QK_FULL : GK_FULL, empty = s_chain ? QK_EMPTY : GK_EMPTY, ready = s_chain ? P_FULL : DS_FULL;
+    const int m_full = s_chain ? GM_FULL : QM_FULL, m_empty = s_chain ? GM_EMPTY : QM_EMPTY;
+    const TileK dB = tile_k(s_chain ? aQk : aGk);
+    const uint64_t dOnes = make_smem_desc(aQk + kOnes, 128, 256, kSwzNone), dStat = make_smem_desc(aQk + kStats + (s_chain ? 0 : 2 * kStatTile), 128, 256, kSwzNone);
+    const TileMN dM = tile_mn(s_chain ? aGm : aQm);
+    Item cur;
+    uint32_t g = 0, r = 0;
+    bool ok = true;
+    // S^T - lse / scale = K Q^T + 1 (-lse / scale), or dP^T - delta, for half h of the queries of the ring's next tile: the queries' statistics, cut in
+    // three TF32 parts, come in as one more K-step, so that the compute warps do not read them (they took a quarter of the warps' time)
+    // `frees`: the item's last, from tensor memory.
+    auto issue_first = [&](int h, bool from_smem, bool frees) -> bool {
+      const uint32_t slot = r & 1, b_off = slot * (kTile >> 4) + h * (kSlab / 2 >> 4);
+      if (h == 0) {
+        if (!mbar_wait_warp(bar(full + slot), (r >> 1) & 1, abort_flag)) return false;
         tc_fence_after_sync();
-        DF_BTRACE(0, 11);
-        if (elect_one()) {
-          batch_ss_128x128((gs & 1) ? tS1 : tS0, dA, dB, idesc_ss);
-          mma_commit(bar(S_FULL0 + (gs & 1)));
-          if (s_it + 1 == s_item.n_it) mma_commit(bar(K_EMPTY));  // last S^T of its item: K may be replaced
-        }
-        __syncwarp();
-        DF_BTRACE(0, 12);
-        ++gs;
-        ++s_it;
-        return true;
-      };
-      Item cur;
-      uint32_t g = 0;
-      bool ok = issue_next_s() && issue_next_s();
-      for (uint32_t n = 0; ok && take_warp(n, &cur); ++n) {
-        for (int it = 0; ok && it < cur.n_it; ++it, ++g) {
-          const bool last = it + 1 == cur.n_it;
-          DF_BTRACE(0, 30);
-          const uint32_t b = g & 1, ph2 = (g >> 1) & 1;
-          const uint32_t m = mbar_test3_warp(bar(P_FULL0 + b), ph2, bar(GM_FULL), b, bar(GM_FULL), b);
-          if ((!(m & 1u) && !mbar_wait_warp(bar(P_FULL0 + b), ph2, abort_flag)) || (!(m & 2u) && !mbar_wait_warp(bar(GM_FULL), b, abort_flag))) {
-            ok = false;
-            break;
-          }
-          DF_BTRACE(0, 31);
-          tc_fence_after_sync();
-          if (elect_one()) {
-            batch_ts_128x64(tDV, b ? tS1 : tS0, dM, idesc_ts, it > 0);  // dV += P^T dO
-            mma_commit(bar(GM_EMPTY));
-            if (last) mma_commit(bar(ACC_FULL));  // the second of its two arrivals completes the item's accumulators
-          }
-          __syncwarp();
-          DF_BTRACE(0, 32);
-          // S^T of step g+2 goes into the buffer dV_g has just been issued on (MMAs of one thread run in order)
-          if (!issue_next_s()) { ok = false; break; }
-        }
       }
-    } else {
-      // ---- chain dP / dK
-      const TileK dA = tile_k(aV), dB = tile_k(aGk);
-      const TileMN dM = tile_mn(aQm);
-      Item cur, nxt;
-      uint32_t g = 0, n = 0;
-      bool ok = take_warp(0, &cur);
-      // dP^T of step gs; `last` = last step of its item: V may then be replaced;
-      // `landed`: the caller has already seen the operand tile's barrier complete (and fenced after that)
-      auto issue_dp = [&](uint32_t gs, bool last, bool landed) -> bool {
-        if (!landed) {
-          if (!mbar_wait_warp(bar(GK_FULL), gs & 1, abort_flag)) return false;
-          tc_fence_after_sync();
-        }
-        if (elect_one()) {
-          batch_ss_128x128(tDP, dA, dB, idesc_ss);
-          mma_commit(bar(DP_FULL));
-          if (last) mma_commit(bar(V_EMPTY));
-        }
-        __syncwarp();
-        return true;
-      };
-      if (ok) ok = mbar_wait_warp(bar(V_FULL), 0, abort_flag);
-      if (ok) ok = issue_dp(0, cur.n_it == 1, false);
-      while (ok) {
-        bool more = true;
-        for (int it = 0; ok && it < cur.n_it; ++it, ++g) {
-          const bool last = it + 1 == cur.n_it;
-          if (last) more = take_warp(n + 1, &nxt);
-          const bool has_next = !last || more;
-          const bool next_last = last ? (nxt.n_it == 1) : (it + 2 == cur.n_it);
-          // One poll covers what dK_g needs and the operand tile of the product issued right after it; only a
-          // barrier that is still open is then waited for on its own.
-          const uint32_t ph = g & 1, phn = ph ^ 1;
-          const uint32_t m = mbar_test3_warp(bar(DS_FULL), ph, bar(QM_FULL), ph, bar(has_next ? GK_FULL : QM_FULL), has_next ? phn : ph);
-          if ((!(m & 1u) && !mbar_wait_warp(bar(DS_FULL), ph, abort_flag)) || (!(m & 2u) && !mbar_wait_warp(bar(QM_FULL), ph, abort_flag))) {
+      if (elect_one()) {
+        mma_tf32_ss(tX + h * (BT / 2), dOnes, dStat + h * (kStatTile >> 4), idesc_st, 0u);
+        if (from_smem) batch_ss_scores(tX + h * (BT / 2), dB, (slot ^ 1) * (kTile >> 4), b_off, idesc_st);
+        else batch_ts_scores(tX + h * (BT / 2), tA, dB, b_off, idesc_st);
+        mma_commit(bar((s_chain ? S_FULL : DP_FULL) + h));
+        if (h == 1) mma_commit(bar(empty + slot));
+        if (h == 1 && frees) mma_commit(bar(s_chain ? K_FREE : V_FREE));
+      }
+      __syncwarp();
+      if (h == 1) ++r;
+      return true;
+    };
+    uint32_t moved = 0;  // items whose K (V) went to tensor memory
+    for (uint32_t n = 0; ok && take_warp(n, &cur); ++n) {
+      const uint32_t slot = r & 1;  // K's, or V's
+      if (n == 0 && !mbar_wait_warp(bar(FIRST), 0, abort_flag)) break;  // the first statistics are staged
+      if (!mbar_wait_warp(bar(full + slot), (r >> 1) & 1, abort_flag)) break;
+      ++r;
+      ok = issue_first(0, true, false) && issue_first(1, true, false);
+      if (ok && cur.n_it > 1) {  // from the second step on K (V) is read from tensor memory
+        ok = mbar_wait_warp(bar(s_chain ? K_READY : V_READY), moved & 1, abort_flag);
+        ++moved;
+      }
+      commit_elected(bar(empty + slot));  // its ring slot is free once the first step's products are done
+      for (int it = 0; ok && it < cur.n_it; ++it, ++g) {
+        const bool last = it + 1 == cur.n_it;
+        const uint32_t ph = g & 1;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint32_t m = mbar_test3_warp(bar(ready + h), ph, bar(m_full + h), ph, bar(m_full + h), ph);
+          if ((!(m & 1u) && !mbar_wait_warp(bar(ready + h), ph, abort_flag)) || (!(m & 2u) && !mbar_wait_warp(bar(m_full + h), ph, abort_flag))) {
             ok = false;
             break;
           }
           tc_fence_after_sync();
-          if (elect_one()) {
-            batch_ts_128x64(tDK, tDP, dM, idesc_ts, it > 0);  // dK += dS^T Q
-            mma_commit(bar(QM_EMPTY));
-            if (last) mma_commit(bar(ACC_FULL));
+          if (elect_one()) {  // dV += P^T dO, or dK += dS^T Q, over this half of the queries
+            if (h == 0) batch_ts_128x64<0>(tR, tX, dM, idesc_ts, it > 0);
+            else batch_ts_128x64<BT / 16>(tR, tX, dM, idesc_ts, true);
+            mma_commit(bar(m_empty + h));
+            if (last && h == 1) mma_commit(bar(ACC_FULL));  // the second of its two arrivals completes the item's accumulators
           }
           __syncwarp();
-          if (has_next) {
-            if (last) {
-              if (!mbar_wait_warp(bar(V_FULL), (n + 1) & 1, abort_flag)) { ok = false; break; }
-              tc_fence_after_sync();
-            }
-            if (!issue_dp(g + 1, next_last, (m & 4u) != 0u)) { ok = false; break; }  // overwrites dS^T_g after dK_g has read it
+          if (!last && !issue_first(h, false, it + 2 == cur.n_it)) {
+            ok = false;
+            break;
           }
         }
-        if (!more) break;
-        cur = nxt;
-        ++n;
       }
     }
   } else {
     // ---------------------------------------------- compute warps: lanes = keys, columns = queries
     const int quarter = warp & 3, sub = (warp - kWarpCompute0) >> 2;
     const int row = quarter * 32 + lane;
-    const int tid = threadIdx.x - kWarpCompute0 * 32;  // 0 .. 128 * NSUB - 1
+    const int stat_q = sub * 64 + (row & 63);  // of the group's 64 queries: half of the threads fetch lse, the others delta
+    const bool stat_lse = row < 64;
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     const int col0 = sub * CPT;
     // result tiles: the first half of the column groups hands over dV, the second half scale * dK, each thread
     // kOutCols dims of its key row starting at out0
-    constexpr int kOutCols = HD / (NSUB / 2);
-    const bool is_dk = sub >= NSUB / 2;
-    const int out0 = (sub % (NSUB / 2)) * kOutCols;
+    constexpr int kOutCols = HD, out0 = 0;
+    const bool is_dk = sub != 0;
     // keys that no query sees (only with a causal shift or more keys than queries): dK = dV = 0. Item idx writes those tiles
     // beyond the items whose number is idx modulo the number of items.
     auto zero_unseen = [&](const Item &im) {
@@ -556,17 +514,21 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
     };
     // row statistics of a query tile: threads 0-127 fetch lse, 128-255 fetch delta (the others none)
     // The value comes back RAW: nothing is computed from it here, so the thread does not stall on the load; it is
-    // turned into what the phases use (`staged`) only when it is written to shared memory, a P phase later.
+    // turned into what the products use (`stage`) only when it is written to shared memory, a phase or two later.
     auto fetch_stat = [&](const Item &im, int it) -> float {
-      const long long q = (im.i_begin + it * ST) * BT + (tid & 127);
-      if (q >= (long long)p.Sq || tid >= 256) return (tid < 128) ? -INFINITY : 0.0f;
+      const long long q = (im.i_begin + it * ST) * BT + stat_q;
+      if (q >= (long long)p.Sq) return stat_lse ? -INFINITY : 0.0f;
       const size_t s_base = ((size_t)im.b * p.H + im.h) * p.Sq;
-      return __ldcg((tid < 128 ? p.lse : p.delta) + s_base + q);  // delta may still be being written when this kernel starts: not cached
+      return __ldcg((stat_lse ? p.lse : p.delta) + s_base + q);  // delta may still be being written when this kernel starts: not cached
     };
-    // lse in log2 units, +inf for a row without visible keys (P = 0); delta as it is
-    auto staged = [&](float raw) -> float {
-      if (tid >= 128) return raw;
-      return (raw == -INFINITY) ? INFINITY : raw * kLog2e;
+    // What the statistics' K-step adds, -lse / scale (-inf for a row without visible keys: P = 0) or -delta, in three TF32 parts
+    auto stage = [&](float raw) {
+      const float x = stat_lse ? -raw * p.inv_scale : -raw;
+      const bool none = stat_lse && raw == -INFINITY;
+      const float hi = none ? -INFINITY : __uint_as_float(cvt_rna_tf32(x)), rest = none ? 0.0f : x - hi, mid = __uint_as_float(cvt_rna_tf32(rest));
+      const uint32_t q = (uint32_t)row & 63;
+      *reinterpret_cast<float4 *>(smem + kStats + ((stat_lse ? 0 : 2) + sub) * kStatTile + (q >> 3) * 256 + (q & 7) * 16) = make_float4(hi, mid, rest - mid, 0.0f);
+      fence_proxy_async_smem();
     };
     // Hands the finished accumulators of the CTA's item number `nd` to the second producer thread: half of the column
     // groups hand over dV, the other half scale * dK. Every MMA of the item has finished by then, so
@@ -595,19 +557,38 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
       DF_BTRACE(1, 61);
       return true;
     };
+    // K (or V) of the CTA's next item from its ring (tile number r there) into tensor memory: as operand A from there it costs the shared-memory port
+    // nothing, and the 64 KB of the two hold a second tile of Q and dO. Items of one step go without. `moved`: items before it that did not.
+    auto load_resident = [&](bool v, uint32_t r, uint32_t moved) -> bool {
+      if (moved > 0 && !mbar_wait_warp(bar(v ? V_FREE : K_FREE), (moved - 1) & 1, abort_flag)) return false;
+      const uint32_t slot = r & 1;
+      if (!mbar_wait_warp(bar((v ? GK_FULL : QK_FULL) + slot), (r >> 1) & 1, abort_flag)) return false;
+      tc_fence_after_sync();
+      const uint8_t *src = smem + ((v ? 2 : 0) + slot) * kTile + sub * kSlab + row * 128;
+#pragma unroll 1
+      for (int c = 0; c < 8; c += 4) {
+        uint32_t rr[16];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const uint4 t = *reinterpret_cast<const uint4 *>(src + (((c + x) ^ (row & 7)) << 4));
+          rr[4 * x] = t.x; rr[4 * x + 1] = t.y; rr[4 * x + 2] = t.z; rr[4 * x + 3] = t.w;
+        }
+        tmem_st16((v ? tV : tK) + lane_base + sub * 32 + c * 4, rr);
+      }
+      tmem_wait_st();
+      tc_fence_before_sync();
+      mbar_arrive(bar(v ? V_READY : K_READY));
+      return true;
+    };
     Item cur, nxt;
-    uint32_t g = 0, n = 0, gb = 0;  // gb = g % 3: the statistics buffer of step g
+    uint32_t g = 0, n = 0, r = 0, moved = 0;  // r: the item's first tile in the rings; moved: items so far whose K and V went to tensor memory
     bool more = take_warp(0, &cur), ok = true;
-    // Row statistics of a step are staged in shared memory ONE STEP AHEAD, in one of three buffers, and published
-    // with a split barrier: every thread arrives in the middle of step g-1 (after its P phase) and waits at the
-    // start of step g, by which time the slowest thread has long arrived. A thread that has passed the wait of step
-    // g knows that all others are at least in step g-1, whose readers use buffers (g-1) % 3 and g % 3: writing buffer
-    // (g+1) % 3 in step g is safe. (A barrier every step, with arrival and wait back to back, cost a quarter of the
-    // compute warps' time: they all stood waiting for the slowest of them.)
+    // Row statistics of a step are staged one step ahead, in the one place there is: the score (dP) product of this step, which read it, is complete
+    // when the compute warps are at its result, and the next one follows their arrival on P_FULL (DS_FULL).
     if (more) {
-      const float s0 = staged(fetch_stat(cur, 0));
-      if (tid < 128) sLse2[tid] = s0; else if (tid < 256) sDelta[tid - 128] = s0;
-      mbar_arrive(bar(STAT_FULL));
+      stage(fetch_stat(cur, 0));
+      mbar_arrive(bar(FIRST));
+      if (cur.n_it > 1) ok = load_resident(false, 0, 0);
     }
     while (more && ok) {
       if (p.zero_tiles > 0) zero_unseen(cur);
@@ -615,22 +596,18 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
         const uint32_t ph = g & 1;
         const long long q0 = (cur.i_begin + it * ST) * BT;
         const long long kj = cur.k0 + row;
-        const float *lse2 = sLse2 + gb * 128, *dlt = sDelta + gb * 128;
-        const uint32_t gb_next = gb == 2 ? 0 : gb + 1;
-        // next step's statistics: loaded now, staged after the P phase below
+        // next step's statistics: loaded now, staged after the phases below
         const bool last = it + 1 == cur.n_it;
         if (last) more = take_warp(n + 1, &nxt);
         const bool has_next_step = !last || more;
         float stat_next = 0.0f;
         if (has_next_step) stat_next = last ? fetch_stat(nxt, 0) : fetch_stat(cur, it + 1);
-        if (!mbar_wait_warp(bar(STAT_FULL), ph, abort_flag)) { ok = false; break; }
         // visible iff key <= query + shift  <=>  column >= kj - shift - q0
         const bool need_mask = p.causal && (q0 + p.shift < cur.k0 + (BT - 1));
         long long cmin_ll = kj - p.shift - q0;
         const int cmin = !need_mask ? 0 : (cmin_ll > BT ? BT : (cmin_ll < 0 ? 0 : (int)cmin_ll));
         DF_BTRACE(1, 50);
-        const uint32_t tS = ph ? tS1 : tS0;
-        if (!mbar_wait_warp(bar(S_FULL0 + ph), (g >> 1) & 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(bar(S_FULL + sub), ph, abort_flag)) { ok = false; break; }
         DF_BTRACE(1, 51);
         tc_fence_after_sync();
         float pr[CPT];
@@ -646,33 +623,31 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
             for (int x = 0; x < 32; ++x)
               if (col0 + c * 32 + x < cmin) rr[x] = 0xff800000u;
           }
-          // the column statistics are the same for every lane: 128-bit broadcast reads
 #pragma unroll
-          for (int x4 = 0; x4 < 32; x4 += 4) {
-            const float4 l4 = *reinterpret_cast<const float4 *>(lse2 + col0 + c * 32 + x4);
-            const float lv[4] = {l4.x, l4.y, l4.z, l4.w};
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const int x = x4 + u;
-              // rounded with the low bits cleared, so that one register serves as the P^T operand of dV and as P for dS
-              // (keeping the unrounded value as well measured slower: 64 more live registers)
-              rr[x] = cvt_rna_tf32(ex2_approx(fmaf(__uint_as_float(rr[x]), p.scale_log2, -lv[u])));
-              pr[c * 32 + x] = __uint_as_float(rr[x]);
-            }
+          for (int x = 0; x < 32; x += 2) {
+            const float2 t = mul2(as_float2(rr[x], rr[x + 1]), make_float2(p.scale_log2, p.scale_log2));
+            // rounded with the low bits cleared, so that one register serves as the P^T operand of dV and as P for dS
+            // (keeping the unrounded value as well measured slower: 64 more live registers)
+            rr[x] = cvt_rna_tf32(ex2_approx(t.x));
+            rr[x + 1] = cvt_rna_tf32(ex2_approx(t.y));
+            pr[c * 32 + x] = __uint_as_float(rr[x]);
+            pr[c * 32 + x + 1] = __uint_as_float(rr[x + 1]);
           }
           tmem_st32(tS + lane_base + col0 + c * 32, rr);
         }
+        if (stat_lse && has_next_step) stage(stat_next);
         tmem_wait_st();
         tc_fence_before_sync();
-        mbar_arrive(bar(P_FULL0 + ph));
-        if (has_next_step) {
-          const float sn = staged(stat_next);
-          if (tid < 128) sLse2[gb_next * 128 + tid] = sn; else if (tid < 256) sDelta[gb_next * 128 + tid - 128] = sn;
-          mbar_arrive(bar(STAT_FULL));
-        }
-        gb = gb_next;
+        mbar_arrive(bar(P_FULL + sub));
         DF_BTRACE(1, 52);
-        if (!mbar_wait_warp(bar(DP_FULL), ph, abort_flag)) { ok = false; break; }
+        // the next item's K: its second step's scores follow soon after; and the very first item's V, which nobody waits for before this
+        if (last) r += cur.n_it + 1;
+        const bool first_v = g == 0 && cur.n_it > 1;
+        if (first_v || (!SPLIT && last && more && nxt.n_it > 1)) {
+          if (!load_resident(first_v, first_v ? 0 : r, moved)) { ok = false; break; }
+          if (first_v) ++moved;
+        }
+        if (!mbar_wait_warp(bar(DP_FULL + sub), ph, abort_flag)) { ok = false; break; }
         DF_BTRACE(1, 53);
         tc_fence_after_sync();
 #pragma unroll
@@ -681,26 +656,24 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
           tmem_ld32(tDP + lane_base + col0 + c * 32, rr);
           tmem_wait_ld();
 #pragma unroll
-          for (int x4 = 0; x4 < 32; x4 += 4) {
-            const float4 d4 = *reinterpret_cast<const float4 *>(dlt + col0 + c * 32 + x4);
-            const float dv[4] = {d4.x, d4.y, d4.z, d4.w};
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const int x = x4 + u;
-              rr[x] = tf32_rna_operand(pr[c * 32 + x] * (__uint_as_float(rr[x]) - dv[u]));
-            }
+          for (int x = 0; x < 32; x += 2) {
+            const float2 t = mul2(make_float2(pr[c * 32 + x], pr[c * 32 + x + 1]), as_float2(rr[x], rr[x + 1]));
+            rr[x] = tf32_rna_operand(t.x);
+            rr[x + 1] = tf32_rna_operand(t.y);
           }
           tmem_st32(tDP + lane_base + col0 + c * 32, rr);
         }
+        if (!stat_lse && has_next_step) stage(stat_next);
         tmem_wait_st();
         tc_fence_before_sync();
-        mbar_arrive(bar(DS_FULL));
+        mbar_arrive(bar(DS_FULL + sub));
         DF_BTRACE(1, 54);
       }
       if (SPLIT) {
         if (ok) ok = mbar_wait_warp(bar(ACC_FULL), n & 1, abort_flag);
         break;
       }
+      if (ok && more && nxt.n_it > 1) ok = load_resident(true, r, moved++);
       if (!ok || !hand_over(n)) { ok = false; break; }
       cur = nxt;
       ++n;
@@ -712,16 +685,25 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
     tc_fence_after_sync();
     const Item it = decode(p, (int)(blockIdx.x / 2));
     const bool own = it.n_it + 1 - (int)rank >= 2, other = it.n_it + (int)rank >= 2;
-    const int row = (warp & 3) * 32 + lane, sub = warp >> 2;  // sub 0 holds the thread's row of dV, sub 1 of dK
-    const uint32_t taddr = (sub ? tDK : tDV) + ((uint32_t)((warp & 3) * 32) << 16);
-    if (warp < kCW && sub != (int)rank && own) send_row<HD>(map_to_rank(aGm, rank ^ 1), row, taddr);
-    cluster_sync();
-    if (warp < kCW && sub == (int)rank) {
-      const long long kj = it.k0 + row;
-      const bool in = kj < (long long)p.Sk;
-      finish_row<HD>(smem + 5 * kTile, row, taddr, own, other, sub ? p.scale : 1.0f,
-                     (sub ? p.dk : p.dv) + ((size_t)it.b * p.Sk + (size_t)(in ? kj : 0)) * dm + it.h * HD, in);
+    // rank 0 finishes dV and rank 1 dK, in the buffer of the MN-major dO tile; the threads of a row have half of its columns each
+    const int row = (warp & 3) * 32 + lane, d0 = (warp >> 2) * 32;
+    const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16, t_own = (rank ? tDK : tDV) + lanes, t_send = (rank ? tDV : tDK) + lanes;
+    if (warp < kCW && own) {
+      send_cols(map_to_rank(aGm, rank ^ 1), row, d0, t_send);
+      send_cols(map_to_rank(aGm, rank ^ 1), row, d0 + 16, t_send);
     }
+    cluster_sync();
+    if (warp < kCW) {
+      finish_cols(smem + 5 * kTile, row, d0, t_own, own, other, rank ? p.scale : 1.0f);
+      finish_cols(smem + 5 * kTile, row, d0 + 16, t_own, own, other, rank ? p.scale : 1.0f);
+      fence_proxy_async_smem();
+      mbar_arrive(bar(EPI_FULL));
+    } else if (warp == kWarpLoadM && lane == 0 && mbar_wait(bar(EPI_FULL), 0, abort_flag)) {
+      for (int sl = 0; sl < 2; ++sl) tma_store_4d(rank ? &tmDK : &tmDV, aGm + sl * kSlab, 32 * sl, (int)it.h, (int)it.k0, (int)it.b);
+      tma_store_commit();
+      tma_store_wait_read_all();
+    }
+    __syncwarp();
     tc_fence_before_sync();
   }
   if (p.early) pdl_wait();  // whoever waits for this kernel waits for the dQ kernel too
@@ -1107,7 +1089,11 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
               if (!(key0 + col0 + c * 32 + x < kmax)) rr[x] = 0xff800000u;
           }
 #pragma unroll
-          for (int x = 0; x < 32; ++x) pr[c * 32 + x] = ex2_approx(fmaf(__uint_as_float(rr[x]), p.scale_log2, -lse2));
+          for (int x = 0; x < 32; x += 2) {
+            const float2 t = fma2(as_float2(rr[x], rr[x + 1]), make_float2(p.scale_log2, p.scale_log2), make_float2(-lse2, -lse2));
+            pr[c * 32 + x] = ex2_approx(t.x);
+            pr[c * 32 + x + 1] = ex2_approx(t.y);
+          }
         }
         tc_fence_before_sync();
         mbar_arrive(bar(S_FREE));
@@ -1122,7 +1108,11 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           tmem_ld32(tDP + lane_base + col0 + c * 32, rr);
           tmem_wait_ld();
 #pragma unroll
-          for (int x = 0; x < 32; ++x) rr[x] = tf32_rna_operand(pr[c * 32 + x] * (__uint_as_float(rr[x]) - dlt));
+          for (int x = 0; x < 32; x += 2) {
+            const float2 t = mul2(make_float2(pr[c * 32 + x], pr[c * 32 + x + 1]), add2(as_float2(rr[x], rr[x + 1]), make_float2(-dlt, -dlt)));
+            rr[x] = tf32_rna_operand(t.x);
+            rr[x + 1] = tf32_rna_operand(t.y);
+          }
           tmem_st32(tDP + lane_base + col0 + c * 32, rr);
         }
         tmem_wait_st();
@@ -1170,16 +1160,21 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     tc_fence_after_sync();
     const Item it = decode(p, (int)(blockIdx.x / 2), n_qt);
     const bool own = it.n_kv + 1 - rank >= 2, other = it.n_kv + rank >= 2;
-    const int row = (warp & 3) * 32 + lane, half = warp >> 2;
-    const uint32_t taddr = tDQ + half * 32 + ((uint32_t)((warp & 3) * 32) << 16);
-    if (warp < 8 && half != rank && own) send_row<32>(map_to_rank(aKm, (uint32_t)(rank ^ 1)), row, taddr);
+    // rank r finishes dims 32 r .. 32 r + 31, in a slab of the buffer of the MN-major K tile; the threads of a row have half of them each
+    const int row = (warp & 3) * 32 + lane, d_own = rank * 32 + (warp >> 2) * 16, d_send = (rank ^ 1) * 32 + (warp >> 2) * 16;
+    const uint32_t taddr = tDQ + ((uint32_t)((warp & 3) * 32) << 16);
+    if (warp < 8 && own) send_cols(map_to_rank(aKm, (uint32_t)(rank ^ 1)), row, d_send, taddr);
     cluster_sync();
-    if (warp < 8 && half == rank) {
-      const long long i = it.q0 + row;
-      const bool in = i < (long long)p.Sq;
-      finish_row<32>(smem + 4 * kTile, row, taddr, own, other, p.scale,
-                     p.dq + ((size_t)it.b * p.Sq + (size_t)(in ? i : 0)) * dm + it.h * HD + half * 32, in);
+    if (warp < 8) {
+      finish_cols(smem + 4 * kTile, row, d_own, taddr, own, other, p.scale);
+      fence_proxy_async_smem();
+      mbar_arrive(bar(EPI_FULL));
+    } else if (warp == 9 && lane == 0 && mbar_wait(bar(EPI_FULL), 0, abort_flag)) {
+      tma_store_4d(&tmDQ, aKm + rank * kSlab, 32 * rank, (int)it.h, (int)it.q0, (int)it.b);
+      tma_store_commit();
+      tma_store_wait_read_all();
     }
+    __syncwarp();
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -1208,7 +1203,7 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 bool tensor_backward_supported(const AttnParams &p) {
   if (option(DF_OPT_DISABLE_TENSOR) != 0) return false;
   if (p.D != HD || p.Sk == 0 || p.Sq == 0 || p.B == 0) return false;
-  if (!(p.scale > 0.0f) || !isfinite(p.scale)) return false;
+  if (!(p.scale > 0.0f) || !isfinite(p.scale) || !isfinite(1.0f / p.scale)) return false;
   const uintptr_t bits = reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k) |
                          reinterpret_cast<uintptr_t>(p.v) | reinterpret_cast<uintptr_t>(p.d_out) |
                          reinterpret_cast<uintptr_t>(p.d_q) | reinterpret_cast<uintptr_t>(p.d_k) |
@@ -1234,8 +1229,8 @@ int device_info(int *n_sm) {
   if (check_cuda(cudaGetDevice(&dev)) != DF_OK || dev < 0 || dev >= 64) return DF_ERR_CUDA;
   DeviceInfo &d = g_dev[dev];
   std::call_once(d.once, [&]() {
-    d.ok = cudaFuncSetAttribute(k_attn_bwd_dkdv_tf32_d64<DF_KV_NSUB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kv::kSmemTotal) == cudaSuccess &&
-           cudaFuncSetAttribute(k_attn_bwd_dkdv_tf32_d64<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kv::kSmemTotal) == cudaSuccess &&
+    d.ok = cudaFuncSetAttribute(k_attn_bwd_dkdv_tf32_d64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kv::kSmemTotal) == cudaSuccess &&
+           cudaFuncSetAttribute(k_attn_bwd_dkdv_tf32_d64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kv::kSmemTotal) == cudaSuccess &&
            cudaFuncSetAttribute(k_attn_bwd_dq_tf32_d64<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dq::kSmemTotal) == cudaSuccess &&
            cudaFuncSetAttribute(k_attn_bwd_dq_tf32_d64<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dq::kSmemTotal) == cudaSuccess &&
            cudaFuncSetAttribute(k_attn_bwd_dq_tf32_d64<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dq::kSmemTotal) == cudaSuccess &&
@@ -1310,9 +1305,9 @@ int tensor_backward(const AttnParams &p, cudaStream_t s) {
   if (!fuse && p.delta_in == nullptr) return DF_ERR_INVALID_ARG;
   CUtensorMap tmQk, tmQm, tmGk, tmGm, tmKk, tmKm, tmVk, tmDQ, tmDK, tmDV, tmO;
   if (!encode_head_tile_map(&tmQk, p.q, false, HD, p.B, p.H, p.Sq, BT, false) ||
-      !encode_head_tile_map(&tmQm, p.q, false, HD, p.B, p.H, p.Sq, BT, true) ||
+      !encode_head_tile_map(&tmQm, p.q, false, HD, p.B, p.H, p.Sq, BT / 2, true) ||
       !encode_head_tile_map(&tmGk, p.d_out, false, HD, p.B, p.H, p.Sq, BT, false) ||
-      !encode_head_tile_map(&tmGm, p.d_out, false, HD, p.B, p.H, p.Sq, BT, true) ||
+      !encode_head_tile_map(&tmGm, p.d_out, false, HD, p.B, p.H, p.Sq, BT / 2, true) ||
       !encode_head_tile_map(&tmKk, p.k, false, HD, p.B, p.H, p.Sk, BT, false) ||
       !encode_head_tile_map(&tmKm, p.k, false, HD, p.B, p.H, p.Sk, BT, true) ||
       !encode_head_tile_map(&tmVk, p.v, false, HD, p.B, p.H, p.Sk, BT, false) ||
@@ -1331,6 +1326,7 @@ int tensor_backward(const AttnParams &p, cudaStream_t s) {
   bp.B = p.B; bp.H = p.H; bp.Sq = p.Sq; bp.Sk = p.Sk;
   bp.scale = p.scale;
   bp.scale_log2 = p.scale * kLog2e;
+  bp.inv_scale = 1.0f / p.scale;
   bp.causal = p.causal;
   bp.shift = p.shift;
   bp.status = device_status_ptr();
@@ -1400,9 +1396,9 @@ int tensor_backward(const AttnParams &p, cudaStream_t s) {
       if (check_cuda(cudaMemsetAsync(p.d_k, 0, k_bytes, s)) != DF_OK || check_cuda(cudaMemsetAsync(p.d_v, 0, k_bytes, s)) != DF_OK) return DF_ERR_CUDA;
       continue;
     }
-    const cudaError_t e = split ? launch_clusters(k_attn_bwd_dkdv_tf32_d64<2, true>, 2, dim3(2 * items_kv), dim3(12 * 32), kv::kSmemTotal, s, tmKk,
+    const cudaError_t e = split ? launch_clusters(k_attn_bwd_dkdv_tf32_d64<true>, 2, dim3(2 * items_kv), dim3(kKvThreads), kv::kSmemTotal, s, tmKk,
                                                   tmVk, tmQk, tmGk, tmQm, tmGm, tmDK, tmDV, bp)
-                          : launch_kernel(k_attn_bwd_dkdv_tf32_d64<DF_KV_NSUB, false>, dim3(items_kv), dim3(kKvThreads), kv::kSmemTotal, s, tmKk, tmVk,
+                          : launch_kernel(k_attn_bwd_dkdv_tf32_d64<false>, dim3(items_kv), dim3(kKvThreads), kv::kSmemTotal, s, tmKk, tmVk,
                                         tmQk, tmGk, tmQm, tmGm, tmDK, tmDV, bp);
     note_launch();
 #if defined(DF_ATTN_TRACE) && !defined(DF_ATTN_TRACE_DQ)

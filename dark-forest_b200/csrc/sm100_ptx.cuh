@@ -432,6 +432,7 @@ __host__ __device__ constexpr uint32_t make_idesc(uint32_t fmt, uint32_t M, uint
 //   [46,48) version = 1 (Blackwell)   [61,64) layout type
 // Layout types used here:
 //   kSwz128      128-byte swizzle, 16-byte atoms (TMA SWIZZLE_128B): 16-byte chunk index XOR (row % 8).
+//   kSwzNone     none: core matrices of 8 rows x 16 bytes, 128 bytes each; LBO = from one to the next along K, SBO = along M/N
 //   kSwz128B32   128-byte swizzle, 32-byte atoms (TMA SWIZZLE_128B_ATOM_32B): 32-byte chunk index
 //                XOR (row % 4). The only layout a 32-bit (TF32) MN-major operand may use.
 // K-major operand (rows of 128 B along K): SBO = distance between 8-row groups (1024 B when
@@ -439,7 +440,7 @@ __host__ __device__ constexpr uint32_t make_idesc(uint32_t fmt, uint32_t M, uint
 // MN-major operand (rows of 128 B along M/N, one row per K index): LBO = distance between
 //   consecutive 128-byte chunks along M/N; SBO = distance between consecutive groups of K rows
 //   (8 rows = 1024 B for kSwz128, 4 rows = 512 B for kSwz128B32 when dense).
-enum : uint32_t { kSwz128 = 2, kSwz128B32 = 1 };
+enum : uint32_t { kSwzNone = 0, kSwz128 = 2, kSwz128B32 = 1 };
 __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes,
                                                    uint32_t layout_type) {
   const uint32_t lo = ((smem_addr & 0x3FFFFu) >> 4) | ((lbo_bytes >> 4) << 16);
@@ -467,7 +468,8 @@ __device__ __forceinline__ float ex2_approx(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// two fp32 fused multiply-adds in one instruction: the pipe's rate is the same, the issue slots are half
+// Two fp32 operations in one instruction: the pipe's rate is the same, the issue slots are half. Compute phases of the attention kernels have two or three
+// warps per scheduler and are bound by how fast one warp issues.
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   float2 d;
   asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
@@ -476,6 +478,21 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
       : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
   return d;
 }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tadd.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmul.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 as_float2(uint32_t x, uint32_t y) { return make_float2(__uint_as_float(x), __uint_as_float(y)); }
 __device__ __forceinline__ float lg2_approx(float x) {
   float y;
   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

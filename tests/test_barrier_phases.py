@@ -1,8 +1,9 @@
-"""Barrier phases of the dQ kernels, on the CPU.
+"""Barrier phases of the backward kernels, on the CPU.
 
 A wait on an mbarrier names a phase by its parity, so a waiter must never be two phases behind: the phase it waits for would look
-as if it had not come yet, and never come again. The roles of a kernel are written down here as the waits and arrivals they
-make; for every wait of every role, that role is held there while all others run as far as they can.
+as if it had not come yet, and never come again. Nor may it come two phases early: the phase before the last would pass for the one it
+waits for. The roles of a kernel are written down here as the waits and arrivals they make; for every wait of every role, that role is held
+there while all others run as far as they can, and for every arrival the arriving role is held ahead of it.
 """
 import os
 import re
@@ -136,8 +137,98 @@ def dq_bf16(n_kv, ds_bars, ring=4):
     return {"load_k": load_k, "load_v": load_v, "scores": scores, "dp_dq": dp_dq, "compute 0": compute, "compute 1": compute}
 
 
-def phases_missed(roles):
-    """(role, barrier, phase) of every wait that can find its barrier two phases on; fails when a role does not reach its end."""
+def dkdv_tf32(items):
+    """k_attn_bwd_dkdv_tf32_d64 for a CTA with items of that many query tiles: each group of compute warps has half of a step's queries."""
+    load_k, load_m = Role(), Role()
+    steps = [(n, i) for n, n_it in enumerate(items) for i in range(n_it)]
+    last = [i + 1 == items[n] for n, i in steps]
+    first_tile = [sum(items[:n]) + n for n in range(len(items) + 1)]  # of an item in the rings: its K (V)
+    for r in range(first_tile[-1]):
+        for tile in ("QK", "GK"):
+            if r > 1:
+                load_k.wait("%s_EMPTY%d" % (tile, r % 2), r // 2 - 1)
+            load_k.arrive("%s_FULL%d" % (tile, r % 2))
+    for g, (n, i) in enumerate(steps):
+        for tile in ("GM", "QM"):
+            for h in range(2):
+                if g > 0:
+                    load_m.wait("%s_EMPTY%d" % (tile, h), g - 1)
+                load_m.arrive("%s_FULL%d" % (tile, h))
+        if last[g]:
+            load_m.wait("EPI_FULL", n)
+
+    moved = [sum(n_it > 1 for n_it in items[:n]) for n in range(len(items) + 1)]  # items before whose K and V went to tensor memory
+
+    def chain(ring, kv, scores, ready, tile):
+        role = Role()
+
+        def first(h, r, frees):
+            if h == 0:
+                role.wait("%s_FULL%d" % (ring, r % 2), r // 2)
+            role.arrive("%s%d" % (scores, h))
+            if h == 1:
+                role.arrive("%s_EMPTY%d" % (ring, r % 2))
+                if frees:
+                    role.arrive(kv + "_FREE")
+
+        g = 0
+        role.wait("FIRST", 0)
+        for n, n_it in enumerate(items):
+            r = first_tile[n]
+            role.wait("%s_FULL%d" % (ring, r % 2), r // 2)
+            first(0, r + 1, False)
+            first(1, r + 1, False)
+            if n_it > 1:
+                role.wait(kv + "_READY", moved[n])
+            role.arrive("%s_EMPTY%d" % (ring, r % 2))
+            for i in range(n_it):
+                for h in range(2):
+                    role.wait("%s%d" % (ready, h), g)
+                    role.wait("%s_FULL%d" % (tile, h), g)
+                    role.arrive("%s_EMPTY%d" % (tile, h))
+                    if i + 1 == n_it and h == 1:
+                        role.arrive("ACC_FULL")
+                    if i + 1 < n_it:
+                        first(h, r + 2 + i, i + 2 == n_it)
+                g += 1
+        return role
+
+    def group(h):
+        role = Role()
+
+        def resident(ring, kv, n):
+            if n < len(items) and items[n] > 1:
+                if moved[n] > 0:
+                    role.wait(kv + "_FREE", moved[n] - 1)
+                role.wait("%s_FULL%d" % (ring, first_tile[n] % 2), first_tile[n] // 2)
+                role.arrive(kv + "_READY")
+
+        role.arrive("FIRST")
+        resident("QK", "K", 0)
+        for g, (n, i) in enumerate(steps):
+            role.wait("S_FULL%d" % h, g)
+            role.arrive("P_FULL%d" % h)
+            if last[g]:
+                resident("QK", "K", n + 1)
+            elif g == 0:
+                resident("GK", "V", 0)
+            role.wait("DP_FULL%d" % h, g)
+            role.arrive("DS_FULL%d" % h)
+            if last[g]:
+                resident("GK", "V", n + 1)
+                role.wait("ACC_FULL", n)
+                role.arrive("EPI_FULL")
+        return role
+
+    roles = {"load_k": load_k, "load_m": load_m, "s_dv": chain("QK", "K", "S_FULL", "P_FULL", "GM"),
+             "dp_dk": chain("GK", "V", "DP_FULL", "DS_FULL", "QM")}
+    for h in range(2):
+        for x in "ab":
+            roles["group %d %s" % (h, x)] = group(h)
+    return roles
+
+
+def _runner(roles):
     counts = {}
     for name, role in roles.items():
         for op, bar, _ in role:
@@ -145,6 +236,7 @@ def phases_missed(roles):
                 counts.setdefault(bar, set()).add(name)
 
     def run(held=None, at=None):
+        """Everybody as far as they can, `held` not past its entry `at`: positions and completed phases."""
         pos, arrived = dict.fromkeys(roles, 0), dict.fromkeys(counts, 0)
         moved = True
         while moved:
@@ -160,6 +252,12 @@ def phases_missed(roles):
                     moved = True
         return pos, {b: arrived[b] // len(counts[b]) for b in counts}
 
+    return run
+
+
+def phases_missed(roles):
+    """(role, barrier, phase) of every wait that can find its barrier two phases on; fails when a role does not reach its end."""
+    run = _runner(roles)
     pos, _ = run()
     assert all(pos[name] == len(role) for name, role in roles.items()), pos
     missed = []
@@ -168,6 +266,22 @@ def phases_missed(roles):
             if op == "wait" and run(name, at)[1][bar] > phase + 1:
                 missed.append((name, bar, phase))
     return missed
+
+
+def phases_early(roles):
+    """(role, barrier, phase) of every wait that can come while the phase before the one it names is still open."""
+    run = _runner(roles)
+    early = set()
+    for held, role in roles.items():
+        done = {}
+        for at, (op, bar, _) in enumerate(role):
+            if op != "arrive":
+                continue
+            open_phase = done[bar] = done.get(bar, -1) + 1  # held ahead of its arrival, this phase stays open
+            pos, _ = run(held, at)
+            for name, other in roles.items():
+                early |= {(name, b, ph) for b, ph in ((b, ph) for o, b, ph in other[:pos[name] + 1] if o == "wait") if b == bar and ph == open_phase + 1}
+    return early
 
 
 def test_one_barrier_for_two_buffers_is_missed():
@@ -181,6 +295,14 @@ def test_tf32_dq_waits_see_every_phase(items):
         enum = re.search(r"namespace dq \{\s*enum Bar \{(.*?)\}", f.read(), re.S).group(1)
     ds_bars = len(re.findall(r"\bDS_FULL\d?\b", enum))
     assert phases_missed(dq_tf32(items, ds_bars)) == []
+    assert phases_early(dq_tf32(items, ds_bars)) == set()
+
+
+@pytest.mark.parametrize("items", [[1], [2], [1, 1, 1], [5, 2, 1, 3], [4, 3]])
+def test_tf32_dkdv_waits_see_their_phase(items):
+    roles = dkdv_tf32(items)
+    assert phases_missed(roles) == []
+    assert phases_early(roles) == set()
 
 
 @pytest.mark.parametrize("n_kv", [1, 2, 3, 9])
