@@ -10,10 +10,11 @@
 //     columns, and each compute thread packs into the first half of the columns it has itself read
 //     (columns [0,32) and [64,96)), so nobody overwrites scores another thread still needs;
 //   * head dimension 64 or 128 (template parameter); gradients are written as bf16.
-// What bounds it: at head dimension 128 the compute warps' two phases per step (tensor pipe 57 to 59 % of active cycles, S = 8192), at 64 the same and the
-// exponentials. The dQ kernel needs nothing of the dK/dV kernel and starts on SMs that it leaves. Backward on B200 with the delta
-// pass, causal, us: D = 64, H = 16, S = 8192 691 -> 580, 8 x 1024 (H = 12) 129 -> 115, S = 512 26.4 -> 15.8; D = 128 S = 8192 848 -> 836,
-// S = 2048 93 -> 78, S = 512 37 -> 24.
+// What bounds it: the compute warps' two phases per step. Hence fp32 arithmetic two elements at a time, and in the dK/dV kernel the queries' statistics
+// (lse / scale and delta, three bf16 parts each) as one more K-step of the products, S^T - lse / scale and dP^T - delta, instead of shared-memory reads for
+// every element. The dQ kernel needs nothing of the dK/dV kernel and starts on SMs that it leaves. Backward on B200 with the delta pass, causal, us, with
+// scalar arithmetic and the reads / now: D = 64, 1 x 16 x 8192 615 / 537, 8 x 12 x 1024 121 / 114, 2 x 12 x 700 21.5 / 20.3; D = 128, 1 x 16 x 8192 911 / 860,
+// 1 x 16 x 2048 73.6 / 70.7, 4 x 8 x 2000 all keys 249 / 236.
 // Every wait is bounded (mbar_wait) and, in roles of whole warps, decided by the warp together; there is no TMA multicast.
 #include <math.h>
 
@@ -34,7 +35,7 @@ struct Bwd16Params {
   const float *delta;
   void *dq, *dk, *dv;   // bf16 or fp32 elements, see Cfg16::OUT_F32
   uint32_t B, H, Sq, Sk;
-  float scale, scale_log2;
+  float scale, scale_log2, inv_scale;
   int causal;
   long long shift;
   int early;  // the dQ kernel begins where the dK/dV kernel leaves SMs and waits for it at its end
@@ -64,11 +65,11 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 // The issue helpers are called by ALL lanes of the MMA warp; one elected lane issues each instruction (see elect_one).
 // [128 x 128] = A[128 x HD] * B[128 x HD]^T, both K-major tiles of kSlabs 128-byte slabs.
 template <class C>
-__device__ __forceinline__ void issue_ss(uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t idesc) {
+__device__ __forceinline__ void issue_ss(uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t idesc, bool accumulate = false) {
 #pragma unroll
   for (int kk = 0; kk < C::kKSteps; ++kk) {
     const uint64_t off = (uint64_t)(((kk >> 2) * kSlab + (kk & 3) * 32) >> 4);
-    if (elect_one()) mma_f16_ss(d_tmem, da + off, db + off, idesc, kk > 0);
+    if (elect_one()) mma_f16_ss(d_tmem, da + off, db + off, idesc, accumulate || kk > 0);
   }
 }
 // [128 x HD] (+)= A[128 x 128 packed bf16 in TMEM] * B[128 rows (K) x HD (N), MN-major].
@@ -111,9 +112,11 @@ __device__ __forceinline__ void store_bf16x32(uint8_t *dst, const uint32_t (&r)[
 namespace kv16 {
 enum Bar { KV_FULL = 0, Q_FULL = 1, Q_EMPTY = 5, G_FULL = 9, G_EMPTY = 13,   // + ring stage
            S_FULL = 17, P_FULL = 19,                                         // + S^T buffer
-           DP_FULL = 21, DS_FULL, STAT_FULL, ACC_FULL, DRAIN, NUM };
-template <class C> __host__ __device__ constexpr uint32_t stats_off() { return (2 + 2 * C::kRing) * C::kTile; }   // K, V, Q ring, dO ring
-template <class C> __host__ __device__ constexpr uint32_t bars_off() { return stats_off<C>() + 6 * 128 * 4; }
+           DP_FULL = 21, DS_FULL, FIRST, ACC_FULL, DRAIN, NUM };
+constexpr uint32_t kOperand = BT * 32;  // 128 rows of 16 bf16: A of the statistics' K-step, (1, 1, 1, 0, ..) in every row, or B, a query's statistic in three parts
+template <class C> __host__ __device__ constexpr uint32_t ones_off() { return (2 + 2 * C::kRing) * C::kTile; }   // K, V, Q ring, dO ring
+template <class C> __host__ __device__ constexpr uint32_t stats_off() { return ones_off<C>() + kOperand; }       // lse per S^T buffer, delta
+template <class C> __host__ __device__ constexpr uint32_t bars_off() { return stats_off<C>() + (C::kSBufs + 1) * kOperand; }
 template <class C> __host__ __device__ constexpr uint32_t smem_total() { return bars_off<C>() + 256 + 1024; }
 }  // namespace kv16
 
@@ -127,8 +130,6 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t aK = smem_u32(smem), aV = aK + kTile, aQ = aK + 2 * kTile, aG = aQ + C::kRing * kTile;  // rings: + stage * kTile
-  float *sLse2 = reinterpret_cast<float *>(smem + stats_off<C>());
-  float *sDelta = sLse2 + 384;   // both [3][128]
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + bars_off<C>());
   volatile uint32_t *abort_flag = reinterpret_cast<volatile uint32_t *>(smem + bars_off<C>() + 224);
   uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(smem + bars_off<C>() + 228);
@@ -163,7 +164,7 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
   if (warp == 8) {
     static_assert(NUM <= 32, "a lane per barrier");
     if (lane < NUM) {
-      const bool compute = lane == P_FULL || lane == P_FULL + 1 || lane == DS_FULL || lane == STAT_FULL;
+      const bool compute = lane == P_FULL || lane == P_FULL + 1 || lane == DS_FULL || lane == FIRST;
       // a Q (dO) tile is read by a product of either issuer; both have to be done with it
       const bool both = (lane >= Q_EMPTY && lane < Q_EMPTY + 4) || (lane >= G_EMPTY && lane < G_EMPTY + 4) || lane == ACC_FULL || lane == DRAIN;
       mbar_init(bar(lane), compute ? 256 : both ? C::kIssuers : 1);
@@ -183,6 +184,12 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
   if (warp == 10) {
     tmem_alloc(smem_u32(tmem_holder), kTmemCols);
     tmem_relinquish();
+  }
+  // unswizzled operands: 16-byte chunk c (of two) of row r at (r / 8) * 256 + c * 128 + (r % 8) * 16
+  if (warp < 8) {
+    for (uint32_t u = threadIdx.x; u < (C::kSBufs + 2) * kOperand / 16; u += 256)
+      *reinterpret_cast<uint4 *>(smem + ones_off<C>() + u * 16) = u < kOperand / 16 && !(u & 8) ? make_uint4(0x3f803f80u, 0x00003f80u, 0u, 0u) : make_uint4(0u, 0u, 0u, 0u);
+    fence_proxy_async_smem();
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -223,13 +230,17 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
     const uint64_t dK = make_smem_desc(aK, 16, 1024, kSwz128), dV = make_smem_desc(aV, 16, 1024, kSwz128);
     const uint64_t dQk = make_smem_desc(aQ, 16, 1024, kSwz128), dGk = make_smem_desc(aG, 16, 1024, kSwz128);
     const uint64_t dQm = make_smem_desc(aQ, kSlab, 1024, kSwz128), dGm = make_smem_desc(aG, kSlab, 1024, kSwz128);
+    const uint64_t dOnes = make_smem_desc(aK + ones_off<C>(), 128, 256, kSwzNone), dStat = make_smem_desc(aK + stats_off<C>(), 128, 256, kSwzNone);
+    const uint32_t stat_dp = C::kSBufs * (kOperand >> 4);
+    // S^T - lse / scale, dP^T - delta: the queries' statistics come in as one more K-step, so that the compute warps do not read them
     auto scores = [&](bool chain_s, int it) -> bool {
       const int st = it % C::kRing;
       const uint64_t off = (uint64_t)(st * (kTile >> 4));
       if (!mbar_wait_warp(bar((chain_s ? Q_FULL : G_FULL) + st), (it / C::kRing) & 1, abort_flag)) return false;
       tc_fence_after_sync();
       const bool second = C::kSBufs == 2 && (it & 1);
-      issue_ss<C>(chain_s ? (second ? tS1 : tS0) : tDP, chain_s ? dK : dV, (chain_s ? dQk : dGk) + off, idesc_ss);
+      if (elect_one()) mma_f16_ss(chain_s ? (second ? tS1 : tS0) : tDP, dOnes, dStat + (chain_s ? (second ? kOperand >> 4 : 0u) : stat_dp), idesc_ss, 0u);
+      issue_ss<C>(chain_s ? (second ? tS1 : tS0) : tDP, chain_s ? dK : dV, (chain_s ? dQk : dGk) + off, idesc_ss, true);
       commit_elected(bar(chain_s ? S_FULL + (second ? 1 : 0) : DP_FULL));
       if (C::kIssuers == 2) commit_elected(bar((chain_s ? Q_EMPTY : G_EMPTY) + st));
       return true;
@@ -246,7 +257,7 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
       commit_elected(bar((chain_s ? G_EMPTY : Q_EMPTY) + st));  // one issuer: the score product of this tile came before
       return true;
     };
-    bool ok = mbar_wait_warp(bar(KV_FULL), 0, abort_flag);
+    bool ok = mbar_wait_warp(bar(KV_FULL), 0, abort_flag) && mbar_wait_warp(bar(FIRST), 0, abort_flag);
     if (C::kIssuers == 2) {
       const bool chain_s = warp == 10;
       const int ahead = chain_s ? C::kSBufs : 1;
@@ -272,32 +283,37 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     const int col0 = half * 64;
     const size_t s_base = ((size_t)b * p.H + h) * p.Sq;
+    // A query's statistic for the K-step of its product, in three bf16 parts: -lse / scale (-inf for a row without visible keys: P = 0) from warps 0-3,
+    // -delta from warps 4-7. Fetched raw at the start of a step, staged behind its phase: the product that read the place before is complete
+    // then (S^T has a place per buffer), and the next one follows this thread's arrival on P_FULL (DS_FULL).
+    const bool stat_lse = half == 0;
     auto fetch_stat = [&](int it) -> float {
-      const long long q = (i_begin + it) * BT + (tid & 127);
-      if (it >= n_it || q >= (long long)p.Sq) return (tid < 128) ? INFINITY : 0.0f;
-      if (tid < 128) {
-        const float v = __ldg(p.lse + s_base + q);
-        return (v == -INFINITY) ? INFINITY : v * kLog2e;
+      const long long q = (i_begin + it) * BT + row;
+      if (it >= n_it || q >= (long long)p.Sq) return stat_lse ? -INFINITY : 0.0f;
+      return __ldg((stat_lse ? p.lse : p.delta) + s_base + q);
+    };
+    auto stage_stat = [&](int it, float raw) {
+      float x = stat_lse ? -raw * p.inv_scale : -raw;
+      const bool none = stat_lse && fabsf(raw) == INFINITY;
+      uint32_t part[3];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {  // each part takes the leading bits that the one before left: exact
+        part[i] = __float_as_uint(x) & 0xffff0000u;
+        x -= __uint_as_float(part[i]);
       }
-      return __ldg(p.delta + s_base + q);
+      const uint32_t place = stat_lse ? (uint32_t)(it % C::kSBufs) : (uint32_t)C::kSBufs;
+      *reinterpret_cast<uint4 *>(smem + stats_off<C>() + place * kOperand + (row >> 3) * 256 + (row & 7) * 16) =
+          none ? make_uint4(0x0000ff80u, 0u, 0u, 0u) : make_uint4((part[0] >> 16) | part[1], part[2] >> 16, 0u, 0u);
+      fence_proxy_async_smem();
     };
-    // Row statistics are staged one step ahead in one of three buffers and published by a split barrier: every thread arrives in
-    // the middle of step i-1 and waits at the start of step i. A thread past that wait knows the others are at least in step i-1,
-    // whose readers use buffers (i-1) % 3 and i % 3, so writing (i+1) % 3 in step i is safe.
-    auto stage_stat = [&](int buf, float v) {
-      if (tid < 128) sLse2[buf * 128 + tid] = v; else sDelta[buf * 128 + tid - 128] = v;
-      mbar_arrive(bar(STAT_FULL));
-    };
-    stage_stat(0, fetch_stat(0));
+    const int ahead = stat_lse ? C::kSBufs : 1;  // of its product
+    for (int it = 0; it < ahead && it < n_it; ++it) stage_stat(it, fetch_stat(it));
+    mbar_arrive(bar(FIRST));
     bool ok = true;
-    int sb = 0;
     for (int it = 0; it < n_it; ++it) {
       const uint32_t ph = it & 1;
       const long long q0 = (i_begin + it) * BT;
-      const float *lse2 = sLse2 + sb * 128, *dlt = sDelta + sb * 128;
-      sb = sb == 2 ? 0 : sb + 1;
-      const float stat_next = fetch_stat(it + 1);
-      if (!mbar_wait_warp(bar(STAT_FULL), ph, abort_flag)) { ok = false; break; }
+      const float stat_next = fetch_stat(it + ahead);
       const bool need_mask = p.causal && (q0 + p.shift < k0 + (BT - 1));
       const long long cmin_ll = kj - p.shift - q0;  // visible iff column >= cmin
       const int cmin = !need_mask ? 0 : (cmin_ll > BT ? BT : (cmin_ll < 0 ? 0 : (int)cmin_ll));
@@ -319,23 +335,20 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
           for (int x = 0; x < 32; ++x)
             if (col0 + c * 32 + x < cmin) r[x] = 0xff800000u;
         }
-        // the column statistics are the same for every lane: 128-bit broadcast reads
 #pragma unroll
-        for (int x4 = 0; x4 < 32; x4 += 4) {
-          const float4 l4 = *reinterpret_cast<const float4 *>(lse2 + col0 + c * 32 + x4);
-          pr[c * 32 + x4] = ex2_approx(fmaf(__uint_as_float(r[x4]), p.scale_log2, -l4.x));
-          pr[c * 32 + x4 + 1] = ex2_approx(fmaf(__uint_as_float(r[x4 + 1]), p.scale_log2, -l4.y));
-          pr[c * 32 + x4 + 2] = ex2_approx(fmaf(__uint_as_float(r[x4 + 2]), p.scale_log2, -l4.z));
-          pr[c * 32 + x4 + 3] = ex2_approx(fmaf(__uint_as_float(r[x4 + 3]), p.scale_log2, -l4.w));
+        for (int x = 0; x < 32; x += 2) {
+          const float2 t = mul2(as_float2(r[x], r[x + 1]), make_float2(p.scale_log2, p.scale_log2));
+          pr[c * 32 + x] = ex2_approx(t.x);
+          pr[c * 32 + x + 1] = ex2_approx(t.y);
         }
 #pragma unroll
         for (int x = 0; x < 16; ++x) packed[c * 16 + x] = pack2(pr[c * 32 + 2 * x], pr[c * 32 + 2 * x + 1]);
       }
       tmem_st32(tS + lane_base + col0, packed);  // packed P^T over the first half of this thread's own columns
+      if (stat_lse && it + ahead < n_it) stage_stat(it + ahead, stat_next);
       tmem_wait_st();
       tc_fence_before_sync();
       mbar_arrive(bar(P_FULL + (second ? 1 : 0)));
-      if (it + 1 < n_it) stage_stat(sb, stat_next);
       if (!mbar_wait_warp(bar(DP_FULL), ph, abort_flag)) { ok = false; break; }
       tc_fence_after_sync();
 #pragma unroll
@@ -344,15 +357,13 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
         tmem_ld32(tDP + lane_base + col0 + c * 32, r);
         tmem_wait_ld();
 #pragma unroll
-        for (int x4 = 0; x4 < 32; x4 += 4) {
-          const float4 d4 = *reinterpret_cast<const float4 *>(dlt + col0 + c * 32 + x4);
-          packed[c * 16 + x4 / 2] = pack2(pr[c * 32 + x4] * (__uint_as_float(r[x4]) - d4.x),
-                                          pr[c * 32 + x4 + 1] * (__uint_as_float(r[x4 + 1]) - d4.y));
-          packed[c * 16 + x4 / 2 + 1] = pack2(pr[c * 32 + x4 + 2] * (__uint_as_float(r[x4 + 2]) - d4.z),
-                                              pr[c * 32 + x4 + 3] * (__uint_as_float(r[x4 + 3]) - d4.w));
+        for (int x = 0; x < 16; ++x) {
+          const float2 t = mul2(make_float2(pr[c * 32 + 2 * x], pr[c * 32 + 2 * x + 1]), as_float2(r[2 * x], r[2 * x + 1]));
+          packed[c * 16 + x] = pack2(t.x, t.y);
         }
       }
       tmem_st32(tDP + lane_base + col0, packed);
+      if (!stat_lse && it + ahead < n_it) stage_stat(it + ahead, stat_next);
       tmem_wait_st();
       tc_fence_before_sync();
       mbar_arrive(bar(DS_FULL));
@@ -615,7 +626,11 @@ k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             if (!(key0 + col0 + c * 32 + x < kmax)) r[x] = 0xff800000u;
         }
 #pragma unroll
-        for (int x = 0; x < 32; ++x) pr[c * 32 + x] = ex2_approx(fmaf(__uint_as_float(r[x]), p.scale_log2, -lse2));
+        for (int x = 0; x < 32; x += 2) {
+          const float2 t = fma2(as_float2(r[x], r[x + 1]), make_float2(p.scale_log2, p.scale_log2), make_float2(-lse2, -lse2));
+          pr[c * 32 + x] = ex2_approx(t.x);
+          pr[c * 32 + x + 1] = ex2_approx(t.y);
+        }
       }
       tc_fence_before_sync();
       mbar_arrive(bar(S_FREE));
@@ -629,9 +644,10 @@ k_attn_bwd_dq_bf16(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tmem_ld32(tDP + lane_base + col0 + c * 32, r);
         tmem_wait_ld();
 #pragma unroll
-        for (int x = 0; x < 16; ++x)
-          packed[c * 16 + x] = pack2(pr[c * 32 + 2 * x] * (__uint_as_float(r[2 * x]) - dlt),
-                                     pr[c * 32 + 2 * x + 1] * (__uint_as_float(r[2 * x + 1]) - dlt));
+        for (int x = 0; x < 16; ++x) {
+          const float2 t = mul2(make_float2(pr[c * 32 + 2 * x], pr[c * 32 + 2 * x + 1]), add2(as_float2(r[2 * x], r[2 * x + 1]), make_float2(-dlt, -dlt)));
+          packed[c * 16 + x] = pack2(t.x, t.y);
+        }
       }
       tmem_st32(tDP + lane_base + col0, packed);
       tmem_wait_st();
@@ -759,6 +775,7 @@ int launch_backward(const AttnParams &p, cudaStream_t s) {
   bp.B = p.B; bp.H = p.H; bp.Sq = p.Sq; bp.Sk = p.Sk;
   bp.scale = p.scale;
   bp.scale_log2 = p.scale * kLog2e;
+  bp.inv_scale = 1.0f / fmaxf(p.scale, 1e-34f);  // finite, and so is its product with a logsumexp; scores times a smaller scale are zero anyway
   bp.causal = p.causal;
   bp.shift = p.shift;
   bp.status = device_status_ptr();

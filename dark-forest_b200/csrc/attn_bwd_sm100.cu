@@ -524,7 +524,7 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
     // What the statistics' K-step adds, -lse / scale (-inf for a row without visible keys: P = 0) or -delta, in three TF32 parts
     auto stage = [&](float raw) {
       const float x = stat_lse ? -raw * p.inv_scale : -raw;
-      const bool none = stat_lse && raw == -INFINITY;
+      const bool none = stat_lse && fabsf(raw) == INFINITY;
       const float hi = none ? -INFINITY : __uint_as_float(cvt_rna_tf32(x)), rest = none ? 0.0f : x - hi, mid = __uint_as_float(cvt_rna_tf32(rest));
       const uint32_t q = (uint32_t)row & 63;
       *reinterpret_cast<float4 *>(smem + kStats + ((stat_lse ? 0 : 2) + sub) * kStatTile + (q >> 3) * 256 + (q & 7) * 16) = make_float4(hi, mid, rest - mid, 0.0f);
@@ -1203,7 +1203,7 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 bool tensor_backward_supported(const AttnParams &p) {
   if (option(DF_OPT_DISABLE_TENSOR) != 0) return false;
   if (p.D != HD || p.Sk == 0 || p.Sq == 0 || p.B == 0) return false;
-  if (!(p.scale > 0.0f) || !isfinite(p.scale) || !isfinite(1.0f / p.scale)) return false;
+  if (!(p.scale > 0.0f) || !isfinite(p.scale) || p.scale < 1e-34f) return false;  // lse / scale is finite
   const uintptr_t bits = reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k) |
                          reinterpret_cast<uintptr_t>(p.v) | reinterpret_cast<uintptr_t>(p.d_out) |
                          reinterpret_cast<uintptr_t>(p.d_q) | reinterpret_cast<uintptr_t>(p.d_k) |
