@@ -1198,6 +1198,326 @@ k_attn_bwd_dq_tf32_d64(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   }
 }
 
+// =========================================================================================
+// One tile: at most 128 queries and 128 keys
+// =========================================================================================
+namespace one {
+// QK_FULL, GV_FULL: two tiles each. The scores and dP exist twice, as [queries, keys] for dQ and as [keys, queries] (.._T) for dK and dV.
+enum Bar { QK_FULL = 0, GV_FULL, O_FULL, GM_FULL, QM_FULL, KM_FULL, LSE_FULL, DELTA_FULL, S_FULL, ST_FULL, DP_FULL, DPT_FULL, PT_FULL, DST_FULL, DS_FULL,
+           DQ_FULL, DV_FULL, DK_FULL, DRAIN, NUM };
+// Sixteen warps that all compute (a seventeenth would leave 96 registers a thread): warp 0 also loads and issues S, dP and dQ, warp 8 the other products.
+constexpr int kThreads = 512;
+constexpr uint32_t kLse = 7 * kTile;             // Q, K, dO, V (K-major), dO, Q, K (MN-major); logsumexp of the queries in log2 units
+constexpr uint32_t kDelta = kLse + BT * 4;       // their row sums in two halves
+constexpr uint32_t kBars = kDelta + 2 * BT * 4;
+constexpr uint32_t kSmemTotal = kBars + 192 + 1024;
+static_assert(NUM * 8 <= 184 && kSmemTotal <= 227 * 1024, "");
+}  // namespace one
+
+// The whole backward of a head whose queries and keys are one tile each. What such a call costs is latency: the chain of two kernels (launch,
+// set-up, first loads, scores, results, twice, the second behind the first's row sums) where one step's products take 1.5 us. Here both sides run at the
+// same time, on tiles that are all loaded at once (224 KB): the score products come out in both orientations (sharing one would mean turning P over
+// through shared memory), for dQ with lanes = queries, for dK and dV with lanes = keys. SPLIT: a CTA for either side, while there are SMs for it; else one
+// CTA has both, eight warps each, and its result accumulators lie over scores that have been read. Every instruction runs once or a few times, so that
+// fetching them is what the phases wait for: short loops instead of straight code. Columns that a warp's rows do not see are skipped (16 at a time).
+// B200, fp32, S = 128, causal, H = 12, us against the two kernels: batch 1 11.6 -> 7.3, 4 12.1 -> 7.3, 8 16.4 -> 8.8, 12 17.6 -> 9.0, 20 23.6 -> 17.0. The
+// parts at batch 1: one kernel 11.0, straight code into loops and no spills 9.2, O through the copy engine and plain stores 8.7, a CTA per side 7.3.
+template <bool SPLIT>
+__global__ void __launch_bounds__(one::kThreads, 1)
+k_attn_bwd_tile_tf32_d64(const __grid_constant__ CUtensorMap tmQk, const __grid_constant__ CUtensorMap tmGk,
+                         const __grid_constant__ CUtensorMap tmKk, const __grid_constant__ CUtensorMap tmVk,
+                         const __grid_constant__ CUtensorMap tmQm, const __grid_constant__ CUtensorMap tmGm,
+                         const __grid_constant__ CUtensorMap tmKm, const __grid_constant__ CUtensorMap tmO, const BwdParams p) {
+  using namespace one;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const uint32_t aQ = smem_u32(smem), aK = aQ + kTile, aG = aQ + 2 * kTile, aV = aQ + 3 * kTile, aGm = aQ + 4 * kTile, aQm = aQ + 5 * kTile, aKm = aQ + 6 * kTile;
+  float *sLse = reinterpret_cast<float *>(smem + kLse), *sDelta = reinterpret_cast<float *>(smem + kDelta);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kBars);
+  volatile uint32_t *abort_flag = reinterpret_cast<volatile uint32_t *>(smem + kBars + 184);
+  uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(smem + kBars + 188);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t bh = SPLIT ? blockIdx.x >> 1 : blockIdx.x, h = bh % p.H, b = bh / p.H;
+  const bool keys = SPLIT ? (blockIdx.x & 1) != 0 : warp >= 8;  // lanes = keys: dV and dK; else lanes = queries: dQ
+  auto bar = [&](int id) { return smem_u32(&bars[id]); };
+  auto load_mn = [&](uint32_t dst, const CUtensorMap *m, int id, int box) {
+    mbar_arrive_expect_tx(bar(id), kTile);
+    for (int row = 0; row < BT; row += box)
+      for (int sl = 0; sl < 2; ++sl) tma_load_4d(dst + sl * kSlab + row * 128, m, bar(id), 32 * sl, (int)h, row, (int)b);
+  };
+  if (warp == 0) {
+    static_assert(NUM <= 32, "a lane per barrier");
+    if (lane < NUM) {
+      const bool two = lane == QK_FULL || lane == GV_FULL || lane == DRAIN;
+      const bool all = (lane >= PT_FULL && lane <= DS_FULL) || lane == DELTA_FULL;
+      mbar_init(bar(lane), two ? 2 : all ? (SPLIT && lane != DELTA_FULL ? 512 : 256) : lane == LSE_FULL ? 128 : 1);
+    }
+    if (lane == 0) *abort_flag = 0;
+    mbar_init_fence();
+    __syncwarp();
+    if (lane == 0) {  // the tiles are under way while the others set up
+      pdl_wait();
+      load_tile(aQ, &tmQk, bar(QK_FULL), (int)h, 0, (int)b);
+      load_tile(aK, &tmKk, bar(QK_FULL), (int)h, 0, (int)b);
+      load_tile(aG, &tmGk, bar(GV_FULL), (int)h, 0, (int)b);
+      load_tile(aV, &tmVk, bar(GV_FULL), (int)h, 0, (int)b);
+      load_tile(aKm, &tmO, bar(O_FULL), (int)h, 0, (int)b);  // K's place is O's at first
+      if (!SPLIT || keys) {
+        load_mn(aGm, &tmGm, GM_FULL, BT / 2);
+        load_mn(aQm, &tmQm, QM_FULL, BT / 2);
+      }
+    }
+    __syncwarp();
+  }
+  if (warp == 8) {
+    tmem_alloc(smem_u32(tmem_holder), kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = *tmem_holder;
+  const uint32_t tS = tmem, tST = tmem + 128, tDP = tmem + 256, tDPT = tmem + 384;
+  const uint32_t tDQ = tS, tDV = tS + 64, tDK = tST;  // over scores that have been read, and over P^T after its product
+  pdl_wait();  // everything above touched only this CTA's shared and tensor memory
+
+  // Products by the calling warp, one elected lane issues; loops, not straight code: every instruction here runs once, and what costs is fetching it.
+  // d = x y^T, of K-major tiles
+  auto scores = [&](uint32_t d, uint32_t x, uint32_t y, int done) {
+    const uint64_t dx = make_smem_desc(x, 16, 1024, kSwz128), dy = make_smem_desc(y, 16, 1024, kSwz128);
+    if (elect_one()) {
+#pragma unroll 1
+      for (uint32_t sl = 0; sl < 2; ++sl)
+#pragma unroll
+        for (uint32_t kk = 0; kk < 4; ++kk) {
+          const uint32_t off = sl * (kSlab >> 4) + kk * 2;
+          mma_tf32_ss_lohi(d, (uint32_t)dx + off, (uint32_t)(dx >> 32), (uint32_t)dy + off, (uint32_t)(dy >> 32), make_idesc(kFmtTF32, BT, BT, 0, 0), sl + kk);
+        }
+      mma_commit(bar(done));
+    }
+    __syncwarp();
+  };
+  // d = x y, x in tensor memory, y an MN-major tile
+  auto result = [&](uint32_t d, uint32_t x, uint32_t y, int done) {
+    tc_fence_after_sync();
+    const uint64_t dy = make_smem_desc(y, kSlab, 512, kSwz128B32);
+    if (elect_one()) {
+#pragma unroll 1
+      for (uint32_t k4 = 0; k4 < BT / 8; k4 += 4)
+#pragma unroll
+        for (uint32_t kk = k4; kk < k4 + 4; ++kk)
+          mma_tf32_ts_lohi(d, x + kk * 8, (uint32_t)dy + kk * (1024 >> 4), (uint32_t)(dy >> 32), make_idesc(kFmtTF32, BT, HD, 0, 1), kk);
+      mma_commit(bar(done));
+    }
+    __syncwarp();
+  };
+  {
+    // a thread has CW columns of its lane's row; half: of the row's dims, where two threads share them
+    constexpr int CW = SPLIT ? 32 : 64;
+    const int row = (warp & 3) * 32 + lane, half = (warp >> 2) & 1, col0 = SPLIT ? (warp >> 2) * 32 : half * 64;
+    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+    auto lse2_of = [](float raw) -> float { return (raw == -INFINITY) ? INFINITY : raw * kLog2e; };
+    bool ok = false;
+    auto row_sums = [&]() -> bool {  // by warps 0-7
+      // row sums of dO o O, dO as rounded by its tensor map: the values that the dP products see
+      if (!mbar_wait_warp(bar(GV_FULL), 0, abort_flag) || !mbar_wait_warp(bar(O_FULL), 0, abort_flag)) return false;
+      const uint8_t *g_row = smem + 2 * kTile + half * kSlab + row * 128, *o_row = smem + 6 * kTile + half * kSlab + row * 128;
+      float acc0 = 0.0f, acc1 = 0.0f;
+#pragma unroll
+      for (int x = 0; x < 8; ++x) {
+        const uint32_t off = (uint32_t)((x ^ (row & 7)) << 4);
+        const float4 gv = *reinterpret_cast<const float4 *>(g_row + off);
+        const float4 ov = *reinterpret_cast<const float4 *>(o_row + off);
+        acc0 = fmaf(gv.x, ov.x, acc0); acc1 = fmaf(gv.y, ov.y, acc1);
+        acc0 = fmaf(gv.z, ov.z, acc0); acc1 = fmaf(gv.w, ov.w, acc1);
+      }
+      sDelta[half * BT + row] = acc0 + acc1;
+      mbar_arrive(bar(DELTA_FULL));
+      return true;
+    };
+    const size_t stat0 = ((size_t)b * p.H + h) * p.Sq;
+    // S = Q K^T and dP = dO V^T, by warp 0; S^T = K Q^T and dP^T = V dO^T, by warp 8
+    if (warp == (keys ? 8 : 0)) {
+#pragma unroll 1
+      for (int x = 0; x < 2; ++x) {
+        if (!mbar_wait_warp(bar(QK_FULL + x), 0, abort_flag)) break;
+        tc_fence_after_sync();
+        const uint32_t lhs = aQ + (2 * x + (keys ? 1 : 0)) * kTile, rhs = aQ + (2 * x + (keys ? 0 : 1)) * kTile;
+        scores((x ? tDP : tS) + (keys ? 128 : 0), lhs, rhs, (x ? DP_FULL : S_FULL) + (keys ? 1 : 0));
+      }
+    }
+    if (!keys) {
+      do {
+        if (warp < 8 && !row_sums()) break;
+        const float lse_raw = row < (int)p.Sq ? __ldg(p.lse + stat0 + row) : -INFINITY;
+        const float lse2 = lse2_of(lse_raw);
+        long long kmax_ll = p.causal ? row + p.shift + 1 : (long long)p.Sk;
+        if (kmax_ll > (long long)p.Sk) kmax_ll = p.Sk;
+        const int kmax = kmax_ll < 0 ? 0 : (int)kmax_ll, k_end = __reduce_max_sync(0xffffffffu, kmax);
+        if (!mbar_wait_warp(bar(DELTA_FULL), 0, abort_flag)) break;
+        if (warp == 0 && lane == 0) load_mn(aKm, &tmKm, KM_FULL, BT);  // O has been read
+        __syncwarp();
+        const float dlt = sDelta[row] + sDelta[BT + row];
+        if (warp < 4 && row < (int)p.Sq) p.delta_out[stat0 + row] = dlt;
+        if (!mbar_wait_warp(bar(S_FULL), 0, abort_flag) || !mbar_wait_warp(bar(DP_FULL), 0, abort_flag)) break;
+        tc_fence_after_sync();
+#pragma unroll 1
+        for (int c = col0; c < col0 + CW; c += 16) {
+          uint32_t rr[16], pr[16];
+          if (c >= k_end) {  // no row of the warp sees these keys
+#pragma unroll
+            for (int x = 0; x < 16; ++x) rr[x] = 0u;
+            tmem_st16(tDP + lane_base + c, rr);
+            continue;
+          }
+          tmem_ld16(tS + lane_base + c, pr);
+          tmem_ld16(tDP + lane_base + c, rr);
+          tmem_wait_ld();
+#pragma unroll
+          for (int x = 0; x < 16; x += 2) {
+            const float2 e = fma2(as_float2(c + x < kmax ? pr[x] : 0xff800000u, c + x + 1 < kmax ? pr[x + 1] : 0xff800000u),
+                                  make_float2(p.scale_log2, p.scale_log2), make_float2(-lse2, -lse2));
+            const float2 y = mul2(make_float2(ex2_approx(e.x), ex2_approx(e.y)), add2(as_float2(rr[x], rr[x + 1]), make_float2(-dlt, -dlt)));
+            rr[x] = tf32_rna_operand(y.x);
+            rr[x + 1] = tf32_rna_operand(y.y);
+          }
+          tmem_st16(tDP + lane_base + c, rr);
+        }
+        tmem_wait_st();
+        tc_fence_before_sync();
+        mbar_arrive(bar(DS_FULL));
+        if (warp == 0) {
+          if (!mbar_wait_warp(bar(DS_FULL), 0, abort_flag) || !mbar_wait_warp(bar(KM_FULL), 0, abort_flag)) break;
+          result(tDQ, tDP, aKm, DQ_FULL);
+        }
+        ok = true;
+      } while (false);
+    } else {
+      do {
+        if ((warp >> 2) == 2) {
+          sLse[row] = lse2_of(row < (int)p.Sq ? __ldg(p.lse + stat0 + row) : -INFINITY);
+          mbar_arrive(bar(LSE_FULL));
+        }
+        // key `row` is visible from query row - shift on
+        long long qmin_ll = p.causal ? row - p.shift : 0;
+        const int qmin = qmin_ll < 0 ? 0 : (qmin_ll > BT ? BT : (int)qmin_ll), q_begin = __reduce_min_sync(0xffffffffu, qmin);
+        auto unseen = [&](int c) { return c + 16 <= q_begin || c >= (int)p.Sq; };  // 16 queries that see no key of the warp
+        const uint32_t zero[16] = {0u};
+        if (!mbar_wait_warp(bar(LSE_FULL), 0, abort_flag) || !mbar_wait_warp(bar(ST_FULL), 0, abort_flag)) break;
+        tc_fence_after_sync();
+#pragma unroll 1
+        for (int c = col0; c < col0 + CW; c += 16) {
+          uint32_t rr[16];
+          if (unseen(c)) {
+            tmem_st16(tST + lane_base + c, zero);
+            continue;
+          }
+          tmem_ld16(tST + lane_base + c, rr);
+          tmem_wait_ld();
+#pragma unroll
+          for (int x = 0; x < 16; x += 2) {
+            const float2 l = *reinterpret_cast<const float2 *>(sLse + c + x);
+            const float2 y = fma2(as_float2(c + x >= qmin ? rr[x] : 0xff800000u, c + x + 1 >= qmin ? rr[x + 1] : 0xff800000u),
+                                  make_float2(p.scale_log2, p.scale_log2), make_float2(-l.x, -l.y));
+            rr[x] = cvt_rna_tf32(ex2_approx(y.x));  // low bits cleared: P of dS, too
+            rr[x + 1] = cvt_rna_tf32(ex2_approx(y.y));
+          }
+          tmem_st16(tST + lane_base + c, rr);
+        }
+        tmem_wait_st();
+        tc_fence_before_sync();
+        mbar_arrive(bar(PT_FULL));
+        if (SPLIT && warp == 8) {
+          if (!mbar_wait_warp(bar(PT_FULL), 0, abort_flag) || !mbar_wait_warp(bar(GM_FULL), 0, abort_flag)) break;
+          result(tDV, tST, aGm, DV_FULL);
+        }
+        if (SPLIT && warp < 8 && !row_sums()) break;
+        if (!mbar_wait_warp(bar(DELTA_FULL), 0, abort_flag) || !mbar_wait_warp(bar(DPT_FULL), 0, abort_flag)) break;
+        tc_fence_after_sync();
+#pragma unroll 1
+        for (int c = col0; c < col0 + CW; c += 16) {
+          uint32_t rr[16], pr[16];
+          if (unseen(c)) {
+            tmem_st16(tDPT + lane_base + c, zero);
+            continue;
+          }
+          tmem_ld16(tST + lane_base + c, pr);
+          tmem_ld16(tDPT + lane_base + c, rr);
+          tmem_wait_ld();
+#pragma unroll
+          for (int x = 0; x < 16; x += 2) {
+            const float2 d = add2(*reinterpret_cast<const float2 *>(sDelta + c + x), *reinterpret_cast<const float2 *>(sDelta + BT + c + x));
+            const float2 y = mul2(as_float2(pr[x], pr[x + 1]), add2(as_float2(rr[x], rr[x + 1]), make_float2(-d.x, -d.y)));
+            rr[x] = tf32_rna_operand(y.x);
+            rr[x + 1] = tf32_rna_operand(y.y);
+          }
+          tmem_st16(tDPT + lane_base + c, rr);
+        }
+        tmem_wait_st();
+        tc_fence_before_sync();
+        mbar_arrive(bar(DST_FULL));
+        if (warp == 8) {
+          if (!SPLIT) {  // dV goes where the scores were, and dK where P^T was
+            if (!mbar_wait_warp(bar(PT_FULL), 0, abort_flag) || !mbar_wait_warp(bar(DS_FULL), 0, abort_flag) || !mbar_wait_warp(bar(GM_FULL), 0, abort_flag)) break;
+            result(tDV, tST, aGm, DV_FULL);
+          }
+          if (!mbar_wait_warp(bar(DST_FULL), 0, abort_flag) || !mbar_wait_warp(bar(QM_FULL), 0, abort_flag)) break;
+          result(tDK, tDPT, aQm, DK_FULL);
+        }
+        ok = true;
+      } while (false);
+    }
+    // Results: dQ, dV and dK. A warp turns 32 rows of 32 columns over in an operand tile that no product reads any more, so that whole 128-byte
+    // lines leave (tensor stores took 1.4 us more: their barrier, their start, and the wait before the tile may go).
+    const int x0 = !keys ? 0 : SPLIT ? 1 + (warp >> 3) : 1, x1 = !keys ? (warp < 8 ? 1 : 0) : SPLIT ? x0 + 1 : 3;
+    const int n_rows = (int)(keys ? p.Sk : p.Sq) - (warp & 3) * 32;
+#pragma unroll 1
+    for (int x = x0; ok && x < x1; ++x) {
+      if (!mbar_wait_warp(bar(DQ_FULL + x), 0, abort_flag)) break;
+      tc_fence_after_sync();
+      const float mul = x == 1 ? 1.0f : p.scale;
+      uint32_t rr[32];
+      tmem_ld32((x == 0 ? tDQ : x == 1 ? tDV : tDK) + lane_base + half * 32, rr);
+      tmem_wait_ld();
+      uint8_t *slab = smem + (x == 0 ? 6 : 3 + x) * kTile + half * kSlab + (warp & 3) * 32 * 128;
+#pragma unroll
+      for (int y = 0; y < 8; ++y)
+        *reinterpret_cast<float4 *>(slab + lane * 128 + ((y ^ (lane & 7)) << 4)) = make_float4(
+            __uint_as_float(rr[4 * y]) * mul, __uint_as_float(rr[4 * y + 1]) * mul, __uint_as_float(rr[4 * y + 2]) * mul, __uint_as_float(rr[4 * y + 3]) * mul);
+      __syncwarp();
+      float *dst = (x == 0 ? p.dq : x == 1 ? p.dv : p.dk) + (((size_t)b * (keys ? p.Sk : p.Sq) + (warp & 3) * 32) * p.H + h) * HD + half * 32 + 4 * (lane & 7);
+#pragma unroll
+      for (int y = 0; y < 32; y += 4) {
+        const int r = y + (lane >> 3);
+        const float4 v = *reinterpret_cast<const float4 *>(slab + r * 128 + (((lane & 7) ^ (r & 7)) << 4));
+        if (r < n_rows) *reinterpret_cast<float4 *>(dst + (size_t)r * p.H * HD) = v;
+      }
+    }
+  }
+
+  // ---------------------------------------------------------------- teardown (all roles)
+  tc_fence_before_sync();
+  __syncthreads();
+  if (*abort_flag != 0u) {
+    if (warp == 0 || warp == 8) {
+      commit_elected(bar(DRAIN));  // by the lanes that issued the MMAs: the election is deterministic; two arrivals
+      for (int t = 0; t < (1 << 16) && !mbar_try_wait(bar(DRAIN), 0); ++t) {
+      }
+    }
+    if (warp == 1 && lane == 0) {  // copies
+      const uint64_t t0 = global_timer_ns();
+      while (global_timer_ns() - t0 < 2000000ull) {
+      }
+    }
+    if (threadIdx.x == 0 && p.status) atomicOr(p.status, DEV_STATUS_WAIT_EXPIRED);
+    __syncthreads();
+  }
+  if (warp == 8) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem, kTmemCols);
+  }
+}
+
 }  // namespace
 
 bool tensor_backward_supported(const AttnParams &p) {
@@ -1234,6 +1554,8 @@ int device_info(int *n_sm) {
            cudaFuncSetAttribute(k_attn_bwd_dq_tf32_d64<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dq::kSmemTotal) == cudaSuccess &&
            cudaFuncSetAttribute(k_attn_bwd_dq_tf32_d64<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dq::kSmemTotal) == cudaSuccess &&
            cudaFuncSetAttribute(k_attn_bwd_dq_tf32_d64<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dq::kSmemTotal) == cudaSuccess &&
+           cudaFuncSetAttribute(k_attn_bwd_tile_tf32_d64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)one::kSmemTotal) == cudaSuccess &&
+           cudaFuncSetAttribute(k_attn_bwd_tile_tf32_d64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)one::kSmemTotal) == cudaSuccess &&
            cudaDeviceGetAttribute(&d.n_sm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && d.n_sm > 0;
   });
   if (!d.ok) {
@@ -1365,6 +1687,17 @@ int tensor_backward(const AttnParams &p, cudaStream_t s) {
       for (const void *in : {(const void *)p.q, (const void *)p.k, (const void *)p.v, (const void *)p.d_out, (const void *)p.o_in, (const void *)p.d_q})
         if (overlap(g, k_bytes, in, in == p.k || in == p.v ? k_bytes : q_bytes)) apart = false;
   bp.early = fuse && prof == nullptr && apart && items_kv > 0 && option(DF_OPT_PDL) != 0;
+  // One tile of queries and of keys: both kernels' work in one (not when the two are to be timed one by one, or kept apart). It has no pipeline over
+  // items, so after some waves of heads the two kernels are faster, sooner where all keys are visible: 25 x 12 heads of 128, 27.0 us (two kernels) against
+  // 24.5, all keys 26.4 and 25.7; 36 x 12 33.0 and 32.2, all keys 32.8 and 34.1; 64 x 12 60.4 and 60.1, all keys 60.0 and 63.7.
+  if (fuse && prof == nullptr && apart && items_kv > 0 && p.Sq <= BT && p.Sk <= BT && (uint64_t)p.B * p.H <= (p.causal ? 3ull : 2ull) * n_sm) {
+    // (d_q may take O's place where one CTA reads O)
+    const bool halves = 2 * p.B * p.H <= (uint32_t)n_sm && !overlap(p.d_q, q_bytes, p.o_in, q_bytes);
+    const cudaError_t e = launch_kernel(halves ? k_attn_bwd_tile_tf32_d64<true> : k_attn_bwd_tile_tf32_d64<false>, dim3(p.B * p.H * (halves ? 2 : 1)),
+                                        dim3(one::kThreads), one::kSmemTotal, s, tmQk, tmGk, tmKk, tmVk, tmQm, tmGm, tmKm, tmO, bp);
+    note_launch();
+    return check_cuda(e);
+  }
   // A profiled call launches each kernel kProfileReps times back to back between its events (the results are the
   // same every time): an event pair around a single launch adds several microseconds to a 70-microsecond kernel.
   const int reps = prof ? kProfileReps : 1;

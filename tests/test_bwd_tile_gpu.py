@@ -1,0 +1,43 @@
+"""The whole TF32 backward of sequences of one tile (128 rows) in one kernel: its forms, at the edges of its 16-column blocks and of the tile."""
+import pytest
+
+import helpers as hp
+from helpers import pkg, to_dev
+
+pytestmark = pytest.mark.gpu
+
+
+# B x H: a CTA for either side of a head, one for both (from 75 heads on a 148-SM device), two and three waves (of causal heads), and past the
+# last wave that the rule takes
+@pytest.mark.parametrize("B,H", [(1, 3), (2, 37), (1, 75), (5, 30), (4, 111), (5, 89)])
+@pytest.mark.parametrize("S", [1, 15, 16, 17, 33, 64, 100, 127, 128])
+@pytest.mark.parametrize("causal", [True, False])
+def test_one_tile_backward_against_float64(B, H, S, causal):
+    import torch
+    from test_split_gpu import _reference
+    p = pkg()
+    from oracle.attn_oracle import Oracle
+    orc = Oracle()
+    q, k, v, go = to_dev(*(orc.fill_normal((B, S, H * 64), 700 + S, i) for i in range(4)))
+    scale = hp.default_scale(64)
+    out, lse = p.forward(q, k, v, H, scale, causal)
+
+    def run(f, o, **kw):
+        delta = torch.full((B, H, S), 9.0, device="cuda")
+        got = f(q, k, v, o, go, lse, H, scale, causal, delta_buf=delta, **kw)[:3]
+        assert p.sync_status() == 0
+        return tuple(got) + (delta,)
+
+    got, again = run(p.backward, out), run(p.backward, out)
+    two = run(p.backward_profile, out)  # timed kernel by kernel, so always in two
+    o = out.clone()
+    in_place = run(p.backward, o, d_q=o)  # d_q in the place of O, which only dQ's side reads
+    refs = _reference(torch, q, k, v, go, H, scale, causal, 0)[2:]
+    for n, name in enumerate(("dq", "dk", "dv")):
+        assert torch.equal(got[n], again[n]) and torch.equal(got[n], in_place[n]), name  # no atomics: the same bits every time
+        size = max(1.0, float(refs[n].abs().max()))
+        err, err_two = (float((x[n].double() - refs[n]).abs().max()) for x in (got, two))
+        assert err <= hp.TOL_GRAD_REL_TF32 * size, name
+        # operands rounded to 11 bits either way, P on the dK side too: half a unit of that is all that may lie between the two
+        assert err <= err_two + 2.0 ** -12 * size, name
+    assert torch.equal(got[3], two[3])  # the row sums are the same sums
