@@ -116,13 +116,6 @@ __device__ __forceinline__ TileMN tile_mn(uint32_t tile_smem) {
   return t;
 }
 // To be called by the elected lane only.
-// 32 lanes x 16 columns of tensor memory from 16 registers per thread
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
-               "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
-               "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-               : "memory");
-}
 // 8 K-steps added to a 128x64x64 TS MMA: A = 64 TMEM columns, B = 64 rows of a K-major tile of a ring (off: their descriptor offset).
 __device__ __forceinline__ void batch_ts_scores(uint32_t d_tmem, uint32_t a_tmem, const TileK &b, uint32_t off, uint32_t idesc) {
 #pragma unroll
@@ -166,13 +159,6 @@ __device__ __forceinline__ void load_tile(uint32_t dst, const CUtensorMap *m, ui
 
 __device__ __forceinline__ void store_cluster(uint32_t addr, float4 v) {
   asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
-                 "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-               : "r"(taddr)
-               : "memory");
 }
 // SPLIT kernels: 16 accumulator columns of a thread's row (dims d0 .. d0 + 15) into the other CTA's staging tile, which has the layout of the store's
 // tensor map (slabs of 32 dims, 16-byte chunk c of row r at c ^ (r % 8)), and there, in place, the sum with the finishing CTA's own columns.

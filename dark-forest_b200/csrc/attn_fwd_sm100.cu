@@ -646,6 +646,189 @@ k_attn_fwd(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
   }
 }
 
+// =========================================================================================
+// One tile: at most 128 queries and 128 keys (fp32)
+// =========================================================================================
+namespace one {
+enum Bar { T_QK_FULL = 0, T_V_FULL, T_S_FULL, T_P_FULL, T_O_FULL, T_DRAIN, T_MAX_FULL, T_NUM = T_MAX_FULL + 4 };  // T_MAX_FULL + quarter of the rows
+constexpr int kThreads = 512;
+constexpr uint32_t kTile = 2 * kSlabBytes;
+constexpr uint32_t kMax = 3 * kTile, kSum = kMax + 4 * BM * 4;  // Q, K, V; a row's maximum and sum over each quarter of the keys
+constexpr uint32_t kBars = kSum + 4 * BM * 4;
+constexpr uint32_t kSmemTotal = kBars + 96 + 1024;
+static_assert(T_NUM * 8 <= 80, "barriers overlap the abort flag");
+}  // namespace one
+
+// The whole forward of a head whose queries and keys are one tile each: a CTA per head, two to an SM, all sixteen warps compute, a thread a quarter of a
+// row; maxima and sums of the rows meet in shared memory. What bounds such a call is latency, and with many heads the ends of items; the kernel
+// above has a tile on four warps (the other slot stands idle) in straight code for a whole row per thread, fetched once to run once.
+// B200, fp32, S = 128, causal, H = 12, us (above / here): batch 1 6.5 / 6.0, 8 7.1 / 6.3, 12 7.9 / 6.4, 24 12.9 / 8.6, 128 60.8 / 53.2; S = 50, batch 128
+// 48.3 / 32.0.
+__global__ void __launch_bounds__(one::kThreads, 2)
+k_attn_fwd_tile(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+                const FwdParams p) {
+  using namespace one;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const uint32_t aQ = smem_u32(smem), aK = aQ + kTile, aV = aQ + 2 * kTile;
+  float *sMax = reinterpret_cast<float *>(smem + kMax), *sSum = reinterpret_cast<float *>(smem + kSum);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kBars);
+  volatile uint32_t *abort_flag = reinterpret_cast<volatile uint32_t *>(smem + kBars + 80);
+  uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(smem + kBars + 84);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t h = blockIdx.x % p.H, b = blockIdx.x / p.H;
+  auto bar = [&](int id) { return smem_u32(&bars[id]); };
+  if (warp == 0) {
+    if (lane < T_NUM) mbar_init(bar(lane), lane == T_QK_FULL ? 2 : lane == T_P_FULL ? kThreads : lane >= T_MAX_FULL ? 128 : 1);
+    if (lane == 0) *abort_flag = 0;
+    mbar_init_fence();
+    __syncwarp();
+    if (lane == 0) {  // the tiles are under way while the others set up
+      pdl_wait();
+      auto load = [&](uint32_t dst, const CUtensorMap *m, int id) {
+        mbar_arrive_expect_tx(bar(id), kTile);
+        for (int sl = 0; sl < 2; ++sl) tma_load_4d(dst + sl * kSlabBytes, m, bar(id), 32 * sl, (int)h, 0, (int)b);
+      };
+      load(aQ, &tmQ, T_QK_FULL);
+      load(aK, &tmK, T_QK_FULL);
+      load(aV, &tmV, T_V_FULL);
+    }
+    __syncwarp();
+  }
+  if (warp == 8) {
+    tmem_alloc(smem_u32(tmem_holder), 256);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tS = *tmem_holder, tO = tS + 128;
+  pdl_wait();  // everything above touched only this CTA's shared and tensor memory
+
+  const int row = (warp & 3) * 32 + lane, group = warp >> 2, col0 = group * 32;
+  const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+  do {
+    if (warp == 0) {  // S = Q K^T
+      if (!mbar_wait_warp(bar(T_QK_FULL), 0, abort_flag)) break;
+      tc_fence_after_sync();
+      const uint64_t dq = make_smem_desc(aQ, 16, 1024, kSwz128), dk = make_smem_desc(aK, 16, 1024, kSwz128);
+      if (elect_one()) {
+#pragma unroll 1
+        for (uint32_t sl = 0; sl < 2; ++sl)
+#pragma unroll
+          for (uint32_t kk = 0; kk < 4; ++kk) {
+            const uint32_t off = sl * (kSlabBytes >> 4) + kk * 2;
+            mma_tf32_ss_lohi(tS, (uint32_t)dq + off, (uint32_t)(dq >> 32), (uint32_t)dk + off, (uint32_t)(dk >> 32), make_idesc(kFmtTF32, BM, BN, 0, 0), sl + kk);
+          }
+        mma_commit(bar(T_S_FULL));
+      }
+      __syncwarp();
+    }
+    long long kmax_ll = p.causal ? row + p.shift + 1 : (long long)p.Sk;
+    if (kmax_ll > (long long)p.Sk) kmax_ll = p.Sk;
+    const int kmax = kmax_ll < 0 ? 0 : (int)kmax_ll, k_end = __reduce_max_sync(0xffffffffu, kmax);  // keys [0, kmax) are visible to this row
+    if (!mbar_wait_warp(bar(T_S_FULL), 0, abort_flag)) break;
+    tc_fence_after_sync();
+    uint32_t r[32];
+    float mx = -INFINITY, l0 = 0.0f, l1 = 0.0f;
+    if (col0 < k_end) {
+      tmem_ld32(tS + lane_base + col0, r);
+      tmem_wait_ld();
+#pragma unroll
+      for (int x = 0; x < 32; ++x) {
+        if (!(col0 + x < kmax)) r[x] = 0xff800000u;  // -inf: exponentiates to 0
+        mx = fmaxf(mx, __uint_as_float(r[x]));
+      }
+    }
+    sMax[group * BM + row] = mx;
+    mbar_arrive(bar(T_MAX_FULL + (warp & 3)));
+    if (!mbar_wait_warp(bar(T_MAX_FULL + (warp & 3)), 0, abort_flag)) break;
+    const float m = fmaxf(fmaxf(sMax[row], sMax[BM + row]), fmaxf(sMax[2 * BM + row], sMax[3 * BM + row])) * p.scale_log2;
+    const float neg_m = m == -INFINITY ? 0.0f : -m;
+    if (col0 < k_end) {
+#pragma unroll
+      for (int x = 0; x < 32; x += 2) {
+        const float2 y = fma2(as_float2(r[x], r[x + 1]), make_float2(p.scale_log2, p.scale_log2), make_float2(neg_m, neg_m));
+        const float e0 = ex2_approx(y.x), e1 = ex2_approx(y.y);
+        l0 += e0;
+        l1 += e1;
+        r[x] = tf32_rna_operand(e0);
+        r[x + 1] = tf32_rna_operand(e1);
+      }
+    } else {
+#pragma unroll
+      for (int x = 0; x < 32; ++x) r[x] = 0u;
+    }
+    tmem_st32(tS + lane_base + col0, r);
+    sSum[group * BM + row] = l0 + l1;
+    tmem_wait_st();
+    tc_fence_before_sync();
+    mbar_arrive(bar(T_P_FULL));
+    if (!mbar_wait_warp(bar(T_P_FULL), 0, abort_flag)) break;
+    if (warp == 0) {  // O = P V
+      if (!mbar_wait_warp(bar(T_V_FULL), 0, abort_flag)) break;
+      tc_fence_after_sync();
+      const uint64_t dv = make_smem_desc(aV, kSlabBytes, 512, kSwz128B32);
+      if (elect_one()) {
+#pragma unroll 1
+        for (uint32_t k4 = 0; k4 < BN / 8; k4 += 4)
+#pragma unroll
+          for (uint32_t kk = k4; kk < k4 + 4; ++kk)
+            mma_tf32_ts_lohi(tO, tS + kk * 8, (uint32_t)dv + kk * (1024 >> 4), (uint32_t)(dv >> 32), make_idesc(kFmtTF32, BM, 64, 0, 1), kk);
+        mma_commit(bar(T_O_FULL));
+      }
+      __syncwarp();
+    }
+    const float l = (sSum[row] + sSum[BM + row]) + (sSum[2 * BM + row] + sSum[3 * BM + row]);
+    const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+    if (group == 0 && p.lse && row < (int)p.Sq) p.lse[((size_t)b * p.H + h) * p.Sq + row] = l > 0.0f ? (m + lg2_approx(l)) * kLn2 : -INFINITY;
+    if (!mbar_wait_warp(bar(T_O_FULL), 0, abort_flag)) break;
+    tc_fence_after_sync();
+    uint32_t ro[16];
+    tmem_ld16(tO + lane_base + group * 16, ro);
+    tmem_wait_ld();
+    // rows that see no key at all: O = 0, lse = -inf (reference guard, attention_fused.cu:104)
+#pragma unroll
+    for (int x = 0; x < 16; ++x) ro[x] = l > 0.0f ? __float_as_uint(__uint_as_float(ro[x]) * inv) : 0u;
+    if (row < (int)p.Sq) {
+      float *dst = reinterpret_cast<float *>(p.out) + (((size_t)b * p.Sq + row) * p.H + h) * 64 + group * 16;
+#pragma unroll
+      for (int x = 0; x < 16; x += 8) {
+        const uint32_t g[8] = {ro[x], ro[x + 1], ro[x + 2], ro[x + 3], ro[x + 4], ro[x + 5], ro[x + 6], ro[x + 7]};
+        if (p.wide) {
+          store_32(dst + x, g);
+        } else {
+          reinterpret_cast<uint4 *>(dst + x)[0] = make_uint4(g[0], g[1], g[2], g[3]);
+          reinterpret_cast<uint4 *>(dst + x)[1] = make_uint4(g[4], g[5], g[6], g[7]);
+        }
+      }
+    }
+  } while (false);
+  __syncwarp();
+
+  // ---------------------------------------------------------------- teardown (all roles)
+  tc_fence_before_sync();
+  __syncthreads();
+  if (*abort_flag != 0u) {
+    if (warp == 0) {
+      commit_elected(bar(T_DRAIN));  // by the lane that issued the MMAs: the election is deterministic
+      for (int t = 0; t < (1 << 16) && !mbar_try_wait(bar(T_DRAIN), 0); ++t) {
+      }
+    }
+    if (warp == 1 && lane == 0) {  // copies
+      const uint64_t t0 = global_timer_ns();
+      while (global_timer_ns() - t0 < 2000000ull) {
+      }
+    }
+    if (threadIdx.x == 0 && p.status) atomicOr(p.status, DEV_STATUS_WAIT_EXPIRED);
+    __syncthreads();
+  }
+  if (warp == 8) {
+    tc_fence_after_sync();
+    tmem_dealloc(tS, 256);
+  }
+}
+
 }  // namespace
 
 bool tensor_forward_supported(const AttnParams &p) {
@@ -663,14 +846,16 @@ bool tensor_forward_supported(const AttnParams &p) {
 }
 
 namespace {
-template <class C>
+template <class C, bool TILE = false>
 int launch_forward(const AttnParams &p, cudaStream_t s) {
+  static_assert(!TILE || (!C::BF16 && C::HD == 64), "");
   static std::once_flag once[64];
   static bool ready[64];
   int dev = 0;
   if (check_cuda(cudaGetDevice(&dev)) != DF_OK || dev < 0 || dev >= 64) return DF_ERR_CUDA;
   std::call_once(once[dev], [&]() {
-    ready[dev] = cudaFuncSetAttribute(k_attn_fwd<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmemTotal) == cudaSuccess;
+    ready[dev] = TILE ? cudaFuncSetAttribute(k_attn_fwd_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)one::kSmemTotal) == cudaSuccess
+                      : cudaFuncSetAttribute(k_attn_fwd<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmemTotal) == cudaSuccess;
   });
   CUtensorMap tmQ, tmK, tmV;
   // V is an MN-major operand: 32-bit elements need the 32-byte-atom swizzle, 16-bit ones do not
@@ -693,7 +878,8 @@ int launch_forward(const AttnParams &p, cudaStream_t s) {
   fp.tiles = tiles;
   fp.n_units = C::SPLIT ? tiles : pairs;
   fp.claims = (uint64_t)fp.n_units * p.B * p.H > (uint64_t)sm_count();
-  const cudaError_t err = launch_kernel(k_attn_fwd<C>, dim3(fp.n_units * p.B * p.H), dim3(C::kThreads), C::kSmemTotal, s, tmQ, tmK, tmV, fp);
+  const cudaError_t err = TILE ? launch_kernel(k_attn_fwd_tile, dim3(p.B * p.H), dim3(one::kThreads), one::kSmemTotal, s, tmQ, tmK, tmV, fp)
+                               : launch_kernel(k_attn_fwd<C>, dim3(fp.n_units * p.B * p.H), dim3(C::kThreads), C::kSmemTotal, s, tmQ, tmK, tmV, fp);
   note_launch();
   return check_cuda(err);
 }
@@ -750,6 +936,10 @@ int tensor_forward(const AttnParams &p, cudaStream_t s) {
   const int n_sm = sm_count();
   if (n_sm <= 0) return DF_ERR_CUDA;
   const bool split = split_items(p, n_sm);
+  // One tile: only a call of many full tiles without a mask has enough steps to a head for the kernel with a pipeline over items (us, that / one tile: 32 x 12
+  // heads of 128, all keys, 15.3 / 13.5, 64 x 12 28.2 / 28.3, 128 x 12 55.3 / 57.0; causal 60.8 / 53.2).
+  if (!p.bf16 && p.Sq <= BM && p.Sk <= BN && option(DF_OPT_FWD_PERSIST) == 1 && (p.causal || p.Sk <= BN / 2 || (uint64_t)p.B * p.H <= 3ull * n_sm))
+    return launch_forward<FwdCfg<64, false, true, false>, true>(p, s);
   if (!p.bf16) return launch_items<64, false, true>(p, split, s);
   if (!split && (p.D == 128 || p.Sq <= BM)) return tensor_forward_row2(p, s);
   if (p.D == 64) return p.out_f32 ? launch_items<64, true, true>(p, split, s) : launch_items<64, true, false>(p, split, s);
