@@ -775,7 +775,7 @@ int launch_backward(const AttnParams &p, cudaStream_t s) {
   bp.B = p.B; bp.H = p.H; bp.Sq = p.Sq; bp.Sk = p.Sk;
   bp.scale = p.scale;
   bp.scale_log2 = p.scale * kLog2e;
-  bp.inv_scale = 1.0f / fmaxf(p.scale, 1e-34f);  // finite, and so is its product with a logsumexp; scores times a smaller scale are zero anyway
+  bp.inv_scale = 1.0f / fmaxf(p.scale, 1e-37f);  // finite, and so is its product with the logsumexp of scores that such a scale has made equal
   bp.causal = p.causal;
   bp.shift = p.shift;
   bp.status = device_status_ptr();

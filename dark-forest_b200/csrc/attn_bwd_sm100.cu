@@ -1509,7 +1509,7 @@ k_attn_bwd_tile_tf32_d64(const __grid_constant__ CUtensorMap tmQk, const __grid_
 bool tensor_backward_supported(const AttnParams &p) {
   if (option(DF_OPT_DISABLE_TENSOR) != 0) return false;
   if (p.D != HD || p.Sk == 0 || p.Sq == 0 || p.B == 0) return false;
-  if (!(p.scale > 0.0f) || !isfinite(p.scale) || p.scale < 1e-34f) return false;  // lse / scale is finite
+  if (!(p.scale > 0.0f) || !isfinite(p.scale)) return false;
   const uintptr_t bits = reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k) |
                          reinterpret_cast<uintptr_t>(p.v) | reinterpret_cast<uintptr_t>(p.d_out) |
                          reinterpret_cast<uintptr_t>(p.d_q) | reinterpret_cast<uintptr_t>(p.d_k) |
@@ -1634,7 +1634,7 @@ int tensor_backward(const AttnParams &p, cudaStream_t s) {
   bp.B = p.B; bp.H = p.H; bp.Sq = p.Sq; bp.Sk = p.Sk;
   bp.scale = p.scale;
   bp.scale_log2 = p.scale * kLog2e;
-  bp.inv_scale = 1.0f / p.scale;
+  bp.inv_scale = 1.0f / fmaxf(p.scale, 1e-37f);  // finite, and so is its product with the logsumexp of scores that such a scale has made equal
   bp.causal = p.causal;
   bp.shift = p.shift;
   bp.status = device_status_ptr();

@@ -41,3 +41,31 @@ def test_one_tile_backward_against_float64(B, H, S, causal):
         # operands rounded to 11 bits either way, P on the dK side too: half a unit of that is all that may lie between the two
         assert err <= err_two + 2.0 ** -12 * size, name
     assert torch.equal(got[3], two[3])  # the row sums are the same sums
+
+
+@pytest.mark.parametrize("S,D,bf16", [(100, 64, False), (300, 64, False), (300, 64, True), (300, 128, True)])
+@pytest.mark.parametrize("scale", [1e-30, 1e-35, 3e-37])
+def test_backward_with_a_scale_that_makes_scores_equal(S, D, bf16, scale):
+    """The logsumexp enters the score products divided by the scale. Such a scale leaves uniform probabilities, dV = means, and dQ = dK = 0 but for the scale."""
+    import torch
+    p = pkg()
+    from oracle.attn_oracle import Oracle
+    orc = Oracle()
+    H = 3
+    q, k, v, go = to_dev(*(orc.fill_normal((1, S, H * D), 500 + S, i) for i in range(4)))
+    fwd, bwd = (p.forward_bf16, p.backward_bf16) if bf16 else (p.forward, p.backward)
+    if bf16:
+        q, k, v, go = (x.to(torch.bfloat16) for x in (q, k, v, go))
+    prev = p.set_variant(p.VARIANT_TENSOR)
+    try:
+        out, lse = fwd(q, k, v, H, scale, True)
+        d_q, d_k, d_v = bwd(q, k, v, out, go, lse, H, scale, True)[:3]
+        assert p.sync_status() == 0
+    finally:
+        p.set_variant(prev)
+    weights = 1.0 / torch.arange(1, S + 1, device="cuda", dtype=torch.float64)
+    ref = torch.flip(torch.cumsum(torch.flip(go.double() * weights[None, :, None], [1]), 1), [1])
+    tol = 2.0 ** -7 if bf16 else hp.TOL_GRAD_REL_TF32
+    assert float((d_v.double() - ref).abs().max()) <= tol * max(1.0, float(ref.abs().max()))
+    for d in (d_q, d_k):
+        assert float(d.double().abs().max()) <= 1e4 * scale
