@@ -18,6 +18,9 @@
 //   Backward on B200, us, before / now: 8 x 12 x 1024 causal 115 / 109, 1 x 12 x 8192 669 / 577, 2 x 16 x 2000 all keys 228 / 203, 1 x 12 x 512 18.0 / 17.4.
 // dQ kernel: a CTA owns 128 queries (lanes = queries) and walks the key tiles they can see:
 //   S = Q K^T, dP = dO V^T (SS), dS in TMEM, dQ += dS K (TS, K tile MN-major: K is fetched twice).
+//   2.55 K cycles a step where the tensor pipe needs 1.54 K: the latency of the issuing and the compute warps' loops (tensor pipe 58 %, exponentials
+//   39 %, issue slots 33 % busy). The dK/dV kernel's halves and operands in tensor memory gave it 2 % at 8192 rows and cost 1-2 % at 8 x 1024 and 512.
+// One-tile kernel (at the end): up to 128 queries and keys, both halves in one launch.
 // MMA issue: tcgen05 MMAs of one thread execute in issue order, which is what lets single shared-memory stages
 // suffice. The dQ kernel has one MMA warp that interleaves the phases of consecutive tiles (.., S_{j+1}, dP_{j+1},
 // dQ_j, ..: dP has two buffers in tensor memory and runs a step ahead of dQ); the dK/dV kernel has one MMA warp per
@@ -26,7 +29,7 @@
 // Both kernels run a CTA's tiles as one uninterrupted pipeline, heaviest tiles first, and hand finished tiles to the copy engine
 // through shared memory. The dQ kernel deals its tiles out in advance; dK/dV CTAs take over tiles whose CTA has not started, and in a
 // whole-sequence call they start on SMs that the dQ kernel has left, as soon as every row sum is written (pdl_trigger). Measured on
-// B200 against two static kernels in turn, us, H = 12: 1 x 128 14.6 -> 11.9, 1 x 1024 37.3 -> 34.4, 1 x 4096 174 -> 167,
+// B200 against two static kernels in turn, us, H = 12: 1 x 1024 37.3 -> 34.4, 1 x 4096 174 -> 167,
 // 1 x 8192 709 -> 690, 8 x 1024 117.1 -> 116.3 (causal; all keys: -2..+2 %). Tiles that become free at different times land on barriers of their own (K and V in the dK/dV
 // kernel, Q and dO/O in the dQ kernel), so that an item's last accumulating product never queues behind the wait for
 // a tile of the next item that it does not need.

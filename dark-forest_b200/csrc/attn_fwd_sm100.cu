@@ -9,7 +9,7 @@
 // key tiles go to slot A and odd ones to slot B, the halves combined at the end through shared memory (items half as long, twice
 // as many: for few or long items, see split_items). Items are numbered heaviest first, a CTA per item in the grid; a running CTA
 // takes over items whose CTA has not started (cluster launch control), so set-up is paid once per SM and SMs of unequal
-// speed end together. The pipeline (rings, barrier phases) runs on across items.
+// speed end together. The pipeline (rings, barrier phases) runs on across items. fp32 sequences of one tile have a kernel of their own, k_attn_fwd_tile.
 //   warps 0-3   softmax of slot A, warps 4-7 of slot B: a thread owns a query row. It reads its 128 scores from tensor memory, masks
 //               the diagonal tile, keeps a lazily updated running maximum (O and l are rescaled only when the maximum grew by more
 //               than 2^8) and writes P = 2^(s * scale * log2e - m) over S, TF32-rounded or packed bf16, handed over in two halves
