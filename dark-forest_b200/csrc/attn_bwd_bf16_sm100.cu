@@ -35,7 +35,8 @@ struct Bwd16Params {
   const float *delta;
   void *dq, *dk, *dv;   // bf16 or fp32 elements, see Cfg16::OUT_F32
   uint32_t B, H, Sq, Sk;
-  float scale, scale_log2, inv_scale;
+  float scale, scale_log2;
+  float inv_scale, kv_scale_log2;  // dK/dV: one over the scale, and log2 e times the number that inv_scale is one over
   int causal;
   long long shift;
   int early;  // the dQ kernel begins where the dK/dV kernel leaves SMs and waits for it at its end
@@ -337,7 +338,7 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
         }
 #pragma unroll
         for (int x = 0; x < 32; x += 2) {
-          const float2 t = mul2(as_float2(r[x], r[x + 1]), make_float2(p.scale_log2, p.scale_log2));
+          const float2 t = mul2(as_float2(r[x], r[x + 1]), make_float2(p.kv_scale_log2, p.kv_scale_log2));
           pr[c * 32 + x] = ex2_approx(t.x);
           pr[c * 32 + x + 1] = ex2_approx(t.y);
         }
@@ -775,7 +776,11 @@ int launch_backward(const AttnParams &p, cudaStream_t s) {
   bp.B = p.B; bp.H = p.H; bp.Sq = p.Sq; bp.Sk = p.Sk;
   bp.scale = p.scale;
   bp.scale_log2 = p.scale * kLog2e;
-  bp.inv_scale = 1.0f / fmaxf(p.scale, 1e-37f);  // finite, and so is its product with the logsumexp of scores that such a scale has made equal
+  // The dK/dV kernel subtracts lse / scale before it multiplies by the scale, so both go by one number. It is 1e-37 at least: below, lse / scale may be
+  // past fp32, and scale * s is below 1e-37 |s| either way, nothing beside lse unless |s| is 1e30 or more.
+  const float kv_scale = fmaxf(p.scale, 1e-37f);
+  bp.inv_scale = 1.0f / kv_scale;
+  bp.kv_scale_log2 = kv_scale * kLog2e;
   bp.causal = p.causal;
   bp.shift = p.shift;
   bp.status = device_status_ptr();

@@ -44,7 +44,7 @@ def test_one_tile_backward_against_float64(B, H, S, causal):
 
 
 @pytest.mark.parametrize("S,D,bf16", [(100, 64, False), (300, 64, False), (300, 64, True), (300, 128, True)])
-@pytest.mark.parametrize("scale", [1e-30, 1e-35, 3e-37])
+@pytest.mark.parametrize("scale", [1e-30, 1e-35, 3e-37, 5e-38, 2e-38, 1e-40])
 def test_backward_with_a_scale_that_makes_scores_equal(S, D, bf16, scale):
     """The logsumexp enters the score products divided by the scale. Such a scale leaves uniform probabilities, dV = means, and dQ = dK = 0 but for the scale."""
     import torch
