@@ -66,11 +66,11 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 // The issue helpers are called by ALL lanes of the MMA warp; one elected lane issues each instruction (see elect_one).
 // [128 x 128] = A[128 x HD] * B[128 x HD]^T, both K-major tiles of kSlabs 128-byte slabs.
 template <class C>
-__device__ __forceinline__ void issue_ss(uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t idesc, bool accumulate = false) {
+__device__ __forceinline__ void issue_ss(uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t idesc) {
 #pragma unroll
   for (int kk = 0; kk < C::kKSteps; ++kk) {
     const uint64_t off = (uint64_t)(((kk >> 2) * kSlab + (kk & 3) * 32) >> 4);
-    if (elect_one()) mma_f16_ss(d_tmem, da + off, db + off, idesc, accumulate || kk > 0);
+    if (elect_one()) mma_f16_ss(d_tmem, da + off, db + off, idesc, kk > 0);
   }
 }
 // [128 x HD] (+)= A[128 x 128 packed bf16 in TMEM] * B[128 rows (K) x HD (N), MN-major].
@@ -233,15 +233,16 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
     const uint64_t dQm = make_smem_desc(aQ, kSlab, 1024, kSwz128), dGm = make_smem_desc(aG, kSlab, 1024, kSwz128);
     const uint64_t dOnes = make_smem_desc(aK + ones_off<C>(), 128, 256, kSwzNone), dStat = make_smem_desc(aK + stats_off<C>(), 128, 256, kSwzNone);
     const uint32_t stat_dp = C::kSBufs * (kOperand >> 4);
-    // S^T - lse / scale, dP^T - delta: the queries' statistics come in as one more K-step, so that the compute warps do not read them
+    // S^T - lse / scale, dP^T - delta: the queries' statistics come in as one more K-step, so that the compute warps do not read them. The last one: the
+    // accumulator truncates, and sums that begin with lse / scale lose bits of a number of that size each time
     auto scores = [&](bool chain_s, int it) -> bool {
       const int st = it % C::kRing;
       const uint64_t off = (uint64_t)(st * (kTile >> 4));
       if (!mbar_wait_warp(bar((chain_s ? Q_FULL : G_FULL) + st), (it / C::kRing) & 1, abort_flag)) return false;
       tc_fence_after_sync();
       const bool second = C::kSBufs == 2 && (it & 1);
-      if (elect_one()) mma_f16_ss(chain_s ? (second ? tS1 : tS0) : tDP, dOnes, dStat + (chain_s ? (second ? kOperand >> 4 : 0u) : stat_dp), idesc_ss, 0u);
-      issue_ss<C>(chain_s ? (second ? tS1 : tS0) : tDP, chain_s ? dK : dV, (chain_s ? dQk : dGk) + off, idesc_ss, true);
+      issue_ss<C>(chain_s ? (second ? tS1 : tS0) : tDP, chain_s ? dK : dV, (chain_s ? dQk : dGk) + off, idesc_ss);
+      if (elect_one()) mma_f16_ss(chain_s ? (second ? tS1 : tS0) : tDP, dOnes, dStat + (chain_s ? (second ? kOperand >> 4 : 0u) : stat_dp), idesc_ss, 1u);
       commit_elected(bar(chain_s ? S_FULL + (second ? 1 : 0) : DP_FULL));
       if (C::kIssuers == 2) commit_elected(bar((chain_s ? Q_EMPTY : G_EMPTY) + st));
       return true;

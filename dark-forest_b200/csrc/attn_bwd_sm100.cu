@@ -120,15 +120,15 @@ __device__ __forceinline__ TileMN tile_mn(uint32_t tile_smem) {
   return t;
 }
 // To be called by the elected lane only.
-// 8 K-steps added to a 128x64x64 TS MMA: A = 64 TMEM columns, B = 64 rows of a K-major tile of a ring (off: their descriptor offset).
+// 128x64x64 TS MMA, 8 K-steps: A = 64 TMEM columns, B = 64 rows of a K-major tile of a ring (off: their descriptor offset).
 __device__ __forceinline__ void batch_ts_scores(uint32_t d_tmem, uint32_t a_tmem, const TileK &b, uint32_t off, uint32_t idesc) {
 #pragma unroll
-  for (int kk = 0; kk < HD / 8; ++kk) mma_tf32_ts_lohi_acc(d_tmem, a_tmem + kk * 8, b.lo[kk] + off, b.hi, idesc);
+  for (int kk = 0; kk < HD / 8; ++kk) mma_tf32_ts_lohi(d_tmem, a_tmem + kk * 8, b.lo[kk] + off, b.hi, idesc, kk > 0 ? 1u : 0u);
 }
 // The same with A, a whole tile, in shared memory too: what an item's first step takes, before its K (V) is in tensor memory.
 __device__ __forceinline__ void batch_ss_scores(uint32_t d_tmem, const TileK &t, uint32_t a_off, uint32_t b_off, uint32_t idesc) {
 #pragma unroll
-  for (int kk = 0; kk < HD / 8; ++kk) mma_tf32_ss_lohi(d_tmem, t.lo[kk] + a_off, t.hi, t.lo[kk] + b_off, t.hi, idesc, 1u);
+  for (int kk = 0; kk < HD / 8; ++kk) mma_tf32_ss_lohi(d_tmem, t.lo[kk] + a_off, t.hi, t.lo[kk] + b_off, t.hi, idesc, kk > 0 ? 1u : 0u);
 }
 // 8 K-steps from FROM on (half) of a 128x64x128 TS MMA: A = 128 TMEM columns, B = MN-major tile.
 template <int FROM>
@@ -419,7 +419,9 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
     uint32_t g = 0, r = 0;
     bool ok = true;
     // S^T - lse / scale = K Q^T + 1 (-lse / scale), or dP^T - delta, for half h of the queries of the ring's next tile: the queries' statistics, cut in
-    // three TF32 parts, come in as one more K-step, so that the compute warps do not read them (they took a quarter of the warps' time)
+    // three TF32 parts, come in as one more K-step, so that the compute warps do not read them (they took a quarter of the warps' time). It is the last
+    // one: the accumulator truncates, so with the statistics first eight sums lose bits of a number as large as lse / scale, with them last only the
+    // difference is rounded. 2 x 12 x 1000, |lse| 291, mean relative error of dV against float64: first 6.5e-6, last 5e-7, subtracted in fp32 5e-7.
     // `frees`: the item's last, from tensor memory.
     auto issue_first = [&](int h, bool from_smem, bool frees) -> bool {
       const uint32_t slot = r & 1, b_off = slot * (kTile >> 4) + h * (kSlab / 2 >> 4);
@@ -428,9 +430,9 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
         tc_fence_after_sync();
       }
       if (elect_one()) {
-        mma_tf32_ss(tX + h * (BT / 2), dOnes, dStat + h * (kStatTile >> 4), idesc_st, 0u);
         if (from_smem) batch_ss_scores(tX + h * (BT / 2), dB, (slot ^ 1) * (kTile >> 4), b_off, idesc_st);
         else batch_ts_scores(tX + h * (BT / 2), tA, dB, b_off, idesc_st);
+        mma_tf32_ss(tX + h * (BT / 2), dOnes, dStat + h * (kStatTile >> 4), idesc_st, 1u);
         mma_commit(bar((s_chain ? S_FULL : DP_FULL) + h));
         if (h == 1) mma_commit(bar(empty + slot));
         if (h == 1 && frees) mma_commit(bar(s_chain ? K_FREE : V_FREE));

@@ -69,3 +69,21 @@ def test_backward_with_a_scale_that_makes_scores_equal(S, D, bf16, scale):
     assert float((d_v.double() - ref).abs().max()) <= tol * max(1.0, float(ref.abs().max()))
     for d in (d_q, d_k):
         assert float(d.double().abs().max()) <= 1e4 * scale
+
+
+def test_large_logsumexps_leave_no_bias():
+    """The logsumexp is subtracted from scores that are about as large (here |lse| is 290). Operands of eight bits, so that products are exact: what is left
+    are errors of either sign, P's rounding to 2^-12 and the logsumexp's own to 290 * 2^-24 = 1.7e-5 of P, over 24000 rows and 1.5 M elements 3e-7 in
+    the mean, and what the accumulators cut off the scores. Sums that began with lse / scale would lose 6e-6 in the mean."""
+    import torch
+    from test_split_gpu import _reference
+    p = pkg()
+    B, H, S, D = 2, 12, 1000, 64
+    for seed in (1, 2):
+        torch.manual_seed(seed)
+        q, k, v, go = (torch.randn(B, S, H * D, device="cuda").to(torch.bfloat16).float() * f for f in (64.0, 1.0, 1.0, 1.0))
+        _, lse, _, _, ref = _reference(torch, q, k, v, go, H, D ** -0.5, True, 0)
+        out, _ = p.forward(q, k, v, H, D ** -0.5, True)
+        got = p.backward_block(q, k, v, go, lse.float(), p.delta(out, go, H), H, D ** -0.5, True)[2]
+        assert p.sync_status() == 0
+        assert abs(float(((got.double() - ref) * ref).sum() / (ref * ref).sum())) <= 2e-6
