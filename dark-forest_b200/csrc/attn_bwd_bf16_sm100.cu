@@ -301,7 +301,7 @@ k_attn_bwd_dkdv_bf16(const __grid_constant__ CUtensorMap tmK, const __grid_const
 #pragma unroll
       for (int i = 0; i < 3; ++i) {  // each part takes the leading bits that the one before left: exact
         part[i] = __float_as_uint(x) & 0xffff0000u;
-        x -= __uint_as_float(part[i]);
+        x = fabsf(x) == INFINITY ? 0.0f : x - __uint_as_float(part[i]);
       }
       const uint32_t place = stat_lse ? (uint32_t)(it % C::kSBufs) : (uint32_t)C::kSBufs;
       *reinterpret_cast<uint4 *>(smem + stats_off<C>() + place * kOperand + (row >> 3) * 256 + (row & 7) * 16) =

@@ -516,8 +516,8 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
     // What the statistics' K-step adds, -lse / scale (-inf for a row without visible keys: P = 0) or -delta, in three TF32 parts
     auto stage = [&](float raw) {
       const float x = stat_lse ? -raw * p.inv_scale : -raw;
-      const bool none = stat_lse && fabsf(raw) == INFINITY;
-      const float hi = none ? -INFINITY : __uint_as_float(cvt_rna_tf32(x)), rest = none ? 0.0f : x - hi, mid = __uint_as_float(cvt_rna_tf32(rest));
+      const float hi = stat_lse && fabsf(raw) == INFINITY ? -INFINITY : __uint_as_float(cvt_rna_tf32(x));
+      const float rest = fabsf(hi) == INFINITY ? 0.0f : x - hi, mid = __uint_as_float(cvt_rna_tf32(rest));
       const uint32_t q = (uint32_t)row & 63;
       *reinterpret_cast<float4 *>(smem + kStats + ((stat_lse ? 0 : 2) + sub) * kStatTile + (q >> 3) * 256 + (q & 7) * 16) = make_float4(hi, mid, rest - mid, 0.0f);
       fence_proxy_async_smem();

@@ -87,3 +87,23 @@ def test_large_logsumexps_leave_no_bias():
         got = p.backward_block(q, k, v, go, lse.float(), p.delta(out, go, H), H, D ** -0.5, True)[2]
         assert p.sync_status() == 0
         assert abs(float(((got.double() - ref) * ref).sum() / (ref * ref).sum())) <= 2e-6
+
+
+@pytest.mark.parametrize("D,bf16", [(64, False), (64, True), (128, True)])
+def test_an_infinite_row_sum_stays_infinite(D, bf16):
+    """delta = inf of one query: its dS is -inf at every key that it sees, and so is dK, with the sign of its Q (or NaN at Q = 0)."""
+    import torch
+    p = pkg()
+    S, H, row = 200, 2, 77
+    torch.manual_seed(3)
+    q, k, v, go = (torch.randn(1, S, H * D, device="cuda") for _ in range(4))
+    q = torch.where(q == 0, 1.0, q)
+    f = (lambda x: x.to(torch.bfloat16)) if bf16 else (lambda x: x)
+    q, k, v, go = map(f, (q, k, v, go))
+    out, lse = (p.forward_bf16 if bf16 else p.forward)(q, k, v, H, D ** -0.5, False)
+    delta = (p.delta_bf16 if bf16 else p.delta)(out, go, H)
+    delta[0, 1, row] = float("inf")
+    d_k, d_v = (p.backward_block_bf16 if bf16 else p.backward_block)(q, k, v, go, lse, delta, H, D ** -0.5, False)[1:3]
+    assert p.sync_status() == 0
+    assert torch.isfinite(d_v).all() and torch.isfinite(d_k[..., :D]).all()
+    assert torch.equal(d_k[0, :, D:].float(), (-torch.sign(q[0, row, D:].float()) * float("inf")).expand(S, D))
