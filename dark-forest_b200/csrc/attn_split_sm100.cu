@@ -1,16 +1,21 @@
 // attn_split_sm100.cu - fp32 attention in full fp32 precision on the tensor cores (sm_100a), for head sizes that the TF32 kernels do not take.
 //
 // Same mathematics as attn_simt.cu (darkforest-cuda/kernels/attention_fused.cu:41-159, 390-516), for sequences of more than kMinSteps - 1 steps.
-// Every fp32 operand is cut into three bf16 parts, a = a1 + a2 + a3: each takes the leading eight significant bits that the one before left, so
-// the cut is exact. A product is the six products of parts whose weights sum to at most 2^-16 (a1 b1, a1 b2, a2 b1, a2 b2, a1 b3, a3 b1), the small
-// ones first; what is left out is below 2^-23 of |a| |b|. The tensor cores add into fp32 with truncation, so sums there are kept short: a step's 64
-// rows are contracted in tensor memory and added to fp32 registers, rounded to nearest, and scores have two accumulators, one of which takes
+// Every fp32 operand is cut into three bf16 parts, a = a1 + a2 + a3, each what is left rounded to bf16: |a2| <= 2^-8 |a|, |a3| <= 2^-17 |a|, and nothing
+// is left after the third. A product is six of the nine products of parts (a1 b1, a1 b2, a2 b1, a2 b2, a1 b3, a3 b1), the small ones first; what is left
+// out, a2 b3 + a3 b2 + a3 b3, is at most 2^-24 of |a| |b| and of either sign. (Parts cut off by truncation would leave out up to 2^-21, always of the sign
+// of a b: dQ 10.4e-7 off with operands near 1 + 2^-7, 2.0e-7 rounded.) The tensor cores add into fp32 with truncation, so sums there are kept short: a
+// step's 64 rows are contracted in tensor memory and added to fp32 registers, rounded to nearest, and scores have two accumulators, one of which takes
 // only half of the largest product. An infinity among the operands gives NaN where it is used (its later parts are inf - inf).
 // Relative error (2-norm) against 64 bits, normal inputs, this / attn_simt.cu, in 1e-7:
-//   B x H x S x D, causal          O            dQ           dK           dV
-//   2 x 8 x 1000 x 128             1.9 / 2.7    3.9 / 4.1    4.2 / 7.9    3.1 / 7.8
-//   2 x 6 x  400 x  32             1.5 / 1.8    3.3 / 3.0    3.6 / 5.0    2.7 / 5.0
-//   1 x 8 x  333 x  80             2.0 / 2.0    3.9 / 3.2    4.1 / 4.9    3.1 / 4.7
+//   B x H x S x D                  O            logsumexp      dQ           dK           dV
+//   2 x 8 x 1000 x 128, causal     1.3 / 2.7    0.31 / 0.28    2.7 / 4.1    3.1 / 8.0    2.5 / 7.8
+//   2 x 6 x  400 x  32, causal     1.0 / 1.8    0.30 / 0.29    2.2 / 3.1    2.5 / 5.1    2.2 / 5.0
+//   1 x 8 x  333 x  80, causal     1.4 / 1.9    0.38 / 0.34    2.7 / 3.2    2.9 / 4.9    2.4 / 4.7
+//   1 x 4 x  260 x 112             1.5 / 3.2    0.29 / 0.33    2.7 / 4.4    2.8 / 4.8    2.5 / 4.6
+//   1 x 4 x 300 x 128, causal, operands near 1 + 2^-7
+//                                  1.0 / 2.3    0.30 / 0.34    2.0 / 3.4    2.3 / 4.9    1.8 / 4.7
+// (of the logsumexp 0.22 are its own rounding to fp32)
 //
 // Four passes from one text, `Pass`:
 //               resident rows A1, A2    streamed rows B1, B2    T (per step)                        result R
@@ -154,13 +159,12 @@ __device__ __forceinline__ void store_cluster(uint32_t addr, float4 v) {
 }
 __device__ __forceinline__ float2 f2(uint32_t x, uint32_t y) { return as_float2(x, y); }
 
-// Cuts two values: out[part] = (part of y) << 16 | part of x. An infinity gives NaN in the second part, and so does a NaN.
+// Cuts two values: out[part] = (part of y) << 16 | part of x. An infinity (or what rounds to one) gives one in the second part, and so NaN; a NaN does.
 __device__ __forceinline__ void cut(float2 x, uint32_t (&out)[3]) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    const uint32_t ux = __float_as_uint(x.x), uy = __float_as_uint(x.y);
-    out[i] = __byte_perm(ux, uy, 0x7632);
-    if (i < 2) x = fma2(f2(ux & 0xffff0000u, uy & 0xffff0000u), make_float2(-1.f, -1.f), x);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(out[i]) : "f"(x.y), "f"(x.x));
+    if (i < 2) x = fma2(f2(out[i] << 16, out[i] & 0xffff0000u), make_float2(-1.f, -1.f), x);
   }
 }
 // 16 rows x 32 values of a warp, as fragments, into the parts of an A operand in tensor memory; what does not go there is left in w[2].
@@ -402,7 +406,7 @@ __device__ __forceinline__ void split_block(const AttnParams &p, uint32_t tile, 
     const uint32_t lanes = (uint32_t)base16 << 16;
     const long long rowA = row0 + base16 + (lane >> 2), rowB = rowA + 8;  // this lane's two rows
     const size_t res_base = C::ROWS_ARE_KEYS ? k_base : q_base;
-    const float scale2 = p.scale * kLog2e;
+    const float scale2 = p.scale_log2;
     // resident tiles: two parts into tensor memory, the third into shared memory
     auto load_resident = [&](const float *src, uint32_t cols, uint32_t third) {
       const uint32_t rA = (uint32_t)(base16 + (lane >> 2)), rB = rA + 8;  // the same modulo 8
@@ -760,12 +764,20 @@ bool allow_smem(uint32_t bytes) {
   return ok[dev];
 }
 
+// What the kernels take from the host beside the caller's parameters. The factor of the scores is rounded once: its error is in every one of them (1 x 4 x
+// 260 x 112: O 2.2e-7 off with scale * log2 e from two roundings, 1.5e-7 so). Formed on the device the same number cost 3-6 %
+// at some head sizes, by other allocations of registers.
+void set_by_host(AttnParams *p) {
+  p->scale_log2 = (float)((double)p->scale * 1.4426950408889634);
+  p->status = device_status_ptr();
+}
+
 template <int DP, int CL>
 int forward_form(AttnParams p, cudaStream_t s) {
   constexpr uint32_t smem = Cfg<DP, FORWARD>::kSmem;
   if (!allow_smem<k_split_fwd<DP, CL>>(smem)) return DF_ERR_CUDA;
   const uint32_t tiles = (p.Sq + BM - 1) / BM;
-  p.status = device_status_ptr();
+  set_by_host(&p);
   launch_clusters(k_split_fwd<DP, CL>, CL > 1 ? CL : 0, dim3(CL * tiles * p.B * p.H), dim3(kThreads), smem, s, p, tiles);
   note_launch();
   return check_cuda(cudaGetLastError());
@@ -775,7 +787,7 @@ int backward_form(AttnParams p, cudaStream_t s) {
   constexpr uint32_t a = Cfg<DP, DK>::kSmem, b = Cfg<DP, DV>::kSmem, smem = a > b ? a : b;
   if (!allow_smem<k_split_bwd<DP, CL>>(smem)) return DF_ERR_CUDA;
   const uint32_t kt = (p.Sk + BM - 1) / BM, qt = (p.Sq + BM - 1) / BM;
-  p.status = device_status_ptr();
+  set_by_host(&p);
   launch_clusters(k_split_bwd<DP, CL>, CL > 1 ? CL : 0, dim3(CL * (2 * kt + qt) * p.B * p.H), dim3(kThreads), smem, s, p, kt, qt);
   note_launch();
   return check_cuda(cudaGetLastError());
@@ -790,7 +802,8 @@ int backward_by_cluster(const AttnParams &p, int cl, cudaStream_t s) {
 }
 
 // From four steps (193 keys) on. Up to two steps attn_simt.cu is as fast (1 x 4 x 100 x 96: forward 9.9 there, 11.1 here; backward 16.8, 14.8); at three it
-// takes 1.3 times as long, but its sums are still short and dQ is more exact there (D = 128, S = 130: 3.3e-7 against 3.8e-7).
+// takes 1.3 times as long, but its sums are still short and dQ was more exact there when the parts here were cut by truncation (D = 128, S = 130: 3.3e-7
+// against 3.8e-7).
 constexpr uint64_t kMinSteps = 4;
 // The longest block's steps, for queries as resident rows and for keys.
 uint64_t query_steps(const AttnParams &p) {

@@ -43,7 +43,8 @@ struct AttnParams {
   float scale = 1.0f;
   int causal = 0;
   long long shift = 0;  // key j visible to query i iff !causal or j <= i + shift
-  unsigned int *status = nullptr;  // device status word (checked builds of the SIMT kernels; set by their launchers)
+  unsigned int *status = nullptr;  // device status word (set by the launchers of the kernels that use it)
+  float scale_log2 = 0.0f;         // scale * log2 e (attn_split_sm100.cu; set by its launchers)
 };
 
 // Sticky per-thread status and launch counter (defined in attn_api.cu).

@@ -59,3 +59,34 @@ def test_split_against_float64(B, H, Sq, Sk, causal, shift, D):
     finally:
         p.set_variant(prev)
     assert not torch.equal(got[4], other[4])  # dV: the rule did choose another kernel
+
+
+# operands: normal; just above 1 + 2^-8 and 1 + 2^-7 in size, where the second and third of three bf16 parts are largest; scores of +-30 and more
+@pytest.mark.parametrize("operands", ["normal", "1+2^-8", "1+2^-7", "large scores"])
+@pytest.mark.parametrize("B,H,S,D,causal", [(2, 6, 400, 32, True), (1, 8, 333, 80, True), (2, 8, 1000, 128, True), (1, 4, 260, 112, False), (1, 4, 1300, 48, True)])
+def test_split_is_as_exact_as_fp32_arithmetic(B, H, S, D, causal, operands):
+    """Error against float64 (2-norm, relative), next to that of the kernel that computes in fp32 throughout: no larger in O and the gradients. The
+    logsumexp bears the rounding of scale * log2 e (2^-24 of the scores at most) and its own (2^-24 of itself): 2^-23."""
+    import torch
+    p = pkg()
+    torch.manual_seed(S + D)
+    x = [torch.randn(B, S, H * D, device="cuda") for _ in range(4)]
+    if operands.startswith("1+"):
+        x = [torch.sign(t) * (1 + 2.0 ** -int(operands[-1]) + 2.0 ** -23 * torch.randint(-99, 100, t.shape, device="cuda")) for t in x]
+    elif operands == "large scores":
+        x[0] *= 10
+    q, k, v, go = x
+    scale = hp.default_scale(D)
+    ref = _reference(torch, q, k, v, go, H, scale, causal, 0)
+    errors = []
+    for variant in (p.VARIANT_AUTO, p.VARIANT_SIMT):
+        prev = p.set_variant(variant)
+        try:
+            out, lse = p.forward(q, k, v, H, scale, causal)
+            got = (out, lse) + tuple(p.backward(q, k, v, out, go, lse, H, scale, causal)[:3])
+            assert p.sync_status() == 0
+        finally:
+            p.set_variant(prev)
+        errors.append([float((g.double() - r).norm() / r.norm()) for g, r in zip(got, ref)])
+    for name, a, b in zip(("out", "lse", "dq", "dk", "dv"), *errors):
+        assert a <= (2.0 ** -23 if name == "lse" else b), (name, a, b)
