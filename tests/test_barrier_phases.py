@@ -1,9 +1,10 @@
-"""Barrier phases of the backward kernels, on the CPU.
+"""Barrier phases of the backward kernels and of the split fp32 kernels, on the CPU.
 
 A wait on an mbarrier names a phase by its parity, so a waiter must never be two phases behind: the phase it waits for would look
 as if it had not come yet, and never come again. Nor may it come two phases early: the phase before the last would pass for the one it
 waits for. The roles of a kernel are written down here as the waits and arrivals they make; for every wait of every role, that role is held
-there while all others run as far as they can, and for every arrival the arriving role is held ahead of it.
+there while all others run as far as they can, and for every arrival the arriving role is held ahead of it. Places that no barrier of their own
+guards (row statistics) are marked where they are written and read, and roles are held at the marks.
 """
 import os
 import re
@@ -21,6 +22,9 @@ class Role(list):
 
     def arrive(self, bar):
         self.append(("arrive", bar, 0))
+
+    def mark(self, what, k):
+        self.append(("mark", what, k))
 
 
 def dq_tf32(items, ds_bars):
@@ -228,6 +232,169 @@ def dkdv_tf32(items):
     return roles
 
 
+def dkdv_bf16(n_it, issuers, s_bufs, ring=4):
+    """k_attn_bwd_dkdv_bf16: two issuing warps and two S^T buffers (head dimension 64), or one of each (128); two threads stand for each half of the
+    compute warps, the one that stages lse and the one that stages delta."""
+    load_q, load_g, chains = Role(), Role(), [Role() for _ in range(issuers)]
+    for it in range(n_it):
+        for role, tile in ((load_q, "Q"), (load_g, "G")):
+            if it >= ring:
+                role.wait("%s_EMPTY%d" % (tile, it % ring), it // ring - 1)
+            role.arrive("%s_FULL%d" % (tile, it % ring))
+
+    def scores(role, chain_s, it):
+        tile = "Q" if chain_s else "G"
+        role.wait("%s_FULL%d" % (tile, it % ring), it // ring)
+        role.mark("lse used" if chain_s else "delta used", it)
+        role.arrive("S_FULL%d" % (it % s_bufs) if chain_s else "DP_FULL")
+        if issuers == 2:
+            role.arrive("%s_EMPTY%d" % (tile, it % ring))
+
+    def gradient(role, chain_s, it):
+        tile = "G" if chain_s else "Q"
+        if issuers == 2:
+            role.wait("%s_FULL%d" % (tile, it % ring), it // ring)
+        role.wait("P_FULL%d" % (it % s_bufs), it // s_bufs) if chain_s else role.wait("DS_FULL", it)
+        role.arrive("%s_EMPTY%d" % (tile, it % ring))
+
+    for role in chains:
+        role.wait("FIRST", 0)
+    if issuers == 2:
+        for role, chain_s in zip(chains, (True, False)):
+            ahead = s_bufs if chain_s else 1
+            for it in range(min(ahead, n_it)):
+                scores(role, chain_s, it)
+            for it in range(n_it):
+                gradient(role, chain_s, it)
+                if it + ahead < n_it:
+                    scores(role, chain_s, it + ahead)
+    else:
+        scores(chains[0], True, 0)
+        scores(chains[0], False, 0)
+        for it in range(n_it):
+            for chain_s in (True, False):
+                gradient(chains[0], chain_s, it)
+                if it + 1 < n_it:
+                    scores(chains[0], chain_s, it + 1)
+    for role in chains:
+        role.arrive("ACC_FULL")
+
+    def half(lse):
+        role, ahead, stat = Role(), s_bufs if lse else 1, "lse" if lse else "delta"
+        for it in range(min(ahead, n_it)):
+            role.mark(stat + " staged", it)
+        role.arrive("FIRST")
+        for it in range(n_it):
+            more = it + ahead < n_it
+            role.wait("S_FULL%d" % (it % s_bufs), it // s_bufs)
+            if lse and more:
+                role.mark("lse staged", it + ahead)
+            role.arrive("P_FULL%d" % (it % s_bufs))
+            role.wait("DP_FULL", it)
+            if not lse and more:
+                role.mark("delta staged", it + ahead)
+            role.arrive("DS_FULL")
+        role.wait("ACC_FULL", 0)
+        return role
+
+    roles = {"load_q": load_q, "load_g": load_g, **{"issuer %d" % i: role for i, role in enumerate(chains)}}
+    roles.update({"%s %s" % (name, x): half(name == "lse") for name in ("lse", "delta") for x in "ab"})
+    return roles
+
+
+def split(n, two, keys, st2):
+    """split_block of attn_split_sm100.cu with n steps. two: DQ and DK, else FORWARD and DV; keys: resident rows are keys (DK, DV), whose steps bring
+    row statistics; st2: buffers of the second streamed tile. Two threads stand for the streaming warps, two for the compute warps."""
+    def stage2(j):
+        return j % st2, j // st2
+
+    def stream():
+        role = Role()
+        for j in range(n):
+            for tile, (st, use) in (("B1", (j % 2, j // 2)), ("B2", stage2(j))):
+                if use > 0:
+                    role.wait("%s_EMPTY%d" % (tile, st), use - 1)
+                role.arrive("%s_FULL%d" % (tile, st))
+        return role
+
+    mma = Role()
+
+    def scores(j):
+        mma.wait("B1_FULL%d" % (j % 2), j // 2)
+        if j > 0:
+            mma.wait("R_FREE" if two else "S_FREE", j - 1)
+        mma.arrive("S_FULL0" if two else "S_FULL%d" % (j % 2))
+        if not two:
+            mma.arrive("B1_EMPTY%d" % (j % 2))
+
+    def dp(j):
+        st, use = stage2(j)
+        mma.wait("B2_FULL%d" % st, use)
+        mma.arrive("DP_FULL")
+        mma.arrive("B2_EMPTY%d" % st)
+
+    def result(j):
+        st, use = stage2(j)
+        if two:
+            mma.wait("T_FULL0", j)
+            mma.wait("T_FULL1", j)
+        else:
+            mma.wait("T_FULL%d" % (j % 2), j // 2)
+            mma.wait("B2_FULL%d" % st, use)
+            if j > 0:
+                mma.wait("R_FREE", j - 1)
+        mma.arrive("R_FULL")
+        mma.arrive("B1_EMPTY%d" % (j % 2) if two else "B2_EMPTY%d" % st)
+
+    mma.wait("A_READY", 0)
+    scores(0)
+    for j in range(n):
+        if two:
+            dp(j)
+            result(j)
+        if j + 1 < n:
+            scores(j + 1)
+        if not two:
+            result(j)
+
+    def compute():
+        role = Role()
+
+        def add_r(j):
+            role.wait("R_FULL", j)
+            role.arrive("R_FREE")
+
+        def stats(j):
+            role.mark("stats written", j)
+            role.arrive("STAT_FULL")
+
+        role.arrive("A_READY")
+        if keys:
+            stats(0)
+        for j in range(n):
+            if two and j > 0:
+                add_r(j - 1)
+            if keys:
+                role.wait("STAT_FULL", j)
+            role.wait("S_FULL0" if two else "S_FULL%d" % (j % 2), j if two else j // 2)
+            if not two:
+                role.arrive("S_FREE")
+            else:
+                role.wait("DP_FULL", j)
+            if keys:
+                role.mark("stats read", j)
+            for x in (0, 1) if two else (j % 2,):
+                role.arrive("T_FULL%d" % x)
+            if keys and j + 1 < n:
+                stats(j + 1)
+            if not two and j > 0:
+                add_r(j - 1)
+        add_r(n - 1)
+        return role
+
+    return {"stream 0": stream(), "stream 1": stream(), "mma": mma, "compute 0": compute(), "compute 1": compute()}
+
+
 def _runner(roles):
     counts = {}
     for name, role in roles.items():
@@ -284,6 +451,17 @@ def phases_early(roles):
     return early
 
 
+def out_of_order(roles, first, second, lag=0):
+    """Marks (second, k + lag) that a role can come to while another is still ahead of its mark (first, k)."""
+    run, found = _runner(roles), set()
+    for held, role in roles.items():
+        for at, (op, what, k) in enumerate(role):
+            if (op, what) == ("mark", first):
+                pos, _ = run(held, at)
+                found |= {(name, second, k + lag) for name, other in roles.items() if name != held and ("mark", second, k + lag) in other[:pos[name]]}
+    return found
+
+
 def test_one_barrier_for_two_buffers_is_missed():
     assert ("mma", "DS_FULL0") in {m[:2] for m in phases_missed(dq_tf32([4], 1))}
     assert ("dp_dq", "DS_FULL0") in {m[:2] for m in phases_missed(dq_bf16(4, 1))}
@@ -316,3 +494,37 @@ def test_bf16_dq_waits_see_every_phase(n_kv):
         at[name] = value
     ds_bars = min(v for v in at.values() if v > at["DS_FULL"]) - at["DS_FULL"]
     assert phases_missed(dq_bf16(n_kv, ds_bars)) == []
+
+
+# head dimension 64: two issuers, two S^T buffers; 128: one of each
+@pytest.mark.parametrize("issuers,s_bufs", [(2, 2), (1, 1)])
+@pytest.mark.parametrize("n_it", [1, 2, 3, 5, 11])
+def test_bf16_dkdv_waits_see_their_phase_and_statistics_stay_until_used(n_it, issuers, s_bufs):
+    with open(os.path.join(CSRC, "attn_bwd_bf16_sm100.cu")) as f:
+        text = f.read()
+    assert re.search(r"kIssuers = HD_ == 64 \? 2 : 1;", text) and re.search(r"kSBufs = HD_ == 64 \? 2 : 1;", text)
+    roles = dkdv_bf16(n_it, issuers, s_bufs)
+    assert phases_missed(roles) == []
+    assert phases_early(roles) == set()
+    for stat, places in (("lse", s_bufs), ("delta", 1)):
+        assert out_of_order(roles, stat + " staged", stat + " used") == set()
+        assert out_of_order(roles, stat + " used", stat + " staged", places) == set()
+    if n_it > s_bufs > 1:  # one place would not do
+        assert out_of_order(roles, "lse used", "lse staged", 1) != set()
+
+
+# passes (FORWARD, DV, DQ, DK) by the head sizes' buffers of the second streamed tile
+@pytest.mark.parametrize("two,keys,st2", [(False, False, 2), (False, True, 2), (True, False, 2), (True, True, 2), (True, False, 1), (True, True, 1)])
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 9])
+def test_split_waits_see_their_phase_and_statistics_stay_until_read(n, two, keys, st2):
+    with open(os.path.join(CSRC, "attn_split_sm100.cu")) as f:
+        text = f.read()
+    assert "ST1 = 2, ST2 = TWO && SLABS == 2 ? 1 : 2;" in text and "sStats + (j % 3) * C::NSTATS * BN" in text
+    roles = split(n, two, keys, st2)
+    assert phases_missed(roles) == []
+    assert phases_early(roles) == set()
+    if keys:
+        assert out_of_order(roles, "stats written", "stats read") == set()
+        assert out_of_order(roles, "stats read", "stats written", 3) == set()
+        if n > 1:
+            assert out_of_order(roles, "stats read", "stats written", 1) != set()  # one buffer would not do
