@@ -6,7 +6,8 @@
 // out, a2 b3 + a3 b2 + a3 b3, is at most 2^-24 of |a| |b| and of either sign. (Parts cut off by truncation would leave out up to 2^-21, always of the sign
 // of a b: dQ 10.4e-7 off with operands near 1 + 2^-7, 2.0e-7 rounded.) The tensor cores add into fp32 with truncation, so sums there are kept short: a
 // step's 64 rows are contracted in tensor memory and added to fp32 registers, rounded to nearest, and scores have two accumulators, one of which takes
-// only half of the largest product. An infinity among the operands gives NaN where it is used (its later parts are inf - inf).
+// only half of the largest product. The bounds hold for operands of 2^-101 and more, where all parts are normal numbers; a smaller one loses bits that are
+// below 2^-133. An infinity has no parts (inf - inf), so rows with a result that is not finite are formed again in fp32 arithmetic (fp32_row).
 // Relative error (2-norm) against 64 bits, normal inputs, this / attn_simt.cu, in 1e-7:
 //   B x H x S x D                  O            logsumexp      dQ           dK           dV
 //   2 x 8 x 1000 x 128, causal     1.3 / 2.7    0.31 / 0.28    2.7 / 4.1    3.1 / 8.0    2.5 / 7.8
@@ -191,6 +192,79 @@ template <int STEPS, class FA, class F>
 __device__ __forceinline__ void product_ss(uint32_t d, uint32_t a_lo, uint32_t a_hi, FA a_step, uint32_t b_lo, uint32_t b_hi, F b_step, uint32_t idesc, uint32_t mine) {
 #pragma unroll
   for (int kk = 0; kk < STEPS; ++kk) mma_ss(d, a_lo + (a_step(kk) >> 4), a_hi, b_lo + (b_step(kk) >> 4), b_hi, idesc, 1u, mine);
+}
+
+// logsumexp in log2 units, negated, in two fp32 numbers: rounded to one, ten times 2^-24 of it goes into every P. No visible key: P = 0.
+__device__ __forceinline__ float neg_lse2(float raw, float *lo) {
+  const float hi = raw * kLog2e;
+  *lo = fabsf(hi) < INFINITY ? -fmaf(raw, 1.92596299e-8f, fmaf(raw, kLog2e, -hi)) : 0.f;  // log2 e = kLog2e + 1.926e-8
+  return raw == -INFINITY ? -INFINITY : -hi;
+}
+
+// One row of a pass in fp32 arithmetic by one warp: the visible streamed rows and no others. An infinity has no parts, and a hidden row's infinity or
+// NaN times a P of zero is NaN too, so what is not finite in a block's results says nothing yet about what the row should be. It is no fast path (a
+// block of 128 rows, D = 128, takes about as long as in attn_simt.cu), nor has it to be one: operands are finite in earnest.
+template <Pass PASS>
+__device__ __forceinline__ void fp32_row(const AttnParams &p, size_t q_base, size_t k_base, size_t s_base, long long row) {
+  constexpr bool KEYS = PASS == DK || PASS == DV, TWO = PASS == DQ || PASS == DK;
+  const uint32_t lane = threadIdx.x & 31;
+  const size_t dm = (size_t)p.H * p.D, res = (KEYS ? k_base : q_base) + (size_t)row * dm, str = KEYS ? q_base : k_base;
+  const float *a1 = (KEYS ? p.k : p.q) + res, *a2 = TWO ? (KEYS ? p.v : p.d_out) + res : a1, *b1 = (KEYS ? p.q : p.k) + str, *b2 = (KEYS ? p.d_out : p.v) + str;
+  long long from = 0, to = KEYS ? p.Sq : p.Sk;
+  if (p.causal && KEYS && row > p.shift) from = row - p.shift;
+  if (p.causal && !KEYS && row + p.shift + 1 < to) to = row + p.shift + 1;
+  auto dot = [&](const float *x, const float *y) {
+    float2 sum = make_float2(0.f, 0.f);
+#pragma unroll 1
+    for (uint32_t d = 0; d < p.D; d += 4) {
+      const float4 u = *reinterpret_cast<const float4 *>(x + d), w = *reinterpret_cast<const float4 *>(y + d);
+      sum = fma2(make_float2(u.z, u.w), make_float2(w.z, w.w), fma2(make_float2(u.x, u.y), make_float2(w.x, w.y), sum));
+    }
+    return sum.x + sum.y;
+  };
+  float m = -INFINITY, l = 0.f, neg = 0.f, lo = 0.f, delta = 0.f;
+  if (PASS == DQ) {
+    neg = neg_lse2(p.lse_in[s_base + row], &lo);
+    delta = p.delta_in[s_base + row];
+  }
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);  // dims 4 lane .. + 3
+#pragma unroll 1
+  for (long long c = from; c < to; c += 32) {
+    const long long j = c + lane;
+    const bool seen = j < to;
+    float t = 0.f;
+    const float s = seen ? dot(a1, b1 + (size_t)j * dm) * p.scale_log2 : -INFINITY;
+    if (PASS == FORWARD) {
+      float top = s;
+#pragma unroll
+      for (int o = 16; o >= 1; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+      const float mn = fmaxf(m, top), alpha = mn == -INFINITY ? 1.f : ex2_approx(m - mn);
+      m = mn;
+      t = ex2_approx(s - (m == -INFINITY ? 0.f : m));
+      float sum = t;
+#pragma unroll
+      for (int o = 16; o >= 1; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      l = fmaf(l, alpha, sum);
+      acc = make_float4(acc.x * alpha, acc.y * alpha, acc.z * alpha, acc.w * alpha);
+    } else if (seen) {
+      if (KEYS) neg = neg_lse2(p.lse_in[s_base + j], &lo);
+      if (PASS == DK) delta = p.delta_in[s_base + j];
+      t = ex2_approx(s + neg + lo);
+      if (TWO) t *= dot(a2, b2 + (size_t)j * dm) - delta;
+    }
+#pragma unroll 1
+    for (int x = 0; x < 32 && c + x < to; ++x) {
+      const float tx = __shfl_sync(0xffffffffu, t, x);
+      if (4 * lane < p.D) {
+        const float4 y = *reinterpret_cast<const float4 *>((TWO ? b1 : b2) + (size_t)(c + x) * dm + 4 * lane);
+        acc = make_float4(fmaf(tx, y.x, acc.x), fmaf(tx, y.y, acc.y), fmaf(tx, y.z, acc.z), fmaf(tx, y.w, acc.w));
+      }
+    }
+  }
+  const float f = PASS == FORWARD ? (l > 0.f ? 1.f / l : 0.f) : PASS == DV ? 1.f : p.scale;  // reference guard, attention_fused.cu:104
+  float *dst = (PASS == FORWARD ? p.out : PASS == DQ ? p.d_q : PASS == DK ? p.d_k : p.d_v) + res;
+  if (4 * lane < p.D) *reinterpret_cast<float4 *>(dst + 4 * lane) = make_float4(acc.x * f, acc.y * f, acc.z * f, acc.w * f);
+  if (PASS == FORWARD && p.lse && lane == 0) p.lse[s_base + row] = l > 0.f ? fmaf(m, kLn2, logf(l)) : -INFINITY;
 }
 
 // One block of 128 resident rows. A cluster of CL CTAs shares it: each takes a range of the steps, rank 0 puts the results together.
@@ -441,12 +515,6 @@ __device__ __forceinline__ void split_block(const AttnParams &p, uint32_t tile, 
     // row statistics: of this lane's rows (queries), or staged for a step's queries one step ahead, in one of three buffers (a thread past the wait
     // of step j knows that all others are past step j - 2)
     float mA = -INFINITY, mB = -INFINITY, lA = 0.f, lB = 0.f, dA = 0.f, dB = 0.f;
-    // logsumexp in log2 units, negated, in two fp32 numbers: rounded to one, ten times 2^-24 of it goes into every P. No visible key: P = 0.
-    auto neg_lse2 = [](float raw, float *lo) -> float {
-      const float hi = raw * kLog2e;
-      *lo = fabsf(hi) < INFINITY ? -fmaf(raw, 1.92596299e-8f, fmaf(raw, kLog2e, -hi)) : 0.f;  // log2 e = kLog2e + 1.926e-8
-      return raw == -INFINITY ? -INFINITY : -hi;
-    };
     float fA = p.scale, fB = p.scale;  // factors of the results
     if (PASS == DQ) {
       if (rowA < n_res) { mA = p.lse_in[s_base + rowA]; dA = -p.delta_in[s_base + rowA]; }
@@ -678,16 +746,30 @@ __device__ __forceinline__ void split_block(const AttnParams &p, uint32_t tile, 
         }
         fA = lA > 0.f ? 1.f / lA : 0.f;  // reference guard, attention_fused.cu:104
         fB = lB > 0.f ? 1.f / lB : 0.f;
-        if (p.lse && t4 == 0) {
-          if (rowA < n_res) p.lse[s_base + rowA] = lA > 0.f ? fmaf(mA, kLn2, logf(lA)) : -INFINITY;
-          if (rowB < n_res) p.lse[s_base + rowB] = lB > 0.f ? fmaf(mB, kLn2, logf(lB)) : -INFINITY;
-        }
+      }
+      // rows with a result or a sum that is not finite (0 * x is NaN): a bit for each, lane 4 i of rows A and B
+      float2 oddA = make_float2(lA * 0.f, 0.f), oddB = make_float2(lB * 0.f, 0.f);
+#pragma unroll
+      for (int g = 0; g < DP / 8; ++g) {
+        oddA = fma2(acc[2 * g], make_float2(0.f, 0.f), oddA);
+        oddB = fma2(acc[2 * g + 1], make_float2(0.f, 0.f), oddB);
+      }
+      auto row_bits = [](bool x) {
+        uint32_t bits = __ballot_sync(0xffffffffu, x);
+        bits |= bits >> 1;
+        return (bits | bits >> 2) & 0x11111111u;
+      };
+      const uint32_t bitsA = row_bits(rowA < n_res && !(oddA.x + oddA.y == 0.f)), bitsB = row_bits(rowB < n_res && !(oddB.x + oddB.y == 0.f));
+      const bool storeA = rowA < n_res && !(bitsA >> (lane & 28) & 1u), storeB = rowB < n_res && !(bitsB >> (lane & 28) & 1u);
+      if (PASS == FORWARD && p.lse && t4 == 0) {
+        if (storeA) p.lse[s_base + rowA] = lA > 0.f ? fmaf(mA, kLn2, logf(lA)) : -INFINITY;
+        if (storeB) p.lse[s_base + rowB] = lB > 0.f ? fmaf(mB, kLn2, logf(lB)) : -INFINITY;
       }
       float *dst = PASS == FORWARD ? p.out : PASS == DQ ? p.d_q : PASS == DK ? p.d_k : p.d_v;
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         const long long row = half ? rowB : rowA;
-        if (row >= n_res) continue;
+        if (!(half ? storeB : storeA)) continue;
         const float f = half ? fB : fA;
         float *at = dst + res_base + (size_t)row * dm;
 #pragma unroll
@@ -696,6 +778,9 @@ __device__ __forceinline__ void split_block(const AttnParams &p, uint32_t tile, 
           if (d < (int)p.D) *reinterpret_cast<float2 *>(at + d) = make_float2(acc[2 * g + half].x * f, acc[2 * g + half].y * f);
         }
       }
+#pragma unroll 1
+      for (int r = 0; r < 16; ++r)
+        if (((r < 8 ? bitsA : bitsB) >> (4 * (r & 7))) & 1u) fp32_row<PASS>(p, q_base, k_base, s_base, row0 + base16 + r);
     }
   }
 

@@ -90,3 +90,61 @@ def test_split_is_as_exact_as_fp32_arithmetic(B, H, S, D, causal, operands):
         errors.append([float((g.double() - r).norm() / r.norm()) for g, r in zip(got, ref)])
     for name, a, b in zip(("out", "lse", "dq", "dk", "dv"), *errors):
         assert a <= (2.0 ** -23 if name == "lse" else b), (name, a, b)
+
+
+def _visible_only(torch, q, k, v, go, lse, delta, scale, causal):
+    """One head in float64, products summed over the visible pairs alone (0 * inf of a hidden pair is no term): out, dq, dk, dv of [S, D]."""
+    S = q.shape[0]
+    hidden = torch.arange(S, device="cuda")[None, :] > torch.arange(S, device="cuda")[:, None] if causal else torch.zeros((S, S), dtype=torch.bool, device="cuda")
+    q, k, v, go, lse, delta = (t.double() for t in (q, k, v, go, lse, delta))
+    each = lambda w, x, dim: torch.where(hidden[..., None], 0.0, w[..., None] * x.unsqueeze(1 - dim)).sum(dim)  # over queries (0) or keys (1)
+    s = (q[:, None] * k[None]).sum(-1) * scale
+    top = torch.nan_to_num(torch.where(hidden, -torch.inf, s), nan=-torch.inf, posinf=torch.inf, neginf=-torch.inf).amax(1, keepdim=True)
+    w = torch.where(hidden, 0.0, torch.exp(s - torch.where(top == -torch.inf, 0.0, top)))
+    out = each(w, v, 1) / w.sum(1, keepdim=True)
+    pr = torch.where(hidden, 0.0, torch.exp(s - torch.where(lse == -torch.inf, torch.inf, lse)[:, None]))
+    ds = torch.where(hidden, 0.0, pr * ((go[:, None] * v[None]).sum(-1) - delta[:, None]))
+    return out, each(ds, k, 1) * scale, each(ds, q, 0) * scale, each(pr, go, 0)
+
+
+# where: tensor, row, value. A CTA a block, two, four.
+@pytest.mark.parametrize("tensor,value", [("v", float("inf")), ("v", float("nan")), ("v", 3.4e38), ("k", float("-inf")), ("k", float("nan")), ("q", float("inf")),
+                                          ("go", float("-inf"))])
+@pytest.mark.parametrize("H,S,D,causal", [(60, 260, 128, True), (2, 300, 32, True), (1, 600, 96, True), (2, 449, 36, False)])
+def test_split_with_operands_that_are_not_finite(H, S, D, causal, tensor, value):
+    """What fp32 arithmetic gives: an infinite V an infinite O, a score of -inf a probability of zero; rows that do not see it stay as they are."""
+    import torch
+    p = pkg()
+    torch.manual_seed(S)
+    x = {n: torch.randn(1, S, H * D, device="cuda") for n in ("q", "k", "v", "go")}
+    x["q"][..., ::D] = x["q"][..., ::D].abs() + 0.1  # against an infinite K in the head's first dim
+    scale = hp.default_scale(D)
+
+    def run():
+        out, lse = p.forward(x["q"], x["k"], x["v"], H, scale, causal)
+        delta = p.delta(out, x["go"], H)
+        got = (out,) + tuple(p.backward_block(x["q"], x["k"], x["v"], x["go"], lse, delta, H, scale, causal)[:3])
+        assert p.sync_status() == 0
+        return lse, delta, got
+
+    clean = run()[2]
+    row, head = S // 2 + 9, H - 1
+    x[tensor][0, row, head * D] = value
+    lse, delta, got = run()
+    cut = slice(head * D, (head + 1) * D)
+    ref = _visible_only(torch, *(x[n][0, :, cut] for n in ("q", "k", "v", "go")), lse[0, head], delta[0, head], scale, causal)
+    for name, a, c, r in zip(("out", "dq", "dk", "dv"), got, clean, ref):
+        if value == 3.4e38 and name in ("dq", "dk"):  # dP is past fp32
+            continue
+        assert torch.equal(a[..., :head * D], c[..., :head * D]), name
+        a, r = a[0, :, cut], r.float()
+        assert torch.equal(torch.isnan(a), torch.isnan(r)), name
+        assert torch.equal(torch.isinf(a) * torch.sign(a).nan_to_num(), torch.isinf(r) * torch.sign(r).nan_to_num()), name
+        seen = torch.isfinite(r)
+        a, r = torch.where(seen, a, 0.0).double(), torch.where(seen, r, 0.0).double()
+        assert bool(((a - r).abs() <= 2e-5 * torch.clamp(r.abs(), min=1.0)).all()), name
+    if causal:  # rows that do not see it
+        before = row if tensor in ("k", "v") else 0
+        assert torch.isfinite(got[0][:, :before]).all() and torch.isfinite(got[1][:, :before]).all()
+        if tensor in ("q", "go"):
+            assert torch.isfinite(got[2][:, row + 1:]).all() and torch.isfinite(got[3][:, row + 1:]).all()
