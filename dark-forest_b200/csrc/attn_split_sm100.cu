@@ -279,7 +279,8 @@ __device__ __forceinline__ void split_block(const AttnParams &p, uint32_t tile, 
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + C::oBars);
   volatile uint32_t *abort_flag = reinterpret_cast<volatile uint32_t *>(smem + C::oBars + 240);
   uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(smem + C::oBars + 244);
-  static_assert(NUM * 8 <= 240, "barriers");
+  uint32_t *again = reinterpret_cast<uint32_t *>(smem + C::oBars + 208);  // of each compute warp: rows to be formed in fp32 arithmetic
+  static_assert(NUM * 8 <= 208, "barriers");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   auto bar = [&](int id) { return smem_u32(&bars[id]); };
 
@@ -544,6 +545,7 @@ __device__ __forceinline__ void split_block(const AttnParams &p, uint32_t tile, 
       mbar_arrive(bar(STAT_FULL));
     };
     bool ok = true;
+    uint32_t odd_rows = 0;
     if (C::ROWS_ARE_KEYS && n > 0) put_stat(0, fetch_stat(0));
     // R of step j into the registers
     auto add_r = [&](int j) -> bool {
@@ -778,10 +780,9 @@ __device__ __forceinline__ void split_block(const AttnParams &p, uint32_t tile, 
           if (d < (int)p.D) *reinterpret_cast<float2 *>(at + d) = make_float2(acc[2 * g + half].x * f, acc[2 * g + half].y * f);
         }
       }
-#pragma unroll 1
-      for (int r = 0; r < 16; ++r)
-        if (((r < 8 ? bitsA : bitsB) >> (4 * (r & 7))) & 1u) fp32_row<PASS>(p, q_base, k_base, s_base, row0 + base16 + r);
+      odd_rows = bitsA | bitsB << 1;
     }
+    if (lane == 0) again[warp] = odd_rows;
   }
 
   if (CL > 1 && warp >= 8) {  // the compute warps' two meetings
@@ -792,6 +793,16 @@ __device__ __forceinline__ void split_block(const AttnParams &p, uint32_t tile, 
   // ---------------------------------------------------------------- teardown (all roles)
   tc_fence_before_sync();
   __syncthreads();
+  // Here, by all warps, and not by the compute warps behind their results: there the loops below cost 2-5 % of every call (registers and instruction
+  // fetch; us, without them / there / here: forward and backward 2 x 8 x 1000 x 128 165.0 / 171.0 / 164.4, 1 x 4 x 700 x 96 48.8 / 50.5 / 49.9).
+  const uint4 again0 = reinterpret_cast<const uint4 *>(again)[0], again1 = reinterpret_cast<const uint4 *>(again)[1];
+  if (__builtin_expect((again0.x | again0.y | again0.z | again0.w | again1.x | again1.y | again1.z | again1.w) != 0u, 0)) {
+#pragma unroll 1
+    for (int i = warp; i < BM; i += kMmaWarp + 1) {  // row i % 16 of the 16 of compute warp i / 16; bit 4 r of its word is row r, 4 r + 1 row r + 8
+      const int w = i >> 4, r = i & 15;
+      if (again[w] >> (4 * (r & 7) + (r >> 3)) & 1u) fp32_row<PASS>(p, q_base, k_base, s_base, row0 + (w & 3) * 32 + (w >> 2) * 16 + r);
+    }
+  }
   if (*abort_flag != 0u) {
     if (warp == kMmaWarp) {
       commit_elected(bar(DRAIN));  // by the lane that issued the MMAs: the election is deterministic
