@@ -194,6 +194,20 @@ __device__ __forceinline__ void product_ss(uint32_t d, uint32_t a_lo, uint32_t a
   for (int kk = 0; kk < STEPS; ++kk) mma_ss(d, a_lo + (a_step(kk) >> 4), a_hi, b_lo + (b_step(kk) >> 4), b_hi, idesc, 1u, mine);
 }
 
+// Index i of W elements of a tensor of n, as it is; range-checked in checked builds where the access is `on` (DF_IDX, df_common.cuh).
+template <int W>
+__device__ __forceinline__ size_t elem(size_t i, size_t n, const AttnParams &p, bool on = true) {
+#ifdef DF_BOUNDS_CHECK
+  return on && df_checked_index(i + W - 1, n, p.status) == i + W - 1 ? i : 0;
+#else
+  return i;
+#endif
+}
+// Elements of the tensors of queries, of keys, and of the row statistics.
+__device__ __forceinline__ size_t q_elements(const AttnParams &p) { return (size_t)p.B * p.Sq * p.H * p.D; }
+__device__ __forceinline__ size_t k_elements(const AttnParams &p) { return (size_t)p.B * p.Sk * p.H * p.D; }
+__device__ __forceinline__ size_t stat_elements(const AttnParams &p) { return (size_t)p.B * p.H * p.Sq; }
+
 // logsumexp in log2 units, negated, in two fp32 numbers: rounded to one, ten times 2^-24 of it goes into every P. No visible key: P = 0.
 __device__ __forceinline__ float neg_lse2(float raw, float *lo) {
   const float hi = raw * kLog2e;
@@ -209,23 +223,24 @@ __device__ __forceinline__ void fp32_row(const AttnParams &p, size_t q_base, siz
   constexpr bool KEYS = PASS == DK || PASS == DV, TWO = PASS == DQ || PASS == DK;
   const uint32_t lane = threadIdx.x & 31;
   const size_t dm = (size_t)p.H * p.D, res = (KEYS ? k_base : q_base) + (size_t)row * dm, str = KEYS ? q_base : k_base;
-  const float *a1 = (KEYS ? p.k : p.q) + res, *a2 = TWO ? (KEYS ? p.v : p.d_out) + res : a1, *b1 = (KEYS ? p.q : p.k) + str, *b2 = (KEYS ? p.d_out : p.v) + str;
+  const size_t n_res = KEYS ? k_elements(p) : q_elements(p), n_str = KEYS ? q_elements(p) : k_elements(p), n_stat = stat_elements(p);
+  const float *a1 = KEYS ? p.k : p.q, *a2 = KEYS ? p.v : p.d_out, *b1 = KEYS ? p.q : p.k, *b2 = KEYS ? p.d_out : p.v;
   long long from = 0, to = KEYS ? p.Sq : p.Sk;
   if (p.causal && KEYS && row > p.shift) from = row - p.shift;
   if (p.causal && !KEYS && row + p.shift + 1 < to) to = row + p.shift + 1;
-  auto dot = [&](const float *x, const float *y) {
+  auto dot = [&](const float *x, const float *y, long long j) {  // of this row and row j of the streamed side
     float2 sum = make_float2(0.f, 0.f);
 #pragma unroll 1
     for (uint32_t d = 0; d < p.D; d += 4) {
-      const float4 u = *reinterpret_cast<const float4 *>(x + d), w = *reinterpret_cast<const float4 *>(y + d);
+      const float4 u = *reinterpret_cast<const float4 *>(x + elem<4>(res + d, n_res, p)), w = *reinterpret_cast<const float4 *>(y + elem<4>(str + (size_t)j * dm + d, n_str, p));
       sum = fma2(make_float2(u.z, u.w), make_float2(w.z, w.w), fma2(make_float2(u.x, u.y), make_float2(w.x, w.y), sum));
     }
     return sum.x + sum.y;
   };
   float m = -INFINITY, l = 0.f, neg = 0.f, lo = 0.f, delta = 0.f;
   if (PASS == DQ) {
-    neg = neg_lse2(p.lse_in[s_base + row], &lo);
-    delta = p.delta_in[s_base + row];
+    neg = neg_lse2(p.lse_in[elem<1>(s_base + row, n_stat, p)], &lo);
+    delta = p.delta_in[elem<1>(s_base + row, n_stat, p)];
   }
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);  // dims 4 lane .. + 3
 #pragma unroll 1
@@ -233,7 +248,7 @@ __device__ __forceinline__ void fp32_row(const AttnParams &p, size_t q_base, siz
     const long long j = c + lane;
     const bool seen = j < to;
     float t = 0.f;
-    const float s = seen ? dot(a1, b1 + (size_t)j * dm) * p.scale_log2 : -INFINITY;
+    const float s = seen ? dot(a1, b1, j) * p.scale_log2 : -INFINITY;
     if (PASS == FORWARD) {
       float top = s;
 #pragma unroll
@@ -247,24 +262,24 @@ __device__ __forceinline__ void fp32_row(const AttnParams &p, size_t q_base, siz
       l = fmaf(l, alpha, sum);
       acc = make_float4(acc.x * alpha, acc.y * alpha, acc.z * alpha, acc.w * alpha);
     } else if (seen) {
-      if (KEYS) neg = neg_lse2(p.lse_in[s_base + j], &lo);
-      if (PASS == DK) delta = p.delta_in[s_base + j];
+      if (KEYS) neg = neg_lse2(p.lse_in[elem<1>(s_base + j, n_stat, p)], &lo);
+      if (PASS == DK) delta = p.delta_in[elem<1>(s_base + j, n_stat, p)];
       t = ex2_approx(s + neg + lo);
-      if (TWO) t *= dot(a2, b2 + (size_t)j * dm) - delta;
+      if (TWO) t *= dot(a2, b2, j) - delta;
     }
 #pragma unroll 1
     for (int x = 0; x < 32 && c + x < to; ++x) {
       const float tx = __shfl_sync(0xffffffffu, t, x);
       if (4 * lane < p.D) {
-        const float4 y = *reinterpret_cast<const float4 *>((TWO ? b1 : b2) + (size_t)(c + x) * dm + 4 * lane);
+        const float4 y = *reinterpret_cast<const float4 *>((TWO ? b1 : b2) + elem<4>(str + (size_t)(c + x) * dm + 4 * lane, n_str, p));
         acc = make_float4(fmaf(tx, y.x, acc.x), fmaf(tx, y.y, acc.y), fmaf(tx, y.z, acc.z), fmaf(tx, y.w, acc.w));
       }
     }
   }
   const float f = PASS == FORWARD ? (l > 0.f ? 1.f / l : 0.f) : PASS == DV ? 1.f : p.scale;  // reference guard, attention_fused.cu:104
-  float *dst = (PASS == FORWARD ? p.out : PASS == DQ ? p.d_q : PASS == DK ? p.d_k : p.d_v) + res;
-  if (4 * lane < p.D) *reinterpret_cast<float4 *>(dst + 4 * lane) = make_float4(acc.x * f, acc.y * f, acc.z * f, acc.w * f);
-  if (PASS == FORWARD && p.lse && lane == 0) p.lse[s_base + row] = l > 0.f ? fmaf(m, kLn2, logf(l)) : -INFINITY;
+  float *dst = PASS == FORWARD ? p.out : PASS == DQ ? p.d_q : PASS == DK ? p.d_k : p.d_v;
+  if (4 * lane < p.D) *reinterpret_cast<float4 *>(dst + elem<4>(res + 4 * lane, n_res, p)) = make_float4(acc.x * f, acc.y * f, acc.z * f, acc.w * f);
+  if (PASS == FORWARD && p.lse && lane == 0) p.lse[elem<1>(s_base + row, n_stat, p)] = l > 0.f ? fmaf(m, kLn2, logf(l)) : -INFINITY;
 }
 
 // One block of 128 resident rows. A cluster of CL CTAs shares it: each takes a range of the steps, rank 0 puts the results together.
@@ -287,6 +302,7 @@ __device__ __forceinline__ void split_block(const AttnParams &p, uint32_t tile, 
   const uint32_t b = bh / p.H, h = bh % p.H;
   const size_t dm = (size_t)p.H * p.D;
   const size_t q_base = (size_t)b * p.Sq * dm + (size_t)h * p.D, k_base = (size_t)b * p.Sk * dm + (size_t)h * p.D, s_base = (size_t)bh * p.Sq;
+  const size_t el_res = C::ROWS_ARE_KEYS ? k_elements(p) : q_elements(p), el_str = C::ROWS_ARE_KEYS ? q_elements(p) : k_elements(p), el_stat = stat_elements(p);
   const long long row0 = (long long)tile * BM;
   const long long n_res = C::ROWS_ARE_KEYS ? p.Sk : p.Sq, n_str = C::ROWS_ARE_KEYS ? p.Sq : p.Sk;
   long long begin = 0, end = n_str;  // streamed rows that any resident row sees
@@ -353,7 +369,8 @@ __device__ __forceinline__ void split_block(const AttnParams &p, uint32_t tile, 
     }
     auto load_tile = [&](int t, int u) {
       const long long row = begin + (long long)(t >> 1) * BN + first_row + C::RPA * u;
-      load4(buf[u], ((t & 1) ? src2 : src1) + str_base + (size_t)min(row, n_str - 1) * dm + 4 * g, dims && first_row + C::RPA * u < BN);
+      const bool valid = dims && first_row + C::RPA * u < BN;
+      load4(buf[u], ((t & 1) ? src2 : src1) + elem<4>(str_base + (size_t)min(row, n_str - 1) * dm + 4 * g, el_str, p, valid), valid);
     };
     if (n > 0) {
 #pragma unroll
@@ -489,8 +506,9 @@ __device__ __forceinline__ void split_block(const AttnParams &p, uint32_t tile, 
 #pragma unroll
       for (int g = 0; g < DP / 8; ++g) {
         const int d = g * 8 + 2 * t4;
-        v[2 * g] = load2(src + res_base + (size_t)rowA * dm + d, rowA < n_res && d < (int)p.D);
-        v[2 * g + 1] = load2(src + res_base + (size_t)rowB * dm + d, rowB < n_res && d < (int)p.D);
+        const bool onA = rowA < n_res && d < (int)p.D, onB = rowB < n_res && d < (int)p.D;
+        v[2 * g] = load2(src + elem<2>(res_base + (size_t)rowA * dm + d, el_res, p, onA), onA);
+        v[2 * g + 1] = load2(src + elem<2>(res_base + (size_t)rowB * dm + d, el_res, p, onB), onB);
       }
 #pragma unroll
       for (int c = 0; c < DP / 32; ++c) {
@@ -518,8 +536,8 @@ __device__ __forceinline__ void split_block(const AttnParams &p, uint32_t tile, 
     float mA = -INFINITY, mB = -INFINITY, lA = 0.f, lB = 0.f, dA = 0.f, dB = 0.f;
     float fA = p.scale, fB = p.scale;  // factors of the results
     if (PASS == DQ) {
-      if (rowA < n_res) { mA = p.lse_in[s_base + rowA]; dA = -p.delta_in[s_base + rowA]; }
-      if (rowB < n_res) { mB = p.lse_in[s_base + rowB]; dB = -p.delta_in[s_base + rowB]; }
+      if (rowA < n_res) { mA = p.lse_in[elem<1>(s_base + rowA, el_stat, p)]; dA = -p.delta_in[elem<1>(s_base + rowA, el_stat, p)]; }
+      if (rowB < n_res) { mB = p.lse_in[elem<1>(s_base + rowB, el_stat, p)]; dB = -p.delta_in[elem<1>(s_base + rowB, el_stat, p)]; }
       float loA, loB;
       mA = neg_lse2(mA, &loA);
       mB = neg_lse2(mB, &loB);
@@ -530,8 +548,8 @@ __device__ __forceinline__ void split_block(const AttnParams &p, uint32_t tile, 
       const int tid = threadIdx.x;
       const long long q = begin + (long long)j * BN + (tid & (BN - 1));
       if (tid >= 2 * BN) return 0.f;
-      if (tid < BN) return q < n_str ? p.lse_in[s_base + q] : -INFINITY;
-      return PASS == DK && q < n_str ? p.delta_in[s_base + q] : 0.f;
+      if (tid < BN) return q < n_str ? p.lse_in[elem<1>(s_base + q, el_stat, p)] : -INFINITY;
+      return PASS == DK && q < n_str ? p.delta_in[elem<1>(s_base + q, el_stat, p)] : 0.f;
     };
     auto put_stat = [&](int j, float raw) {
       float *to = sStats + (j % 3) * C::NSTATS * BN;
@@ -764,8 +782,8 @@ __device__ __forceinline__ void split_block(const AttnParams &p, uint32_t tile, 
       const uint32_t bitsA = row_bits(rowA < n_res && !(oddA.x + oddA.y == 0.f)), bitsB = row_bits(rowB < n_res && !(oddB.x + oddB.y == 0.f));
       const bool storeA = rowA < n_res && !(bitsA >> (lane & 28) & 1u), storeB = rowB < n_res && !(bitsB >> (lane & 28) & 1u);
       if (PASS == FORWARD && p.lse && t4 == 0) {
-        if (storeA) p.lse[s_base + rowA] = lA > 0.f ? fmaf(mA, kLn2, logf(lA)) : -INFINITY;
-        if (storeB) p.lse[s_base + rowB] = lB > 0.f ? fmaf(mB, kLn2, logf(lB)) : -INFINITY;
+        if (storeA) p.lse[elem<1>(s_base + rowA, el_stat, p)] = lA > 0.f ? fmaf(mA, kLn2, logf(lA)) : -INFINITY;
+        if (storeB) p.lse[elem<1>(s_base + rowB, el_stat, p)] = lB > 0.f ? fmaf(mB, kLn2, logf(lB)) : -INFINITY;
       }
       float *dst = PASS == FORWARD ? p.out : PASS == DQ ? p.d_q : PASS == DK ? p.d_k : p.d_v;
 #pragma unroll
@@ -773,11 +791,10 @@ __device__ __forceinline__ void split_block(const AttnParams &p, uint32_t tile, 
         const long long row = half ? rowB : rowA;
         if (!(half ? storeB : storeA)) continue;
         const float f = half ? fB : fA;
-        float *at = dst + res_base + (size_t)row * dm;
 #pragma unroll
         for (int g = 0; g < DP / 8; ++g) {
           const int d = 8 * g + 2 * t4;
-          if (d < (int)p.D) *reinterpret_cast<float2 *>(at + d) = make_float2(acc[2 * g + half].x * f, acc[2 * g + half].y * f);
+          if (d < (int)p.D) *reinterpret_cast<float2 *>(dst + elem<2>(res_base + (size_t)row * dm + d, el_res, p)) = make_float2(acc[2 * g + half].x * f, acc[2 * g + half].y * f);
         }
       }
       odd_rows = bitsA | bitsB << 1;

@@ -62,11 +62,12 @@ int option(int which);
 constexpr unsigned int DEV_STATUS_WAIT_EXPIRED = 1u;
 constexpr unsigned int DEV_STATUS_BOUNDS = 2u;
 
-// Optional checked build (make EXTRA=-DDF_BOUNDS_CHECK): every global-memory index of the SIMT kernels goes through
+// Optional checked build (make EXTRA=-DDF_BOUNDS_CHECK): every global-memory index of the SIMT kernels and of the split fp32 kernels goes through
 // DF_IDX(i, n, status): an index outside [0, n) ORs DEV_STATUS_BOUNDS into the device status word and is replaced by 0,
 // so the access itself stays inside the tensor and the context stays usable; df_sync_status then returns
-// DF_ERR_DEVICE_BOUNDS. In the normal build the macro is the index itself. (The tensor-core kernels move their
-// tiles with TMA, whose tensor maps bound every copy in hardware.)
+// DF_ERR_DEVICE_BOUNDS. In the normal build the macro is the index itself. (The other tensor-core
+// kernels move their tiles with TMA, whose tensor maps bound every copy in hardware; the row statistics, and the results of the one-tile kernels and of
+// the forward, they move by plain accesses behind a comparison with the number of rows, which no build checks.)
 #ifdef DF_BOUNDS_CHECK
 #ifdef __CUDACC__
 __device__ __forceinline__ size_t df_checked_index(size_t i, size_t n, unsigned int *status) {

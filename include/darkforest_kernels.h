@@ -427,7 +427,7 @@ DF_API const char *df_attn_status_string(int status);
 DF_API int df_attn_selftest_wait_expiry(uint32_t budget_ms, void *stream);
 
 /* Checked builds (make EXTRA=-DDF_BOUNDS_CHECK; no counterpart in the reference, which runs unchecked): the
- * SIMT kernels range-check every global-memory index; an index outside its tensor sets a bit in the device status word
+ * SIMT kernels and the split fp32 kernels range-check every global-memory index; an index outside its tensor sets a bit in the device status word
  * and is replaced by 0, so nothing outside the tensor is touched and the context stays usable, and df_sync_status
  * returns DF_ERR_DEVICE_BOUNDS once. This call makes one thread ask the checker for an out-of-range element, which is
  * how a test sees the path work without a bad access. In a normal build it returns DF_ERR_UNSUPPORTED. */

@@ -1,11 +1,12 @@
-"""The checked build of the library (make EXTRA=-DDF_BOUNDS_CHECK): the SIMT kernels range-check every global index.
+"""The checked build of the library (make EXTRA=-DDF_BOUNDS_CHECK): the SIMT kernels and the split fp32 kernels range-check every global index.
 
-The test builds that variant into a scratch directory (nvcc, about a minute), runs ragged shapes through the SIMT
-path in a child process and expects (a) the same results as the oracle, (b) a clean device status word, and (c) that
+The test builds that variant into a scratch directory (nvcc, about a minute), runs ragged shapes through both
+paths in a child process and expects (a) the same results as the oracle, (b) a clean device status word, and (c) that
 the checker's own self-test - one thread asking for element 5 of a 4-element tensor - is reported as
 DF_ERR_DEVICE_BOUNDS exactly once while the context stays usable. No out-of-range access is made anywhere."""
 import json
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -30,7 +31,11 @@ CHILD = textwrap.dedent("""
     L = pkg.lib()
     prev = pkg.set_variant(pkg.VARIANT_SIMT)
     rng = np.random.default_rng(11)
-    for (B, H, S, D, causal) in ((1, 1, 5, 4, True), (2, 3, 33, 3, True), (1, 2, 129, 64, True), (1, 2, 77, 128, False), (1, 12, 257, 32, True)):
+    simt = ((1, 1, 5, 4, True), (2, 3, 33, 3, True), (1, 2, 129, 64, True), (1, 2, 77, 128, False), (1, 12, 257, 32, True))
+    split = ((2, 3, 257, 36, True), (1, 1, 601, 96, True), (4, 15, 195, 128, False), (1, 2, 449, 4, False))  # two CTAs a block, four, one, four
+    for i, (B, H, S, D, causal) in enumerate(simt + split):
+        if i == len(simt):
+            pkg.set_variant(pkg.VARIANT_AUTO)
         q, k, v, go = (rng.standard_normal((B, S, H * D), dtype=np.float32) for _ in range(4))
         tq, tk, tv, tg = (torch.from_numpy(x).cuda() for x in (q, k, v, go))
         scale = 1.0 / np.sqrt(D)
@@ -44,6 +49,10 @@ CHILD = textwrap.dedent("""
                              "err_dq": float(np.abs(dq.cpu().numpy() - dq_ref).max()),
                              "err_dk": float(np.abs(dk.cpu().numpy() - dk_ref).max()),
                              "err_dv": float(np.abs(dv.cpu().numpy() - dv_ref).max())}})
+    # rows that are computed in fp32 arithmetic: an infinite V, seen by the last row alone
+    v[0, S - 1, 0] = np.inf
+    out, lse = pkg.forward(tq, tk, torch.from_numpy(v).cuda(), H, scale, True)
+    res["infinite"] = [int(torch.isinf(out).sum()), int(torch.isfinite(out).sum()), out.numel(), pkg.sync_status()]
     pkg.set_variant(prev)
     res["selftest_launch"] = L.df_attn_selftest_bounds_check(None)
     res["status_after_selftest"] = pkg.sync_status()
@@ -70,9 +79,12 @@ def test_checked_build_runs_clean_and_reports_a_bad_index(tmp_path):
     assert child.returncode == 0, child.stdout[-3000:] + child.stderr[-3000:]
     line = [l for l in child.stdout.splitlines() if l.startswith("RESULT ")][-1]
     res = json.loads(line[len("RESULT "):])
+    assert len(res["cases"]) == 9
     for c in res["cases"]:
         assert c["status"] == 0, c
-        assert max(c["err_o"], c["err_dq"], c["err_dk"], c["err_dv"]) <= 2e-4, c   # fp32 SIMT path against the fp32 oracle
+        assert max(c["err_o"], c["err_dq"], c["err_dk"], c["err_dv"]) <= 2e-4, c   # fp32 kernels against the fp32 oracle
+    inf, finite, n, status = res["infinite"]
+    assert inf == 1 and finite == n - 1 and status == 0, res["infinite"]
     assert res["selftest_launch"] == 0
     assert res["status_after_selftest"] == 9      # DF_ERR_DEVICE_BOUNDS, reported once
     assert res["status_again"] == 0
@@ -87,3 +99,14 @@ def test_normal_build_has_no_checker():
     p = pkg()
     assert p.lib().df_attn_selftest_bounds_check(None) == p.DF_ERR_UNSUPPORTED
     p.lib().df_attn_last_status()
+
+
+def test_split_kernels_check_every_global_index():
+    """In the source: global tensors are indexed through elem<> (range-checked in checked builds) and by nothing else."""
+    with open(os.path.join(ROOT, "dark-forest_b200", "csrc", "attn_split_sm100.cu")) as f:
+        text = f.read()
+    body = text[text.index("fp32_row"):text.index("Heaviest blocks first")]
+    assert len(re.findall(r"p\.(?:lse|lse_in|delta_in)\[elem<1>\(", body)) == 13
+    assert re.findall(r"p\.(?:lse|lse_in|delta_in)\[(?!elem<1>\()", body) == []
+    moves = re.findall(r"load[24]\((?!float4 |const float )[^;]*;", body) + re.findall(r"reinterpret_cast<(?:const )?float[24] \*>\((?:x|y|dst|\(TWO)[^;]*;", body)
+    assert len(moves) == 7 and all("elem<" in m for m in moves), moves
