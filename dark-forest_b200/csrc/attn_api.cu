@@ -109,7 +109,11 @@ int forward_dispatch(const AttnParams &p, cudaStream_t s) {
   const bool tensor_ok = p.out != nullptr && tensor_forward_supported(p);
   if (t_variant == DF_VARIANT_TENSOR) return tensor_ok ? tensor_forward(p, s) : DF_ERR_UNSUPPORTED;
   if (tensor_ok) return tensor_forward(p, s);
-  return split_forward_wanted(p) ? split_forward(p, s) : generic_forward(p, s);
+  if (split_forward_wanted(p)) {
+    const int st = split_forward(p, s);
+    if (st != DF_ERR_UNSUPPORTED) return st;
+  }
+  return generic_forward(p, s);
 }
 
 int backward_dispatch(const AttnParams &p, cudaStream_t s) {
@@ -117,7 +121,10 @@ int backward_dispatch(const AttnParams &p, cudaStream_t s) {
   const bool tensor_ok = tensor_backward_supported(p);
   if (t_variant == DF_VARIANT_TENSOR && !tensor_ok) return DF_ERR_UNSUPPORTED;
   if (t_variant != DF_VARIANT_SIMT && tensor_ok) return tensor_backward(p, s);
-  if (t_variant == DF_VARIANT_AUTO && split_backward_wanted(p)) return split_backward(p, s);
+  if (t_variant == DF_VARIANT_AUTO && split_backward_wanted(p)) {
+    const int st = split_backward(p, s);
+    if (st != DF_ERR_UNSUPPORTED) return st;
+  }
   return generic_backward(p, s);
 }
 

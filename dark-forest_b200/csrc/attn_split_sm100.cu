@@ -862,19 +862,25 @@ __global__ void __launch_bounds__(kThreads, 1) k_split_bwd(const AttnParams p, c
   else split_block<Cfg<DP, DV>, CL>(p, rank, bh);
 }
 
+// The registers a thread that the kernels are taken to be built with. Another number than kLaunchRegs refuses them all (tests build such a library).
+#ifndef DF_SPLIT_BUILT_REGS
+#define DF_SPLIT_BUILT_REGS kLaunchRegs
+#endif
+// DF_OK when the kernel can be launched on the current device. Built for fewer registers it would wait for ever in setmaxnreg: DF_ERR_UNSUPPORTED, and the
+// dispatch takes the SIMT kernels.
 template <auto K>
-bool allow_smem(uint32_t bytes) {
+int ready(uint32_t bytes) {
   static std::once_flag once[64];
-  static bool ok[64];
+  static int status[64];
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  if (check_cuda(cudaGetDevice(&dev)) != DF_OK || dev < 0 || dev >= 64) return DF_ERR_CUDA;
   std::call_once(once[dev], [&]() {
-    cudaFuncAttributes attr;  // a kernel built for fewer registers would wait for ever in setmaxnreg: it is not launched
-    ok[dev] = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess &&
-              cudaFuncGetAttributes(&attr, K) == cudaSuccess && attr.numRegs == kLaunchRegs;
+    cudaFuncAttributes attr;
+    status[dev] = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess || cudaFuncGetAttributes(&attr, K) != cudaSuccess
+                      ? DF_ERR_CUDA
+                  : attr.numRegs != DF_SPLIT_BUILT_REGS ? DF_ERR_UNSUPPORTED : DF_OK;
   });
-  if (!ok[dev]) note_status(DF_ERR_CUDA);
-  return ok[dev];
+  return status[dev];
 }
 
 // What the kernels take from the host beside the caller's parameters. The factor of the scores is rounded once: its error is in every one of them (1 x 4 x
@@ -888,7 +894,7 @@ void set_by_host(AttnParams *p) {
 template <int DP, int CL>
 int forward_form(AttnParams p, cudaStream_t s) {
   constexpr uint32_t smem = Cfg<DP, FORWARD>::kSmem;
-  if (!allow_smem<k_split_fwd<DP, CL>>(smem)) return DF_ERR_CUDA;
+  if (const int st = ready<k_split_fwd<DP, CL>>(smem)) return st;
   const uint32_t tiles = (p.Sq + BM - 1) / BM;
   set_by_host(&p);
   launch_clusters(k_split_fwd<DP, CL>, CL > 1 ? CL : 0, dim3(CL * tiles * p.B * p.H), dim3(kThreads), smem, s, p, tiles);
@@ -898,7 +904,7 @@ int forward_form(AttnParams p, cudaStream_t s) {
 template <int DP, int CL>
 int backward_form(AttnParams p, cudaStream_t s) {
   constexpr uint32_t a = Cfg<DP, DK>::kSmem, b = Cfg<DP, DV>::kSmem, smem = a > b ? a : b;
-  if (!allow_smem<k_split_bwd<DP, CL>>(smem)) return DF_ERR_CUDA;
+  if (const int st = ready<k_split_bwd<DP, CL>>(smem)) return st;
   const uint32_t kt = (p.Sk + BM - 1) / BM, qt = (p.Sq + BM - 1) / BM;
   set_by_host(&p);
   launch_clusters(k_split_bwd<DP, CL>, CL > 1 ? CL : 0, dim3(CL * (2 * kt + qt) * p.B * p.H), dim3(kThreads), smem, s, p, kt, qt);

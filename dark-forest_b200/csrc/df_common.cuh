@@ -92,6 +92,7 @@ int accumulate(float *dst, const float *src, uint64_t n, cudaStream_t s);
 // ---- fp32 in full precision on the tensor cores (attn_split_sm100.cu): head sizes without a TF32 kernel, from 193 keys on ----
 bool split_forward_wanted(const AttnParams &p);   // out, and lse if asked for; no row sums
 bool split_backward_wanted(const AttnParams &p);
+// DF_ERR_UNSUPPORTED, and nothing launched, when this build's kernels have other register counts than their hand-over of registers needs.
 int split_forward(const AttnParams &p, cudaStream_t s);
 int split_backward(const AttnParams &p, cudaStream_t s);  // needs lse_in, delta_in
 

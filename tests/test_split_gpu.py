@@ -1,5 +1,11 @@
 """fp32 attention on the tensor cores with operands cut into three bf16 parts (head sizes other than 64, four steps of 64 keys or more): the forms
 that its rules choose between, at the edges of its tiles, against float64. The bar is that of the other fp32 kernels, 2e-5 of the result's scale."""
+import os
+import shutil
+import subprocess
+import sys
+import textwrap
+
 import pytest
 
 import helpers as hp
@@ -148,3 +154,38 @@ def test_split_with_operands_that_are_not_finite(H, S, D, causal, tensor, value)
         assert torch.isfinite(got[0][:, :before]).all() and torch.isfinite(got[1][:, :before]).all()
         if tensor in ("q", "go"):
             assert torch.isfinite(got[2][:, row + 1:]).all() and torch.isfinite(got[3][:, row + 1:]).all()
+
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+OTHER_REGISTERS = textwrap.dedent("""
+    import sys
+    sys.path.insert(0, {root!r})
+    import torch
+    from __graft_entry__ import load_package
+    p = load_package()
+    p.LIB_PATH = {lib!r}
+    torch.manual_seed(1)
+    for B, H, S, D in ((1, 2, 449, 36), (2, 3, 300, 96), (4, 15, 260, 128)):
+        q, k, v, go = (torch.randn(B, S, H * D, device="cuda") for _ in range(4))
+        got = []
+        for variant in (p.VARIANT_AUTO, p.VARIANT_SIMT):
+            p.set_variant(variant)
+            out, lse = p.forward(q, k, v, H, D ** -0.5, True)
+            got.append([out, lse] + list(p.backward(q, k, v, out, go, lse, H, D ** -0.5, True)[:3]))
+            assert p.sync_status() == 0
+        assert all(torch.equal(a, b) for a, b in zip(*got))
+    print("SAME")
+""")
+
+
+def test_split_kernels_with_other_registers_leave_calls_to_the_simt_kernels(tmp_path):
+    """A library whose split kernels are taken to have been built with 127 registers a thread launches none of them, and answers all the same."""
+    if shutil.which("nvcc") is None and not os.path.exists("/usr/local/cuda/bin/nvcc"):
+        pytest.skip("nvcc is not available: the variant cannot be built here")
+    out_dir = str(tmp_path / "lib")
+    lib = os.path.join(out_dir, "libdarkforest_kernels.so")
+    r = subprocess.run(["make", "-C", os.path.join(ROOT, "dark-forest_b200"), "-j8", f"OUT={out_dir}", "EXTRA=-DDF_SPLIT_BUILT_REGS=127", lib],
+                       capture_output=True, text=True, timeout=900)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
+    child = subprocess.run([sys.executable, "-c", OTHER_REGISTERS.format(root=ROOT, lib=lib)], capture_output=True, text=True, timeout=600)
+    assert child.returncode == 0 and "SAME" in child.stdout, child.stdout[-3000:] + child.stderr[-3000:]
