@@ -245,6 +245,8 @@ def dkdv_bf16(n_it, issuers, s_bufs, ring=4):
     def scores(role, chain_s, it):
         tile = "Q" if chain_s else "G"
         role.wait("%s_FULL%d" % (tile, it % ring), it // ring)
+        if it < s_bufs:
+            role.wait("FIRST", 0)
         role.mark("lse used" if chain_s else "delta used", it)
         role.arrive("S_FULL%d" % (it % s_bufs) if chain_s else "DP_FULL")
         if issuers == 2:
@@ -257,8 +259,6 @@ def dkdv_bf16(n_it, issuers, s_bufs, ring=4):
         role.wait("P_FULL%d" % (it % s_bufs), it // s_bufs) if chain_s else role.wait("DS_FULL", it)
         role.arrive("%s_EMPTY%d" % (tile, it % ring))
 
-    for role in chains:
-        role.wait("FIRST", 0)
     if issuers == 2:
         for role, chain_s in zip(chains, (True, False)):
             ahead = s_bufs if chain_s else 1
