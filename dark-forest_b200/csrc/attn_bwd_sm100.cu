@@ -417,7 +417,7 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
     const TileMN dM = tile_mn(s_chain ? aGm : aQm);
     Item cur;
     uint32_t g = 0, r = 0;
-    bool ok = true;
+    bool ok = true, staged = false;
     // S^T - lse / scale = K Q^T + 1 (-lse / scale), or dP^T - delta, for half h of the queries of the ring's next tile: the queries' statistics, cut in
     // three TF32 parts, come in as one more K-step, so that the compute warps do not read them (they took a quarter of the warps' time). It is the last
     // one: the accumulator truncates, so with the statistics first eight sums lose bits of a number as large as lse / scale, with them last only the
@@ -429,9 +429,17 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
         if (!mbar_wait_warp(bar(full + slot), (r >> 1) & 1, abort_flag)) return false;
         tc_fence_after_sync();
       }
+      if (from_smem) {
+        if (elect_one()) batch_ss_scores(tX + h * (BT / 2), dB, (slot ^ 1) * (kTile >> 4), b_off, idesc_st);
+        __syncwarp();
+        if (!staged) {  // the CTA's first statistics come out of global memory while its first tiles do
+          if (!mbar_wait_warp(bar(FIRST), 0, abort_flag)) return false;
+          tc_fence_after_sync();
+          staged = true;
+        }
+      }
       if (elect_one()) {
-        if (from_smem) batch_ss_scores(tX + h * (BT / 2), dB, (slot ^ 1) * (kTile >> 4), b_off, idesc_st);
-        else batch_ts_scores(tX + h * (BT / 2), tA, dB, b_off, idesc_st);
+        if (!from_smem) batch_ts_scores(tX + h * (BT / 2), tA, dB, b_off, idesc_st);
         mma_tf32_ss(tX + h * (BT / 2), dOnes, dStat + h * (kStatTile >> 4), idesc_st, 1u);
         mma_commit(bar((s_chain ? S_FULL : DP_FULL) + h));
         if (h == 1) mma_commit(bar(empty + slot));
@@ -444,7 +452,6 @@ k_attn_bwd_dkdv_tf32_d64(const __grid_constant__ CUtensorMap tmK, const __grid_c
     uint32_t moved = 0;  // items whose K (V) went to tensor memory
     for (uint32_t n = 0; ok && take_warp(n, &cur); ++n) {
       const uint32_t slot = r & 1;  // K's, or V's
-      if (n == 0 && !mbar_wait_warp(bar(FIRST), 0, abort_flag)) break;  // the first statistics are staged
       if (!mbar_wait_warp(bar(full + slot), (r >> 1) & 1, abort_flag)) break;
       ++r;
       ok = issue_first(0, true, false) && issue_first(1, true, false);

@@ -169,6 +169,8 @@ def dkdv_tf32(items):
         def first(h, r, frees):
             if h == 0:
                 role.wait("%s_FULL%d" % (ring, r % 2), r // 2)
+            if h == 0 and r == 1:
+                role.wait("FIRST", 0)
             role.arrive("%s%d" % (scores, h))
             if h == 1:
                 role.arrive("%s_EMPTY%d" % (ring, r % 2))
@@ -176,7 +178,6 @@ def dkdv_tf32(items):
                     role.arrive(kv + "_FREE")
 
         g = 0
-        role.wait("FIRST", 0)
         for n, n_it in enumerate(items):
             r = first_tile[n]
             role.wait("%s_FULL%d" % (ring, r % 2), r // 2)
