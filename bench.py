@@ -31,8 +31,8 @@ sys.path.insert(0, ROOT)
 CFG = dict(B=8, H=12, S=1024, D=64)
 # DRAM bytes (read + write) of one launch of each kernel of the step at exactly the benchmark size, from one ncu
 # capture; TRAFFIC_CAPTURE names the build the capture was taken from
-TRAFFIC = {"fwd": 81.2e6, "dq": 148.9e6, "dkdv": 126.2e6}
-TRAFFIC_CAPTURE = "ncu, dram__bytes_read.sum + dram__bytes_write.sum of bench.py --kernel-case fwd / bwd --batch 8 --seq 1024 --iters 3, kernels as of commit e09812d"
+TRAFFIC = {"fwd": 80.7e6, "dq": 147.1e6, "dkdv": 125.5e6}
+TRAFFIC_CAPTURE = "ncu, dram__bytes_read.sum + dram__bytes_write.sum of bench.py --kernel-case fwd / bwd --batch 8 --seq 1024 --iters 3, kernels as of commit 57da17c"
 METRIC = "causal_attention_fwd_bwd_tflops"
 UNIT = "TFLOP/s"
 

@@ -13,13 +13,13 @@
 //   different shared-memory swizzle (32-byte atoms) than a K-major one, so Q and dO tiles are fetched twice by TMA, once per layout.  The queries'
 //   statistics come in as one more K-step of the first two products: S^T - lse / scale, dP^T - delta.  A step's queries are two halves with barriers of
 //   their own: warps 0-3 turn one half's S^T into P^T and dP^T into dS^T in place in TMEM, warps 4-7 the other's, and neither group waits for the other.
-//   What bounds it: the compute warps, two of which share a scheduler. Of a step's 3.4 K cycles 3.1 K were theirs when they read the statistics from
-//   shared memory (a quarter of their time) and went in step; now it takes 2.7 K, of which the tensor pipe needs 2.2 K.
+//   What bounds it: the tensor pipe, with 2.18 K of the 2.50 K cycles that a step takes at 1 x 12 x 16384 (87 % busy); in short sequences the ends of items
+//   (8 x 12 x 1024: 54 %). When the compute warps read the statistics from shared memory (a quarter of their time) and went in step it was 3.4 K.
 //   Backward on B200, us, before / now: 8 x 12 x 1024 causal 115 / 109, 1 x 12 x 8192 669 / 577, 2 x 16 x 2000 all keys 228 / 203, 1 x 12 x 512 18.0 / 17.4.
 // dQ kernel: a CTA owns 128 queries (lanes = queries) and walks the key tiles they can see:
 //   S = Q K^T, dP = dO V^T (SS), dS in TMEM, dQ += dS K (TS, K tile MN-major: K is fetched twice).
-//   2.55 K cycles a step where the tensor pipe needs 1.54 K: the latency of the issuing and the compute warps' loops (tensor pipe 58 %, exponentials
-//   39 %, issue slots 33 % busy). The dK/dV kernel's halves and operands in tensor memory gave it 2 % at 8192 rows and cost 1-2 % at 8 x 1024 and 512.
+//   2.55 K cycles a step at 1 x 12 x 4096 (2.24 K at 16384) where the tensor pipe needs 1.54 K: the latency of the issuing and the compute warps' loops
+//   (at 4096 tensor pipe 58 %, exponentials 39 %, issue slots 33 % busy). The dK/dV kernel's halves and operands in tensor memory gave it 2 % at 8192 rows and cost 1-2 % at 8 x 1024 and 512.
 // One-tile kernel (at the end): up to 128 queries and keys, both halves in one launch.
 // MMA issue: tcgen05 MMAs of one thread execute in issue order, which is what lets single shared-memory stages
 // suffice. The dQ kernel has one MMA warp that interleaves the phases of consecutive tiles (.., S_{j+1}, dP_{j+1},
@@ -61,9 +61,10 @@ constexpr uint32_t kSlab = 128 * 128;
 constexpr uint32_t kTile = 2 * kSlab;
 constexpr uint32_t kTmemCols = 512;
 
-// Optional phase trace (build with -DDF_ATTN_TRACE): (event id, SM clock) pairs recorded by the
-// MMA thread (slot 0) and lane 0 of compute warp 0 (slot 1) of CTA 0 of the dK/dV kernel; the
-// launcher prints them when DF_ATTN_TRACE_DUMP is set. Compiled out by default.
+// Optional phase trace (build with -DDF_ATTN_TRACE): (event id, SM clock) pairs recorded by lane 0 of compute warp 0
+// (slot 1) of CTA 0 of the dK/dV kernel, or with -DDF_ATTN_TRACE_DQ of the dQ kernel, there by its MMA warp as well
+// (slot 0; in the dK/dV kernel that slot has the kernel's start alone); the launcher prints them when
+// DF_ATTN_TRACE_DUMP is set. Compiled out by default.
 #ifdef DF_ATTN_TRACE
 __device__ unsigned long long g_bwd_trace[2 * 1024];
 #define DF_BTRACE(slot, id)                                           \

@@ -38,7 +38,7 @@
 // 18, 4.9 K, and takes 8.5 K: the issue (50 cycles an MMA of 64 columns, 32 in the pipe), and in DQ and DK the way from dP to T, which the pipe waits
 // for since tensor memory is full. Instructions count too (six of sixteen warps' issue slots go into the cuts), hence two fp32 operations per
 // instruction wherever they come in pairs.
-// Measured on B200, us, this / attn_simt.cu, forward and backward with the row sums, causal, 2 x 8 x 1000 x 128: 38 / 115, 122 / 371; 1 x 4 x 700 x 96:
+// Measured on B200, us, this / attn_simt.cu, forward and backward with the row sums, causal, 2 x 8 x 1000 x 128: 39 / 115, 122 / 371; 1 x 4 x 700 x 96:
 // 18 / 42, 32 / 72; 2 x 8 x 500 x 96: 18 / 36, 38 / 88; 1 x 8 x 1000 x 16: 15 / 30, 36 / 66; 1 x 6 x 192 x 128: 13.5 / 17.7, 24 / 30.
 #include <math.h>
 

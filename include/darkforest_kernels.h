@@ -241,7 +241,7 @@ DF_API int df_attn_init(void);
  * kernel four times back to back, then the dK/dV kernel four times (an event pair around a single
  * launch would add several microseconds to a 70-microsecond kernel), with events before, between
  * and after the two groups; synchronises the stream and returns the two durations per launch in
- * milliseconds (0 when the SIMT path ran, which runs once). Creates and destroys three events per
+ * milliseconds (0 when another kernel than the TF32 pair ran, which runs once). Creates and destroys three events per
  * call: a measurement aid, not part of the allocation-free contract. Results are the same as
  * df_attn_backward's. No counterpart in the reference. */
 DF_API int df_attn_backward_profile(const float *q, const float *k, const float *v, const float *out,
