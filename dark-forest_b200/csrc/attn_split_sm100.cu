@@ -217,7 +217,7 @@ __device__ __forceinline__ float neg_lse2(float raw, float *lo) {
 
 // One row of a pass in fp32 arithmetic by one warp: the visible streamed rows and no others. An infinity has no parts, and a hidden row's infinity or
 // NaN times a P of zero is NaN too, so what is not finite in a block's results says nothing yet about what the row should be. It is no fast path:
-// lanes read rows of their own, and when every row needs it a call takes 15 to 30 times as long as attn_simt.cu (B200, ms, forward / backward, 2 x 8 x 1000 x
+// lanes read rows of their own, and when every row needs it a call takes 17 to 42 times as long as attn_simt.cu (B200, ms, forward / backward, 2 x 8 x 1000 x
 // 128, V infinite at key 0: 3.6 / 6.5 here, 0.13 / 0.38 there; one NaN in Q: forward 0.21). Loops unrolled eight times made that 3.0 / 5.2 and calls with
 // finite operands, which are the ones that matter, up to 5 % slower.
 template <Pass PASS>
